@@ -197,15 +197,6 @@ def reference_arm(args):
     return 0
 
 
-# DRAM bytes per staged flood brick visit: dram__bytes_read.sum +
-# dram__bytes_write.sum of one k_relax launch over the first 48 jobs of
-# mixed-256 (ncu --set full, one GB300: 1.899087 GB + 184.804864 MB), divided
-# by the 35370 visits of that launch that staged their brick (36922 visits,
-# 1552 found nothing new).  The roofline's `traffic` is this figure times the
-# staged visits of the timed launch.
-K_RELAX_DRAM_BYTES_PER_VISIT = (1899086592 + 184804864) / 35370
-
-
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -283,9 +274,7 @@ def main():
     R.barrier()
     ctx.synchronize()
     L.vf_ctx_event_record(ctx.h, 0)
-    launches, flood_ms, flood_bytes, visits, passes, sweeps, maxit = 0, 0.0, 0, 0, 0, 0, 0
-    act_rows, key_changes, busy_warps, empty = 0, 0, 0, 0
-    phase = {}
+    launches, flood_ms, flood_bytes, visits, passes, key_changes = 0, 0.0, 0, 0, 0, 0
     stage_tot = {}
     for _ in range(args.steps):
         rb.execute(download=False)
@@ -294,16 +283,9 @@ def main():
         flood_ms += st["flood_ms"]
         flood_bytes += st["flood_bytes"]
         visits += st["flood_visits"]
-        empty += st["flood_empty_visits"]
         passes += st["flood_passes"]
-        sweeps += st["flood_sweeps"]
-        maxit += st["flood_maxit_hits"]
-        act_rows += st["flood_active_row_sweeps"]
         key_changes += st["flood_key_changes"]
-        busy_warps += st["flood_busy_warp_sweeps"]
         pass_sizes = ctx.flood_pass_sizes()
-        for k, v in st["flood_phase_cycles"].items():
-            phase[k] = phase.get(k, 0) + v
         for k, v in ctx.stage_ms().items():
             stage_tot[k] = stage_tot.get(k, 0.0) + v
     L.vf_ctx_event_record(ctx.h, 1)
@@ -435,32 +417,23 @@ def main():
     flood_launch_ms = flood_ms / args.steps
     flood_launch_bytes = flood_bytes / args.steps
     achieved = (flood_launch_bytes / 1e9) / (flood_launch_ms / 1000.0) if flood_launch_ms else 0.0
-    roof = {"kernel": "k_relax (flood brick relaxation, one cooperative launch per step)",
+    roof = {"kernel": "k_wave (bit-parallel flood waves, one cooperative launch per step)",
             "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_kind": f"{peak_kind} copy bandwidth",
             "algorithmic_bytes_per_launch": flood_launch_bytes,
-            "bytes_rule": "4 B (u16 label read + write) per voxel of every brick visit",
-            "brick_visits_per_launch": visits / args.steps,
-            "empty_visits_per_launch": empty / args.steps,
-            "passes_per_launch": passes / args.steps,
-            "sweeps_per_visit": sweeps / max(visits, 1),
-            "visits_at_sweep_cap": maxit / args.steps,
-            "active_rows_per_sweep": act_rows / max(sweeps, 1),
-            "busy_warps_per_sweep": busy_warps / max(sweeps, 1),
-            "key_changes_per_visit": key_changes / max(visits, 1),
-            "bricks_per_pass_last_step": pass_sizes,
-            "phase_share": {k: round(v / max(sum(phase.values()), 1), 4) for k, v in phase.items()},
-            "phase_kcycles_per_visit": {k: round(v / max(visits, 1) / 1000.0, 2) for k, v in phase.items()},
-            "launch_ms": flood_launch_ms,
-            "traffic": K_RELAX_DRAM_BYTES_PER_VISIT * (visits - empty) / args.steps,
-            "traffic_source": "ncu DRAM bytes per brick visit (48-job capture) x visits of this launch"}
+            "bytes_rule": "4 B (u16 label read + write) per voxel of every row visit (32 voxels)",
+            "row_visits_per_launch": visits / args.steps,
+            "waves_per_launch": passes / args.steps,
+            "claims_per_visit": key_changes / max(visits, 1),
+            "rows_per_wave_last_step": pass_sizes,
+            "launch_ms": flood_launch_ms}
     line = {"metric": METRIC, "value": value, "unit": "voxels/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "u16",
             "data": "synthetic",
             "config": workload_config(jobs),
             "setup": {"parallelism": "replicas" if world > 1 else "single GPU",
-                      "path": "batched (one persistent brick-queue kernel per stage)",
+                      "path": "batched (every stage once over all jobs; one persistent flood launch)",
                       "cuda_graph": bool(getattr(rb, "graph", False)),
                       "tuning": tuning},
             "e2e": {"value": e2e_value, "unit": "voxels/s", "h2d_bytes_per_step": h2d,
@@ -616,7 +589,7 @@ def single_configs(args):
         t = time.perf_counter()
         lab, cnt, _ = O.run_job(v, f, spec.dims, spec.aabb[0], spec.aabb[1], q)
         cpu_ms = 1000.0 * (time.perf_counter() - t)
-        flood_bytes = 4.0 * 8192 * st["flood_visits"]
+        flood_bytes = st["flood_bytes"]
         print(json.dumps({
             "config": name, "dims": list(spec.dims), "voxels": vox, "triangles": int(spec.faces.shape[0]),
             "batched_device_ms": dev_ms, "batched_voxels_per_s": vox / (dev_ms / 1e3),
@@ -625,8 +598,8 @@ def single_configs(args):
             "plain_bfs_waves": int(pr.flood_passes),
             "cpu_oracle_ms": cpu_ms, "cpu_voxels_per_s": vox / (cpu_ms / 1e3), "cpu_cores": os.cpu_count(),
             "stages_ms": stages,
-            "flood": {"k_relax_ms": st["flood_ms"], "brick_visits": st["flood_visits"],
-                      "passes": st["flood_passes"],
+            "flood": {"k_wave_ms": st["flood_ms"], "row_visits": st["flood_visits"],
+                      "waves": st["flood_passes"],
                       "hbm_frac": (flood_bytes / (st["flood_ms"] / 1e3) / 1e9) / _peaks()[0]
                       if st["flood_ms"] else None},
             "labels_equal_oracle": bool(np.array_equal(got, lab)),

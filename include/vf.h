@@ -333,7 +333,7 @@ typedef struct vf_job_result {
   uint64_t voxels;         /* X*Y*Z */
   uint64_t occupied;       /* labelled voxels after the pipeline */
   uint32_t fragments;      /* distinct labels counted */
-  uint32_t flood_passes;   /* brick passes (batched) or BFS waves (plain) */
+  uint32_t flood_passes;   /* BFS waves of the flood that claimed voxels (plain: that ran) */
   double submit_ms;        /* server: submit time, ms since server start */
   double done_ms;          /* server: result-on-host time */
   uint64_t user_tag;
@@ -401,8 +401,8 @@ vf_status vf_pipeline_destroy(vf_pipeline* p);
  * file-scope device array of 32 MiB inside the library, held by every GPU
  * that loads it until exit; grids needing more (about 5 million voxels)
  * return VF_ERR_RANGE.  Calls share that array: calls that overlap on the
- * GPU race.  The flood inside is a cooperative launch with a grid-wide
- * barrier, so a call must not overlap a context's batched flood
+ * GPU race.  The flood inside is a cooperative launch whose CTAs wait for one
+ * another, so a call must not overlap a context's batched flood
  * (vf_batch_run, vf_pipeline_*, vf_server_*) on another stream either (the
  * barrier's bounded wait could run out: VF_ERR_TIMEOUT).  The first call on
  * a device looks up the array's address; make it before any stream capture.
@@ -418,8 +418,9 @@ vf_status vf_flood_noalloc(const uint16_t* d_grid, uint16_t* d_labels, uint32_t 
 /* ---- timing helpers for benchmarks (CUDA events on the context stream) --- */
 vf_status vf_ctx_event_record(vf_ctx* ctx, int slot);
 vf_status vf_ctx_event_elapsed(vf_ctx* ctx, int slot_a, int slot_b, float* ms);
-/* per-kernel statistics of the last vf_batch_run: launches and device ms of
- * the flood relaxation kernel (for the roofline) */
+/* per-kernel statistics of the last vf_batch_run: launches, device ms of the
+ * flood's wave kernel, its algorithmic bytes (u16 label read and write of every
+ * voxel of every visited row), rows visited (for the roofline) */
 vf_status vf_ctx_last_stats(vf_ctx* ctx, uint64_t* kernel_launches,
                             float* flood_ms, uint64_t* flood_bytes,
                             uint64_t* flood_brick_visits);
@@ -429,26 +430,16 @@ vf_status vf_ctx_last_stats(vf_ctx* ctx, uint64_t* kernel_launches,
  * bricks, [5] seeds, [6] fracture, [7] perturb, [8] erode/boundaries,
  * [9] counts, [10] download (n <= 11 entries written) */
 vf_status vf_ctx_stage_ms(vf_ctx* ctx, float* ms, uint32_t n);
-/* flood relaxation of the last batched run: passes (grid-wide rounds),
- * brick sweeps summed over all visits, visits that hit the sweep cap */
+/* flood of the last batched run: passes = waves; sweeps and maxit_hits are 0
+ * (counts of an earlier flood that relaxed bricks) */
 vf_status vf_ctx_flood_stats(vf_ctx* ctx, uint64_t* passes, uint64_t* sweeps,
                              uint64_t* maxit_hits);
-/* raw flood counters of the last batched run: [0] brick visits, [1] passes,
- * [2] warps with work summed over sweeps (8 warps per brick), [3] barrier
- * timeouts, [4] sweeps, [5] visits at the sweep cap, [6] active rows summed
- * over sweeps, [7] voxel key changes, [8] 0, or the kind of the first
- * out-of-range access the relaxation skipped (1 brick id, 2 job id, 3 key
- * read, 4 queued brick id, 5 key write; the batch then fails with
- * VF_ERR_TIMEOUT) with [9], [10] its brick and index, [11..15] SM cycles / 256
- * summed over the relaxation CTAs in each phase of their work: [11] claiming
- * a brick, [12] staging its keys, [13] sweeps, [14] write-back and enqueue of
- * neighbours, [15] from the last claim of a pass through the pass barrier,
- * [16] visits that found no change around the brick and staged nothing
- * (included in [0]), [17] visits that staged their brick but changed no key.
- * n <= 20 are filled, the rest zeroed. */
+/* raw flood counters of the last batched run: [0] rows (32 voxels) visited,
+ * [1] waves of the longest gang, [3] barrier timeouts, [7] voxels claimed; the
+ * others are 0.  n <= 20 are filled, the rest zeroed. */
 vf_status vf_ctx_flood_counters(vf_ctx* ctx, uint64_t* out, uint32_t n);
-/* bricks queued for each pass of the last batched flood (first 256 passes;
- * zero beyond the pass count). */
+/* rows visited in each wave of the last batched flood (first 256 waves; zero
+ * beyond the wave count). */
 vf_status vf_ctx_flood_pass_sizes(vf_ctx* ctx, uint32_t* out, uint32_t n);
 /* *replayed = 1 when the last vf_batch_execute ran its stage chain as a
  * CUDA graph (captured on the first execute after vf_batch_prepare, replayed
@@ -457,15 +448,16 @@ vf_status vf_ctx_last_graph(vf_ctx* ctx, int* replayed);
 
 /* ---- tuning (no counterpart in the reference) ----------------------------
  * Launch settings of a context, in this order: [0] parity-fill CTAs per SM,
- * [1] shell-test CTAs per SM, [2] flood relaxation sweeps per brick visit
- * (BFS waves a brick advances per pass before it re-queues itself),
- * [3] flood CTAs per SM (0: as many as fit).  Results never depend on them. */
+ * [1] shell-test CTAs per SM, [2] flood sweeps (kept and range-checked for
+ * callers that set it; the flood has no such bound any more), [3] flood CTAs
+ * per SM (0: as many as fit).  Results never depend on them. */
 vf_status vf_ctx_set_tuning(vf_ctx* ctx, const int32_t* values, uint32_t n);
-/* Spin limit of the flood relaxation's pass barrier on this context (polls
- * of about 64 ns each; 0 restores the default 2^26, about 4 s).  When the
- * limit runs out the kernel sets its error word and returns, and the call
- * fails with VF_ERR_TIMEOUT; the context stays usable.  A small limit makes
- * the bounded device wait run out on purpose (tests of the error path). */
+/* Poll limit of the flood's wave barrier on this context (polls of about half
+ * a microsecond each; 0 restores the default 2^23, about 4 s).  When the limit
+ * runs out the kernel sets its error word and returns, and the call fails with
+ * VF_ERR_TIMEOUT; the context stays usable.  With a limit every flood runs on
+ * at least two CTAs, so that the wait exists: a small one makes it run out on
+ * purpose (tests of the error path). */
 vf_status vf_ctx_set_flood_wait_limit(vf_ctx* ctx, uint32_t spins);
 vf_status vf_ctx_get_tuning(vf_ctx* ctx, int32_t* values, uint32_t n);
 /* Autotuner: prepares `jobs` as a resident batch (as vf_batch_prepare, which

@@ -258,7 +258,7 @@ class Context:
         return dict(zip(self.TUNING, list(v)))
 
     def flood_pass_sizes(self):
-        """Bricks queued per pass of the last batched flood."""
+        """Rows visited in each wave of the last batched flood (the first 256)."""
         a = (C.c_uint32 * 256)()
         _check(lib().vf_ctx_flood_pass_sizes(self.h, a, 256))
         return [v for v in a if v]
@@ -276,6 +276,9 @@ class Context:
         return a.value, b.value
 
     def last_stats(self):
+        """Statistics of the last batched run.  The flood's visits are rows of 32
+        voxels, its passes waves, its key changes claimed voxels; the counts of
+        brick visits, sweeps and phases of an earlier flood are 0."""
         la, vis, by = C.c_uint64(), C.c_uint64(), C.c_uint64()
         ms = C.c_float()
         _check(lib().vf_ctx_last_stats(self.h, C.byref(la), C.byref(ms), C.byref(by), C.byref(vis)))
@@ -289,11 +292,9 @@ class Context:
                 "flood_busy_warp_sweeps": cn[2],
                 "flood_key_changes": cn[7],
                 "flood_barrier_timeouts": cn[3],
-                # first out-of-range access the relaxation skipped (0: none)
                 "flood_anomaly": (cn[8], cn[9], cn[10]),
                 "flood_empty_visits": cn[16],
                 "flood_visits_no_change": cn[17],
-                # SM cycles summed over the relaxation CTAs, per phase of their work
                 "flood_phase_cycles": {k: 256 * cn[11 + i] for i, k in enumerate(
                     ("claim", "staging", "sweeps", "writeback_enqueue", "pass_barrier"))}}
 

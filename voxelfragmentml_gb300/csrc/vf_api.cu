@@ -1092,9 +1092,11 @@ vf_status vf_fracture_plain(vf_grid* g, int distance, const uint32_t* seeds, uin
   vfr::Batch& B = g->b;
   const vf_job* jp = &g->job;
   B.stages = vfr::ST_SEED | vfr::ST_FRACTURE;
+  B.plain = true;
   vf_status s = B.plan(&jp, 1);
   vf_job_result r;
   if (!s) s = B.enqueue_plain_and_wait(&r, /*skip_vox=*/true);
+  B.plain = false;
   if (!s && waves_out) *waves_out = r.flood_passes;
   g->b.given.clear();
   g->job.params = saved;
@@ -1373,8 +1375,10 @@ vf_status vf_plain_run(vf_ctx* ctx, const vf_job* jobs, uint32_t njobs, vf_job_r
     const vf_job* jp = jobs + i;
     B.stages = vfr::ST_ALL;
     B.given.clear();
+    B.plain = true;
     vf_status s = B.plan(&jp, 1);
     if (!s) s = B.enqueue_plain_and_wait(results ? results + i : nullptr, false);
+    B.plain = false;
     launches += B.launches;
     if (s && results) results[i].status = s;
     if (s && !first) first = s;
@@ -1400,9 +1404,8 @@ vf_status vf_ctx_last_stats(vf_ctx* ctx, uint64_t* launches, float* flood_ms, ui
   if (!ctx) return fail(VF_ERR_INVALID, "ctx is NULL");
   if (launches) *launches = ctx->c.last_launches;
   if (flood_ms) *flood_ms = ctx->c.last_flood_ms;
-  // algorithmic bytes of a brick visit: every voxel's label read and written
-  if (flood_bytes)  // visits that staged the brick (4 B per voxel, label read + write)
-    *flood_bytes = (ctx->c.last_flood_visits - ctx->c.last_flood_counters[16]) * (uint64_t)VF_BRICK_VOXELS * 4u;
+  // algorithmic bytes of a row visit: the labels of its 32 voxels read and written
+  if (flood_bytes) *flood_bytes = ctx->c.last_flood_visits * (uint64_t)VF_BZ * 4u;
   if (flood_visits) *flood_visits = ctx->c.last_flood_visits;
   return VF_OK;
 }

@@ -2,7 +2,9 @@
 //
 // Memory layout in HBM (per job):
 //   grid, grid2 : uint16 [X][Y][Zp], Zp = roundup(Z, 8)   (labels, ping-pong)
-//   keys        : uint32 [X][Y][Zk], Zk = roundup(Z, 4)   (flood state)
+//   wstate      : uint32 [rows][8, 12 or 16] (flood state: bit planes of 32
+//                 voxels along z, vf_flood.cu)
+//   keys        : uint32 [X][Y][Zk], Zk = roundup(Z, 4)   (plain flood state)
 //   par, shell  : uint32 [X][Y][Zw], Zw = ceil(Z / 32)     (voxelizer bit planes,
 //                 bit z&31 of word z>>5)
 // Rows along z are contiguous, so every brick row is one coalesced segment.
@@ -28,7 +30,7 @@
 #define VOXEL_EMPTY 0u
 #define VOXEL_FREE 1u
 
-// flood key encoding: key = ~((dist << 12) | seed_slot); 0 = wall (EMPTY),
+// plain flood key encoding: key = ~((dist << 12) | seed_slot); 0 = wall (EMPTY),
 // 1 = occupied, not reached.  A larger key is closer (then a lower slot).
 #define VF_KEY_WALL 0u
 #define VF_KEY_UNREACHED 1u
@@ -51,7 +53,13 @@ struct JobDesc {
   uint32_t nbx, nby, nbz, brick_base, nbricks;
   uint16_t* grid;   // stage source (and in-place target)
   uint16_t* grid2;  // stage destination for double-buffered stages
-  uint32_t* keys;
+  uint32_t* keys;   // plain path only
+  // flood: row states of wsw words, what reaches their ends, candidate bits; row
+  // (x, z word, y) is wrow0 + x * wsx + word * wsy + y (vfk::WaveJob)
+  uint32_t* wstate;
+  uint2* win;
+  uint32_t* wcand;
+  uint32_t wsw, wrow0, wsx, wsy;
   uint32_t* par;
   uint32_t* shell;
   // mesh

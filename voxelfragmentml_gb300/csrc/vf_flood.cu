@@ -6,23 +6,57 @@
 // among its wave-(t-1) neighbours", the label of every voxel is the label of
 // the seed nearest to it in grid-graph distance through occupied voxels
 // (6-neighbourhood for Manhattan, 26 for Euclidean and Chebyshev), ties to
-// the lowest seed index.  That fixed point does not depend on the order in
-// which voxels are relaxed, so the GPU computes it by relaxation:
+// the lowest seed index.
 //
-//   key(v) = ~((dist << 12) | seed_slot)      (0 = EMPTY, 1 = unreached)
-//   key(v) <- max(key(v), max_{u in N(v)} key(u) - 4096)
+// The GPU runs those waves bit-parallel.  32 voxels along z are one word of
+// bit planes:
 //
-// Bricks of 16x16x32 voxels are relaxed to local convergence in shared
-// memory (many BFS waves per visit).  A sweep runs only the rows next to new
-// halo data (sweep 0, from the brick's change record) or to a row that
-// changed in the previous sweep, compacted onto the lowest warps; a row
-// update is one forward and one backward pass along its 32-voxel z row.  A
-// brick whose boundary voxels changed records what changed in its
-// neighbours' change records and puts them on the next pass's queue
-// (deduplicated by a pass epoch, appended with warp ballot/popc).  All passes
-// of all jobs of a batch run in ONE cooperative persistent kernel; passes are
-// separated by a software grid barrier whose spin is bounded (it sets an
-// error word and the kernel returns instead of hanging).
+//   A, B         00 EMPTY, 01 occupied and not claimed yet (U), 10 / 11 claimed
+//                in a wave of even / odd parity (E0, E1)
+//   L0 .. L(n-1) the claiming seed's slot, bit by bit
+//
+// and, apart from them, the smallest slot that reaches the word's two end
+// voxels from the words below and above (in), kept by the claims there.
+//
+// A wave t dilates the bits claimed in wave t (E(t & 1)) over the
+// neighbourhood, carries the smallest slot along with bit-sliced minima, and
+// claims the unclaimed occupied bits it reaches into E((t + 1) & 1).  Every
+// voxel is claimed once.  E(t & 1) also holds the bits of waves t-2, t-4,
+// ..., but no unclaimed voxel is next to one of those (it would have been
+// claimed by the following wave), so they change nothing; and a word's
+// owner changes only bits that the same wave's readers mask out.  So there
+// is no frontier to clear and no race between the words of a wave.
+//
+// A lane takes one row (x, y, word) of 32 voxels with its 8 neighbour rows.
+// Rows are numbered linearly with rows of zeros around each axis (WaveJob), so
+// a neighbour is an index difference and no bounds are tested.  Which rows a
+// wave looks at is a candidate bit per row, set by the claims of the previous
+// wave: a row is a candidate when a claimed bit reaches one of its unclaimed
+// bits.  A wave scans the candidate words of its jobs (4 bytes per 32 rows, so
+// there are no queues), lists the rows in shared memory and deals them to the
+// lanes: the rows of a front are few and scattered, and a warp per run of
+// neighbouring rows left 27 of 32 lanes idle.
+//
+// All waves of all jobs of a batch run in ONE cooperative launch, on gangs of
+// CTAs that flood a set of jobs in step (vfk::WaveGang): wave t of all of them,
+// then the gang's barrier.  A batch has two gangs of one CTA per SM, so that
+// one gang's scan and barrier run under the other's visits; jobs of a batch of
+// small ones, and a small job alone, have a CTA each, which synchronises with
+// __syncthreads and keeps the candidate words in shared memory.  The barrier
+// of a larger gang is a counter in global memory whose spin is bounded (it
+// sets an error word and the kernel returns instead of hanging).
+//
+// What bounds it: the latency of a wave's four steps (scan, row list, visits,
+// barrier), each 1300 to 4000 cycles, while the front is small, and the L1's
+// tag lookups of the 9 row loads while it is large (about 20 lines per warp
+// load).  Flood launch of a batch of 128 uneven jobs: 3.96 ms, where relaxing
+// bricks of keys in shared memory to local convergence, a queue of bricks per
+// pass, took 10.56 ms (7 key updates per voxel claimed, bound by the chain
+// along each row); 48 jobs 1.64 against 4.01 ms; one job of 476 x 476 x 512
+// 0.87 against 2.15 ms, of 240 x 240 x 256 0.56 against 1.36 ms; of 60 x 57 x
+// 64 0.29 against 0.26 ms.  A gang per job in proportion to its size instead of
+// two gangs in step took 6.1 ms for the 128 jobs (the longest job's gang
+// finished last), a word of 30 neighbouring rows per warp 15.3 ms.
 //
 // Sub-seed prefixes (extra seeds merged into fragments, Seeder.cpp:115-152)
 // then go through the reference's competition and disjoint cleanup
@@ -30,1095 +64,788 @@
 // connected component of one fragment the lowest prefix wins; per fragment
 // only voxels with the fragment's minimum prefix survive; the rest is
 // re-flooded from all survivors (ties to the lowest label value).
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
-#include <mutex>
+#include <algorithm>
+#include <vector>
 
 #include "vf_kernels.h"
 
 namespace {
 
-using vfk::FLOOD_FDIR;
+typedef unsigned long long u64;
+using vfk::WaveArrays;
+using vfk::WaveCta;
+using vfk::WaveEntry;
+using vfk::WaveGang;
+using vfk::WaveJob;
 
-constexpr int KP = 36;                 // smem row pitch (u32): conflict-free 16 B loads
-constexpr int KNX = VF_BX + 2, KNY = VF_BY + 2;
-constexpr int KROWS = KNX * KNY;
-constexpr int TILE_BYTES = KROWS * KP * 4;
-constexpr int TILE_SMEM = TILE_BYTES + 128;  // dynamic shared memory: the tile, aligned to 128
-constexpr int MAXIT = 96;              // default cap of relaxation sweeps per brick visit
+constexpr unsigned FULL = 0xFFFFFFFFu;
+constexpr uint32_t MAX_LEVEL = 0xFFFFEu;  // largest geodesic distance a flood takes
+constexpr int SCAN = 4;                   // times 32 candidate words a warp reads per round
+constexpr uint32_t WORDS = 1024;          // words with candidates listed per round
+constexpr uint32_t LIST = 2048;           // rows of each kind listed per round
+constexpr uint32_t UNITS = 2048;          // units of 256 rows a CTA keeps a list of
+// floods of at most this many rows get a CTA of their own: a wave of theirs is one
+// or two passes of 512 threads, and without a global barrier 60 x 57 x 64 voxels
+// (10.8 k rows) take 0.29 ms against 0.31 on three CTAs and 0.33 on six
+constexpr uint32_t SMALL_ROWS = 16384;
+constexpr uint32_t PRUNE = 16;            // waves between dropping the finished jobs' units
 
-struct FloodArgs {
-  const JobDesc* jobs;
+struct WaveArgs {
+  WaveArrays arr;
+  const WaveJob* jobs;
+  const WaveGang* gangs;
+  const WaveCta* cta;        // [gridDim.x] its entries
+  const WaveEntry* entries;  // gang, rank, gang size
   JobState* st;
-  const uint32_t* brick_job;
-  const uint8_t* live;
-  uint32_t* queue[3];
-  uint32_t* qcount;  // [3]
-  uint32_t* qhead;   // [3]
-  uint32_t* epoch;
-  uint32_t* bar;     // [2]
+  uint32_t* bar;             // [gangs][WAVE_BAR_WORDS] arrivals, last wave with candidates (zeroed)
+  uint32_t* last;            // [wave jobs] a wave with claims, + 1 (zeroed)
   uint32_t* err;
-  uint32_t* stats;   // [0] visits, [1] passes, [2] busy warp-sweeps, [3] timeout, [4] sweeps,
-                     // [5] visits at the sweep cap, [6] active row-sweeps, [7] key changes,
-                     // [8..10] first out-of-range access (code, two values),
-                     // [11..15] SM cycles / 256 per phase of the CTAs' work,
-                     // [16] visits that found nothing new and staged nothing,
-                     // [17] visits that staged their brick but changed no key
-  uint32_t max_passes;
-  int max_sweeps;    // sweeps per brick visit before the brick re-queues itself
-  uint32_t* pass_sizes;  // bricks queued for each of the first 256 passes (or null)
-  uint32_t* fdir;        // [nbricks][FLOOD_FDIR] change record (read and cleared by each visit)
-  uint32_t nbricks;      // bricks of the batch (queue entries and brick ids are below)
-  uint32_t njobs;        // jobs of the batch
-  uint32_t wait_spins;   // spins of the pass barrier before it gives up
-  const unsigned char* tmaps;  // [njobs] keys tensor maps (KEYS_MAP_BYTES each)
+  uint32_t* stats;           // [0] rows visited, [1] waves, [3] timeouts, [7] voxels claimed
+  uint32_t* wave_sizes;      // rows visited in each of the first 256 waves (or null)
+  uint32_t wait_spins;       // polls of a gang barrier before it gives up
+  uint32_t smem_words;       // candidate words that fit the shared memory of a one-CTA gang
 };
-
-// ---- TMA tile loads (cp.async.bulk.tensor) with mbarrier completion -------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t mbar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t mbar, uint32_t phase) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok) : "r"(mbar), "r"(phase) : "memory");
-  return ok != 0;
-}
-// bounded wait for the phase `phase` of the mbarrier to complete
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase) {
-  for (uint32_t i = 0; i < (1u << 22); ++i)
-    if (mbar_try_wait(mbar, phase)) return true;
-  return false;
-}
-// box of the 3-D tensor `map` at (c0 innermost, c1, c2) into shared memory,
-// completion counted in bytes on the mbarrier
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* map, int c0, int c1, int c2,
-                                            uint32_t mbar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(mbar) : "memory");
-}
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+__device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void red_release(uint32_t* p, uint32_t v) {
+  asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 
-// A brick id, job id or key address outside its buffer: the access is
-// skipped, the flood's error word gets bit 3 (the batch reports the job as
-// failed) and the first case is kept in stats[8..10] (code, two values).
-__device__ __noinline__ void flood_anomaly(const FloodArgs& a, uint32_t code, uint32_t v0,
-                                           uint32_t v1) {
-  atomicOr(a.err, 8u);
-  if (atomicCAS(a.stats + 8, 0u, code) == 0u) {
-    a.stats[9] = v0;
-    a.stats[10] = v1;
+// words per row state with n slot planes: A, B and the planes, in units of 16
+// bytes
+__host__ __device__ constexpr int state_words(int n) { return (n + 2 + 3) / 4 * 4; }
+
+// the row state at p (rows of 32 bytes in one access)
+template <int NB>
+__device__ __forceinline__ void load_row(const uint32_t* p, uint32_t (&w)[state_words(NB)]) {
+  constexpr int SW = state_words(NB);
+  if (SW % 8 == 0) {
+#pragma unroll
+    for (int i = 0; i + 7 < SW; i += 8)
+      asm volatile("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(w[i]), "=r"(w[i + 1]), "=r"(w[i + 2]), "=r"(w[i + 3]), "=r"(w[i + 4]), "=r"(w[i + 5]),
+                     "=r"(w[i + 6]), "=r"(w[i + 7])
+                   : "l"(p + i)
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int i = 0; i < SW; i += 4) {
+      const uint4 v = *reinterpret_cast<const uint4*>(p + i);
+      w[i] = v.x; w[i + 1] = v.y; w[i + 2] = v.z; w[i + 3] = v.w;
+    }
   }
 }
 
-// software grid barrier with a bounded spin (wait_spins polls, 2^26 or about
-// 4 s by default); false on timeout
-__device__ bool grid_sync(uint32_t* bar, uint32_t nblocks, uint32_t* err, uint32_t* stats,
-                          uint32_t wait_spins) {
-  __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ok = 1;
-    const uint32_t gen = ld_acquire(bar + 1);
-    __threadfence();
-    const uint32_t arrived = atomicAdd(bar, 1u) + 1u;
-    if (arrived == nblocks) {
-      atomicExch(bar, 0u);
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      uint32_t spins = 0;
-      while (ld_acquire(bar + 1) == gen) {
-        if (++spins > wait_spins || ld_acquire(err) != 0) {
-          atomicOr(err, 2u);
-          atomicAdd(stats + 3, 1u);
-          ok = 0;
+// Per bit, the smallest slot among K sources (bit-sliced: F[i] says which
+// bits source i has, P[i] its planes) by elimination from the top plane: where
+// some source left has a 0, the sources with a 1 drop out.
+template <int NB, int K>
+__device__ __forceinline__ uint32_t min_slots(uint32_t (&F)[K], const uint32_t (&P)[K][NB], uint32_t (&L)[NB]) {
+  uint32_t f = 0;
+#pragma unroll
+  for (int i = 0; i < K; ++i) f |= F[i];
+#pragma unroll
+  for (int b = NB - 1; b >= 0; --b) {
+    uint32_t z3[3] = {0, 0, 0};  // three short chains
+#pragma unroll
+    for (int i = 0; i < K; ++i) z3[i % 3] |= F[i] & ~P[i][b];
+    const uint32_t z = z3[0] | z3[1] | z3[2];
+    L[b] = ~z;
+#pragma unroll
+    for (int i = 0; i < K; ++i) F[i] &= ~(z & P[i][b]);
+  }
+  return f;
+}
+
+template <int V>
+struct Int {
+  static constexpr int value = V;
+};
+
+// a job of the gang in shared memory: rows between x, between words (bit 31:
+// 6-neighbourhood), the rows that are visited
+struct JobRow {
+  uint32_t sx, sy, lo, hi;
+};
+
+// key of a claim of level `level` by `slot` in WaveJob::in; a later level is smaller
+__device__ __forceinline__ uint32_t in_key(uint32_t level, uint32_t slot) { return ((0xFFFFFu - level) << 12) | slot; }
+
+// reductions without a result (the atomics of CUDA C++ return one on generic
+// pointers, used or not)
+template <bool SMEM>
+__device__ __forceinline__ void red_or(uint32_t* p, uint32_t v) {
+  if (SMEM)
+    asm volatile("red.relaxed.cta.shared::cta.or.b32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(p)), "r"(v)
+                 : "memory");
+  else
+    asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ void red_min(uint32_t* p, uint32_t v) {
+  asm volatile("red.relaxed.gpu.global.min.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// candidate bits of the rows i - 1, i, i + 1 (bits 0 .. 2 of m)
+template <bool SMEM>
+__device__ __forceinline__ void set_candidates(uint32_t* cand, uint32_t i, uint32_t m) {
+  const uint32_t k = i - 1, sh = k & 31u;
+  uint32_t* c = cand + (k >> 5);
+  if (m) red_or<SMEM>(c, m << sh);
+  const uint32_t hi = (m >> 1) >> (31u - sh);
+  if (hi) red_or<SMEM>(c + 1, hi);
+}
+
+// One row in wave t: claims and the next wave's candidates.  Returns whether
+// a candidate was set (bit 0) and whether a voxel was claimed (bit 1).
+template <int NB, int CONN, bool SMEM>
+__device__ __forceinline__ uint32_t visit_row(const WaveArrays& arr, const JobRow& J, uint32_t i, uint32_t t,
+                                              uint32_t* next, uint32_t* err, uint32_t& claims) {
+  constexpr int SW = state_words(NB);
+  const uint32_t sy = J.sy & 0x7FFFFFFFu, sx = J.sx;
+  // a claim at a word end names rows beyond it unseen: the ones in the zeros
+  // around the grid whose own neighbours would lie outside the job
+  if (i < J.lo || i >= J.hi) return 0;
+  const bool par = t & 1u;
+  uint32_t* const p0 = arr.state + (size_t)i * SW;
+  const size_t xs = (size_t)sx * SW;
+  const uint32_t pm = par ? 0u : FULL;  // A & (B ^ pm): claimed with this wave's parity
+  uint32_t A4, B4, O[NB], U[9], F[9], P[9][NB];
+  // the 3 x 3 rows around the row (6: the cross)
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    const int dx = r / 3 - 1, dy = r % 3 - 1;
+    if (CONN == 6 && dx && dy) {
+      U[r] = F[r] = 0;
+      continue;
+    }
+    uint32_t w[SW];
+    load_row<NB>((dx < 0 ? p0 - xs : (dx > 0 ? p0 + xs : p0)) + dy * SW, w);
+    U[r] = w[1] & ~w[0];
+    F[r] = w[0] & (w[1] ^ pm);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) P[r][b] = w[2 + b];
+    if (r == 4) {
+      A4 = w[0];
+      B4 = w[1];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) O[b] = w[2 + b];
+    }
+  }
+  // slots that claims of this wave's level bring in from the words below / above
+  const uint2 in = arr.in[2 * (size_t)i + (t & 1u)];
+  const uint32_t base = in_key(t, 0), dlo = in.x - base, dhi = in.y - base;
+  const uint32_t lo_f = dlo < 4095u ? 1u : 0u, hi_f = dhi < 4095u ? 1u << 31 : 0u;  // slots are below 4095
+  uint32_t L[NB], f;
+  if (CONN == 26) {
+    uint32_t W[NB];  // over the 3 x 3 rows, then z - 1, z, z + 1
+    const uint32_t g = min_slots<NB, 9>(F, P, W);
+    uint32_t G[3] = {g, (g << 1) | lo_f, (g >> 1) | hi_f}, Q[3][NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      Q[0][b] = W[b];
+      Q[1][b] = __funnelshift_l(dlo << (31 - b), W[b], 1);
+      Q[2][b] = __funnelshift_r(W[b], dhi >> b, 1);
+    }
+    f = min_slots<NB, 3>(G, Q, L);
+  } else {
+    const uint32_t g = F[4];
+    uint32_t G[6] = {F[1], F[3], F[5], F[7], (g << 1) | lo_f, (g >> 1) | hi_f}, Q[6][NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      Q[0][b] = P[1][b];
+      Q[1][b] = P[3][b];
+      Q[2][b] = P[5][b];
+      Q[3][b] = P[7][b];
+      Q[4][b] = __funnelshift_l(dlo << (31 - b), P[4][b], 1);
+      Q[5][b] = __funnelshift_r(P[4][b], dhi >> b, 1);
+    }
+    f = min_slots<NB, 6>(G, Q, L);
+  }
+  const uint32_t N = f & U[4];
+  if (!N) return 0;
+  if (t >= MAX_LEVEL) {  // the claims would lie beyond the largest distance
+    atomicOr(err, VF_JERR_DIST_OVERFLOW);
+    return 0;
+  }
+  claims += (uint32_t)__popc(N);
+  U[4] &= ~N;
+  {
+    uint32_t w[SW];
+    w[0] = A4 | N;
+    w[1] = par ? B4 & ~N : B4;  // B is set for U: claims of odd waves + 1 clear it
+#pragma unroll
+    for (int b = 0; b < SW - 2; ++b) w[2 + b] = b < NB ? (O[b < NB ? b : 0] & ~N) | (L[b < NB ? b : 0] & N) : 0u;
+#pragma unroll
+    for (int k = 0; k < SW; k += 4)
+      *reinterpret_cast<uint4*>(p0 + k) = make_uint4(w[k], w[k + 1], w[k + 2], w[k + 3]);
+  }
+  // rows the claims reach: exactly in this word (their unclaimed bits as read:
+  // a row claimed meanwhile is looked at in vain), row by row in the words
+  // below and above
+  const uint32_t nz = N | (N << 1) | (N >> 1);
+  uint32_t any = 0;
+#pragma unroll
+  for (int dx = -1; dx <= 1; ++dx) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy) {
+      const int r = (dx + 1) * 3 + dy + 1;
+      const uint32_t reach = CONN == 26 ? nz : (r == 4 ? (N << 1) | (N >> 1) : N);
+      m |= (reach & U[r]) ? 1u << (dy + 1) : 0u;
+    }
+    set_candidates<SMEM>(next, i + (uint32_t)dx * sx, m);
+    any |= m;
+  }
+  if ((N & 0x80000001u) != 0) {
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+      if (k == 0 ? !(N & 1u) : !(N >> 31)) continue;
+      uint32_t slot = 0;
+#pragma unroll
+      for (int b = 0; b < NB; ++b) slot |= (k ? L[b] >> 31 : L[b] & 1u) << b;
+      const uint32_t key = in_key(t + 1u, slot);
+      // row i is below (k = 1) or above the rows j it reaches: their .x / .y
+      const uint32_t j = k ? i + sy : i - sy;
+      uint32_t* const to = reinterpret_cast<uint32_t*>(arr.in + 2 * (size_t)j + ((t + 1) & 1u)) + (1 - k);
+#pragma unroll
+      for (int dx = -1; dx <= 1; ++dx) {
+        if (CONN == 6 && dx) continue;
+        uint32_t* const q = to + 4 * (dx < 0 ? -(ptrdiff_t)sx : (dx > 0 ? (ptrdiff_t)sx : 0));
+        red_min(q, key);
+        if (CONN == 26) {
+          red_min(q - 4, key);
+          red_min(q + 4, key);
+        }
+        set_candidates<SMEM>(next, j + (uint32_t)dx * sx, CONN == 26 ? 7u : 2u);
+      }
+    }
+    any = 1;
+  }
+  return any ? 3u : 2u;
+}
+
+// the dynamic shared memory of k_wave; the candidate words of a one-CTA gang follow
+struct WaveShared {
+  JobRow job[vfk::WAVE_GANG_JOBS];
+  uint32_t last[vfk::WAVE_GANG_JOBS];  // this CTA's last wave with claims, + 1
+  uint8_t live[vfk::WAVE_GANG_JOBS];
+  uint32_t bits[WORDS], word[WORDS];   // the round's words with candidates
+  uint8_t wjob[WORDS];                 // their jobs
+  uint32_t row[2][LIST];               // the round's rows: 26- / 6-neighbourhood
+  uint8_t rjob[2][LIST];               // their jobs
+  uint32_t unit[UNITS];                // this CTA's units | job << 24
+};
+
+template <int NB, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_wave(WaveArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  WaveShared& S = *reinterpret_cast<WaveShared*>(smem_raw);
+  uint32_t* const s_cand = reinterpret_cast<uint32_t*>(smem_raw + sizeof(WaveShared));
+  __shared__ WaveGang G;
+  __shared__ uint32_t s_n[2][2], s_w[2], s_any[2], s_again[2], s_go, s_ok, s_units, s_rank, s_size;
+  __shared__ uint32_t s_stat[2];
+  constexpr uint32_t warps = THREADS / 32;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const WaveCta mine = a.cta[blockIdx.x];
+  if (tid < 2) s_stat[tid] = 0;
+  uint32_t claims = 0;  // this thread's
+  for (uint32_t e = 0; e < mine.count; ++e) {
+    __syncthreads();
+    if (tid == 0) {
+      const WaveEntry en = a.entries[mine.first + e];
+      G = a.gangs[en.gang];
+      s_rank = en.rank;
+      s_size = en.size;
+      s_n[0][0] = s_n[0][1] = s_n[1][0] = s_n[1][1] = s_w[0] = s_w[1] = s_any[0] = s_any[1] = s_again[0] = s_again[1] = 0;
+    }
+    __syncthreads();
+    const uint32_t rank = s_rank, size = s_size, first = G.first, njobs = G.count;
+    const uint32_t word_lo = G.unit_lo * 8, words = G.units * 8;
+    for (uint32_t j = tid; j < njobs; j += THREADS) {
+      const WaveJob& W = a.jobs[first + j];
+      S.job[j] = {W.sx, W.sy | (W.conn6 << 31), W.row0, W.base + W.nrows - (W.sx + W.sy + 1)};
+      S.last[j] = 0;
+    }
+    const bool in_smem = size == 1 && 2 * words <= a.smem_words;
+    if (in_smem)
+      for (uint32_t i = tid; i < words; i += THREADS) {
+        s_cand[i] = a.arr.cand[word_lo + i];
+        s_cand[words + i] = 0;
+      }
+    __syncthreads();
+    // Candidate words in units of 8 (256 rows, one job); the gang's units are
+    // dealt to its CTAs in turn, so that the rows of a front spread evenly.
+    // The job of a unit: the last whose rows start at or before it.
+    auto unit_of = [&](uint32_t k) {
+      const uint32_t u = G.unit_lo + k * size + rank;
+      uint32_t lo = 0, hi = njobs - 1;
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (a.jobs[first + mid].base <= u * 256u) lo = mid; else hi = mid - 1;
+      }
+      return u | (lo << 24);
+    };
+    uint32_t nunits = G.units > rank ? (G.units - rank + size - 1) / size : 0;
+    const bool listed = nunits <= UNITS;
+    if (listed)
+      for (uint32_t k = tid; k < nunits; k += THREADS) S.unit[k] = unit_of(k);
+    if (tid == 0) s_units = nunits;
+    __syncthreads();
+    uint32_t* const bar = a.bar + (size_t)(size > 1 ? a.entries[mine.first + e].gang : 0) * vfk::WAVE_BAR_WORDS;
+    uint32_t rr = 0;  // rounds done: parity of the list counters
+    uint32_t t = 0;
+    for (;; ++t) {
+      uint32_t* const gcur = a.arr.cand + (t & 1u) * (size_t)a.arr.nwords;
+      uint32_t* const gnext = a.arr.cand + ((t + 1) & 1u) * (size_t)a.arr.nwords;
+      uint32_t* const scur = s_cand + (t & 1u) * words - word_lo;
+      uint32_t* const snext = s_cand + ((t + 1) & 1u) * words - word_lo;
+      bool any = false, stop = false;
+      uint32_t active = t;  // the last wave with candidates (thread 0; a gang's word of it)
+      if (tid == 0 && size > 1 && t) active = ld_relaxed(bar + 16);
+      nunits = s_units;
+      const uint32_t rounds = (nunits + 4 * warps * SCAN - 1) / (4 * warps * SCAN);
+      for (bool again = true, once = true; again; ++rr, once = false) {
+        // 1. the words with candidates: SCAN loads of the next round in flight
+        // while a round's words are listed
+        uint32_t b[SCAN], g[SCAN];
+        auto read = [&](uint32_t r) {
+#pragma unroll
+          for (int k = 0; k < SCAN; ++k) {
+            const uint32_t q = 4 * ((r * SCAN + k) * warps + warp) + lane / 8;
+            b[k] = g[k] = 0;
+            if (q < nunits) {
+              g[k] = listed ? S.unit[q] : unit_of(q);  // unit | job << 24
+              const uint32_t w = (g[k] & 0xFFFFFFu) * 8 + lane % 8;
+              b[k] = in_smem ? scur[w] : gcur[w];
+            }
+          }
+        };
+        read(0);
+#pragma unroll 1
+        for (uint32_t r = 0; r < rounds; ++r) {
+          uint32_t c[SCAN], h[SCAN], full = 0;
+          unsigned m[SCAN];
+#pragma unroll
+          for (int k = 0; k < SCAN; ++k) {
+            c[k] = b[k];
+            h[k] = g[k];
+          }
+          if (r + 1 < rounds) read(r + 1);
+#pragma unroll
+          for (int k = 0; k < SCAN; ++k) {
+            m[k] = __ballot_sync(FULL, c[k] != 0);
+            full += (uint32_t)__popc(m[k]);
+          }
+          if (!full) continue;
+          uint32_t pos = 0;
+          if (lane == 0) pos = atomicAdd(&s_w[rr & 1u], full);
+          pos = __shfl_sync(FULL, pos, 0);
+          if (pos + full > WORDS) {  // no room: these words stay for another round
+            for (uint32_t i = pos + lane; i < min(WORDS, pos + full); i += 32) S.bits[i] = 0;
+            if (lane == 0) s_again[rr & 1u] = 1u;
+            continue;
+          }
+#pragma unroll
+          for (int k = 0; k < SCAN; ++k) {
+            if (c[k]) {
+              const uint32_t i = pos + __popc(m[k] & ((1u << lane) - 1u)), w = (h[k] & 0xFFFFFFu) * 8 + lane % 8;
+              S.bits[i] = c[k];
+              S.word[i] = w;
+              S.wjob[i] = (uint8_t)(h[k] >> 24);
+              if (in_smem) scur[w] = 0; else gcur[w] = 0;  // wave t + 2 starts with empty words
+            }
+            pos += (uint32_t)__popc(m[k]);
+          }
+        }
+        if (tid == 0 && once) s_go = (int32_t)(active - t) >= 0 ? 1u : 0u;
+        __syncthreads();
+        if (once && !s_go) {
+          stop = true;
           break;
         }
-        __nanosleep(64);
-      }
-    }
-    __threadfence();
-  }
-  __syncthreads();
-  return ok != 0;
-}
-
-__device__ __forceinline__ uint32_t brick_id(const JobDesc& J, int bx, int by, int bz) {
-  return J.brick_base + ((uint32_t)bx * J.nby + (uint32_t)by) * J.nbz + (uint32_t)bz;
-}
-
-__device__ __forceinline__ void enqueue(const FloodArgs& a, uint32_t b, uint32_t next_pass,
-                                        bool want) {
-  // warp-aggregated append of the bricks this warp wants on the next queue
-  const int lane = threadIdx.x & 31;
-  bool push = false;
-  if (want && b >= a.nbricks) {
-    flood_anomaly(a, 4u, b, next_pass);
-    want = false;
-  }
-  if (want) push = atomicMax(&a.epoch[b], next_pass + 1u) < next_pass + 1u;
-  const unsigned m = __ballot_sync(0xFFFFFFFFu, push);
-  if (!m) return;
-  const uint32_t q = next_pass % 3u;
-  uint32_t base = 0;
-  const int leader = __ffs(m) - 1;
-  if (lane == leader) base = atomicAdd(&a.qcount[q], (uint32_t)__popc(m));
-  base = __shfl_sync(0xFFFFFFFFu, base, leader);
-  if (push) a.queue[q][base + __popc(m & ((1u << lane) - 1u))] = b;
-}
-
-// relaxation candidate from a neighbour key: one step further (0 when the
-// neighbour is EMPTY or unreached)
-__device__ __forceinline__ uint32_t step_from(uint32_t m) {
-  return m >= 2u * VF_KEY_STEP ? m - VF_KEY_STEP : 0u;
-}
-// key of a voxel (kk) relaxed by the best neighbour key m; EMPTY stays EMPTY.
-// step_from is monotone, so relaxing by max(m1, m2) equals relaxing by m1
-// and then by m2.
-__device__ __forceinline__ uint32_t relax(uint32_t kk, uint32_t m) {
-  return kk ? max(kk, step_from(m)) : 0u;
-}
-// One step of an in-row chain: relax(kk, max(w, prev)) with the part that
-// does not depend on prev, a = relax(kk, w), computed ahead of the chain.
-// step_from is monotone, so relax(kk, max(w, prev)) = kk ? max(a, step_from(
-// prev)) : 0, and a = 0 when kk = 0: on the chain there is one select (the
-// step, taken only for occupied voxels) and one max.
-__device__ __forceinline__ uint32_t chain_step(uint32_t a, bool occ, uint32_t prev) {
-  const uint32_t s = (occ && prev >= 2u * VF_KEY_STEP) ? prev - VF_KEY_STEP : 0u;
-  return max(a, s);
-}
-// a key at the largest distance the key format holds (its neighbours would
-// overflow the distance field)
-__device__ __forceinline__ bool at_limit(uint32_t m) {
-  return m - VF_KEY_MIN_REACHED < VF_KEY_STEP;
-}
-__device__ __forceinline__ uint4 max4(uint4 a, uint4 b) {
-  return make_uint4(max(a.x, b.x), max(a.y, b.y), max(a.z, b.z), max(a.w, b.w));
-}
-__device__ __forceinline__ uint4 lds4(const uint32_t* p) {
-  return *reinterpret_cast<const uint4*>(p);
-}
-
-// Shared state of the sweeps of one brick visit.
-struct SweepShared {
-  uint32_t rfw[16];      // [2][8] rows that changed in the previous sweep (bit per row)
-  uint32_t wmask[8];     // active rows of each warp in this sweep (bit per lane)
-  uint32_t hl[256];      // per row: z halo candidate below the brick (z0-1)
-  uint32_t hh[256];      //          z halo candidate above the brick (z0+32)
-  uint32_t rowchg[256];  // per row: z positions changed during the visit
-  uint8_t occ8[256];     // per row: bit q set when its keys 4q .. 4q+3 hold an occupied voxel
-};
-
-// position of the k-th (from 0) set bit of m; k < popc(m)
-__device__ __forceinline__ int nth_set_bit(uint32_t m, uint32_t k) {
-  int pos = 0;
+        // 2. their rows, a lane per half word
+        const uint32_t nwords = min(s_w[rr & 1u], WORDS);
+        for (uint32_t k0 = warp * 16; k0 < nwords; k0 += warps * 16) {
+          const uint32_t k = k0 + lane / 2;
+          uint32_t bits = 0, w = 0, jid = 0;
+          if (k < nwords) {
+            bits = S.bits[k];
+            w = S.word[k];
+            jid = S.wjob[k];
+          }
+          bits &= lane & 1 ? 0xFFFF0000u : 0xFFFFu;
+          if (!__any_sync(FULL, bits != 0)) continue;
+          // both kinds in one scan: rows of the 6-neighbourhood in the high half
+          const uint32_t six = S.job[jid].sy >> 31, n = (uint32_t)__popc(bits) << (16 * six);
+          uint32_t incl = n;
 #pragma unroll
-  for (int w = 16; w >= 1; w >>= 1) {
-    const uint32_t lo = (uint32_t)__popc(m & ((1u << w) - 1u));
-    if (k >= lo) {
-      k -= lo;
-      m >>= w;
-      pos += w;
-    }
-  }
-  return pos;
-}
-
-// Column maximum of the 3 x 3 rows around own_row at row slot s (one z).
-__device__ __forceinline__ uint32_t colmax1(const uint32_t* own_row, int s) {
-  uint32_t m = 0;
-#pragma unroll
-  for (int r = 0; r < 9; ++r) m = max(m, own_row[((r / 3 - 1) * KNY + (r % 3 - 1)) * KP + s]);
-  return m;
-}
-// Column maxima of the 3 x 3 rows around own_row at row slots s .. s+3.
-__device__ __forceinline__ uint4 colmax4(const uint32_t* own_row, int s) {
-  uint4 C = make_uint4(0, 0, 0, 0);
-#pragma unroll
-  for (int r = 0; r < 9; ++r) C = max4(C, lds4(own_row + ((r / 3 - 1) * KNY + (r % 3 - 1)) * KP + s));
-  return C;
-}
-
-// Relaxes one row of the staged tile (own_row) in place, on a pair of
-// adjacent lanes: lane h = 0 takes the chunks 0..3 (z 0..15), h = 1 the
-// chunks 4..7 (z 16..31).  A row update is a forward pass (cross-row
-// candidates fused with the increasing-z in-row chain) and a backward pass
-// (the decreasing-z chain), both starting from the row's z halo candidates
-// hlo / hhi.  occ8 has bit q set when the row's 4-key chunk q holds an
-// occupied voxel: empty chunks keep their zero keys and break the in-row
-// chain, so both passes skip them (a thin wall crosses a row in a few
-// chunks).
-// Each lane runs both chains over its half from a lower bound of the chain
-// value at the boundary (a key as read: keys only grow), then takes the
-// exact boundary value from the other lane by a shuffle.  Along an occupied
-// run the chain is max-plus linear: the value a chain carries in from the
-// boundary adds step^d(P) at distance d, so the lane raises its keys from
-// the boundary while step^d(P) exceeds them (past the first key it does not
-// exceed, none it reaches can be exceeded; an empty voxel ends the run).
-// The result equals one lane's sequential pass over the whole row for the
-// same reads.  All lanes of pair_mask call this (two shuffles each).
-// Returns the lane's changed z positions.
-template <int CONN>
-__device__ __forceinline__ uint32_t relax_half(uint32_t* own_row, int h, uint32_t hlo,
-                                               uint32_t hhi, uint32_t occ8, bool full_backward,
-                                               unsigned pair_mask) {
-  const int q0 = 4 * h, q1 = q0 + 4;
-  const uint32_t om = (occ8 >> q0) & 0xFu;
-  uint32_t chg = 0;
-  // forward: lane 0 from the halo candidate hlo, lane 1 from the key at z 15
-  uint32_t prev = h == 0 ? hlo : own_row[4 + 15];
-  int last = q0 - 2;  // the chunk relaxed last
-  if (CONN == 26) {
-    uint4 C = make_uint4(0, 0, 0, 0);
-    uint32_t cp = hlo;
-#pragma unroll 1
-    for (uint32_t m = om; m; m &= m - 1u) {
-      const int q = q0 + __ffs(m) - 1;
-      if (q != last + 1) {
-        C = colmax4(own_row, 4 + 4 * q);
-        if (q > 0) {
-          cp = colmax1(own_row, 3 + 4 * q);
-          if (q != q0) prev = 0u;  // after an empty chunk
+          for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t v = __shfl_up_sync(FULL, incl, o);
+            if (lane >= (uint32_t)o) incl += v;
+          }
+          const uint32_t total = __shfl_sync(FULL, incl, 31);
+          uint32_t pos = 0;
+          if (lane < 2) pos = atomicAdd(&s_n[rr & 1u][lane], (total >> (16 * lane)) & 0xFFFFu);
+          const uint32_t pos0 = __shfl_sync(FULL, pos, 0), pos1 = __shfl_sync(FULL, pos, 1);
+          const uint32_t end = six ? pos1 + (total >> 16) : pos0 + (total & 0xFFFFu);
+          pos = (six ? pos1 : pos0) + (((incl - n) >> (16 * six)) & 0xFFFFu);
+          if (end > LIST) {  // no room: back into the word
+            if (bits) {
+              if (in_smem) atomicOr(scur + w, bits); else atomicOr(gcur + w, bits);
+              s_again[rr & 1u] = 1u;
+            }
+            const uint32_t stop = min(LIST, pos + (uint32_t)__popc(bits));
+            for (; pos < stop; ++pos) S.row[six][pos] = 0xFFFFFFFFu;
+            bits = 0;
+          }
+          while (bits) {
+            const uint32_t bit = (uint32_t)__ffs(bits) - 1;
+            bits &= bits - 1;
+            S.row[six][pos] = (w << 5) | bit;
+            S.rjob[six][pos++] = (uint8_t)jid;
+          }
         }
+        __syncthreads();
+        const uint32_t n26 = min(s_n[rr & 1u][0], LIST), n6 = min(s_n[rr & 1u][1], LIST);
+        again = s_again[rr & 1u] != 0;
+        if (tid == 0) {
+          s_n[(rr + 1) & 1u][0] = s_n[(rr + 1) & 1u][1] = 0;
+          s_w[(rr + 1) & 1u] = s_again[(rr + 1) & 1u] = 0;
+          if (once) s_any[(t + 1) & 1u] = 0;
+          s_stat[0] += n26 + n6;
+          if (a.wave_sizes && n26 + n6 && t < 256) atomicAdd(a.wave_sizes + t, n26 + n6);
+        }
+        auto visit = [&](auto conn, uint32_t i) {
+          constexpr int CONN = decltype(conn)::value;
+          const uint32_t row = S.row[CONN == 6][i], j = S.rjob[CONN == 6][i];
+          if (row == 0xFFFFFFFFu) return;
+          const JobRow J = S.job[j];
+          uint32_t* const err = &a.st[a.jobs[first + j].job].err;
+          const uint32_t f = in_smem ? visit_row<NB, CONN, true>(a.arr, J, row, t, snext, err, claims)
+                                     : visit_row<NB, CONN, false>(a.arr, J, row, t, gnext, err, claims);
+          any |= (f & 1u) != 0;
+          if (f) S.last[j] = t + 1;
+        };
+        for (uint32_t i = tid; i < n26; i += THREADS) visit(Int<26>{}, i);
+        // the 6-neighbourhood rows start at the warp after the others' last one
+        const uint32_t off = ((n26 + 31) / 32 % warps) * 32;
+        for (uint32_t i = (tid + THREADS - off) % THREADS; i < n6; i += THREADS) visit(Int<6>{}, i);
+        if (any) s_any[t & 1u] = 1u;
+        __syncthreads();
       }
-      uint4 Cn = make_uint4(hhi, 0, 0, 0);
-      if (q + 1 < 8) {
-        if (q + 1 < q1 && ((om >> (q + 1 - q0)) & 1u)) Cn = colmax4(own_row, 8 + 4 * q);
-        else Cn.x = colmax1(own_row, 8 + 4 * q);
-      }
-      const uint4 kv = lds4(own_row + 4 + 4 * q);
-      const uint32_t w[4] = {max(cp, max(C.x, C.y)), max(C.x, max(C.y, C.z)),
-                             max(C.y, max(C.z, C.w)), max(C.z, max(C.w, Cn.x))};
-      const uint32_t kk[4] = {kv.x, kv.y, kv.z, kv.w};
-      uint32_t f[4], av[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) av[j] = relax(kk[j], w[j]);  // off the chain
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        f[j] = chain_step(av[j], kk[j] != 0u, prev);
-        prev = f[j];
-        if (f[j] != kk[j]) chg |= 1u << (4 * q + j);
-      }
-      if ((chg >> (4 * q)) & 0xFu)
-        *reinterpret_cast<uint4*>(own_row + 4 + 4 * q) = make_uint4(f[0], f[1], f[2], f[3]);
-      cp = C.w; C = Cn; last = q;
-    }
-  } else {
-#pragma unroll 1
-    for (uint32_t m = om; m; m &= m - 1u) {
-      const int q = q0 + __ffs(m) - 1;
-      if (q != last + 1 && q != q0) prev = 0u;  // after an empty chunk
-      const uint4 M = max4(max4(lds4(own_row - KNY * KP + 4 + 4 * q), lds4(own_row + KNY * KP + 4 + 4 * q)),
-                           max4(lds4(own_row - KP + 4 + 4 * q), lds4(own_row + KP + 4 + 4 * q)));
-      const uint4 kv = lds4(own_row + 4 + 4 * q);
-      const uint32_t w[4] = {M.x, M.y, M.z, M.w};
-      const uint32_t kk[4] = {kv.x, kv.y, kv.z, kv.w};
-      uint32_t f[4], av[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) av[j] = relax(kk[j], w[j]);  // off the chain
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        f[j] = chain_step(av[j], kk[j] != 0u, prev);
-        prev = f[j];
-        if (f[j] != kk[j]) chg |= 1u << (4 * q + j);
-      }
-      if ((chg >> (4 * q)) & 0xFu)
-        *reinterpret_cast<uint4*>(own_row + 4 + 4 * q) = make_uint4(f[0], f[1], f[2], f[3]);
-      last = q;
-    }
-  }
-  // lane 1 takes lane 0's exact chain value at z 15 (zero when chunk 3 is empty)
-  const uint32_t P = __shfl_xor_sync(pair_mask, last == 3 ? prev : 0u, 1);
-  if (h == 1) {
-    uint32_t v = P;
-#pragma unroll 1
-    for (int z = 16; z < 32; ++z) {
-      const uint32_t k = own_row[4 + z];
-      v = (k != 0u && v >= 2u * VF_KEY_STEP) ? v - VF_KEY_STEP : 0u;
-      if (v <= k) break;  // also ends the run at an empty voxel (v = 0)
-      own_row[4 + z] = v;
-      chg |= 1u << z;
-    }
-  }
-  // Backward over the lane's half: from its top chunk (full_backward; lane 1
-  // from the halo candidate hhi, lane 0 from the key at z 16) or from its
-  // highest chunk the forward pass changed, down to where nothing changes and
-  // no forward change lies below.  The row was consistent along z before
-  // this pass, so nothing above the highest changed chunk needs it.
-  int q = q1 - 1;
-  bool run = full_backward;
-  if (!run && chg) {
-    run = true;
-    q = (31 - __clz(chg)) >> 2;
-  }
-  if (run) {
-    prev = q == 7 ? hhi : own_row[4 + 4 * q + 4];
-#pragma unroll 1
-    for (; q >= q0; --q) {
-      if (!((om >> (q - q0)) & 1u)) {
-        if ((chg & (0xFFFFFFFFu >> (28 - 4 * q))) == 0u) break;
-        prev = 0u;
+      if (stop) break;
+      if (size == 1) {
+        if (!s_any[t & 1u]) {
+          ++t;
+          break;
+        }
         continue;
       }
-      const uint4 kv = lds4(own_row + 4 + 4 * q);
-      const uint32_t kk[4] = {kv.x, kv.y, kv.z, kv.w};
-      uint32_t f[4];
-      uint32_t cq = 0;
-#pragma unroll
-      for (int j = 3; j >= 0; --j) {
-        f[j] = chain_step(kk[j], kk[j] != 0u, prev);
-        prev = f[j];
-        if (f[j] != kk[j]) cq |= 1u << j;
+      const bool prune = listed && njobs > 1 && t % PRUNE == PRUNE - 1;
+      if (prune) {
+        for (uint32_t j = tid; j < njobs; j += THREADS)
+          if (S.last[j] == t + 1) atomicMax(a.last + first + j, t + 1);
+        __syncthreads();
       }
-      if (cq) {
-        *reinterpret_cast<uint4*>(own_row + 4 + 4 * q) = make_uint4(f[0], f[1], f[2], f[3]);
-        chg |= cq << (4 * q);
-      } else if ((chg & (0xFFFFFFFFu >> (28 - 4 * q))) == 0u) {
-        break;  // this chunk and everything below it unchanged: consistent
-      }
-    }
-  }
-  // lane 0 takes lane 1's final key at z 16
-  const uint32_t P2 = __shfl_xor_sync(pair_mask, h == 1 ? own_row[4 + 16] : 0u, 1);
-  if (h == 0) {
-    uint32_t v = P2;
-#pragma unroll 1
-    for (int z = 15; z >= 0; --z) {
-      const uint32_t k = own_row[4 + z];
-      v = (k != 0u && v >= 2u * VF_KEY_STEP) ? v - VF_KEY_STEP : 0u;
-      if (v <= k) break;
-      own_row[4 + z] = v;
-      chg |= 1u << z;
-    }
-  }
-  return chg;
-}
-
-// The values of a visit that the code after the sweeps needs.  Thread 0
-// keeps them in shared memory, and the code after the sweeps reads them back
-// there: held in registers across the sweeps they cost spills at 64
-// registers per thread (4 CTAs per SM).
-struct VisitInfo {
-  const JobDesc* J;
-  uint32_t b, jid, pass;
-  int bx, by, bz;
-  int sweeps;  // sweeps run (the loop counter at its end)
-};
-
-template <int CONN>
-__device__ bool visit_tail(const FloodArgs& a, uint32_t* tile, uint32_t* live27, uint32_t* dirs,
-                           int* reenq, SweepShared& sw, unsigned long long* ph, uint32_t* scnt,
-                           const VisitInfo* vi);
-
-// One visit of brick b.  False when its tile load did not complete in
-// time (the error word is set; the kernel stops).
-template <int CONN>
-__device__ bool relax_brick(const FloodArgs& a, const JobDesc& J, uint32_t jid, uint32_t b,
-                            uint32_t pass, uint32_t* tile, uint32_t* live27, uint32_t* dirs,
-                            int* reenq, SweepShared& sw, uint32_t* fbits,
-                            unsigned long long* ph, uint32_t i, uint32_t qn, uint32_t* pre,
-                            uint32_t mbar, uint32_t& phase, uint32_t* scnt, VisitInfo* vi) {
-  // ph (thread 0): SM cycles of [1] live map + staging, [2] sweeps, [3] write-back + enqueue
-  // phase timing (thread 0): ph[k] += cycles since the last mark, kept in
-  // shared memory so no 64-bit clock lives in registers across the sweeps
-  if (threadIdx.x == 0) ph[5] = clock64();
-  const uint32_t lb = b - J.brick_base;
-  const int bz = lb % J.nbz, by = (lb / J.nbz) % J.nby, bx = lb / (J.nbz * J.nby);
-  const int x0 = bx * VF_BX, y0 = by * VF_BY, z0 = bz * VF_BZ;
-  const int t = threadIdx.x;
-  // What changed next to the brick since its last visit (read and cleared).
-  // A flag set after the keys it covers were written (writer: fence, then
-  // flag) makes the staging loads below see those keys (reader: flag, fence,
-  // barrier, loads); a flag this visit does not see stays for the next visit,
-  // which the same writer queued.
-  uint32_t fv = 0;
-  if (t < (int)FLOOD_FDIR) {  // exchange with acquire semantics
-    asm volatile("atom.acquire.gpu.global.exch.b32 %0, [%1], %2;"
-                 : "=r"(fv) : "l"(a.fdir + (size_t)b * FLOOD_FDIR + t), "r"(0u) : "memory");
-    fbits[t] = fv;
-  }
-  if (t >= 32 && t < 32 + 27) {  // live map of the 27 bricks around (warp 1)
-    const int n = t - 32;
-    const int dx = n / 9 - 1, dy = (n / 3) % 3 - 1, dz = n % 3 - 1;
-    const int nx = bx + dx, ny = by + dy, nz = bz + dz;
-    uint32_t l = 0;
-    if (nx >= 0 && ny >= 0 && nz >= 0 && nx < (int)J.nbx && ny < (int)J.nby && nz < (int)J.nbz)
-      l = a.live[brick_id(J, nx, ny, nz)];
-    live27[n] = l;
-  }
-  if (t == 0) {
-    atomicMax(&a.st[jid].passes, pass + 1);
-    *dirs = 0; *reenq = 0; scnt[0] = 0; scnt[1] = 0; scnt[2] = 0;
-    vi->J = &J; vi->b = b; vi->jid = jid; vi->pass = pass;
-    vi->bx = bx; vi->by = by; vi->bz = bz;
-  }
-  if (!__syncthreads_or(fv != 0)) {  // nothing new around the brick
-    if (t == 0) atomicAdd(a.stats + 16, 1u);
-    return true;
-  }
-  // Stage the keys of the brick and its one-voxel halo.  One TMA load (a
-  // 3-D box of 36 x 18 x 18 keys at z0-4, y0-1, x0-1 of the job's keys
-  // tensor) fills the 18 x 18 rows [x0-1, x0+17) x [y0-1, y0+17) with the
-  // keys z0-4 .. z0+31: [3] holds z0-1 and [4 + z] the key z0 + z; keys
-  // outside the grid arrive as zero (EMPTY).  The keys z0+32 (slot [0]) are
-  // loaded by the threads meanwhile.  Keys of neighbour bricks without
-  // occupied voxels are never initialised, so their parts of the tile are
-  // cleared once the load has landed.  Thread 224 also claims this CTA's
-  // next brick of the pass (while much of the pass is left), so the next
-  // visit starts without a claim round trip.
-  if (t == 0) {
-    // the neighbours' key writes acquired with the change record, and this
-    // CTA's own accesses to the tile, ordered before the async-proxy copy
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    asm volatile("fence.proxy.async.global;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    mbar_arrive_expect_tx(mbar, (uint32_t)TILE_BYTES);
-    tma_load_3d(smem_u32(tile), a.tmaps + (size_t)jid * vfk::KEYS_MAP_BYTES, z0 - 4, y0 - 1,
-                x0 - 1, mbar);
-  }
-  uint32_t htop[2];
-  bool bad = false;
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int q = t + u * 256;
-    htop[u] = 0;
-    if (q < KROWS) {
-      const int lx = q / KNY - 1, ly = q % KNY - 1;
-      const int x = x0 + lx, y = y0 + ly, z = z0 + VF_BZ;
-      if (x >= 0 && y >= 0 && x < (int)J.X && y < (int)J.Y && z < (int)J.Zk) {
-        const int dx = lx < 0 ? 0 : (lx >= VF_BX ? 2 : 1);
-        const int dy = ly < 0 ? 0 : (ly >= VF_BY ? 2 : 1);
-        if (live27[dx * 9 + dy * 3 + 2]) {
-          const size_t ki = vf_kidx(J, x, y, z);
-          if (ki < (size_t)J.X * J.Y * J.Zk) htop[u] = __ldcg(J.keys + ki);
-          else bad = true;
-        }
-      }
-    }
-  }
-  if (t == 224 && i + 2u * gridDim.x < qn) {
-    const uint32_t c = atomicAdd(&a.qhead[pass % 3u], 1u);
-    if (c < qn) *pre = c;
-  }
-  if (bad) flood_anomaly(a, 3u, b, (uint32_t)t);
-  const bool landed = mbar_wait(mbar, phase);
-  if (__syncthreads_or(!landed)) {
-    // the copy did not complete in time: report it, give it one more bounded
-    // wait so that nothing is in flight into this CTA's tile, and stop
-    if (t == 0) atomicOr(a.err, 16u);
-    mbar_wait(mbar, phase);
-    return false;
-  }
-  phase ^= 1u;
-  // clear the parts of bricks without occupied voxels, place the keys z0+32
-#pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int q = t + u * 256;
-    if (q < KROWS) {
-      uint32_t* row = tile + q * KP;
-      const int lx = q / KNY, ly = q % KNY;
-      const int dx = lx == 0 ? 0 : (lx == KNX - 1 ? 2 : 1);
-      const int dy = ly == 0 ? 0 : (ly == KNY - 1 ? 2 : 1);
-      if (!live27[dx * 9 + dy * 3 + 1]) {
-#pragma unroll
-        for (int c = 0; c < VF_BZ / 4; ++c)
-          *reinterpret_cast<uint4*>(row + 4 + 4 * c) = make_uint4(0, 0, 0, 0);
-      }
-      if (!live27[dx * 9 + dy * 3 + 0]) row[3] = 0u;
-      row[0] = htop[u];
-    }
-  }
-  __syncthreads();
-  if (t == 0) { const unsigned long long now = clock64(); ph[1] += now - ph[5]; ph[5] = now; }
-  const int tx = t / VF_BY, ty = t % VF_BY;
-  uint32_t* own_row = tile + ((tx + 1) * KNY + (ty + 1)) * KP;
-  // Row layout (KP u32): [0] key z0+32, [3] key z0-1, [4 + z] key z0 + z.  The
-  // z halo candidates are fixed for the visit (other bricks' keys).
-  uint32_t hlo, hhi;
-  if (CONN == 26) {
-    hlo = 0; hhi = 0;
-#pragma unroll
-    for (int r = 0; r < 9; ++r) {
-      const uint32_t* rp = own_row + ((r / 3 - 1) * KNY + (r % 3 - 1)) * KP;
-      hlo = max(hlo, rp[3]);
-      hhi = max(hhi, rp[0]);
-    }
-  } else {
-    hlo = own_row[3];
-    hhi = own_row[0];
-  }
-  // scnt: [0] active row-sweeps, [2] busy warp-sweeps (thread 0), [1] key changes
-  sw.hl[t] = hlo;
-  sw.hh[t] = hhi;
-  sw.rowchg[t] = 0;
-  uint32_t occ8 = 0;
-#pragma unroll
-  for (int q = 0; q < VF_BZ / 4; ++q) {
-    const uint4 kv = lds4(own_row + 4 + 4 * q);
-    if ((kv.x | kv.y | kv.z | kv.w) != 0u) occ8 |= 1u << q;
-  }
-  sw.occ8[t] = (uint8_t)occ8;
-  // Sweep 0 runs the rows that read a changed key: x/y face, edge and corner
-  // neighbours mark whole faces and edges, the z neighbours the changed rows
-  // (26: widened by one row in x and y); bit 13 marks every row.
-  bool act0;
-  {
-    const uint32_t d = fbits[0];
-    const uint32_t dxm = 2u | (tx == 0 ? 1u : 0u) | (tx == VF_BX - 1 ? 4u : 0u);
-    const uint32_t dym = 2u | (ty == 0 ? 1u : 0u) | (ty == VF_BY - 1 ? 4u : 0u);
-    uint32_t hit = 0;
-#pragma unroll
-    for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-      for (int dy = 0; dy < 3; ++dy)
-        if ((dxm >> dx) & (dym >> dy) & 1u) hit |= (d >> (dx * 9 + dy * 3)) & 7u;
-    // the z neighbours name exactly the rows whose end voxel they improve
-    const uint32_t zc = (((fbits[1 + (tx >> 1)] | fbits[9 + (tx >> 1)]) >> ((tx & 1) * 16)) & 0xFFFFu);
-    hit |= (zc >> ty) & 1u;
-    act0 = hit != 0 && occ8 != 0u;  // a row without occupied voxels never changes
-  }
-  // Sweeps.  The rows to run are compacted onto the lowest threads (one list
-  // per sweep), so a sweep with n active rows keeps ceil(n / 32) warps busy.
-  // A row runs when a neighbour row changed in the previous sweep (its own
-  // changes are already final along z against the neighbour values it read);
-  // sweep 0 runs the rows next to new halo data (act0).  sw.rfw[s & 1] holds
-  // the rows that changed in sweep s - 1 (bit row & 31 of word row >> 5, row
-  // t = x * 16 + y, so word w holds x-rows 2w and 2w + 1).
-  const int lane = t & 31, wid = t >> 5;
-  int it = 0, cur = 0;
-  for (; it < a.max_sweeps; ++it) {
-    const uint32_t* pw = sw.rfw + cur * 8;
-    bool active;
-    if (it == 0) {
-      active = act0;
-    } else {
-      const uint32_t m0 = tx > 0 ? (pw[(tx - 1) >> 1] >> (((tx - 1) & 1) * 16)) & 0xFFFFu : 0u;
-      const uint32_t m1 = (pw[tx >> 1] >> ((tx & 1) * 16)) & 0xFFFFu;
-      const uint32_t m2 = tx < VF_BX - 1 ? (pw[(tx + 1) >> 1] >> (((tx + 1) & 1) * 16)) & 0xFFFFu : 0u;
-      if (CONN == 26)
-        active = ((((m0 | m2) << 1) & (7u << ty)) | ((m1 << 1) & (5u << ty))) != 0;
-      else
-        active = ((((m0 | m2) >> ty) & 1u) | ((m1 << 1) & (5u << ty))) != 0;
-      active = active && sw.occ8[t] != 0;
-    }
-    const unsigned bal = __ballot_sync(0xFFFFFFFFu, active);
-    if (lane == 0) sw.wmask[wid] = bal;
-    if (t < 8) sw.rfw[(cur ^ 1) * 8 + t] = 0u;  // filled by this sweep's changes
-    __syncthreads();
-    // The lane pair (t, t ^ 1) takes the idx-th active row, idx = t / 2 (and
-    // 128 more per round when more than 128 rows are active): the k-th
-    // active lane of warp ws.
-    uint32_t n = 0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) n += (uint32_t)__popc(sw.wmask[i]);
-    uint32_t chg = 0;
-    for (uint32_t base = 0; base < n; base += 128u) {
-      const uint32_t idx = base + ((uint32_t)t >> 1);
-      const unsigned pm = __ballot_sync(0xFFFFFFFFu, idx < n);
-      if (idx < n) {
-        uint32_t acc = 0, k = 0;
-        int ws = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint32_t c = (uint32_t)__popc(sw.wmask[i]);
-          if (idx >= acc && idx < acc + c) {
-            ws = i;
-            k = idx - acc;
+      // Gang barrier: one arrival counter that only grows, which every CTA
+      // polls.  Whether a wave follows is in a word of its own, the last wave
+      // with candidates; it is read while the next wave scans.
+      if (tid == 0) {
+        if (s_any[t & 1u]) atomicMax(bar + 16, t + 1u);
+        red_release(bar, 1u);
+        const uint32_t target = (t + 1u) * size;
+        uint32_t spins = 0, ok = 1;
+        while ((int32_t)(ld_acquire(bar) - target) < 0) {
+          if (++spins > a.wait_spins || ((spins & 63u) == 0 && ld_acquire(a.err) != 0)) {
+            atomicOr(a.err, 2u);
+            atomicAdd(a.stats + 3, 1u);
+            ok = 0;
+            break;
           }
-          acc += c;
         }
-        const int row = 32 * ws + nth_set_bit(sw.wmask[ws], k);
-        uint32_t* rr = tile + (((row >> 4) + 1) * KNY + ((row & 15) + 1)) * KP;
-        const uint32_t c = relax_half<CONN>(rr, t & 1, sw.hl[row], sw.hh[row], sw.occ8[row],
-                                            it == 0, pm);
-        if (c) {
-          atomicOr(&sw.rfw[(cur ^ 1) * 8 + (row >> 5)], 1u << (row & 31));
-          atomicOr(&sw.rowchg[row], c);
-          chg |= c;
-        }
-      }
-    }
-    cur ^= 1;
-    if (t == 0) { scnt[0] += n; scnt[2] += (2u * n + 31u) / 32u; }
-    if (chg) atomicAdd(&scnt[1], (uint32_t)__popc(chg));
-    if (!__syncthreads_or(chg != 0)) break;
-  }
-  if (t == 0) vi->sweeps = it;
-  return visit_tail<CONN>(a, tile, live27, dirs, reenq, sw, ph, scnt, vi);
-}
-
-// The rest of a visit, after the sweeps: the distance limit, write-back,
-// notifications and statistics.
-template <int CONN>
-__device__ bool visit_tail(const FloodArgs& a, uint32_t* tile, uint32_t* live27, uint32_t* dirs,
-                           int* reenq, SweepShared& sw, unsigned long long* ph, uint32_t* scnt,
-                           const VisitInfo* vi) {
-  const int t = threadIdx.x;
-  const JobDesc& J = *vi->J;
-  const uint32_t b = vi->b, jid = vi->jid, pass = vi->pass;
-  const int bx = vi->bx, by = vi->by, bz = vi->bz;
-  const int x0 = bx * VF_BX, y0 = by * VF_BY, z0 = bz * VF_BZ;
-  const int tx = t / VF_BY, ty = t % VF_BY;
-  uint32_t* own_row = tile + ((tx + 1) * KNY + (ty + 1)) * KP;
-  uint32_t overflow = 0;
-  const uint32_t changed = sw.rowchg[t];
-  // Distance limit: an unreached voxel next to a key at the largest distance
-  // the key format holds.  Checked on the converged tile, and only when some
-  // key of the tile (row or halo) is at that distance.
-  {
-    bool lim = false;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const uint4 v = lds4(own_row + 4 + 4 * q);
-      lim |= at_limit(v.x) | at_limit(v.y) | at_limit(v.z) | at_limit(v.w);
-    }
-    lim |= at_limit(own_row[0]) | at_limit(own_row[3]);
-    if (t < 2 * KNY + 2 * VF_BX) {  // the 68 halo rows of the 18 x 18 tile
-      const int lx = t < KNY ? 0 : t < 2 * KNY ? KNX - 1 : 1 + (t - 2 * KNY) % VF_BX;
-      const int ly = t < KNY ? t : t < 2 * KNY ? t - KNY : (t < 2 * KNY + VF_BX ? 0 : KNY - 1);
-      const uint32_t* hr = tile + (lx * KNY + ly) * KP;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const uint4 v = lds4(hr + 4 + 4 * q);
-        lim |= at_limit(v.x) | at_limit(v.y) | at_limit(v.z) | at_limit(v.w);
-      }
-      lim |= at_limit(hr[0]) | at_limit(hr[3]);
-    }
-    if (__syncthreads_or(lim)) {
-      // key at z (-1 .. 32) of a row: [3] z0-1, [4 + z], [0] z0+32
-      auto at = [](const uint32_t* r, int z) { return r[z < 0 ? 3 : (z >= VF_BZ ? 0 : 4 + z)]; };
-      for (int z = 0; z < VF_BZ; ++z) {
-        if (own_row[4 + z] != VF_KEY_UNREACHED) continue;
-        uint32_t m = max(at(own_row, z - 1), at(own_row, z + 1));
-        if (CONN == 26) {
-          for (int r = 0; r < 9; ++r) {
-            const uint32_t* rp = own_row + ((r / 3 - 1) * KNY + (r % 3 - 1)) * KP;
-            m = max(m, max(at(rp, z - 1), max(at(rp, z), at(rp, z + 1))));
-          }
-        } else {
-          m = max(m, max(max(own_row[-KNY * KP + 4 + z], own_row[KNY * KP + 4 + z]),
-                         max(own_row[-KP + 4 + z], own_row[KP + 4 + z])));
-        }
-        if (at_limit(m)) overflow = 1;
-      }
-    }
-  }
-  if (t == 0) { const unsigned long long now = clock64(); ph[2] += now - ph[5]; ph[5] = now; }
-  const int x = x0 + tx, y = y0 + ty;
-  if (changed && x < (int)J.X && y < (int)J.Y) {
-    // write back the changed 32-byte sectors of the row
-    const int nq = min(VF_BZ, (int)J.Zk - z0) / 4;
-    const size_t ki = vf_kidx(J, x, y, z0);
-    uint4* dst = reinterpret_cast<uint4*>(J.keys + ki);
-    if (ki + 4 * (size_t)nq <= (size_t)J.X * J.Y * J.Zk && (reinterpret_cast<uintptr_t>(dst) & 15u) == 0) {
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        if (q < nq && ((changed >> (8 * (q >> 1))) & 0xFFu)) __stcg(dst + q, lds4(own_row + 4 + 4 * q));
-    } else {
-      flood_anomaly(a, 5u, b, (uint32_t)ki);
-    }
-  }
-  if (overflow) atomicOr(&a.st[jid].err, VF_JERR_DIST_OVERFLOW);
-  // Notifications.  A neighbour brick is queued (and its change record set)
-  // only when a voxel this visit changed can improve one of its voxels,
-  // judged against the neighbour's keys staged in the halo.  Staged keys can
-  // only be lower than the neighbour's current ones (keys never decrease),
-  // so a halo voxel that no changed voxel improves here cannot be improved
-  // in the neighbour either: skipping it loses nothing.  This drops the
-  // visits a front would otherwise send back to the brick it came from.
-  // changed key of interior row r (brick coordinates) at z, or 0
-  auto chg_key = [&](int rx, int ry, int z) -> uint32_t {
-    const uint32_t c = sw.rowchg[rx * VF_BY + ry];
-    return ((c >> z) & 1u) ? tile[((rx + 1) * KNY + (ry + 1)) * KP + 4 + z] : 0u;
-  };
-  // (a) the z faces, per interior row: the halo voxels below (z0-1) and
-  //     above (z0+32) the row, against the changed keys of the window rows
-  //     at z0 and z0+31 (26: the interior rows of the 3x3 around; 6: the row)
-  bool lo_imp = false, hi_imp = false;
-  {
-    const uint32_t klo = own_row[3], khi = own_row[0];
-    if (klo | khi) {
-      uint32_t mlo = 0, mhi = 0;
-      if (CONN == 26) {
-#pragma unroll
-        for (int r = 0; r < 9; ++r) {
-          const int rx = tx + r / 3 - 1, ry = ty + r % 3 - 1;
-          if (rx < 0 || ry < 0 || rx >= VF_BX || ry >= VF_BY) continue;
-          mlo = max(mlo, chg_key(rx, ry, 0));
-          mhi = max(mhi, chg_key(rx, ry, VF_BZ - 1));
-        }
-      } else {
-        mlo = chg_key(tx, ty, 0);
-        mhi = chg_key(tx, ty, VF_BZ - 1);
-      }
-      lo_imp = klo != 0u && step_from(mlo) > klo;
-      hi_imp = khi != 0u && step_from(mhi) > khi;
-    }
-  }
-  // (b) the x/y faces, edges and corners: one thread per halo row of the
-  //     tile's perimeter.  C(z) = the largest changed key at z among the
-  //     interior rows next to the halo row; a halo voxel at z is improvable
-  //     when step(max of C over its z window) beats its key.  Chunks of four
-  //     keys with one chunk of look-ahead, as in relax_half.
-  if (t < 2 * KNY + 2 * VF_BX) {
-    const int lx = t < KNY ? 0 : t < 2 * KNY ? KNX - 1 : 1 + (t - 2 * KNY) % VF_BX;
-    const int ly = t < KNY ? t : t < 2 * KNY ? t - KNY : (t < 2 * KNY + VF_BX ? 0 : KNY - 1);
-    const uint32_t* hr = tile + (lx * KNY + ly) * KP;
-    // Interior rows next to this halo row, as a line of up to three rows
-    // (brick coordinates): the halo row's inward neighbour (ix, iy) and, for
-    // 26, its two neighbours along the halo edge (dx, dy) when inside.  A
-    // corner halo row has one (26) or none (6).  Rows outside get a zero mask.
-    const bool xs = lx == 0 || lx == KNX - 1, ys = ly == 0 || ly == KNY - 1;
-    const int ix = lx == 0 ? 0 : (lx == KNX - 1 ? VF_BX - 1 : lx - 1);
-    const int iy = ly == 0 ? 0 : (ly == KNY - 1 ? VF_BY - 1 : ly - 1);
-    const int ex = xs ? 0 : 1, ey = xs ? 1 : 0;  // direction along the edge
-    uint32_t cm[3] = {0u, 0u, 0u};
-    int base_row = (ix + 1) * KNY + (iy + 1);    // tile row of the middle row
-    const int stride_row = ex * KNY + ey;        // tile rows between the three
-    if (CONN == 26 || xs != ys) {
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        const int rx = ix + (k - 1) * ex, ry = iy + (k - 1) * ey;
-        const bool in = (CONN == 26 || k == 1) && rx >= 0 && ry >= 0 && rx < VF_BX && ry < VF_BY &&
-                        !(xs && ys && k != 1);
-        cm[k] = in ? sw.rowchg[rx * VF_BY + ry] : 0u;
-      }
-    }
-    const uint32_t u = cm[0] | cm[1] | cm[2];
-    if (u) {
-      // changed keys of the adjacent rows at chunk q, column maximum
-      auto chunkC = [&](int q) -> uint4 {
-        uint4 c = make_uint4(0, 0, 0, 0);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const uint32_t m = cm[k] >> (4 * q);
-          if (!(m & 0xFu)) continue;
-          const uint4 v = lds4(tile + (base_row + (k - 1) * stride_row) * KP + 4 + 4 * q);
-          c.x = max(c.x, (m & 1u) ? v.x : 0u);
-          c.y = max(c.y, (m & 2u) ? v.y : 0u);
-          c.z = max(c.z, (m & 4u) ? v.z : 0u);
-          c.w = max(c.w, (m & 8u) ? v.w : 0u);
-        }
-        return c;
-      };
-      auto imp = [](uint32_t w, uint32_t kh) { return kh != 0u && step_from(w) > kh; };
-      bool face = false, below = false, above = false;
-      uint4 Cc = chunkC(0);
-      uint32_t cprev = 0;
-      if (CONN == 26) below = imp(Cc.x, hr[3]);  // z0-1 reads C(z0)
-#pragma unroll 1
-      for (int q = 0; q < 8; ++q) {
-        // changed keys at z = 4q-1 .. 4q+4 reach this chunk's halo voxels
-        const uint32_t win = q == 0 ? (u & 0x1Fu) : ((u >> (4 * q - 1)) & 0x3Fu);
-        if (win) {
-          const uint4 Cn = (CONN == 26 && q < 7) ? chunkC(q + 1) : make_uint4(0, 0, 0, 0);
-          const uint4 kh = lds4(hr + 4 + 4 * q);
-          uint32_t w0, w1, w2, w3;
-          if (CONN == 26) {
-            w0 = max(cprev, max(Cc.x, Cc.y));
-            w1 = max(Cc.x, max(Cc.y, Cc.z));
-            w2 = max(Cc.y, max(Cc.z, Cc.w));
-            w3 = max(Cc.z, max(Cc.w, Cn.x));
-          } else {
-            w0 = Cc.x; w1 = Cc.y; w2 = Cc.z; w3 = Cc.w;
-          }
-          face |= imp(w0, kh.x) | imp(w1, kh.y) | imp(w2, kh.z) | imp(w3, kh.w);
-          cprev = Cc.w;
-          Cc = CONN == 26 ? Cn : (q < 7 ? chunkC(q + 1) : Cc);
-        } else {
-          cprev = 0u;
-          Cc = q < 7 ? chunkC(q + 1) : Cc;
-        }
-      }
-      if (CONN == 26) above = imp(cprev, hr[0]);  // z0+32 reads C(z0+31)
-      const int sx = lx == 0 ? 0 : (lx == KNX - 1 ? 2 : 1);
-      const int sy = ly == 0 ? 0 : (ly == KNY - 1 ? 2 : 1);
-      const uint32_t dmh = (below ? 1u << (sx * 9 + sy * 3 + 0) : 0u) |
-                           (face ? 1u << (sx * 9 + sy * 3 + 1) : 0u) |
-                           (above ? 1u << (sx * 9 + sy * 3 + 2) : 0u);
-      if (dmh) atomicOr(dirs, dmh);
-    }
-  }
-  // rows of the z neighbours that read an improvable key (exact row masks)
-  const unsigned zlo = __ballot_sync(0xFFFFFFFFu, lo_imp);
-  const unsigned zhi = __ballot_sync(0xFFFFFFFFu, hi_imp);
-  if ((t & 31) == 0 && (zlo | zhi))
-    atomicOr(dirs, (zlo ? 1u << (1 * 9 + 1 * 3 + 0) : 0u) | (zhi ? 1u << (1 * 9 + 1 * 3 + 2) : 0u));
-  // statistics: active row-sweeps and key changes (block sums in shared memory)
-  if (t == 0) {
-    const int it = vi->sweeps;
-    if (it == a.max_sweeps) *reenq = 1;
-    atomicAdd(a.stats + 4, (uint32_t)it + 1u);  // sweeps (statistics)
-    if (it == a.max_sweeps) atomicAdd(a.stats + 5, 1u);
-  }
-  __syncthreads();
-  if (t == 0) {
-    atomicAdd(a.stats + 6, scnt[0]);
-    atomicAdd(a.stats + 7, scnt[1]);
-    atomicAdd(a.stats + 2, scnt[2]);
-    if (scnt[1] == 0) atomicAdd(a.stats + 17, 1u);  // staged, but no key changed
-  }
-  // change records of the neighbours, after the key writes above (fence), then
-  // the neighbours go on the next pass's queue
-  if (t < 32 || (t & 31) == 0) asm volatile("fence.acq_rel.gpu;" ::: "memory");
-  if ((t & 31) == 0) {
-    const int w = t >> 5;
-    if (zlo && live27[1 * 9 + 1 * 3 + 0]) {  // below: its keys at z0'+32 are our bottom layer
-      const uint32_t nb = brick_id(J, bx, by, bz - 1);
-      if (nb < a.nbricks) atomicOr(&a.fdir[(size_t)nb * FLOOD_FDIR + 9 + w], zlo);
-    }
-    if (zhi && live27[1 * 9 + 1 * 3 + 2]) {  // above: its keys at z0'-1 are our top layer
-      const uint32_t nb = brick_id(J, bx, by, bz + 1);
-      if (nb < a.nbricks) atomicOr(&a.fdir[(size_t)nb * FLOOD_FDIR + 1 + w], zhi);
-    }
-  }
-  if (t < 32) {
-    const uint32_t dm = *dirs;
-    bool want = false;
-    uint32_t nb = 0;
-    if (t < 27 && ((dm >> t) & 1u) && live27[t]) {
-      want = true;
-      nb = brick_id(J, bx + t / 9 - 1, by + (t / 3) % 3 - 1, bz + t % 3 - 1);
-      // seen from nb this brick is in direction 26 - t; z faces use the row masks
-      if (t != 1 * 9 + 1 * 3 + 0 && t != 1 * 9 + 1 * 3 + 2 && nb < a.nbricks)
-        atomicOr(&a.fdir[(size_t)nb * FLOOD_FDIR], 1u << (26 - t));
-    }
-    if (t == 27 && *reenq) {  // sweep cap: the brick comes back with every row
-      want = true;
-      nb = b;
-      atomicOr(&a.fdir[(size_t)b * FLOOD_FDIR], 1u << 13);
-    }
-    enqueue(a, nb, pass + 1, want);
-  }
-  if (t == 0) ph[3] += clock64() - ph[5];
-  return true;
-}
-
-__global__ void __launch_bounds__(256, 4) k_relax(FloodArgs args) {
-  // The arguments are read from a shared copy: the kernel and the functions
-  // it calls take them by reference, and a shared-memory struct is an
-  // ordinary addressable object (no address of the parameter space is taken).
-  __shared__ FloodArgs a;
-  if (threadIdx.x == 0) a = args;
-  __syncthreads();
-  // the tile, a TMA destination: 128-byte aligned inside the dynamic shared
-  // memory (TILE_SMEM = TILE_BYTES + 128)
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  uint32_t* tile = reinterpret_cast<uint32_t*>(smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u));
-  __shared__ uint32_t live27[27];
-  __shared__ uint32_t dirs;
-  __shared__ int reenq;
-  __shared__ uint32_t item;
-  __shared__ uint32_t pre;  // queue index of the next brick, claimed ahead (~0: none)
-  __shared__ SweepShared sw;
-  __shared__ uint32_t fbits[FLOOD_FDIR];
-  // thread 0: SM cycles per phase (see flush below); [5] the phase mark of a
-  // visit, [6] the clock at the last claim
-  __shared__ unsigned long long ph[7];
-  __shared__ uint32_t scnt[3];   // per visit: active row-sweeps, key changes, busy warp-sweeps
-  __shared__ VisitInfo vinfo;
-  // the pass, its queue length and its visits: read back from shared memory
-  // around each visit (registers held across a visit cost spills)
-  __shared__ uint32_t pass_p, pass_qn, pass_visits;
-  __shared__ __align__(8) unsigned long long tile_bar;  // completion of the tile loads
-  const uint32_t mbar = smem_u32(&tile_bar);
-  uint32_t phase = 0;  // parity of the tile load in flight (uniform across the CTA)
-  if (threadIdx.x < 5) ph[threadIdx.x] = 0;
-  if (threadIdx.x == 0) {
-    pre = 0xFFFFFFFFu;
-    pass_p = 0;
-    mbar_init(mbar, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  for (;;) {
-    const uint32_t p0 = pass_p;
-    if (p0 >= a.max_passes) break;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      a.qcount[(p0 + 2) % 3] = 0;
-      a.qhead[(p0 + 2) % 3] = 0;
-    }
-    if (threadIdx.x == 0) {
-      pass_qn = ld_acquire(&a.qcount[p0 % 3u]);
-      pass_visits = 0;
-      if (a.pass_sizes && blockIdx.x == 0 && p0 < 256) a.pass_sizes[p0] = pass_qn;
-    }
-    for (;;) {
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        ph[6] = clock64();
-        item = pre != 0xFFFFFFFFu ? pre : atomicAdd(&a.qhead[pass_p % 3u], 1u);
-        pre = 0xFFFFFFFFu;
+        s_ok = ok;
       }
       __syncthreads();
-      const uint32_t i = item, p = pass_p, qn = pass_qn, cur = p % 3u;
-      if (i >= qn) break;
-      const uint32_t b = a.queue[cur][i];
-      if (b >= a.nbricks) {
-        if (threadIdx.x == 0) flood_anomaly(a, 1u, b, i);
-        continue;
-      }
-      const uint32_t jid = a.brick_job[b];
-      if (jid >= a.njobs) {
-        if (threadIdx.x == 0) flood_anomaly(a, 2u, b, jid);
-        continue;
-      }
-      const JobDesc& J = a.jobs[jid];
-      const int conn6 = J.distance == 1;
-      if (threadIdx.x == 0) ph[0] += clock64() - ph[6];
-      const bool ok =
-          conn6 ? relax_brick<6>(a, J, jid, b, p, tile, live27, &dirs, &reenq, sw, fbits, ph, i,
-                                 qn, &pre, mbar, phase, scnt, &vinfo)
-                : relax_brick<26>(a, J, jid, b, p, tile, live27, &dirs, &reenq, sw, fbits, ph, i,
-                                  qn, &pre, mbar, phase, scnt, &vinfo);
-      if (!ok) return;  // tile load timed out (error word set; the others stop at the barrier)
-      if (threadIdx.x == 0) ++pass_visits;
-    }
-    const uint32_t p = pass_p;
-    if (threadIdx.x == 0 && pass_visits) atomicAdd(&a.stats[0], pass_visits);
-    const bool synced = grid_sync(a.bar, gridDim.x, a.err, a.stats, a.wait_spins);
-    if (threadIdx.x == 0) {
-      // phase cycles: [0] claim, [1] staging, [2] sweeps, [3] write-back +
-      // enqueue, [4] from the failed claim through the pass barrier; added to
-      // stats[11..15] in units of 256 cycles
-      ph[4] += clock64() - ph[6];
-      for (int i = 0; i < 5; ++i) {
-        const uint32_t c = (uint32_t)(ph[i] >> 8);
-        if (c) atomicAdd(a.stats + 11 + i, c);
-        ph[i] &= 255u;
+      if (!s_ok) return;  // timed out: the error word is set
+      if (prune) {
+        // a job without claims in this wave has no candidates any more: its
+        // units leave the list (warp 0, in place)
+        for (uint32_t j = tid; j < njobs; j += THREADS) S.live[j] = ld_relaxed(a.last + first + j) == t + 1;
+        __syncthreads();
+        if (warp == 0) {
+          uint32_t out = 0;
+          for (uint32_t k0 = 0; k0 < nunits; k0 += 32) {
+            const uint32_t k = k0 + lane, u = k < nunits ? S.unit[k] : 0u;
+            const bool live = k < nunits && S.live[u >> 24];
+            const unsigned m = __ballot_sync(FULL, live);
+            if (live) S.unit[out + __popc(m & ((1u << lane) - 1u))] = u;
+            __syncwarp();
+            out += __popc(m);
+          }
+          if (lane == 0) s_units = out;
+        }
+        __syncthreads();
       }
     }
-    if (!synced) return;
-    const uint32_t nn = ld_acquire(&a.qcount[(p + 1) % 3]);
-    if (nn == 0 || ld_acquire(a.err) != 0) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) a.stats[1] = p + 1;
-      return;
-    }
-    if (threadIdx.x == 0) pass_p = p + 1;
-    __syncthreads();
+    for (uint32_t j = tid; j < njobs; j += THREADS)
+      if (S.last[j]) atomicMax(&a.st[a.jobs[first + j].job].passes, S.last[j]);
+    if (tid == 0 && rank == 0) atomicMax(a.stats + 1, t);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    a.stats[1] = a.max_passes;
-    atomicOr(a.err, 4u);  // did not converge
+  claims = __reduce_add_sync(FULL, claims);
+  if (lane == 0 && claims) atomicAdd(&s_stat[1], claims);
+  __syncthreads();
+  if (tid == 0) {
+    if (s_stat[0]) atomicAdd(a.stats + 0, s_stat[0]);
+    if (s_stat[1]) atomicAdd(a.stats + 7, s_stat[1]);
   }
 }
 
 // ---------------------------------------------------------------------------
-// keys from the label grid: EMPTY -> 0, occupied -> 1 (unreached)
-//
-// Row kernels over live bricks (k_init_keys, k_finalize): one brick per CTA
-// iteration, eight lanes per (x, y) row with the lanes along z.  A lane
-// handles 4 voxels (8 bytes of labels, 16 bytes of keys), so one warp
-// instruction covers 4 rows of the brick with contiguous bytes per row.  A
-// thread takes rows r, r + 32, ... r + 224 and issues all 8 loads before
-// its stores.
-constexpr int ROW_UNITS = VF_BX * VF_BY * (VF_BZ / 4) / 256;
-
-__global__ void __launch_bounds__(256) k_init_keys(const JobDesc* jobs, const uint32_t* list,
-                                                   const uint32_t* count, const uint32_t* brick_job) {
-  const uint32_t n = *count;
+// Row states from the label grid: occupied voxels unclaimed, all else zero,
+// the rows around the grid included (bricks without occupied voxels are not
+// read).  A CTA takes 256 consecutive rows of one job, eight lanes per row, 4
+// voxels per lane (a warp instruction reads 4 whole 64-byte rows); the lanes
+// then write the row's state together.
+__global__ void __launch_bounds__(256) k_wave_init(const JobDesc* jobs, WaveArrays arr, const WaveJob* wj,
+                                                   uint32_t njobs, const uint8_t* live) {
+  uint32_t lo = 0, hi = njobs - 1;  // the job of these rows: the last that starts at or before them
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi + 1) >> 1;
+    if (wj[mid].base <= blockIdx.x * 256u) lo = mid; else hi = mid - 1;
+  }
+  const WaveJob& W = wj[lo];
+  const JobDesc& J = jobs[W.job];
   const uint32_t q = threadIdx.x & 7, r0 = threadIdx.x >> 3;
-  for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
-    const uint32_t b = list[it];
-    const JobDesc& J = jobs[brick_job[b]];
-    if (!J.active) continue;
-    const uint32_t lb = b - J.brick_base;
-    const uint32_t bz = lb % J.nbz, by = (lb / J.nbz) % J.nby, bx = lb / (J.nbz * J.nby);
-    const uint32_t z = bz * VF_BZ + 4 * q;
-    // Zk is a multiple of 4 and Zp >= Zk: the lane's 4 keys and 4 labels
-    // are inside the row when z < Zk
-    if (z >= J.Zk) continue;
-    uint2 a[ROW_UNITS];
-    bool ok[ROW_UNITS];
+  const uint32_t first = blockIdx.x * 256u;
+  uint2 a[8];
 #pragma unroll
-    for (int i = 0; i < ROW_UNITS; ++i) {
-      const uint32_t r = r0 + 32u * i;
-      const uint32_t x = bx * VF_BX + r / VF_BY, y = by * VF_BY + r % VF_BY;
-      ok[i] = x < J.X && y < J.Y;
-      a[i] = ok[i] ? *reinterpret_cast<const uint2*>(J.grid + vf_gidx(J, x, y, z)) : make_uint2(0, 0);
-    }
+  for (int i = 0; i < 8; ++i) {
+    a[i] = make_uint2(0, 0);
+    const uint32_t row = first + r0 + 32u * i;
+    if (row < W.row0) continue;
+    const uint32_t r = row - W.row0, x = r / W.sx, yz = r - x * W.sx, zw = yz / W.sy, y = yz - zw * W.sy;
+    if (x >= J.X || y >= J.Y || zw >= J.nbz) continue;
+    const uint32_t z = zw * VF_BZ + 4 * q;
+    // Zp >= Zk: the lane's 4 labels are inside the row
+    if (z < J.Zk && live[J.brick_base + ((x / VF_BX) * J.nby + y / VF_BY) * J.nbz + zw])
+      a[i] = *reinterpret_cast<const uint2*>(J.grid + vf_gidx(J, x, y, z));
+  }
 #pragma unroll
-    for (int i = 0; i < ROW_UNITS; ++i) {
-      if (!ok[i]) continue;
-      const uint32_t r = r0 + 32u * i;
-      const uint32_t x = bx * VF_BX + r / VF_BY, y = by * VF_BY + r % VF_BY;
-      __stcg(reinterpret_cast<uint4*>(J.keys + vf_kidx(J, x, y, z)),
-             make_uint4((a[i].x & 0xFFFFu) ? 1u : 0u, (a[i].x >> 16) ? 1u : 0u,
-                        (a[i].y & 0xFFFFu) ? 1u : 0u, (a[i].y >> 16) ? 1u : 0u));
-    }
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t row = first + r0 + 32u * i;
+    uint32_t w = ((a[i].x & 0xFFFFu) ? 1u : 0u) | ((a[i].x >> 16) ? 2u : 0u) | ((a[i].y & 0xFFFFu) ? 4u : 0u) |
+                 ((a[i].y >> 16) ? 8u : 0u);
+    w <<= 4 * q;
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) w |= __shfl_xor_sync(FULL, w, o);
+    uint32_t* d = arr.state + (size_t)row * J.wsw;  // up to the next job's base
+
+    for (uint32_t k = q; k < J.wsw; k += 8) d[k] = k == 1 ? w : 0u;
+    if (q < 4) reinterpret_cast<uint32_t*>(arr.in + 2 * (size_t)row)[q] = 0xFFFFFFFFu;
   }
 }
 
-// seed bricks must be live (a caller may seed an EMPTY voxel)
-__global__ void k_seed_bricks(const JobDesc* jobs, JobState* st, int njobs, uint8_t* live,
-                              uint32_t* list, uint32_t* count) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= njobs) return;
-  const JobDesc& J = jobs[j];
+// seed bricks must be live (a caller may seed an EMPTY voxel); seeds are
+// checked, the fragments' prefix minima reset.  One CTA per job.
+__global__ void __launch_bounds__(128) k_seed_bricks(const JobDesc* jobs, JobState* st, uint8_t* live,
+                                                     uint32_t* list, uint32_t* count) {
+  __shared__ int dead;
+  const JobDesc& J = jobs[blockIdx.x];
   if (!J.active) return;
-  JobState& s = st[j];
-  for (int f = 0; f < 256; ++f) s.minprefix[f] = 0xFFFFFFFFu;
-  s.passes = 0;
-  s.disjoint = 0;
+  JobState& s = st[blockIdx.x];
+  for (int f = threadIdx.x; f < 256; f += blockDim.x) s.minprefix[f] = 0xFFFFFFFFu;
+  if (threadIdx.x == 0) {
+    s.passes = 0;
+    s.disjoint = 0;
+    dead = 0;
+  }
+  __syncthreads();
   const uint32_t ns = s.nseeds;
-  for (uint32_t i = 0; i < ns; ++i) {
-    const uint32_t x = J.seeds[4 * i], y = J.seeds[4 * i + 1], z = J.seeds[4 * i + 2],
-                   w = J.seeds[4 * i + 3];
+  auto brick = [&](uint32_t i) {
+    return J.brick_base + ((J.seeds[4 * i] / VF_BX) * J.nby + J.seeds[4 * i + 1] / VF_BY) * J.nbz +
+           J.seeds[4 * i + 2] / VF_BZ;
+  };
+  auto valid = [&](uint32_t i) {
     // label = frag | prefix << 8 (Seeder.cpp:150), fragment id >= 2
-    if (x >= J.X || y >= J.Y || z >= J.Z || w > 0x7FFFu || (w & 0xFFu) <= VOXEL_FREE) {
-      s.err |= VF_JERR_INVALID;
-      continue;
+    const uint32_t w = J.seeds[4 * i + 3];
+    return J.seeds[4 * i] < J.X && J.seeds[4 * i + 1] < J.Y && J.seeds[4 * i + 2] < J.Z && w <= 0x7FFFu &&
+           (w & 0xFFu) > VOXEL_FREE;
+  };
+  for (uint32_t i = threadIdx.x; i < ns; i += blockDim.x) {
+    if (!valid(i)) atomicOr(&s.err, VF_JERR_INVALID);
+    else if (!live[brick(i)]) dead = 1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && dead)
+    for (uint32_t i = 0; i < ns; ++i) {
+      if (!valid(i)) continue;
+      const uint32_t b = brick(i);
+      if (!live[b]) {
+        live[b] = 1;
+        list[atomicAdd(count, 1u)] = b;
+      }
     }
-    const uint32_t b = J.brick_base + ((x / VF_BX) * J.nby + y / VF_BY) * J.nbz + z / VF_BZ;
-    if (!live[b]) {
-      live[b] = 1;
-      list[atomicAdd(count, 1u)] = b;
+}
+
+// Seeds into the row states (later seeds win a shared voxel, as grid.set in
+// list order does, FloodFracturer.cpp:101-103), the rows around them into
+// wave 0's candidate masks.  One CTA per job; works on any axis order (the
+// seed's axis a is coordinate ax[a] of the state).
+__device__ void seed_waves(const WaveArrays& arr, const WaveJob& W, const uint32_t* seeds, uint32_t ns, uint32_t sw, int nb,
+                           uint32_t order, u64* pos) {
+  const int t = threadIdx.x;
+  auto coord = [&](uint32_t i, int a) { return seeds[4 * i + ((order >> (4 * a)) & 15u)]; };
+  for (uint32_t i = t; i < ns; i += blockDim.x)
+    pos[i] = ((u64)coord(i, 0) << 40) | ((u64)coord(i, 1) << 20) | coord(i, 2);
+  __syncthreads();
+  for (uint32_t i = t; i < ns; i += blockDim.x) {
+    bool won = true;
+    for (uint32_t k = i + 1; k < ns && won; ++k) won = pos[k] != pos[i];
+    if (!won) continue;
+    const uint32_t x = (uint32_t)(pos[i] >> 40), y = (uint32_t)(pos[i] >> 20) & 0xFFFFFu,
+                   z = (uint32_t)pos[i] & 0xFFFFFu;
+    const uint32_t zw = z >> 5, bit = 1u << (z & 31u);
+    const uint32_t row = W.row0 + x * W.sx + zw * W.sy + y;
+    uint32_t* d = arr.state + (size_t)row * sw;
+    atomicOr(d, bit);  // E0
+    atomicAnd(d + 1, ~bit);
+    for (int b = 0; b < nb; ++b)
+      if ((i >> b) & 1u) atomicOr(d + 2 + b, bit);
+    const bool lo = (z & 31u) == 0, hi = (z & 31u) == 31;
+    for (int dx = -1; dx <= 1; ++dx) {
+      const uint32_t r = row + (uint32_t)dx * W.sx;
+      set_candidates<false>(arr.cand, r, 7u);
+      if (lo) set_candidates<false>(arr.cand, r - W.sy, 7u);
+      if (hi) set_candidates<false>(arr.cand, r + W.sy, 7u);
+      for (int dy = -1; dy <= 1; ++dy) {
+        if (W.conn6 && (dx || dy)) continue;  // level 0 reaches wave 0
+        if (lo) atomicMin(&arr.in[2 * (size_t)(r - W.sy + dy)].y, in_key(0, i));
+        if (hi) atomicMin(&arr.in[2 * (size_t)(r + W.sy + dy)].x, in_key(0, i));
+      }
     }
   }
 }
 
-// seeds into the keys (later seeds win a shared voxel, as grid.set in list
-// order does, FloodFracturer.cpp:101-103) and their bricks onto queue 0
-__global__ void k_seed_keys(const JobDesc* jobs, JobState* st, int njobs, uint32_t* epoch,
-                            uint32_t* queue0, uint32_t* qcount, uint32_t* fdir) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= njobs) return;
-  const JobDesc& J = jobs[j];
-  if (!J.active) return;
-  JobState& s = st[j];
-  if (s.err) return;
-  const uint32_t ns = s.nseeds;
-  for (uint32_t i = 0; i < ns; ++i) {
-    const uint32_t x = J.seeds[4 * i], y = J.seeds[4 * i + 1], z = J.seeds[4 * i + 2];
-    J.keys[vf_kidx(J, x, y, z)] = ~i;
-    const uint32_t b = J.brick_base + ((x / VF_BX) * J.nby + y / VF_BY) * J.nbz + z / VF_BZ;
-    atomicOr(&fdir[(size_t)b * FLOOD_FDIR], 1u << 13);  // first visit: every row
-    if (atomicMax(&epoch[b], 1u) < 1u) queue0[atomicAdd(qcount, 1u)] = b;
+__global__ void __launch_bounds__(256) k_wave_seed(const JobDesc* jobs, const JobState* st, WaveArrays arr,
+                                                   const WaveJob* wj) {
+  __shared__ u64 pos[4096];
+  const WaveJob& W = wj[blockIdx.x];
+  const JobDesc& J = jobs[W.job];
+  const JobState& s = st[W.job];
+  if (!J.active || s.err) return;
+  seed_waves(arr, W, J.seeds, min(s.nseeds, 4096u), J.wsw, (int)J.wsw - 2, 0x210u, pos);
+}
+
+// ---- a flood on a caller's unpadded device grid, any axis order -----------
+// (vf_flood_noalloc).  Voxel (a, b, c) of the state, c along the words, is the
+// caller's element a * sa + b * sb + c * sc.
+// One warp per row, a lane per voxel; consecutive warps take consecutive words
+// of a grid row, whose voxels are contiguous.
+__device__ __forceinline__ bool flat_row(const WaveJob& W, const vfk::FlatAxes& A, uint32_t k, uint32_t lane,
+                                         uint32_t& row, size_t& at) {
+  // k numbers the rows of the padded box [nx + 2][ny + 1][nw + 1], words fastest
+  const uint32_t nw1 = W.sx / W.sy, zw = k % nw1, y = (k / nw1) % W.sy, x = k / W.sx;
+  row = W.row0 - W.sx + x * W.sx + zw * W.sy + y;  // base 0
+  const uint32_t z = 32 * zw + lane;
+  at = (x - 1) * A.s[0] + y * A.s[1] + z * A.s[2];
+  return x >= 1 && x <= A.nx && y < A.ny && z < A.nz;
+}
+
+__global__ void __launch_bounds__(256) k_flat_init(const uint16_t* grid, WaveArrays arr, WaveJob W,
+                                                   vfk::FlatAxes A, uint32_t sw) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t box = (A.nx + 2) * W.sx, nwarps = (gridDim.x * blockDim.x) >> 5;
+  auto put = [&](uint32_t row, uint32_t m) {
+    if (lane < sw) arr.state[(size_t)row * sw + lane] = lane == 1 ? m : 0u;
+    if (lane < 4) reinterpret_cast<uint32_t*>(arr.in + 2 * (size_t)row)[lane] = 0xFFFFFFFFu;
+  };
+  for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < box; k += nwarps) {
+    uint32_t row;
+    size_t at;
+    const bool in = flat_row(W, A, k, lane, row, at);
+    put(row, __ballot_sync(FULL, in && grid[at] != VOXEL_EMPTY));
+  }
+  // the rows before and after the box
+  const uint32_t before = W.row0 - W.sx, after = W.nrows - before - box;
+  for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < before + after; k += nwarps)
+    put(k < before ? k : box + k, 0u);
+}
+
+// wave job and gang table, then the seeds (labels 2..255 without prefix)
+__global__ void __launch_bounds__(256) k_flat_seed(WaveArrays arr, WaveJob W, vfk::FlatAxes A, uint32_t sw,
+                                                   const uint32_t* seeds, uint32_t ns, uint32_t size,
+                                                   uint32_t blocks, JobState* st, WaveJob* jobs, WaveGang* gang,
+                                                   WaveCta* cta, WaveEntry* entries) {
+  __shared__ u64 pos[4096];
+  __shared__ uint32_t bad, prefix;
+  if (threadIdx.x == 0) {
+    *jobs = W;
+    *gang = {0, 1, 0, (W.nrows + 255) / 256};
+    bad = prefix = 0;
+  }
+  for (uint32_t c = threadIdx.x; c < blocks; c += blockDim.x) {
+    cta[c] = {c, c < size ? 1u : 0u};
+    entries[c] = {0, c, size, 0};
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.x; i < ns; i += blockDim.x) {
+    const uint32_t w = seeds[4 * i + 3];
+    if (seeds[4 * i] >= A.dims[0] || seeds[4 * i + 1] >= A.dims[1] || seeds[4 * i + 2] >= A.dims[2] ||
+        w > 0x7FFFu || (w & 0xFFu) <= VOXEL_FREE)
+      bad = 1;
+    if (w > 0xFFu) prefix = 1;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    st->nseeds = ns;
+    st->err = bad ? VF_JERR_INVALID : 0u;
+    st->has_prefix = prefix;
+  }
+  if (!bad && !prefix) seed_waves(arr, W, seeds, ns, sw, (int)sw - 2, A.order, pos);
+}
+
+__global__ void __launch_bounds__(256) k_flat_labels(WaveArrays arr, WaveJob W, vfk::FlatAxes A, uint32_t sw,
+                                                     const uint32_t* seeds, uint16_t* labels) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t box = (A.nx + 2) * W.sx, nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < box; k += nwarps) {
+    uint32_t row;
+    size_t at;
+    const bool in = flat_row(W, A, k, lane, row, at);
+    if (!__any_sync(FULL, in)) continue;
+    const uint32_t word = lane < sw ? arr.state[(size_t)row * sw + lane] : 0u;
+    const uint32_t v = __shfl_sync(FULL, word, 0);
+    const uint32_t u = __shfl_sync(FULL, word, 1) & ~v;
+    uint32_t l = (u >> lane) & 1u;
+    if (v) {  // uniform
+      uint32_t slot = 0;
+      for (uint32_t b = 0; b + 2 < sw; ++b) slot |= ((__shfl_sync(FULL, word, 2 + b) >> lane) & 1u) << b;
+      if ((v >> lane) & 1u) l = seeds[4 * slot + 3] & 0xFFu;
+    }
+    if (in) labels[at] = (uint16_t)l;
   }
 }
 
-// keys -> labels (undoMask fused: & 0xFF unless prefixes must survive)
-__global__ void __launch_bounds__(256) k_finalize(const JobDesc* jobs, const JobState* st,
-                                                  const uint32_t* list, const uint32_t* count,
-                                                  const uint32_t* brick_job, int pass2) {
+// 8 bits -> 8 bytes of 0 / 1 (low four in .x)
+__device__ __forceinline__ uint2 spread8(uint32_t b) {
+  return make_uint2(((b & 15u) * 0x00204081u) & 0x01010101u, ((b >> 4) * 0x00204081u) & 0x01010101u);
+}
+
+// row states -> labels (undoMask fused: & 0xFF unless prefixes must survive).
+// Live bricks, one per CTA; four lanes per row, each 8 voxels (16 bytes of
+// labels).  EMPTY 0, unclaimed FREE, claimed: the slot's label.
+__global__ void __launch_bounds__(256) k_wave_labels(const JobDesc* jobs, const JobState* st,
+                                                     const uint32_t* list, const uint32_t* count,
+                                                     const uint32_t* brick_job, int pass2) {
   // label of each seed slot for the job of the current brick (reloaded when
   // the job changes): the seed's label (pass 1) or the pass-2 rank value,
   // reduced to the fragment byte unless the sub-seed prefixes are kept
@@ -1133,7 +860,7 @@ __global__ void __launch_bounds__(256) k_finalize(const JobDesc* jobs, const Job
     const JobDesc& J = jobs[j];
     if (!J.active) continue;  // uniform across the CTA
     const JobState& s = st[j];
-    if (pass2 && !s.has_prefix) continue;  // keys of every prefix job are final here
+    if (pass2 && !s.has_prefix) continue;  // only the prefix jobs flood twice
     if ((int)j != cached) {  // uniform: cached changes only between barriers
       __syncthreads();
       const bool keep_prefix = !pass2 && s.has_prefix;
@@ -1146,36 +873,48 @@ __global__ void __launch_bounds__(256) k_finalize(const JobDesc* jobs, const Job
       if (threadIdx.x == 0) cached = (int)j;
       __syncthreads();
     }
-    // rows as in k_init_keys: 8 lanes per row along z, 4 keys per lane
     const uint32_t lb = b - J.brick_base;
     const uint32_t bz = lb % J.nbz, by = (lb / J.nbz) % J.nby, bx = lb / (J.nbz * J.nby);
-    const uint32_t z = bz * VF_BZ + 4 * (threadIdx.x & 7), r0 = threadIdx.x >> 3;
-    if (z >= J.Zk) continue;
-    uint4 k4[ROW_UNITS];
-    bool ok[ROW_UNITS];
+    const uint32_t part = threadIdx.x & 3u, z = bz * VF_BZ + 8 * part;
+    if (z >= J.Zp) continue;
+    const uint32_t nq = J.wsw / 4;
 #pragma unroll
-    for (int i = 0; i < ROW_UNITS; ++i) {
-      const uint32_t r = r0 + 32u * i;
-      const uint32_t x = bx * VF_BX + r / VF_BY, y = by * VF_BY + r % VF_BY;
-      ok[i] = x < J.X && y < J.Y;
-      k4[i] = ok[i] ? __ldcg(reinterpret_cast<const uint4*>(J.keys + vf_kidx(J, x, y, z)))
-                    : make_uint4(0, 0, 0, 0);
-    }
+    for (int pass = 0; pass < 4; ++pass) {
+      const uint32_t row = (threadIdx.x >> 2) + 64u * pass;
+      const uint32_t x = bx * VF_BX + row / VF_BY, y = by * VF_BY + row % VF_BY;
+      if (x >= J.X || y >= J.Y) continue;
+      const uint4* src = reinterpret_cast<const uint4*>(J.wstate + (size_t)(J.wrow0 + x * J.wsx + bz * J.wsy + y) * J.wsw);
+      const uint4 a = __ldcs(src);
+      const uint32_t sh = 8 * part;
+      const uint32_t v = (a.x >> sh) & 0xFFu, u = ((a.y & ~a.x) >> sh) & 0xFFu;
+      uint4 out = make_uint4(0, 0, 0, 0);
+      if (v | u) {
+        const uint2 us = spread8(u);
+        const uint2 l0 = spread8((a.z >> sh) & 0xFFu), l1 = spread8((a.w >> sh) & 0xFFu);
+        uint2 lo = make_uint2(l0.x | (l1.x << 1), l0.y | (l1.y << 1)), hi = make_uint2(0, 0);  // slot bits 0-7, 8-
+        for (uint32_t k = 1; k < nq; ++k) {
+          const uint4 c = src[k];
+          const uint32_t p[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
-    for (int i = 0; i < ROW_UNITS; ++i) {
-      if (!ok[i]) continue;
-      const uint32_t r = r0 + 32u * i;
-      const uint32_t x = bx * VF_BX + r / VF_BY, y = by * VF_BY + r % VF_BY;
-      const uint32_t ks[4] = {k4[i].x, k4[i].y, k4[i].z, k4[i].w};
-      uint32_t lv[4];
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t bit = 4 * k - 2 + i;  // slot bit of plane word 4 k + i
+            const uint2 sp = spread8((p[i] >> sh) & 0xFFu);
+            if (bit < 8) { lo.x |= sp.x << bit; lo.y |= sp.y << bit; }
+            else { hi.x |= sp.x << (bit - 8); hi.y |= sp.y << (bit - 8); }
+          }
+        }
+        uint32_t l[8];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const uint32_t key = ks[h];
-        // reached: the slot's label; else 0 EMPTY, 1 FREE
-        lv[h] = key >= VF_KEY_MIN_REACHED ? (uint32_t)lab[(~key) & 0xFFFu] : key;
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t by8 = 8 * (i & 3);
+          const uint32_t slot = (((i < 4 ? lo.x : lo.y) >> by8) & 0xFFu) |
+                                ((((i < 4 ? hi.x : hi.y) >> by8) & 0xFu) << 8);
+          const uint32_t fr = ((i < 4 ? us.x : us.y) >> by8) & 1u;
+          l[i] = (v >> i) & 1u ? (uint32_t)lab[slot] : fr;
+        }
+        out = make_uint4(l[0] | (l[1] << 16), l[2] | (l[3] << 16), l[4] | (l[5] << 16), l[6] | (l[7] << 16));
       }
-      *reinterpret_cast<uint2*>(J.grid + vf_gidx(J, x, y, z)) =
-          make_uint2(lv[0] | (lv[1] << 16), lv[2] | (lv[3] << 16));
+      *reinterpret_cast<uint4*>(J.grid + vf_gidx(J, x, y, z)) = out;
     }
   }
 }
@@ -1256,8 +995,11 @@ __global__ void k_ranks(const JobDesc* jobs, JobState* st, int njobs) {
   s.nranks = nr;
 }
 
-// disjointSetStack: non-minimal prefixes -> FREE; survivors keyed by slot
-__global__ void __launch_bounds__(256) k_disjoint_reset(const JobDesc* jobs, JobState* st,
+// disjointSetStack: voxels of non-minimal prefixes -> unclaimed; the
+// survivors are the second flood's wave 0, keyed by their rank.  One thread
+// per row of a live brick; every row with unclaimed voxels becomes a
+// candidate of wave 0.
+__global__ void __launch_bounds__(256) k_disjoint_reset(const JobDesc* jobs, const JobState* st,
                                                         const uint32_t* list, const uint32_t* count,
                                                         const uint32_t* brick_job) {
   const uint32_t n = *count;
@@ -1266,47 +1008,48 @@ __global__ void __launch_bounds__(256) k_disjoint_reset(const JobDesc* jobs, Job
     const uint32_t j = brick_job[b];
     const JobDesc& J = jobs[j];
     if (!J.active || !st[j].has_prefix) continue;
-    JobState& s = st[j];
+    const JobState& s = st[j];
     const uint32_t lb = b - J.brick_base;
     const uint32_t bz = lb % J.nbz, by = (lb / J.nbz) % J.nby, bx = lb / (J.nbz * J.nby);
     const uint32_t x = bx * VF_BX + threadIdx.x / VF_BY, y = by * VF_BY + threadIdx.x % VF_BY;
     const uint32_t z0 = bz * VF_BZ;
-    uint32_t reset = 0;
-    if (x < J.X && y < J.Y) {
-      for (uint32_t z = z0; z < min(z0 + VF_BZ, J.Zk); ++z) {
-        uint32_t key = 0;
-        if (z < J.Z) {
-          uint16_t* gp = J.grid + vf_gidx(J, x, y, z);
-          const uint32_t g = *gp;
-          if (g == VOXEL_FREE) key = VF_KEY_UNREACHED;
-          else if (g > VOXEL_FREE) {
-            if ((g >> 8) != s.minprefix[g & 0xFFu]) {
-              *gp = VOXEL_FREE;
-              key = VF_KEY_UNREACHED;
-              ++reset;
-            } else {
-              key = ~s.value_rank[g & 0xFFu];
-            }
-          }
-        }
-        J.keys[vf_kidx(J, x, y, z)] = key;
+    if (x >= J.X || y >= J.Y) continue;
+    uint32_t w[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) w[k] = 0;
+    for (uint32_t z = z0; z < min(z0 + VF_BZ, J.Z); ++z) {
+      const uint32_t g = J.grid[vf_gidx(J, x, y, z)], bit = 1u << (z - z0);
+      if (g == VOXEL_EMPTY) continue;
+      if (g == VOXEL_FREE || (g >> 8) != s.minprefix[g & 0xFFu]) {
+        w[1] |= bit;
+        continue;
       }
+      w[0] |= bit;
+      const uint32_t slot = s.value_rank[g & 0xFFu];  // ranks are below 256
+#pragma unroll
+      for (int k = 0; k < 8; ++k) w[2 + k] |= (slot >> k) & 1u ? bit : 0u;
     }
-    if (reset) atomicAdd(&s.disjoint, reset);
-  }
-}
-
-__global__ void k_enqueue_pass2(const JobDesc* jobs, const JobState* st, const uint32_t* list,
-                                const uint32_t* count, const uint32_t* brick_job,
-                                uint32_t* epoch, uint32_t* queue0, uint32_t* qcount,
-                                uint32_t* fdir) {
-  const uint32_t n = *count;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const uint32_t b = list[i];
-    const uint32_t j = brick_job[b];
-    if (!jobs[j].active || !st[j].has_prefix || !st[j].disjoint) continue;
-    fdir[(size_t)b * FLOOD_FDIR] = 1u << 13;  // keys were reset: every row
-    if (atomicMax(&epoch[b], 1u) < 1u) queue0[atomicAdd(qcount, 1u)] = b;
+    const uint32_t row = J.wrow0 + x * J.wsx + bz * J.wsy + y;
+    uint32_t* d = J.wstate + (size_t)row * J.wsw;
+#pragma unroll
+    for (uint32_t k = 0; k < 16; ++k)
+      if (k < J.wsw) d[k] = w[k];
+    // wave 0's claims at the word's ends, for the rows below and above (their
+    // `in` still holds keys of the first flood's levels: cleared before)
+    for (int k = 0; k < 2; ++k) {
+      if (k == 0 ? !(w[0] & 1u) : !(w[0] >> 31)) continue;
+      uint32_t slot = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) slot |= (k ? w[2 + q] >> 31 : w[2 + q] & 1u) << q;
+      const uint32_t j = k ? row + J.wsy : row - J.wsy;
+      for (int dx = -1; dx <= 1; ++dx)
+        for (int dy = -1; dy <= 1; ++dy) {
+          if (J.distance == 1 && (dx || dy)) continue;
+          uint2* to = J.win + 2 * (size_t)(j + (uint32_t)dx * J.wsx + dy);
+          atomicMin(k ? &to->x : &to->y, in_key(0, slot));
+        }
+    }
+    if (w[1]) atomicOr(&J.wcand[row >> 5], 1u << (row & 31u));
   }
 }
 
@@ -1314,124 +1057,207 @@ __global__ void k_enqueue_pass2(const JobDesc* jobs, const JobState* st, const u
 
 namespace vfk {
 
-namespace {
-PFN_cuTensorMapEncodeTiled_v12000 g_encode_tiled = nullptr;
-std::once_flag g_encode_once;
-}  // namespace
-
-bool encode_keys_map(void* map128, const uint32_t* keys, uint32_t X, uint32_t Y, uint32_t Zk,
-                     std::string* err) {
-  std::call_once(g_encode_once, [] {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault,
-                                         &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      g_encode_tiled = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(fn);
-    cudaGetLastError();
-  });
-  if (!g_encode_tiled) {
-    if (err) *err = "cuTensorMapEncodeTiled is not available from the CUDA driver";
-    return false;
-  }
-  // dims innermost first: z (Zk, a multiple of 4: 16-byte row strides), y, x
-  const cuuint64_t dims[3] = {Zk, Y, X};
-  const cuuint64_t strides[2] = {(cuuint64_t)Zk * 4u, (cuuint64_t)Zk * 4u * Y};
-  const cuuint32_t box[3] = {(cuuint32_t)KP, (cuuint32_t)KNY, (cuuint32_t)KNX};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUresult r = g_encode_tiled(
-      static_cast<CUtensorMap*>(map128), CU_TENSOR_MAP_DATA_TYPE_UINT32, 3,
-      const_cast<uint32_t*>(keys), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-      CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    if (err) *err = "cuTensorMapEncodeTiled failed (CUresult " + std::to_string((int)r) + ")";
-    return false;
-  }
-  return true;
-}
-
 static inline int brick_grid(uint32_t max_count) {
   uint32_t g = max_count ? max_count : 1;
   return (int)(g > (1u << 20) ? (1u << 20) : g);
 }
 
-void flood_init_keys(cudaStream_t st, const JobDesc* dj, const uint32_t* list,
-                     const uint32_t* count, uint32_t max_count, const uint32_t* brick_job,
-                     const uint8_t*) {
-  if (max_count) k_init_keys<<<brick_grid(max_count), 256, 0, st>>>(dj, list, count, brick_job);
+uint32_t wave_state_words(uint32_t nseeds) {
+  // 6 planes (64 slots) fill 32 bytes with A and B, one 256-bit load per row; 10
+  // planes fill 48; 12 hold every slot (4095 seeds) in 64
+  return (uint32_t)(nseeds <= 64 ? state_words(6) : (nseeds <= 1024 ? state_words(10) : state_words(12)));
+}
+uint64_t wave_rows(uint32_t nx, uint32_t ny, uint32_t nw) {
+  const uint64_t sy = ny + 1ull, sx = (nw + 1ull) * sy;
+  return (nx + 2ull) * sx + sy + 3;
+}
+void wave_layout(WaveJob& W, uint32_t base, uint32_t nx, uint32_t ny, uint32_t nw) {
+  W.base = base;
+  W.sy = ny + 1;
+  W.sx = (nw + 1) * W.sy;
+  W.row0 = base + W.sx + W.sy + 1;
+  W.nrows = (uint32_t)wave_rows(nx, ny, nw);
 }
 
 void flood_seed_bricks(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs, uint8_t* live,
                        uint32_t* list, uint32_t* count) {
-  if (njobs > 0) k_seed_bricks<<<(njobs + 127) / 128, 128, 0, st>>>(dj, ds, njobs, live, list, count);
+  if (njobs > 0) k_seed_bricks<<<njobs, 128, 0, st>>>(dj, ds, live, list, count);
 }
 
-void flood_seed(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs,
-                const FloodScratch& fs, const uint8_t*) {
-  cudaMemsetAsync(fs.epoch, 0, sizeof(uint32_t) * fs.total_bricks, st);
-  cudaMemsetAsync(fs.qcount, 0, sizeof(uint32_t) * 3, st);
-  cudaMemsetAsync(fs.qhead, 0, sizeof(uint32_t) * 3, st);
-  cudaMemsetAsync(fs.barrier, 0, sizeof(uint32_t) * 2, st);
-  cudaMemsetAsync(fs.fdir, 0, sizeof(uint32_t) * FLOOD_FDIR * fs.total_bricks, st);
-  if (njobs > 0)
-    k_seed_keys<<<(njobs + 127) / 128, 128, 0, st>>>(dj, ds, njobs, fs.epoch, fs.queue[0], fs.qcount,
-                                                      fs.fdir);
+void flood_init(cudaStream_t st, const JobDesc* dj, const FloodScratch& fs, const uint8_t* live) {
+  if (fs.units) k_wave_init<<<fs.units, 256, 0, st>>>(dj, fs.arr, fs.jobs, fs.njobs, live);
 }
 
-static int relax_blocks(int num_sms) {
+// launch shape of k_wave: threads per CTA and dynamic shared memory
+namespace {
+constexpr size_t WAVE_SMEM = sizeof(WaveShared) + 2 * 4 * (SMALL_ROWS / 32 + 8);
+
+template <int NB, int THREADS>
+int wave_per_sm() {
   static int per_sm[64] = {};  // per device: the attribute is set on each device
   const int dv = cur_dev();
   if (per_sm[dv] < 1) {
     int n = 0;
-    cudaFuncSetAttribute(k_relax, cudaFuncAttributeMaxDynamicSharedMemorySize, TILE_SMEM);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_relax, 256, TILE_SMEM) != cudaSuccess)
-      n = 1;
+    const auto k = k_wave<NB, THREADS>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WAVE_SMEM);
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, THREADS, WAVE_SMEM) != cudaSuccess) n = 1;
     per_sm[dv] = n < 1 ? 1 : n;
   }
-  return per_sm[dv] * num_sms;
+  return per_sm[dv];
+}
+template <int THREADS>
+int wave_per_sm(uint32_t sw) {
+  return sw <= 8 ? wave_per_sm<6, THREADS>() : (sw <= 12 ? wave_per_sm<10, THREADS>() : wave_per_sm<12, THREADS>());
+}
+template <int THREADS>
+const void* wave_kernel(uint32_t sw) {
+  return sw <= 8 ? (const void*)k_wave<6, THREADS>
+                 : (sw <= 12 ? (const void*)k_wave<10, THREADS> : (const void*)k_wave<12, THREADS>);
+}
+}  // namespace
+
+WaveShape flood_shape(uint32_t sw, uint32_t njobs, int num_sms, int ctas_per_sm) {
+  WaveShape s;
+  s.sms = num_sms;
+  // one flood: the rows of a wave fit one CTA per SM, whose 16 warps hide each
+  // other's latency; a batch: two CTAs, one of each gang
+  s.threads = njobs < 2 ? 512 : 256;
+  int per = s.threads == 512 ? wave_per_sm<512>(sw) : wave_per_sm<256>(sw);
+  if (ctas_per_sm > 0) per = std::min(per, ctas_per_sm);
+  s.blocks = per * num_sms;
+  return s;
 }
 
-void flood_prepare(int num_sms) { (void)relax_blocks(num_sms); }
+uint32_t flood_gang(uint64_t rows, uint32_t blocks, uint32_t min_size) {
+  // rows per CTA: 525 k rows (240 x 240 x 256) take 0.56 ms with 4096, 0.59
+  // with 2048 and 0.62 with 8192
+  constexpr uint64_t GANG_ROWS = 4096;
+  if (rows <= SMALL_ROWS) return std::min(min_size, blocks);
+  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>((rows + GANG_ROWS - 1) / GANG_ROWS, 2), blocks);
+}
 
-cudaError_t flood_relax(cudaStream_t st, const JobDesc* dj, JobState* ds,
-                        const uint32_t* brick_job, const uint8_t* live,
-                        const FloodScratch& fs, int num_sms, int* blocks_used) {
-  FloodArgs a;
-  a.jobs = dj;
+uint32_t flood_gangs(const uint64_t* rows, uint32_t n, uint32_t* gang_of) {
+  bool small = true;
+  for (uint32_t i = 0; i < n; ++i) small &= rows[i] <= SMALL_ROWS;
+  if (small) {
+    for (uint32_t i = 0; i < n; ++i) gang_of[i] = i;
+    return n;
+  }
+  if (n < 2) {
+    gang_of[0] = 0;
+    return 1;
+  }
+  // two sets of equal size, the largest job first, each to the smaller set
+  // (more sets where a set would have too many jobs)
+  const uint32_t k = std::max(2u, (n + WAVE_GANG_JOBS / 2 - 1) / (WAVE_GANG_JOBS / 2));
+  std::vector<uint32_t> order(n);
+  for (uint32_t i = 0; i < n; ++i) order[i] = i;
+  std::sort(order.begin(), order.end(),
+            [&](uint32_t a, uint32_t b) { return rows[a] != rows[b] ? rows[a] > rows[b] : a < b; });
+  std::vector<uint64_t> load(k, 0);
+  std::vector<uint32_t> count(k, 0);
+  for (uint32_t i : order) {
+    uint32_t best = k;
+    for (uint32_t g = 0; g < k; ++g)
+      if (count[g] < WAVE_GANG_JOBS && (best == k || load[g] < load[best])) best = g;
+    gang_of[i] = best;
+    load[best] += rows[i];
+    ++count[best];
+  }
+  return k;
+}
+
+// One-CTA gangs are dealt to all CTAs, the largest first, each to the least
+// loaded one; larger gangs alternate between as many sets of CTAs as fit an SM.
+uint32_t flood_schedule(const WaveGang* gangs, uint32_t n, const WaveShape& shape, uint32_t min_size, WaveCta* cta,
+                        WaveEntry* entries) {
+  const uint32_t C = (uint32_t)shape.blocks;
+  std::vector<std::vector<WaveEntry>> lists(C);
+  const uint32_t sets = n > 1 ? std::max(1u, std::min(n, C / (uint32_t)std::max(shape.sms, 1))) : 1u;
+  const uint32_t width = std::max(1u, std::min(C / sets, (uint32_t)std::max(shape.sms, 1)));
+  std::vector<uint32_t> small;
+  for (uint32_t g = 0; g < n; ++g) {
+    const uint32_t size = flood_gang((uint64_t)gangs[g].units * 256, width, min_size);
+    if (size < 2) {
+      small.push_back(g);
+      continue;
+    }
+    const uint32_t at = (g % sets) * width;
+    for (uint32_t r = 0; r < size; ++r) lists[at + r].push_back({g, r, size, 0});
+  }
+  std::sort(small.begin(), small.end(), [&](uint32_t a, uint32_t b) {
+    return gangs[a].units != gangs[b].units ? gangs[a].units > gangs[b].units : a < b;
+  });
+  std::vector<uint64_t> load(C, 0);
+  for (uint32_t c = 0; c < C; ++c)
+    for (const WaveEntry& e : lists[c]) load[c] += gangs[e.gang].units / e.size + 1;
+  auto later = [&](uint32_t a, uint32_t b) { return load[a] != load[b] ? load[a] > load[b] : a > b; };
+  std::vector<uint32_t> heap(C);
+  for (uint32_t c = 0; c < C; ++c) heap[c] = c;
+  std::make_heap(heap.begin(), heap.end(), later);
+  for (uint32_t g : small) {
+    std::pop_heap(heap.begin(), heap.end(), later);
+    const uint32_t c = heap.back();
+    lists[c].push_back({g, 0, 1, 0});
+    load[c] += gangs[g].units;
+    std::push_heap(heap.begin(), heap.end(), later);
+  }
+  uint32_t at = 0;
+  for (uint32_t c = 0; c < C; ++c) {
+    cta[c] = {at, (uint32_t)lists[c].size()};
+    for (const WaveEntry& e : lists[c]) entries[at++] = e;
+  }
+  return at;
+}
+
+cudaError_t flood_seed(cudaStream_t st, const JobDesc* dj, const JobState* ds, const FloodScratch& fs) {
+  cudaError_t e = cudaMemsetAsync(fs.zero, 0, fs.zero_bytes, st);
+  if (e == cudaSuccess && fs.njobs) k_wave_seed<<<fs.njobs, 256, 0, st>>>(dj, ds, fs.arr, fs.jobs);
+  return e;
+}
+
+cudaError_t flood_waves(cudaStream_t st, JobState* ds, const FloodScratch& fs) {
+  WaveArgs a;
+  a.arr = fs.arr;
+  a.jobs = fs.jobs;
+  a.gangs = fs.gangs;
+  a.last = fs.last;
+  a.cta = fs.cta;
+  a.entries = fs.entries;
   a.st = ds;
-  a.brick_job = brick_job;
-  a.live = live;
-  a.queue[0] = fs.queue[0];
-  a.queue[1] = fs.queue[1];
-  a.queue[2] = fs.queue[2];
-  a.qcount = fs.qcount;
-  a.qhead = fs.qhead;
-  a.epoch = fs.epoch;
-  a.bar = fs.barrier;
+  a.bar = fs.bar;
   a.err = fs.err;
   a.stats = fs.stats;
-  a.max_passes = fs.max_passes;
-  a.max_sweeps = (fs.max_sweeps > 0 && fs.max_sweeps <= MAXIT) ? fs.max_sweeps : MAXIT;
-  a.pass_sizes = fs.pass_sizes;
-  a.fdir = fs.fdir;
-  a.nbricks = fs.total_bricks;
-  a.njobs = fs.njobs;
-  a.wait_spins = fs.wait_spins ? fs.wait_spins : (1u << 26);
-  a.tmaps = static_cast<const unsigned char*>(fs.tmaps);
-  if (!a.tmaps) return cudaErrorInvalidValue;
-  int blocks = relax_blocks(num_sms);
-  if (fs.ctas_per_sm > 0 && fs.ctas_per_sm * num_sms < blocks) blocks = fs.ctas_per_sm * num_sms;
-  if (blocks_used) *blocks_used = blocks;
+  a.wave_sizes = fs.wave_sizes;
+  a.wait_spins = fs.wait_spins ? fs.wait_spins : (1u << 23);
+  a.smem_words = (uint32_t)((WAVE_SMEM - sizeof(WaveShared)) / 4);
   void* args[] = {&a};
-  return cudaLaunchCooperativeKernel((const void*)k_relax, dim3(blocks), dim3(256), args,
-                                     TILE_SMEM, st);
+  return cudaLaunchCooperativeKernel(fs.shape.threads == 512 ? wave_kernel<512>(fs.sw) : wave_kernel<256>(fs.sw),
+                                     dim3(fs.shape.blocks), dim3(fs.shape.threads), args, WAVE_SMEM, st);
 }
 
-void flood_finalize(cudaStream_t st, const JobDesc* dj, const JobState* ds, const uint32_t* list,
-                    const uint32_t* count, uint32_t max_count, const uint32_t* brick_job,
-                    int pass2) {
-  if (max_count) k_finalize<<<brick_grid(max_count), 256, 0, st>>>(dj, ds, list, count, brick_job, pass2);
+static int flat_grid(const WaveJob& W) {
+  return (int)std::max<uint32_t>(1, std::min<uint32_t>((W.nrows + 7) / 8, 2432));
+}
+void flat_init(cudaStream_t st, const uint16_t* grid, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A,
+               uint32_t sw) {
+  k_flat_init<<<flat_grid(W), 256, 0, st>>>(grid, arr, W, A, sw);
+}
+void flat_seed(cudaStream_t st, const WaveJob& W, const FlatAxes& A, const FloodScratch& fs, const uint32_t* seeds,
+               uint32_t ns, JobState* ds) {
+  const uint32_t size = flood_gang(W.nrows, (uint32_t)std::min(fs.shape.blocks, fs.shape.sms), 1);
+  k_flat_seed<<<1, 256, 0, st>>>(fs.arr, W, A, fs.sw, seeds, ns, size, (uint32_t)fs.shape.blocks, ds,
+                                 const_cast<WaveJob*>(fs.jobs), const_cast<WaveGang*>(fs.gangs),
+                                 const_cast<WaveCta*>(fs.cta), const_cast<WaveEntry*>(fs.entries));
+}
+void flat_labels(cudaStream_t st, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A, uint32_t sw,
+                 const uint32_t* seeds, uint16_t* labels) {
+  k_flat_labels<<<flat_grid(W), 256, 0, st>>>(arr, W, A, sw, seeds, labels);
+}
+
+void flood_labels(cudaStream_t st, const JobDesc* dj, const JobState* ds, const uint32_t* list,
+                  const uint32_t* count, uint32_t max_count, const uint32_t* brick_job, int pass2) {
+  if (max_count) k_wave_labels<<<brick_grid(max_count), 256, 0, st>>>(dj, ds, list, count, brick_job, pass2);
 }
 
 void flood_competition(cudaStream_t st, const JobDesc* dj, JobState* ds, const uint32_t* list,
@@ -1439,20 +1265,17 @@ void flood_competition(cudaStream_t st, const JobDesc* dj, JobState* ds, const u
   if (max_count) k_competition<<<brick_grid(max_count), 256, 0, st>>>(dj, ds, list, count, brick_job);
 }
 
-void flood_disjoint(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs,
-                    const uint32_t* list, const uint32_t* count, uint32_t max_count,
-                    const uint32_t* brick_job, const FloodScratch& fs, const uint8_t*) {
-  if (!max_count) return;
+cudaError_t flood_disjoint(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs,
+                           const uint32_t* list, const uint32_t* count, uint32_t max_count,
+                           const uint32_t* brick_job, const FloodScratch& fs) {
+  cudaError_t e = cudaMemsetAsync(fs.zero, 0, fs.zero_bytes, st);
+  if (e != cudaSuccess || !max_count) return e;
+  e = cudaMemsetAsync(fs.arr.in, 0xFF, fs.in_bytes, st);
+  if (e != cudaSuccess) return e;
   k_minprefix<<<brick_grid(max_count), 256, 0, st>>>(dj, ds, list, count, brick_job);
   k_ranks<<<(njobs + 127) / 128, 128, 0, st>>>(dj, ds, njobs);
   k_disjoint_reset<<<brick_grid(max_count), 256, 0, st>>>(dj, ds, list, count, brick_job);
-  cudaMemsetAsync(fs.epoch, 0, sizeof(uint32_t) * fs.total_bricks, st);
-  cudaMemsetAsync(fs.qcount, 0, sizeof(uint32_t) * 3, st);
-  cudaMemsetAsync(fs.qhead, 0, sizeof(uint32_t) * 3, st);
-  cudaMemsetAsync(fs.barrier, 0, sizeof(uint32_t) * 2, st);
-  cudaMemsetAsync(fs.fdir, 0, sizeof(uint32_t) * FLOOD_FDIR * fs.total_bricks, st);
-  k_enqueue_pass2<<<brick_grid((max_count + 255) / 256), 256, 0, st>>>(
-      dj, ds, list, count, brick_job, fs.epoch, fs.queue[0], fs.qcount, fs.fdir);
+  return cudaSuccess;
 }
 
 }  // namespace vfk

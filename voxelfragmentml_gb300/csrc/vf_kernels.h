@@ -182,13 +182,6 @@ void remove_isolated(cudaStream_t st, const JobDesc* dj, const uint32_t* list,
 void count_values(cudaStream_t st, const JobDesc* dj, JobState* ds, const uint32_t* list,
                   const uint32_t* count, uint32_t max_count, const uint32_t* brick_job);
 
-// ---- flood (vf_flood.cu) ----
-// Words per brick of the flood's change record: [0] neighbour directions
-// (bit dx*9 + dy*3 + dz: the brick at offset (dx-1, dy-1, dz-1) changed keys
-// this brick reads; bit 13: every row), [1..8] rows whose key at z0-1 changed,
-// [9..16] rows whose key at z0+32 changed (bit t & 31 of word t >> 5, row
-// t = x * 16 + y within the brick).
-constexpr uint32_t FLOOD_FDIR = 17;
 // the current device, as an index into per-device caches of launch
 // attributes (a kernel's shared-memory limit is set once per device)
 inline int cur_dev() {
@@ -197,53 +190,107 @@ inline int cur_dev() {
   return d & 63;
 }
 
-// TMA descriptor (CUtensorMap, 128 bytes, 64-byte aligned) of one job's
-// flood keys uint32 [X][Y][Zk], encoded on the host for k_relax's tile
-// loads: boxes of 36 x 18 x 18 keys (z, y, x), zeros outside the grid.
-constexpr size_t KEYS_MAP_BYTES = 128;
-// false (message in *err) when the driver cannot encode the map
-bool encode_keys_map(void* map128, const uint32_t* keys, uint32_t X, uint32_t Y, uint32_t Zk,
-                     std::string* err);
-
-struct FloodScratch {
-  uint32_t* queue[3];    // brick ids, capacity total_bricks each (rotating)
-  uint32_t* qcount;      // [3]
-  uint32_t* qhead;       // [3]
-  uint32_t* epoch;       // [total_bricks]
-  uint32_t* fdir;        // [total_bricks][FLOOD_FDIR] change record, zero between floods
-  uint32_t* barrier;     // [2] count, generation
-  uint32_t* err;         // [1] global error word
-  uint32_t* stats;       // [4] brick visits, passes, overflow, timeout
-  uint32_t max_passes;
-  uint32_t total_bricks;
-  uint32_t njobs = 1;    // job descriptors in the table
-  int max_sweeps = 0;    // tuning: sweeps per brick visit (0: default cap)
-  int ctas_per_sm = 0;   // tuning: resident CTAs per SM (0: as many as fit)
-  uint32_t wait_spins = 0;  // spins of the pass barrier before it gives up (0: 2^26, ~4 s)
-  const void* tmaps = nullptr;  // [njobs] keys tensor maps (KEYS_MAP_BYTES each, device)
-  uint32_t* pass_sizes = nullptr;  // statistics: bricks queued per pass (256)
+// ---- flood (vf_flood.cu) ----
+// The floods of a batch share arrays of rows, 32 voxels along a word axis
+// each.
+struct WaveArrays {
+  uint32_t* state;  // [rows] state words (wave_state_words)
+  uint2* in;        // [rows][2] what reaches the word ends from below (.x) / above (.y), by wave parity
+  uint32_t* cand;   // [2][nwords] a candidate bit per row, by wave parity
+  uint32_t nwords;  // rows / 32
 };
-void flood_init_keys(cudaStream_t st, const JobDesc* dj, const uint32_t* list,
-                     const uint32_t* count, uint32_t max_count, const uint32_t* brick_job,
-                     const uint8_t* live);
+// One flood: rows base .. base + nrows of the arrays (base a multiple of 256, up
+// to the next job's base).  Row (outer x, word, y) is row0 + x * sx + word * sy
+// + y, with at least one row of zeros on each side of every axis, so the
+// neighbours of a row are rows +- sx, +- sy, +- 1.  A job's axes are (x, y, z) with
+// words along z, or any permutation.
+struct WaveJob {
+  uint32_t base, nrows, row0, sx, sy;
+  uint32_t conn6;  // 6-neighbourhood (Manhattan), else 26
+  uint32_t job;    // its JobState
+};
+uint64_t wave_rows(uint32_t nx, uint32_t ny, uint32_t nw);
+void wave_layout(WaveJob& W, uint32_t base, uint32_t nx, uint32_t ny, uint32_t nw);
+// Jobs flooded in step: wave jobs first .. first + count, whose rows are units
+// unit_lo .. unit_lo + units of 256 rows
+struct WaveGang {
+  uint32_t first, count, unit_lo, units;
+};
+constexpr uint32_t WAVE_GANG_JOBS = 256;  // most jobs of a gang
+struct WaveEntry {
+  uint32_t gang, rank, size, pad;  // this CTA's rank in the gang, CTAs of the gang
+};
+struct WaveCta {
+  uint32_t first, count;  // entries of one CTA, run in order
+};
+// u32 words of a row state for floods of up to nseeds seeds (8, 12 or 16)
+uint32_t wave_state_words(uint32_t nseeds);
+constexpr uint32_t WAVE_BAR_WORDS = 32;  // barrier words per gang
+
+struct WaveShape {
+  int blocks = 0, threads = 256, sms = 0;
+};
+struct FloodScratch {
+  WaveArrays arr = {};
+  uint32_t units = 0;                  // 256-row units of all jobs
+  const WaveJob* jobs = nullptr;       // device, njobs
+  uint32_t njobs = 0;
+  const WaveGang* gangs = nullptr;     // device
+  const WaveCta* cta = nullptr;        // device, shape.blocks
+  const WaveEntry* entries = nullptr;  // device
+  WaveShape shape;                     // of the launch (flood_shape)
+  uint32_t sw = 8;                     // state words of every job of the batch
+  uint32_t* bar = nullptr;             // [gangs][WAVE_BAR_WORDS]
+  uint32_t* last = nullptr;            // [njobs]
+  void* zero = nullptr;                // candidate words, bar, last: cleared before a flood
+  size_t zero_bytes = 0;
+  size_t in_bytes = 0;                 // of arr.in
+  uint32_t* err = nullptr;             // [1] global error word
+  uint32_t* stats = nullptr;           // [VF_FLOOD_NCOUNTERS]
+  uint32_t* wave_sizes = nullptr;      // statistics: rows visited per wave (256)
+  uint32_t wait_spins = 0;             // polls of a gang barrier before it gives up (0: 2^23, ~4 s)
+};
+// launch shape of the waves of njobs floods (ctas_per_sm > 0: at most that many
+// CTAs per SM); also sets the kernel's attributes (once per device, outside a
+// stream capture)
+WaveShape flood_shape(uint32_t sw, uint32_t njobs, int num_sms, int ctas_per_sm);
+// the gangs of n floods of rows[i] rows: their number, the gang of each
+uint32_t flood_gangs(const uint64_t* rows, uint32_t n, uint32_t* gang_of);
+// CTAs of a gang
+uint32_t flood_gang(uint64_t rows, uint32_t blocks, uint32_t min_size);
+// the CTAs of n gangs: cta[shape.blocks], entries (at most n * shape.sms + n);
+// returns the entries
+uint32_t flood_schedule(const WaveGang* gangs, uint32_t n, const WaveShape& shape, uint32_t min_size, WaveCta* cta,
+                    WaveEntry* entries);
 void flood_seed_bricks(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs, uint8_t* live,
                        uint32_t* list, uint32_t* count);
-void flood_seed(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs,
-                const FloodScratch& fs, const uint8_t* live);
-// sets k_relax's shared-memory attribute and occupancy (once per process)
-void flood_prepare(int num_sms);
-cudaError_t flood_relax(cudaStream_t st, const JobDesc* dj, JobState* ds,
-                        const uint32_t* brick_job, const uint8_t* live,
-                        const FloodScratch& fs, int num_sms, int* blocks_used);
-void flood_finalize(cudaStream_t st, const JobDesc* dj, const JobState* ds,
-                    const uint32_t* list, const uint32_t* count, uint32_t max_count,
-                    const uint32_t* brick_job, int pass2);
+// row states from the labels
+void flood_init(cudaStream_t st, const JobDesc* dj, const FloodScratch& fs, const uint8_t* live);
+cudaError_t flood_seed(cudaStream_t st, const JobDesc* dj, const JobState* ds, const FloodScratch& fs);
+cudaError_t flood_waves(cudaStream_t st, JobState* ds, const FloodScratch& fs);
+void flood_labels(cudaStream_t st, const JobDesc* dj, const JobState* ds, const uint32_t* list,
+                  const uint32_t* count, uint32_t max_count, const uint32_t* brick_job, int pass2);
 // sub-seed prefix competition and the disjoint cleanup
 void flood_competition(cudaStream_t st, const JobDesc* dj, JobState* ds, const uint32_t* list,
                        const uint32_t* count, uint32_t max_count, const uint32_t* brick_job);
-void flood_disjoint(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs,
-                    const uint32_t* list, const uint32_t* count, uint32_t max_count,
-                    const uint32_t* brick_job, const FloodScratch& fs, const uint8_t* live);
+cudaError_t flood_disjoint(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs,
+                           const uint32_t* list, const uint32_t* count, uint32_t max_count,
+                           const uint32_t* brick_job, const FloodScratch& fs);
+
+// ---- a flood on an unpadded device grid (vf_flood_noalloc) ----
+struct FlatAxes {
+  size_t s[3];       // element strides of the state's axes (outer, rows, words)
+  uint32_t nx, ny, nz;  // voxels along them
+  uint32_t dims[3];  // X, Y, Z
+  uint32_t order;    // nibble a: the grid axis of state axis a
+};
+void flat_init(cudaStream_t st, const uint16_t* grid, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A,
+               uint32_t sw);
+// checks and places the seeds; writes the wave job and its gang's tables
+void flat_seed(cudaStream_t st, const WaveJob& W, const FlatAxes& A, const FloodScratch& fs, const uint32_t* seeds,
+               uint32_t ns, JobState* ds);
+void flat_labels(cudaStream_t st, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A, uint32_t sw,
+                 const uint32_t* seeds, uint16_t* labels);
 
 // ---- plain (reference-shaped) per-voxel kernels for one job ----
 void plain_init_keys(cudaStream_t st, const JobDesc* dj, const JobDesc& hj);

@@ -118,7 +118,7 @@ vf_status Batch::execute_resident(bool download) {
   if (!graphs_ok || host_steps) return enqueue_batched(false, download);
   const int gi = download ? 1 : 0;
   if (!gexec[gi]) {
-    vfk::flood_prepare(ctx->num_sms);  // function attributes outside the capture
+    vfk::flood_shape(wsw, (uint32_t)wave_jobs.size(), ctx->num_sms, 0);  // function attributes outside the capture
     if (cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
       cudaGetLastError();
       graphs_ok = false;
@@ -152,9 +152,9 @@ void Batch::release() {
   if (!ctx) return;
   for (DevBuf* b : {&grid0, &grid1, &keys, &par, &tets, &range, &ys, &seeds, &counts, &lat,
                     &verts, &faces, &emask, &etab, &tables, &state, &brick_job, &live, &list, &lcount,
-                    &q[0], &q[1], &q[2], &scal, &epoch, &fdir, &front[0], &front[1], &pcnt, &pbase,
+                    &scal, &wst, &win, &wzero, &wsched, &front[0], &front[1], &pcnt, &pbase,
                     &psums, &srec, &stage_out, &rle_cnt, &rle_base, &rle_sums, &rle_tot, &rle_starts,
-                    &rle_rec, &tmaps})
+                    &rle_rec})
     ctx->free_buf(*b);
   if (h_tables) cudaFreeHost(h_tables);
   if (h_state) cudaFreeHost(h_state);
@@ -278,17 +278,23 @@ static uint32_t edge_slots(uint32_t nfaces) {
   return (uint32_t)std::min<uint64_t>(c, 1ull << 31);
 }
 
+// most seeds a flood of these parameters can have (Batch::plan's given seeds aside)
+static uint32_t wave_seeds(const vf_params& q) {
+  const int32_t n = q.num_seeds + (q.num_impacts > 0 ? q.bias_seeds : 0);
+  return (uint32_t)std::max(q.num_extra_seeds > 0 ? 2 * n + q.num_extra_seeds : n, 1);
+}
+
 size_t job_footprint(const vf_job& j) {
   uint32_t d[3] = {j.dims[0], j.dims[1], j.dims[2]};
   if (!d[0] && !d[1] && !d[2]) d[0] = d[1] = d[2] = j.max_dim;
   const size_t X = d[0], Y = d[1], Z = d[2];
-  const size_t Zp = vf_roundup((uint32_t)Z, 8), Zk = vf_roundup((uint32_t)Z, 4), Zw = (Z + 31) / 32;
+  const size_t Zp = vf_roundup((uint32_t)Z, 8), Zw = (Z + 31) / 32;
   size_t b = X * Y * Zp * 2 * 2 + X * Y * Zw * 4 * 2 + (size_t)j.nfaces * (48 + 4 + 12) +
              (size_t)edge_slots(j.nfaces) * 8 + (size_t)j.nverts * 12 + 65536;
-  if (j.params.algorithm == VF_FLOOD) b += X * Y * Zk * 4;
-  // per brick: owner, live flag, list, 3 queues, epoch, change record
-  b += ((X + VF_BX - 1) / VF_BX) * ((Y + VF_BY - 1) / VF_BY) * ((Z + VF_BZ - 1) / VF_BZ) *
-       (4 + 1 + 4 + 12 + 4 + 4 * vfk::FLOOD_FDIR);
+  if (j.params.algorithm == VF_FLOOD)  // row states, what reaches their ends, two sets of candidate words
+    b += vfk::wave_rows((uint32_t)X, (uint32_t)Y, (uint32_t)Zw) * (4 * vfk::wave_state_words(wave_seeds(j.params)) + 17);
+  // per brick: owner, live flag, list
+  b += ((X + VF_BX - 1) / VF_BX) * ((Y + VF_BY - 1) / VF_BY) * ((Z + VF_BZ - 1) / VF_BZ) * (4 + 1 + 4);
   return b;
 }
 
@@ -298,6 +304,11 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
   jobs.assign(js, js + n);
   plans.assign(n, JobPlan());
   sz = Sizes();
+  wsw = 8;
+  for (uint32_t i = 0; i < n; ++i)
+    if (js[i]->params.algorithm == VF_FLOOD)
+      wsw = std::max(wsw, vfk::wave_state_words(i < given.size() && given[i].second ? given[i].second
+                                                                                    : wave_seeds(js[i]->params)));
   for (uint32_t i = 0; i < n; ++i) {
     const vf_job& j = *js[i];
     JobPlan& p = plans[i];
@@ -343,10 +354,14 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
       p.lat_ny = (p.Y - 1) / j.params.noise_period + 2;
       p.lat_nz = (p.Z - 1) / j.params.noise_period + 2;
     }
-    p.prefix_possible = j.params.algorithm == VF_FLOOD && (j.params.num_extra_seeds > 0 || ngiven > 0);
+    // given seeds are in host memory: sub-seed prefixes are seen in their labels
+    bool given_prefix = false;
+    for (uint32_t k = 0; k < ngiven; ++k) given_prefix |= given[i].first[4 * (size_t)k + 3] > 0xFFu;
+    p.prefix_possible = j.params.algorithm == VF_FLOOD && (ngiven ? given_prefix : j.params.num_extra_seeds > 0);
     const size_t vox = (size_t)p.X * p.Y;
     p.o_grid = sz.grid; sz.grid += align_up(vox * p.Zp, 128);
-    p.o_keys = sz.keys; if (j.params.algorithm == VF_FLOOD) sz.keys += align_up(vox * p.Zk, 64);
+    p.o_keys = sz.keys;
+    if (j.params.algorithm == VF_FLOOD && plain) sz.keys += align_up(vox * p.Zk, 64);
     p.o_par = sz.par; sz.par += align_up(vox * p.Zw, 64);
     p.o_tets = sz.tets; sz.tets += align_up((size_t)j.nfaces * 3, 16);
     p.o_range = sz.range; sz.range += align_up(j.nfaces, 64);
@@ -368,6 +383,54 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
     sz.faces_total += j.nfaces;
     if (j.params.erode) sz.max_iters = std::max(sz.max_iters, (uint32_t)j.params.erosion_iterations);
   }
+  // The floods of the batch: gangs, and the rows of each job gang by gang
+  wave_jobs.clear();
+  wave_gangs.clear();
+  wave_units = 0;
+  if (!plain) {
+    std::vector<uint32_t> fl, gang;
+    std::vector<uint64_t> rows;
+    for (uint32_t i = 0; i < n; ++i)
+      if (js[i]->params.algorithm == VF_FLOOD) {
+        fl.push_back(i);
+        rows.push_back(vfk::wave_rows(plans[i].X, plans[i].Y, plans[i].nbz));
+      }
+    gang.resize(fl.size());
+    const uint32_t ng = fl.empty() ? 0u : vfk::flood_gangs(rows.data(), (uint32_t)fl.size(), gang.data());
+    std::vector<uint32_t> order(fl.size());
+    for (uint32_t k = 0; k < order.size(); ++k) order[k] = k;
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t a, uint32_t b) { return gang[a] < gang[b]; });
+    uint64_t units = 0;
+    wave_gangs.assign(ng, {0, 0, 0, 0});
+    for (uint32_t k : order) {
+      const uint32_t i = fl[k];
+      const uint64_t u = (rows[k] + 255) / 256;
+      if ((units + u) * 256 > 1ull << 31) return fail(VF_ERR_RANGE, "the batch's floods have 2^31 rows or more");
+      vfk::WaveJob w = {};
+      vfk::wave_layout(w, (uint32_t)(units * 256), plans[i].X, plans[i].Y, plans[i].nbz);
+      w.conn6 = js[i]->params.distance == VF_MANHATTAN ? 1u : 0u;
+      w.job = i;
+      vfk::WaveGang& g = wave_gangs[gang[k]];
+      if (!g.count) {
+        g.first = (uint32_t)wave_jobs.size();
+        g.unit_lo = (uint32_t)units;
+      }
+      ++g.count;
+      g.units += (uint32_t)u;
+      wave_jobs.push_back(w);
+      units += u;
+    }
+    wave_units = (uint32_t)units;
+  }
+  const size_t wrows = (size_t)wave_units * 256;
+  // wave jobs, then the CTA table and the gang entries of the widest launch
+  const size_t max_blocks = 8 * (size_t)std::max(ctx->num_sms, 1);
+  size_t max_entries = max_blocks;
+  for (const vfk::WaveGang& g : wave_gangs)
+    max_entries += vfk::flood_gang((uint64_t)g.units * 256, (uint32_t)std::max(ctx->num_sms, 2), 2);
+  const size_t wave_bytes = (sizeof(vfk::WaveJob) + sizeof(vfk::WaveGang)) * (wave_jobs.size() + 1) +
+                            sizeof(vfk::WaveCta) * max_blocks +
+                            sizeof(vfk::WaveEntry) * max_entries + 128;
   // arenas (grow-only)
   Ctx& c = *ctx;
   vf_status s;
@@ -396,9 +459,10 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
   ALLOC(live, nb);
   ALLOC(list, nb * 4);
   ALLOC(lcount, 256);
-  for (int i = 0; i < 3; ++i) ALLOC(q[i], nb * 4);
-  ALLOC(epoch, nb * 4);
-  ALLOC(fdir, nb * vfk::FLOOD_FDIR * 4);
+  ALLOC(wst, std::max<size_t>(wrows * wsw * 4, 256));
+  ALLOC(win, std::max<size_t>(wrows * 16, 256));
+  ALLOC(wzero, std::max<size_t>(wave_zero_bytes(), 256));
+  ALLOC(wsched, wave_bytes);
   ALLOC(scal, 4096);
   const size_t nf = std::max<uint32_t>(sz.faces_total, 1);
   ALLOC(pcnt, nf * 4);
@@ -406,7 +470,6 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
   ALLOC(psums, ((nf + 1023) / 1024 + 1) * 8);
   ALLOC(srec, nf * 96);
   if (sz.out) ALLOC(stage_out, sz.out * 2);
-  ALLOC(tmaps, vfk::KEYS_MAP_BYTES * std::max<size_t>(n, 1));
 #undef ALLOC
     return VF_OK;
   };
@@ -433,15 +496,15 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
   s = alloc_all();
   c.grow = 0.0;
   if (s) return s;
-  // pinned staging: stage tables, erosion masks, then the keys tensor maps
-  // (128-byte aligned, as CUtensorMap requires 64)
-  tmap_off = align_up(sizeof(JobDesc) * ntables * std::max<size_t>(n, 1) + sz.emask * 4, 128);
-  const size_t tbytes = tmap_off + vfk::KEYS_MAP_BYTES * std::max<size_t>(n, 1) + 256;
+  // pinned staging: stage tables, the erosion masks, the flood's tables
+  const size_t wave_off = align_up(sizeof(JobDesc) * ntables * std::max<size_t>(n, 1) + sz.emask * 4, 128);
+  const size_t tbytes = wave_off + wave_bytes;
   if (tbytes > h_tables_cap) {
     if (h_tables) cudaFreeHost(h_tables);
     h_tables_cap = align_up(tbytes * 2, 1 << 16);
     VF_CK(cudaMallocHost(&h_tables, h_tables_cap));
   }
+  h_wave = static_cast<char*>(h_tables) + wave_off;
   const size_t sbytes = sizeof(JobState) * std::max<size_t>(n, 1);
   if (sbytes > h_state_cap) {
     if (h_state) cudaFreeHost(h_state);
@@ -464,13 +527,11 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
     uint16_t* g0 = static_cast<uint16_t*>(grid0.p) + p.o_grid;
     uint16_t* g1 = static_cast<uint16_t*>(grid1.p) + p.o_grid;
     d.keys = static_cast<uint32_t*>(keys.p) + p.o_keys;
-    {
-      void* map = static_cast<char*>(h_tables) + tmap_off + vfk::KEYS_MAP_BYTES * i;
-      std::memset(map, 0, vfk::KEYS_MAP_BYTES);
-      std::string why;
-      if (j.params.algorithm == VF_FLOOD && !vfk::encode_keys_map(map, d.keys, p.X, p.Y, p.Zk, &why))
-        return fail(VF_ERR_CUDA, "job " + std::to_string(i) + ": " + why);
-    }
+    d.wstate = static_cast<uint32_t*>(wst.p);
+    d.win = static_cast<uint2*>(win.p);
+    d.wcand = static_cast<uint32_t*>(wzero.p);
+    d.wsw = wsw;
+    d.wrow0 = d.wsx = d.wsy = 0;  // from its wave job, below
     d.par = static_cast<uint32_t*>(par.p) + p.o_par;
     d.shell = static_cast<uint32_t*>(par.p) + sz.par + p.o_par;
     d.verts = static_cast<float*>(verts.p) + p.o_verts;
@@ -562,7 +623,18 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
     brick_base += p.nbricks;
     face_base += j.nfaces;
   }
+  for (const vfk::WaveJob& w : wave_jobs)
+    for (uint32_t t = 0; t < nt; ++t) {
+      JobDesc& d = T[(size_t)t * n + w.job];
+      d.wrow0 = w.row0;
+      d.wsx = w.sx;
+      d.wsy = w.sy;
+    }
   return VF_OK;
+}
+
+size_t Batch::wave_zero_bytes() const {
+  return (size_t)wave_units * 64 + (vfk::WAVE_BAR_WORDS * wave_gangs.size() + wave_jobs.size()) * 4;
 }
 
 // --------------------------------------------------------------------------
@@ -606,8 +678,6 @@ static vf_status upload_inputs_impl(Batch& B) {
   if (B.sz.emask)
     VF_CK(cudaMemcpyAsync(B.emask.p, static_cast<char*>(B.h_tables) + tb, B.sz.emask * 4,
                           cudaMemcpyHostToDevice, st));
-  VF_CK(cudaMemcpyAsync(B.tmaps.p, static_cast<char*>(B.h_tables) + B.tmap_off,
-                        vfk::KEYS_MAP_BYTES * n, cudaMemcpyHostToDevice, st));
   return VF_OK;
 }
 
@@ -665,33 +735,52 @@ static void voxelize_stages(Batch& B, const std::function<void(int)>& mark) {
 
 static vfk::FloodScratch flood_scratch(Batch& B) {
   vfk::FloodScratch fs;
-  for (int i = 0; i < 3; ++i) fs.queue[i] = static_cast<uint32_t*>(B.q[i].p);
   uint32_t* sc = static_cast<uint32_t*>(B.scal.p);
-  fs.qcount = sc + 0;    // [3]
-  fs.qhead = sc + 4;     // [3]
-  fs.barrier = sc + 8;   // [2]
+  fs.arr = {static_cast<uint32_t*>(B.wst.p), static_cast<uint2*>(B.win.p), static_cast<uint32_t*>(B.wzero.p),
+            B.wave_units * 8};
+  fs.units = B.wave_units;
+  fs.njobs = (uint32_t)B.wave_jobs.size();
+  fs.sw = B.wsw;
+  // candidate words, barriers, last waves
+  fs.zero = B.wzero.p;
+  fs.zero_bytes = B.wave_zero_bytes();
+  fs.bar = fs.arr.cand + (size_t)B.wave_units * 16;
+  fs.last = fs.bar + vfk::WAVE_BAR_WORDS * B.wave_gangs.size();
+  fs.in_bytes = (size_t)B.wave_units * 256 * 16;
   fs.err = sc + 12;      // [1]
-  fs.stats = sc + 16;    // [VF_FLOOD_NCOUNTERS]: visits, passes, busy warp-sweeps, timeouts, sweeps,
-                         // sweep-cap hits, active row-sweeps, changed voxels, the
-                         // first out-of-range access (code, two values), the SM
-                         // cycles / 256 of five phases of the relaxation CTAs and
-                         // the visits that found nothing new
-  fs.epoch = static_cast<uint32_t*>(B.epoch.p);
-  fs.fdir = static_cast<uint32_t*>(B.fdir.p);
-  fs.max_passes = 1u << 20;
-  fs.total_bricks = B.sz.bricks;
-  fs.njobs = (uint32_t)B.jobs.size();
-  fs.max_sweeps = B.ctx->tune.flood_sweeps;
-  fs.ctas_per_sm = B.ctx->tune.flood_ctas;
+  fs.stats = sc + 16;    // [VF_FLOOD_NCOUNTERS]
+  fs.wave_sizes = sc + 128;  // [256]
   fs.wait_spins = B.ctx->tune.flood_wait_spins;
-  fs.tmaps = B.tmaps.p;
-  fs.pass_sizes = sc + 128;  // [256]
   return fs;
 }
 
-// the flood relaxation, after the last one issued on the context (any stream)
-cudaError_t Batch::relax_serialized(cudaStream_t st, const JobDesc* tf, JobState* ds,
-                                    const uint32_t* bj, const uint8_t* lv, const vfk::FloodScratch& fs) {
+// the wave jobs, their gangs and the gangs' CTAs of those that fit the GPU: one
+// table, uploaded before the flood.  A context with a wait limit of
+// its own gets gangs of at least two CTAs, so that the limited wait exists.
+vf_status Batch::wave_tables(vfk::FloodScratch& fs) {
+  const size_t n = wave_jobs.size(), ng = wave_gangs.size();
+  fs.shape = vfk::flood_shape(wsw, (uint32_t)n, ctx->num_sms, ctx->tune.flood_ctas);
+  fs.shape.blocks = std::min(fs.shape.blocks, 8 * ctx->num_sms);
+  const size_t o_gang = align_up(sizeof(vfk::WaveJob) * n, 16);
+  const size_t o_cta = align_up(o_gang + sizeof(vfk::WaveGang) * ng, 16);
+  const size_t o_ent = align_up(o_cta + sizeof(vfk::WaveCta) * (size_t)fs.shape.blocks, 16);
+  char* const h = h_wave;
+  char* const d = static_cast<char*>(wsched.p);
+  std::memcpy(h, wave_jobs.data(), sizeof(vfk::WaveJob) * n);
+  std::memcpy(h + o_gang, wave_gangs.data(), sizeof(vfk::WaveGang) * ng);
+  const uint32_t used = vfk::flood_schedule(wave_gangs.data(), (uint32_t)ng, fs.shape, fs.wait_spins ? 2 : 1,
+                                            reinterpret_cast<vfk::WaveCta*>(h + o_cta),
+                                            reinterpret_cast<vfk::WaveEntry*>(h + o_ent));
+  fs.jobs = reinterpret_cast<const vfk::WaveJob*>(d);
+  fs.gangs = reinterpret_cast<const vfk::WaveGang*>(d + o_gang);
+  fs.cta = reinterpret_cast<const vfk::WaveCta*>(d + o_cta);
+  fs.entries = reinterpret_cast<const vfk::WaveEntry*>(d + o_ent);
+  VF_CK(cudaMemcpyAsync(d, h, o_ent + sizeof(vfk::WaveEntry) * (size_t)used, cudaMemcpyHostToDevice, stream));
+  return VF_OK;
+}
+
+// the flood's waves, after the last ones issued on the context (any stream)
+cudaError_t Batch::waves_serialized(cudaStream_t st, JobState* ds, const vfk::FloodScratch& fs) {
   const bool chain = !capturing && ctx->ev_relax;
   std::unique_lock<std::mutex> lk(ctx->relax_mu, std::defer_lock);
   if (chain) lk.lock();
@@ -699,7 +788,7 @@ cudaError_t Batch::relax_serialized(cudaStream_t st, const JobDesc* tf, JobState
     cudaError_t e = cudaStreamWaitEvent(st, ctx->ev_relax, 0);
     if (e != cudaSuccess) return e;
   }
-  cudaError_t e = vfk::flood_relax(st, tf, ds, bj, lv, fs, ctx->num_sms, &relax_blocks);
+  cudaError_t e = vfk::flood_waves(st, ds, fs);
   if (e == cudaSuccess && chain) {
     e = cudaEventRecord(ctx->ev_relax, st);
     ctx->ev_relax_used = e == cudaSuccess;
@@ -767,15 +856,16 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
   vfk::FloodScratch fs = flood_scratch(*this);
   if (any_flood) {
     const JobDesc* tf = dtable(T_FLOOD);
+    if ((s = wave_tables(fs))) return s;
     vfk::flood_seed_bricks(st, tf, ds, n, lv, lst, lc);
-    vfk::flood_init_keys(st, tf, lst, lc, maxc, bj, lv);
-    vfk::flood_seed(st, tf, ds, n, fs, lv);
+    vfk::flood_init(st, tf, fs, lv);
+    VF_CK(vfk::flood_seed(st, tf, ds, fs));
     VF_CK(record_event(ev_flood0, st));
-    cudaError_t e = relax_serialized(st, tf, ds, bj, lv, fs);
-    if (e != cudaSuccess) return fail(VF_ERR_CUDA, std::string("flood relax launch: ") + cudaGetErrorString(e));
+    cudaError_t e = waves_serialized(st, ds, fs);
+    if (e != cudaSuccess) return fail(VF_ERR_CUDA, std::string("flood launch: ") + cudaGetErrorString(e));
     VF_CK(record_event(ev_flood1, st));
     flood_timed = true;
-    vfk::flood_finalize(st, tf, ds, lst, lc, maxc, bj, 0);
+    vfk::flood_labels(st, tf, ds, lst, lc, maxc, bj, 0);
     launches += 5;
     if (any_prefix) {
       // competition to a fixed point (host loop), disjoint cleanup, re-flood
@@ -790,11 +880,11 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
         for (uint32_t i = 0; i < n; ++i) any |= h_state[i].changed != 0;
         if (!any) break;
       }
-      vfk::flood_disjoint(st, tf, ds, n, lst, lc, maxc, bj, fs, lv);
-      e = relax_serialized(st, tf, ds, bj, lv, fs);
-      if (e != cudaSuccess) return fail(VF_ERR_CUDA, std::string("flood relax launch: ") + cudaGetErrorString(e));
-      vfk::flood_finalize(st, tf, ds, lst, lc, maxc, bj, 1);
-      launches += 6;
+      VF_CK(vfk::flood_disjoint(st, tf, ds, n, lst, lc, maxc, bj, fs));
+      e = waves_serialized(st, ds, fs);
+      if (e != cudaSuccess) return fail(VF_ERR_CUDA, std::string("flood launch: ") + cudaGetErrorString(e));
+      vfk::flood_labels(st, tf, ds, lst, lc, maxc, bj, 1);
+      launches += 5;
     }
   }
   if (any_naive) { vfk::naive(st, dtable(T_NAIVE), ds, lst, lc, maxc, bj); launches += 1; }
@@ -876,7 +966,7 @@ vf_status Batch::finish(vf_job_result* res) {
       first = st;
       set_error("job " + std::to_string(i) + ": " +
                 (st == VF_ERR_SEED_SEARCH ? "seed search exceeded 1e6 tries"
-                 : st == VF_ERR_TIMEOUT   ? ((ferr & 8u) ? "flood relaxation skipped an out-of-range brick or key access"
+                 : st == VF_ERR_TIMEOUT   ? ((ferr & 8u) ? "flood skipped an out-of-range access"
                                                         : "flood did not converge (bounded wait expired)")
                  : st == VF_ERR_RANGE     ? "value out of range (prefix, distance or count)"
                                           : "invalid seeds or parameters"));

@@ -64,11 +64,18 @@ struct Batch {
   DevBuf grid0, grid1, keys, par, tets, range, ys, seeds, counts, lat, verts, faces, emask;
   DevBuf etab;  // mesh edge parity tables (voxelizer)
   DevBuf rle_cnt, rle_base, rle_sums, rle_tot, rle_starts, rle_rec;  // RLE export scratch
-  DevBuf tables, state, brick_job, live, list, lcount, q[3], scal, epoch, fdir, front[2];
+  DevBuf tables, state, brick_job, live, list, lcount, scal, front[2];
+  DevBuf wst, win, wzero, wsched;  // flood: row states; what reaches their ends; candidates + barriers; wave jobs + gangs
   DevBuf pcnt, pbase, psums, srec;  // flattened per-face work lists, shell setup
   DevBuf stage_out;  // packed labels of the DMA download
-  DevBuf tmaps;      // [jobs] TMA descriptors of the flood keys (vfk::KEYS_MAP_BYTES each)
-  size_t tmap_off = 0;  // their host copy inside h_tables
+  // the plain path floods on u32 keys, the batched one on row states
+  bool plain = false;
+  uint32_t wsw = 8;                     // state words of the batch's floods
+  std::vector<vfk::WaveJob> wave_jobs;  // the batch's floods
+  std::vector<vfk::WaveGang> wave_gangs;
+  uint32_t wave_units = 0;              // their 256-row units
+  size_t wave_zero_bytes() const;       // candidate words, barriers, last waves
+  char* h_wave = nullptr;               // in h_tables: wave jobs, gangs, CTA table, gang entries
   // download by DMA: labels are copied to out_labels by the copy engine, from
   // the label grid when its rows have no padding, else packed first into a
   // device staging buffer (no kernel writes host memory, so the download of
@@ -98,14 +105,13 @@ struct Batch {
   // per-launch bookkeeping
   uint64_t launches = 0;
   bool flood_timed = false;
-  int relax_blocks = 0;
 
   vf_status init(Ctx* c, bool own);
   void release();
   vf_status plan(const vf_job* const* js, uint32_t n);
   vf_status enqueue_batched(bool upload_inputs = true, bool download = true);
-  cudaError_t relax_serialized(cudaStream_t st, const JobDesc* tf, JobState* ds, const uint32_t* bj,
-                               const uint8_t* lv, const vfk::FloodScratch& fs);
+  cudaError_t waves_serialized(cudaStream_t st, JobState* ds, const vfk::FloodScratch& fs);
+  vf_status wave_tables(vfk::FloodScratch& fs);
   // the resident stage chain (no uploads) as a CUDA graph: captured on the
   // first execute after plan(), replayed afterwards; falls back to direct
   // launches when the chain has host steps (sub-seed prefix competition) or
@@ -129,9 +135,9 @@ struct Batch {
 struct Tuning {
   int32_t parity_grid = 16;   // k_parity_flat CTAs per SM
   int32_t shell_grid = 12;    // k_shell_flat CTAs per SM
-  int32_t flood_sweeps = 96;  // relaxation sweeps per brick visit (waves per pass)
-  int32_t flood_ctas = 0;     // k_relax resident CTAs per SM (0: as many as fit)
-  uint32_t flood_wait_spins = 0;  // grid-barrier spin limit of k_relax (0: the default)
+  int32_t flood_sweeps = 96;  // kept for callers that set it; the wave flood has no such bound
+  int32_t flood_ctas = 0;     // k_wave resident CTAs per SM (0: as many as fit)
+  uint32_t flood_wait_spins = 0;  // gang-barrier poll limit of k_wave (0: the default)
 };
 
 struct Ctx {

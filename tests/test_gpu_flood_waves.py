@@ -68,3 +68,36 @@ def _check_batch(vf, ctx, sizes):
                          ids=["one_cta_each", "two_gangs", "more_jobs_than_a_gang"])
 def test_flood_gangs(vf, ctx, sizes):
     _check_batch(vf, ctx, sizes)
+
+
+@pytest.mark.parametrize("dfunc", [1, 2])
+@pytest.mark.parametrize("shape,frac,nseeds,nfrag,nprefix", [
+    ((20, 33, 40), 0.45, 9, 2, 3), ((31, 32, 65), 0.4, 64, 7, 4), ((40, 20, 96), 0.35, 65, 30, 2),
+    ((33, 47, 33), 0.6, 300, 5, 100), ((24, 24, 70), 0.3, 1100, 254, 5)])
+def test_flood_prefix_sets(vf, ctx, shape, frac, nseeds, nfrag, nprefix, dfunc):
+    """Sub-seed prefixes: labels shared by several seeds, seeds on one voxel, fragments
+    in several components, at every plane count."""
+    rng = np.random.default_rng(sum(shape) + nseeds)
+    occ = (rng.random(shape) < frac).astype(np.uint16)
+    seeds = _seeds(occ, nseeds, rng)
+    n = len(seeds)
+    seeds[:, 3] = (rng.integers(0, nfrag, n) + 2) | (rng.integers(0, nprefix, n) << 8)
+    seeds[n // 2, :3] = seeds[0, :3]  # the later one holds the voxel
+    seeds = seeds[rng.permutation(n)]
+    assert np.array_equal(_flood(vf, ctx, occ, seeds, dfunc), O.flood(occ, seeds, dfunc)[0])
+
+
+def test_flood_prefixes_in_a_batch(vf, ctx):
+    # jobs with and without sub-seeds in one batch, in step
+    specs, wants = [], []
+    for i, (z, extra) in enumerate([(40, 0), (96, 12), (33, 5), (100, 0), (64, 30)]):
+        v, f = Vs.vessel_mesh(20, 15, i)
+        mn, mx = Vs.mesh_aabb(v)
+        p = vf.Params.default(distance=i % 3, num_seeds=4 + i, num_extra_seeds=extra, seed=i + 1)
+        specs.append(vf.JobSpec(v, f, p, dims=(z - 3, z, z), aabb=(mn, mx), ncounts=256))
+        q = O.Params()
+        for name, _ in O.Params._fields_:
+            setattr(q, name, getattr(p, name))
+        wants.append(O.run_job(v, f, specs[-1].dims, mn, mx, q, ncounts=256)[:2])
+    for r, s, (lab, cnt) in zip(vf.batch_run(specs, ctx), specs, wants):
+        assert r.status == 0 and np.array_equal(s.labels, lab) and np.array_equal(s.counts, cnt)

@@ -60,6 +60,7 @@ struct JobDesc {
   uint2* win;
   uint32_t* wcand;
   uint32_t wsw, wrow0, wsx, wsy;
+  uint32_t* uf;     // [seeds_cap] union-find over the slots (null: no sub-seed prefixes)
   uint32_t* par;
   uint32_t* shell;
   // mesh
@@ -111,7 +112,7 @@ struct JobState {
   uint32_t nseeds;
   uint32_t err;
   uint32_t has_prefix;      // any seed label with a sub-seed prefix
-  uint32_t disjoint;        // voxels reset by the disjoint cleanup
+  uint32_t disjoint;        // the disjoint cleanup reset voxels (plain path: how many)
   uint32_t changed;         // generic convergence flag
   uint32_t minprefix[256];  // per fragment
   uint32_t rank_value[256]; // pass-2 slot -> label value

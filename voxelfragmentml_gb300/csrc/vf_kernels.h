@@ -244,7 +244,6 @@ struct FloodScratch {
   uint32_t* last = nullptr;            // [njobs]
   void* zero = nullptr;                // candidate words, bar, last: cleared before a flood
   size_t zero_bytes = 0;
-  size_t in_bytes = 0;                 // of arr.in
   uint32_t* err = nullptr;             // [1] global error word
   uint32_t* stats = nullptr;           // [VF_FLOOD_NCOUNTERS]
   uint32_t* wave_sizes = nullptr;      // statistics: rows visited per wave (256)
@@ -269,13 +268,10 @@ void flood_init(cudaStream_t st, const JobDesc* dj, const FloodScratch& fs, cons
 cudaError_t flood_seed(cudaStream_t st, const JobDesc* dj, const JobState* ds, const FloodScratch& fs);
 cudaError_t flood_waves(cudaStream_t st, JobState* ds, const FloodScratch& fs);
 void flood_labels(cudaStream_t st, const JobDesc* dj, const JobState* ds, const uint32_t* list,
-                  const uint32_t* count, uint32_t max_count, const uint32_t* brick_job, int pass2);
-// sub-seed prefix competition and the disjoint cleanup
-void flood_competition(cudaStream_t st, const JobDesc* dj, JobState* ds, const uint32_t* list,
-                       const uint32_t* count, uint32_t max_count, const uint32_t* brick_job);
-cudaError_t flood_disjoint(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs,
-                           const uint32_t* list, const uint32_t* count, uint32_t max_count,
-                           const uint32_t* brick_job, const FloodScratch& fs);
+                  const uint32_t* count, uint32_t max_count, const uint32_t* brick_job);
+// sub-seed prefix competition and the disjoint cleanup after a flood: the jobs
+// whose voxels were reset are ready for the second flood
+cudaError_t flood_prefixes(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs, const FloodScratch& fs);
 
 // ---- a flood on an unpadded device grid (vf_flood_noalloc) ----
 struct FlatAxes {

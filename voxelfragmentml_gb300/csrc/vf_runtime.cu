@@ -112,10 +112,12 @@ void Batch::drop_graphs() {
 }
 
 vf_status Batch::execute_resident(bool download) {
-  bool host_steps = false;
-  for (const JobPlan& p : plans) host_steps |= p.prefix_possible;
+  // batches with sub-seed prefixes run with direct launches, as callers of
+  // vf_ctx_last_graph know them
+  bool prefixes = false;
+  for (const JobPlan& p : plans) prefixes |= p.prefix_possible;
   last_run_graph = false;
-  if (!graphs_ok || host_steps) return enqueue_batched(false, download);
+  if (!graphs_ok || prefixes) return enqueue_batched(false, download);
   const int gi = download ? 1 : 0;
   if (!gexec[gi]) {
     vfk::flood_shape(wsw, (uint32_t)wave_jobs.size(), ctx->num_sms, 0);  // function attributes outside the capture
@@ -152,7 +154,7 @@ void Batch::release() {
   if (!ctx) return;
   for (DevBuf* b : {&grid0, &grid1, &keys, &par, &tets, &range, &ys, &seeds, &counts, &lat,
                     &verts, &faces, &emask, &etab, &tables, &state, &brick_job, &live, &list, &lcount,
-                    &scal, &wst, &win, &wzero, &wsched, &front[0], &front[1], &pcnt, &pbase,
+                    &scal, &uf, &wst, &win, &wzero, &wsched, &front[0], &front[1], &pcnt, &pbase,
                     &psums, &srec, &stage_out, &rle_cnt, &rle_base, &rle_sums, &rle_tot, &rle_starts,
                     &rle_rec})
     ctx->free_buf(*b);
@@ -369,6 +371,7 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
     p.o_etab = sz.etab; sz.etab += p.ecap;
     p.o_ys = sz.ys; sz.ys += align_up(p.Y, 64);
     p.o_seeds = sz.seeds; sz.seeds += align_up(4 * (size_t)p.seeds_cap, 64);
+    p.o_uf = sz.uf; if (p.prefix_possible && !plain) sz.uf += align_up(p.seeds_cap, 64);
     p.o_counts = sz.counts; sz.counts += align_up(p.ncounts, 64);
     p.o_lat = sz.lat; sz.lat += align_up((size_t)p.lat_nx * p.lat_ny * p.lat_nz * 3, 64);
     p.o_verts = sz.verts; sz.verts += align_up((size_t)j.nverts * 3, 64);
@@ -459,6 +462,7 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
   ALLOC(live, nb);
   ALLOC(list, nb * 4);
   ALLOC(lcount, 256);
+  ALLOC(uf, std::max<size_t>(sz.uf * 4, 256));
   ALLOC(wst, std::max<size_t>(wrows * wsw * 4, 256));
   ALLOC(win, std::max<size_t>(wrows * 16, 256));
   ALLOC(wzero, std::max<size_t>(wave_zero_bytes(), 256));
@@ -532,6 +536,7 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
     d.wcand = static_cast<uint32_t*>(wzero.p);
     d.wsw = wsw;
     d.wrow0 = d.wsx = d.wsy = 0;  // from its wave job, below
+    d.uf = p.prefix_possible && !plain ? static_cast<uint32_t*>(uf.p) + p.o_uf : nullptr;
     d.par = static_cast<uint32_t*>(par.p) + p.o_par;
     d.shell = static_cast<uint32_t*>(par.p) + sz.par + p.o_par;
     d.verts = static_cast<float*>(verts.p) + p.o_verts;
@@ -746,7 +751,6 @@ static vfk::FloodScratch flood_scratch(Batch& B) {
   fs.zero_bytes = B.wave_zero_bytes();
   fs.bar = fs.arr.cand + (size_t)B.wave_units * 16;
   fs.last = fs.bar + vfk::WAVE_BAR_WORDS * B.wave_gangs.size();
-  fs.in_bytes = (size_t)B.wave_units * 256 * 16;
   fs.err = sc + 12;      // [1]
   fs.stats = sc + 16;    // [VF_FLOOD_NCOUNTERS]
   fs.wave_sizes = sc + 128;  // [256]
@@ -865,27 +869,16 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
     if (e != cudaSuccess) return fail(VF_ERR_CUDA, std::string("flood launch: ") + cudaGetErrorString(e));
     VF_CK(record_event(ev_flood1, st));
     flood_timed = true;
-    vfk::flood_labels(st, tf, ds, lst, lc, maxc, bj, 0);
-    launches += 5;
+    launches += 4;
     if (any_prefix) {
-      // competition to a fixed point (host loop), disjoint cleanup, re-flood
-      for (int it = 0; it < 1 << 20; ++it) {
-        for (uint32_t i = 0; i < n; ++i)
-          VF_CK(cudaMemsetAsync(&ds[i].changed, 0, sizeof(uint32_t), st));
-        vfk::flood_competition(st, tf, ds, lst, lc, maxc, bj);
-        VF_CK(cudaMemcpyAsync(h_state, ds, sizeof(JobState) * n, cudaMemcpyDeviceToHost, st));
-        VF_CK(cudaStreamSynchronize(st));
-        launches += 1;
-        bool any = false;
-        for (uint32_t i = 0; i < n; ++i) any |= h_state[i].changed != 0;
-        if (!any) break;
-      }
-      VF_CK(vfk::flood_disjoint(st, tf, ds, n, lst, lc, maxc, bj, fs));
+      // competition, disjoint cleanup, second flood of the jobs it reset
+      VF_CK(vfk::flood_prefixes(st, tf, ds, n, fs));
       e = waves_serialized(st, ds, fs);
       if (e != cudaSuccess) return fail(VF_ERR_CUDA, std::string("flood launch: ") + cudaGetErrorString(e));
-      vfk::flood_labels(st, tf, ds, lst, lc, maxc, bj, 1);
       launches += 5;
     }
+    vfk::flood_labels(st, tf, ds, lst, lc, maxc, bj);
+    launches += 1;
   }
   if (any_naive) { vfk::naive(st, dtable(T_NAIVE), ds, lst, lc, maxc, bj); launches += 1; }
   mark(7);

@@ -29,7 +29,7 @@ struct DevBuf {
 struct JobPlan {
   uint32_t X, Y, Z, Zp, Zk, Zw, nbx, nby, nbz, nbricks;
   float amin[3], amax[3];
-  size_t o_grid, o_keys, o_par, o_tets, o_range, o_ys, o_seeds, o_counts, o_lat, o_verts,
+  size_t o_grid, o_keys, o_par, o_tets, o_range, o_ys, o_seeds, o_uf, o_counts, o_lat, o_verts,
       o_faces, o_emask, o_etab;
   uint32_t ecap, ncounts, seeds_cap, lat_nx, lat_ny, lat_nz, ek;
   float elimit;
@@ -42,7 +42,7 @@ struct JobPlan {
 };
 
 struct Sizes {
-  size_t grid = 0, keys = 0, par = 0, tets = 0, range = 0, ys = 0, seeds = 0, counts = 0,
+  size_t grid = 0, keys = 0, par = 0, tets = 0, range = 0, ys = 0, seeds = 0, uf = 0, counts = 0,
          lat = 0, verts = 0, faces = 0, emask = 0, etab = 0;
   uint32_t bricks = 0, faces_total = 0, max_iters = 0;
   uint64_t rows = 0;  // sum of X * Y over the jobs
@@ -65,6 +65,7 @@ struct Batch {
   DevBuf etab;  // mesh edge parity tables (voxelizer)
   DevBuf rle_cnt, rle_base, rle_sums, rle_tot, rle_starts, rle_rec;  // RLE export scratch
   DevBuf tables, state, brick_job, live, list, lcount, scal, front[2];
+  DevBuf uf;         // union-find over the seed slots of jobs with sub-seed prefixes
   DevBuf wst, win, wzero, wsched;  // flood: row states; what reaches their ends; candidates + barriers; wave jobs + gangs
   DevBuf pcnt, pbase, psums, srec;  // flattened per-face work lists, shell setup
   DevBuf stage_out;  // packed labels of the DMA download
@@ -114,8 +115,7 @@ struct Batch {
   vf_status wave_tables(vfk::FloodScratch& fs);
   // the resident stage chain (no uploads) as a CUDA graph: captured on the
   // first execute after plan(), replayed afterwards; falls back to direct
-  // launches when the chain has host steps (sub-seed prefix competition) or
-  // cannot be captured
+  // launches when the chain has sub-seed prefixes or cannot be captured
   vf_status execute_resident(bool download);
   void drop_graphs();
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};  // [download]

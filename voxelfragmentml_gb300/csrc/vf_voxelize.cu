@@ -301,12 +301,17 @@ __global__ void k_scan_add(unsigned long long* out, const unsigned long long* su
 }
 
 // Warp-interleaved runs over a flattened work list (faces in batch order,
-// items of a face contiguous): a warp owns WARP_RUN consecutive items and
+// items of a face contiguous): a warp owns a run of consecutive items and
 // lane l takes items base + l, base + l + 32, ...  Neighbouring lanes work on
 // neighbouring items of the same face, so control flow stays coherent and no
 // lane idles when a face has few items.  One binary search per warp run; each
-// lane then steps its face cursor forward.
-constexpr uint32_t WARP_RUN = 32 * 16;
+// lane then steps its face cursor forward.  A run is an even share of the items
+// per warp, 32 to 512: with 512 always, a 12 k face mesh kept one warp per SM
+// busy for 16 items in a row (parity 73 us against 14, shell 63 against 14).
+__device__ __forceinline__ uint32_t warp_run(unsigned long long total, unsigned long long nwarps) {
+  const unsigned long long share = (total + nwarps - 1) / nwarps;
+  return 32u * (uint32_t)min(16ull, max(1ull, (share + 31) / 32));
+}
 
 __device__ __forceinline__ uint32_t face_of_item(const unsigned long long* base, uint32_t nfaces,
                                                  unsigned long long p) {
@@ -325,12 +330,13 @@ __global__ void __launch_bounds__(256) k_parity_flat(const JobDesc* jobs, int nj
                                                   uint32_t total_faces) {
   const unsigned long long total = *ptotal;
   const int lane = threadIdx.x & 31;
-  const unsigned long long nwruns = (total + WARP_RUN - 1) / WARP_RUN;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+  const uint32_t run = warp_run(total, nwarps);
+  const unsigned long long nwruns = (total + run - 1) / run;
   for (unsigned long long wr = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
        wr < nwruns; wr += nwarps) {
-    const unsigned long long base = wr * WARP_RUN;
-    const unsigned long long end = min(base + WARP_RUN, total);
+    const unsigned long long base = wr * run;
+    const unsigned long long end = min(base + run, total);
     uint32_t g = 0;
     if (lane == 0) g = face_of_item(pbase, total_faces, base);
     g = __shfl_sync(0xFFFFFFFFu, g, 0);
@@ -767,12 +773,13 @@ __global__ void __launch_bounds__(256, 3) k_shell_flat(const JobDesc* jobs, cons
                                                        uint32_t total_faces, const float4* srec) {
   const unsigned long long total = *stotal;
   const int lane = threadIdx.x & 31;
-  const unsigned long long nwruns = (total + WARP_RUN - 1) / WARP_RUN;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+  const uint32_t run = warp_run(total, nwarps);
+  const unsigned long long nwruns = (total + run - 1) / run;
   for (unsigned long long wr = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
        wr < nwruns; wr += nwarps) {
-    const unsigned long long base = wr * WARP_RUN;
-    const unsigned long long end = min(base + WARP_RUN, total);
+    const unsigned long long base = wr * run;
+    const unsigned long long end = min(base + run, total);
     uint32_t g = 0;
     if (lane == 0) g = face_of_item(sbase, total_faces, base);
     g = __shfl_sync(0xFFFFFFFFu, g, 0);

@@ -127,18 +127,23 @@ __device__ bool uniform_block(const JobDesc& J, SeedSmem& S, uint32_t n, uint64_
     S.cand[t] = key;
     __syncthreads();
     if (warp == 0) {
+      // 32 attempts at a time, only the valid ones compared: 64 seeds in a hollow
+      // 192 voxel model 23 us (62 us one attempt at a time)
       uint32_t cnt = S.cnt;
-      for (int i = 0; i < 1024 && cnt < n; ++i) {
-        const unsigned long long k = S.cand[i];
-        if (k == ~0ull) continue;
-        bool dup = false;
-        for (uint32_t m = lane; m < cnt; m += 32) dup |= (S.acc[m] == k);
-        dup = __any_sync(0xFFFFFFFFu, dup);
-        if (!dup) {
-          if (lane == 0) S.acc[cnt] = k;
-          ++cnt;
+      for (int i0 = 0; i0 < 1024 && cnt < n; i0 += 32) {
+        const unsigned long long mine = S.cand[i0 + lane];
+        unsigned m = __ballot_sync(0xFFFFFFFFu, mine != ~0ull);
+        for (; m && cnt < n; m &= m - 1) {
+          const unsigned long long k = __shfl_sync(0xFFFFFFFFu, mine, __ffs(m) - 1);
+          bool dup = false;
+          for (uint32_t q = lane; q < cnt; q += 32) dup |= (S.acc[q] == k);
+          dup = __any_sync(0xFFFFFFFFu, dup);
+          if (!dup) {
+            if (lane == 0) S.acc[cnt] = k;
+            ++cnt;
+          }
+          __syncwarp();
         }
-        __syncwarp();
       }
       if (lane == 0) S.cnt = cnt;
     }

@@ -293,69 +293,232 @@ __global__ void __launch_bounds__(1024) k_seeds(const JobDesc* jobs, JobState* s
 }
 
 // ===========================================================================
+// A brick's 256 label rows between global memory and shared memory (34-u16 row
+// pitch: the u16 of one z from 32 threads falls on 32 distinct banks), 4 lanes
+// per row along z; units at or past Zp are zero / not written.
+constexpr int ROW_PITCH = VF_BZ + 2;
+__device__ __forceinline__ void rows_in(const JobDesc& J, const uint16_t* src, uint32_t x0, uint32_t y0, uint32_t z0,
+                                        uint16_t* rows) {
+  const uint32_t nz = min((uint32_t)VF_BZ, J.Zp - z0);
+  uint4 w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t u = i * 256 + threadIdx.x, row = u >> 2, q = u & 3;
+    const uint32_t x = x0 + row / VF_BY, y = y0 + row % VF_BY;
+    w[i] = (x < J.X && y < J.Y && 8 * q < nz) ? *reinterpret_cast<const uint4*>(src + vf_gidx(J, x, y, z0 + 8 * q))
+                                              : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t u = i * 256 + threadIdx.x, row = u >> 2, q = u & 3;
+    // 4-byte aligned: 68-byte row pitch, 16-byte units
+    uint32_t* d = reinterpret_cast<uint32_t*>(rows + row * ROW_PITCH + 8 * q);
+    d[0] = w[i].x; d[1] = w[i].y; d[2] = w[i].z; d[3] = w[i].w;
+  }
+}
+__device__ __forceinline__ void rows_out(const JobDesc& J, uint16_t* dst, uint32_t x0, uint32_t y0, uint32_t z0,
+                                         const uint16_t* rows) {
+  const uint32_t nz = min((uint32_t)VF_BZ, J.Zp - z0);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t u = i * 256 + threadIdx.x, row = u >> 2, q = u & 3;
+    const uint32_t x = x0 + row / VF_BY, y = y0 + row % VF_BY;
+    if (x < J.X && y < J.Y && 8 * q < nz) {
+      const uint32_t* r = reinterpret_cast<const uint32_t*>(rows + row * ROW_PITCH + 8 * q);
+      *reinterpret_cast<uint4*>(dst + vf_gidx(J, x, y, z0 + 8 * q)) = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+  }
+}
+// bit z: voxel z of 32 (16 u16 pairs) is above `floor`
+__device__ __forceinline__ uint32_t pair_bits(uint32_t w, uint32_t floor, int k) {
+  const uint32_t g = __vsetgtu2(w, floor * 0x00010001u);
+  return ((g | (g >> 15)) & 3u) << (2 * k);
+}
+__device__ __forceinline__ uint32_t voxels_above(const uint16_t* row /* 4-byte aligned */, uint32_t floor) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int k = 0; k < VF_BZ / 2; ++k) m |= pair_bits(reinterpret_cast<const uint32_t*>(row)[k], floor, k);
+  return m;
+}
+__device__ __forceinline__ uint32_t tile_voxels_above(const uint16_t* row /* 16-byte aligned */, uint32_t floor) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int k = 0; k < VF_BZ / 8; ++k) {
+    const uint4 w = reinterpret_cast<const uint4*>(row)[k];
+    m |= pair_bits(w.x, floor, 4 * k) | pair_bits(w.y, floor, 4 * k + 1) | pair_bits(w.z, floor, 4 * k + 2) |
+         pair_bits(w.w, floor, 4 * k + 3);
+  }
+  return m;
+}
+// The voxels of a brick chosen by m (bit z of the thread's row, row = thread), as
+// row << 5 | z in row order, into vq (all 256 threads call it; wq: 8 words).
+// The voxels of a thin wall are few and uneven per row: dealt from the queue
+// they keep every lane busy.
+__device__ __forceinline__ uint32_t queue_voxels(uint32_t m, uint16_t* vq, uint32_t* wq) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t c = (uint32_t)__popc(m);
+  uint32_t incl = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += u;
+  }
+  if (lane == 31) wq[warp] = incl;
+  __syncthreads();
+  uint32_t base = incl - c, total = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    base += w < warp ? wq[w] : 0u;
+    total += wq[w];
+  }
+  while (m) {
+    const uint32_t z = (uint32_t)__ffs(m) - 1;
+    m &= m - 1;
+    vq[base++] = (uint16_t)((t << 5) | z);
+  }
+  __syncthreads();
+  return total;
+}
+
 // NaiveFracturer::buildCPU (NaiveFracturer.cpp:26-68): every occupied voxel
 // takes the label of the nearest seed; strict '<' keeps the lowest index.
+//
+// Per brick, only the seeds that can be nearest to one of its voxels are
+// compared: a seed is dropped when its distance to the brick's box exceeds the
+// largest distance some other seed has to it.  The bounds are whole numbers
+// (squares for VF_EUCLIDEAN); a 2^-18 margin on squares is far above the
+// rounding of the float distances (2^-23), so a dropped seed never ties.  Seeds
+// far outside every grid (no rule refuses them) are always compared.
+// Bound by the distance arithmetic of the voxels left: 64 seeds on 180 x 179 x
+// 192 voxels 25 us (531 us with every seed against all voxels of the rows).
+constexpr uint32_t NAIVE_SEEDS = 256;  // compared per round, plus at most as many
+constexpr uint32_t SEED_NEAR = 8192;  // twice the largest grid side; squares of coordinates below it add up in u32
 __global__ void __launch_bounds__(256) k_naive(const JobDesc* jobs, const JobState* st,
                                                const uint32_t* list, const uint32_t* count,
                                                const uint32_t* brick_job) {
-  __shared__ uint4 sd[512];
+  __shared__ uint4 sd[2 * NAIVE_SEEDS];  // position, index
+  __shared__ __align__(16) uint16_t rows[256 * ROW_PITCH];
+  __shared__ uint16_t vq[256 * VF_BZ];
+  __shared__ uint32_t wq[8], s_bound;
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const uint32_t n = *count;
   for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
     const uint32_t b = list[it];
     const uint32_t j = brick_job[b];
     const JobDesc& J = jobs[j];
-    if (!J.active) continue;
     const uint32_t ns = st[j].nseeds;
+    if (!J.active || ns == 0) continue;  // uniform across the CTA
+    const uint4* const seeds = reinterpret_cast<const uint4*>(J.seeds);
+    const int dist = J.distance;
     uint32_t x0, y0, z0;
     brick_coords(J, b, x0, y0, z0);
-    const uint32_t x = x0 + threadIdx.x / VF_BY, y = y0 + threadIdx.x % VF_BY;
-    const bool row_ok = x < J.X && y < J.Y;
-    uint16_t v[VF_BZ];
-    float best[VF_BZ];
-    if (row_ok) {
-      const uint4* src = reinterpret_cast<const uint4*>(J.grid + vf_gidx(J, x, y, z0));
-      const uint32_t nz = min((uint32_t)VF_BZ, J.Zp - z0);
+    __syncthreads();  // the previous brick is done with the shared arrays
+    rows_in(J, J.grid, x0, y0, z0, rows);
+    if (t == 0) s_bound = 0xFFFFFFFFu;
+    __syncthreads();
+    const uint32_t total = queue_voxels(voxels_above(rows + t * ROW_PITCH, VOXEL_EMPTY), vq, wq);
+    // smallest (near) and largest (far) distance of a seed to the brick's voxels
+    auto reach = [&](const uint4& sp, uint32_t& near, uint32_t& far) {
+      const uint32_t p[3] = {sp.x, sp.y, sp.z}, lo[3] = {x0, y0, z0};
+      const uint32_t hi[3] = {min(x0 + VF_BX, J.X) - 1, min(y0 + VF_BY, J.Y) - 1, min(z0 + VF_BZ, J.Z) - 1};
+      near = 0;
+      far = 0xFFFFFFFFu;
+      if (max(max(sp.x, sp.y), sp.z) >= SEED_NEAR) return;
+      far = 0;
 #pragma unroll
-      for (int q = 0; q < VF_BZ / 8; ++q) {
-        uint4 w = (q * 8 < (int)nz) ? src[q] : make_uint4(0, 0, 0, 0);
-        v[8 * q + 0] = w.x & 0xFFFF; v[8 * q + 1] = w.x >> 16;
-        v[8 * q + 2] = w.y & 0xFFFF; v[8 * q + 3] = w.y >> 16;
-        v[8 * q + 4] = w.z & 0xFFFF; v[8 * q + 5] = w.z >> 16;
-        v[8 * q + 6] = w.w & 0xFFFF; v[8 * q + 7] = w.w >> 16;
+      for (int a = 0; a < 3; ++a) {
+        const uint32_t l = p[a] < lo[a] ? lo[a] - p[a] : (p[a] > hi[a] ? p[a] - hi[a] : 0u);
+        const uint32_t f = max(p[a] > lo[a] ? p[a] - lo[a] : lo[a] - p[a], p[a] > hi[a] ? p[a] - hi[a] : hi[a] - p[a]);
+        if (dist == 0) { near += l * l; far += f * f; }
+        else if (dist == 1) { near += l; far += f; }
+        else { near = max(near, l); far = max(far, f); }
       }
+    };
+    uint32_t bound = 0xFFFFFFFFu;
+    for (uint32_t i = t; i < ns; i += 256) {
+      uint32_t near, far;
+      reach(seeds[i], near, far);
+      bound = min(bound, far);
     }
-#pragma unroll
-    for (int z = 0; z < VF_BZ; ++z) best[z] = FLT_MAX;
-    for (uint32_t c0 = 0; c0 < ns; c0 += 512) {
+    bound = __reduce_min_sync(0xFFFFFFFFu, bound);
+    if (lane == 0) atomicMin(&s_bound, bound);
+    __syncthreads();
+    bound = s_bound;
+    if (dist == 0 && bound != 0xFFFFFFFFu) bound += (bound >> 18) + 1;
+    // From here a voxel's entry holds the index of its nearest seed so far.
+    uint32_t kept = 0;
+    bool first = true;
+    for (uint32_t c0 = 0; c0 < ns; c0 += 256) {
+      uint4 sp = make_uint4(0, 0, 0, 0);
+      bool keep = false;
+      if (c0 + t < ns) {
+        sp = seeds[c0 + t];
+        uint32_t near, far;
+        reach(sp, near, far);
+        keep = near <= bound;
+      }
+      const uint32_t m = __ballot_sync(0xFFFFFFFFu, keep);
+      if (lane == 0) wq[warp] = (uint32_t)__popc(m);
       __syncthreads();
-      for (uint32_t i = threadIdx.x; i < 512 && c0 + i < ns; i += blockDim.x)
-        sd[i] = reinterpret_cast<const uint4*>(J.seeds)[c0 + i];
-      __syncthreads();
-      if (!row_ok) continue;
-      const uint32_t cn = min(512u, ns - c0);
-      for (uint32_t s = 0; s < cn; ++s) {
-        const uint4 sp = sd[s];
-        const int dx = (int)x - (int)sp.x, dy = (int)y - (int)sp.y;
+      uint32_t at = kept + (uint32_t)__popc(m & ((1u << lane) - 1u));
 #pragma unroll
-        for (int z = 0; z < VF_BZ; ++z) {
-          const int dz = (int)(z0 + z) - (int)sp.z;
-          float d;
-          if (J.distance == 0) {
-            const float fx = (float)dx, fy = (float)dy, fz = (float)dz;
-            d = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy)), __fmul_rn(fz, fz)));
-          } else if (J.distance == 1) {
-            d = (float)(abs(dx) + abs(dy) + abs(dz));
-          } else {
-            d = (float)max(abs(dx), max(abs(dy), abs(dz)));
+      for (uint32_t w = 0; w < 8; ++w) {
+        at += w < warp ? wq[w] : 0u;
+        kept += wq[w];
+      }
+      if (keep) sd[at] = make_uint4(sp.x, sp.y, sp.z, c0 + t);
+      __syncthreads();
+      if (kept < NAIVE_SEEDS && c0 + 256 < ns) continue;  // room for another 256
+      for (uint32_t i = t; i < total; i += 256) {
+        const uint32_t e = vq[i], row = e >> 5, z = e & 31u;
+        const int x = (int)(x0 + row / VF_BY), y = (int)(y0 + row % VF_BY), gz = (int)(z0 + z);
+        uint16_t* const v = rows + row * ROW_PITCH + z;
+        uint32_t lead = first ? 0u : *v;
+        if (dist == 0) {
+          // the square root keeps the order, so only a smaller square can be a
+          // smaller distance; equal roots of unequal squares go to the lower index
+          float best = FLT_MAX, best2 = FLT_MAX;
+          auto square = [&](const uint4& q) {
+            const float fx = (float)(x - (int)q.x), fy = (float)(y - (int)q.y), fz = (float)(gz - (int)q.z);
+            return __fadd_rn(__fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy)), __fmul_rn(fz, fz));
+          };
+          if (!first) {
+            best2 = square(seeds[lead]);
+            best = __fsqrt_rn(best2);
           }
-          if (v[z] != VOXEL_EMPTY && d < best[z]) { best[z] = d; v[z] = (uint16_t)sp.w; }
+          for (uint32_t k = 0; k < kept; ++k) {
+            const uint4 q = sd[k];
+            const float d2 = square(q);
+            if (d2 < best2) {
+              const float d = __fsqrt_rn(d2);
+              if (d < best) { best = d; best2 = d2; lead = q.w; }
+            }
+          }
+        } else {
+          auto steps = [&](const uint4& q) {
+            const int dx = abs(x - (int)q.x), dy = abs(y - (int)q.y), dz = abs(gz - (int)q.z);
+            return (float)(dist == 1 ? dx + dy + dz : max(dx, max(dy, dz)));
+          };
+          float best = first ? FLT_MAX : steps(seeds[lead]);
+          for (uint32_t k = 0; k < kept; ++k) {
+            const uint4 q = sd[k];
+            const float d = steps(q);
+            if (d < best) { best = d; lead = q.w; }
+          }
         }
+        *v = (uint16_t)lead;
       }
+      kept = 0;
+      first = false;
+      __syncthreads();
     }
-    if (row_ok) {
-      // padding voxels stay 0 (they are EMPTY and never labelled)
-      store_row(J, J.grid, x, y, z0, v);
+    for (uint32_t i = t; i < total; i += 256) {
+      const uint32_t e = vq[i];
+      uint16_t* const v = rows + (e >> 5) * ROW_PITCH + (e & 31u);
+      *v = (uint16_t)seeds[*v].w;
     }
+    __syncthreads();
+    rows_out(J, J.grid, x0, y0, z0, rows);
   }
 }
 
@@ -385,15 +548,10 @@ __global__ void __launch_bounds__(256) k_perturb(const JobDesc* jobs, const uint
   // and 32 z values, t = (c mod P) / P rounded as the oracle divides
   __shared__ float t0s[VF_BX], t1s[VF_BY], t2s[VF_BZ];
   __shared__ uint32_t i0s[VF_BX], i1s[VF_BY], i2s[VF_BZ];
-  // the thread's row of labels (34-u16 pitch: the u16 of one z from 32
-  // threads falls on 32 distinct banks)
-  __shared__ __align__(16) uint16_t vrows[256 * 34];
-  // the brick's labelled voxels (row << 5 | z), dealt to all threads: the
-  // labelled voxels of a thin wall are few and uneven per row
+  __shared__ __align__(16) uint16_t vrows[256 * ROW_PITCH];
   __shared__ uint16_t vq[256 * VF_BZ];
   __shared__ uint32_t wq[8];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  uint16_t* v = vrows + t * 34;
+  const int t = threadIdx.x;
   const uint32_t n = *count;
   for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
     const uint32_t b = list[it];
@@ -417,58 +575,10 @@ __global__ void __launch_bounds__(256) k_perturb(const JobDesc* jobs, const uint
       t1s[t - VF_BZ - VF_BX] = __fdiv_rn((float)(gy % P), fp);
       i1s[t - VF_BZ - VF_BX] = gy / P;
     }
-    const uint32_t x = x0 + t / VF_BY, y = y0 + t % VF_BY;
-    const bool rowok = x < J.X && y < J.Y;
     const uint16_t* src = J.grid;
-    // the brick's label rows into shared memory, 4 lanes per row along z (a
-    // warp instruction reads 8 whole 64-byte rows); chunks at or past Zp are
-    // zero
-    const uint32_t nz = min((uint32_t)VF_BZ, J.Zp - z0);
-    {
-      uint4 w[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t u = i * 256 + t, row = u >> 2, q = u & 3;
-        const uint32_t xr = x0 + row / VF_BY, yr = y0 + row % VF_BY;
-        w[i] = (xr < J.X && yr < J.Y && 8 * q < nz)
-                   ? *reinterpret_cast<const uint4*>(src + vf_gidx(J, xr, yr, z0 + 8 * q))
-                   : make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t u = i * 256 + t, row = u >> 2, q = u & 3;
-        // 4-byte aligned: 68-byte row pitch, 16-byte chunks
-        uint32_t* d = reinterpret_cast<uint32_t*>(vrows + row * 34 + 8 * q);
-        d[0] = w[i].x; d[1] = w[i].y; d[2] = w[i].z; d[3] = w[i].w;
-      }
-    }
+    rows_in(J, src, x0, y0, z0, vrows);
     __syncthreads();
-    uint32_t m = 0;  // labelled z of this row
-    if (rowok) {
-#pragma unroll
-      for (int z = 0; z < VF_BZ; ++z) m |= (uint32_t)(v[z] > VOXEL_FREE) << z;
-    }
-    const uint32_t c = (uint32_t)__popc(m);
-    uint32_t incl = c;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-      if (lane >= o) incl += u;
-    }
-    if (lane == 31) wq[warp] = incl;
-    __syncthreads();
-    uint32_t base = incl - c, total = 0;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) {
-      base += w < warp ? wq[w] : 0u;
-      total += wq[w];
-    }
-    while (m) {
-      const uint32_t z = (uint32_t)__ffs(m) - 1;
-      m &= m - 1;
-      vq[base++] = (uint16_t)((t << 5) | z);
-    }
-    __syncthreads();
+    const uint32_t total = queue_voxels(voxels_above(vrows + t * ROW_PITCH, VOXEL_FREE), vq, wq);
     // Per labelled voxel: a 3-channel trilinear value noise n(v / P) from the
     // lattice (lerp along z, then y, then x, as the oracle), offset
     // floor(A * n + 0.5) per axis, and the label found there if it is labelled.
@@ -493,20 +603,10 @@ __global__ void __launch_bounds__(256) k_perturb(const JobDesc* jobs, const uint
       const long ux = (long)xr + o[0], uy = (long)yr + o[1], uz = (long)gz + o[2];
       if (ux < 0 || uy < 0 || uz < 0 || ux >= (long)J.X || uy >= (long)J.Y || uz >= (long)J.Z) continue;
       const uint16_t u = src[vf_gidx(J, (uint32_t)ux, (uint32_t)uy, (uint32_t)uz)];
-      if (u > VOXEL_FREE) vrows[row * 34 + z] = u;
+      if (u > VOXEL_FREE) vrows[row * ROW_PITCH + z] = u;
     }
     __syncthreads();
-    // rows back out as they came in, 4 lanes per row
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t u = i * 256 + t, row = u >> 2, q = u & 3;
-      const uint32_t xr = x0 + row / VF_BY, yr = y0 + row % VF_BY;
-      if (xr < J.X && yr < J.Y && 8 * q < nz) {
-        const uint32_t* r32 = reinterpret_cast<const uint32_t*>(vrows + row * 34 + 8 * q);
-        *reinterpret_cast<uint4*>(J.grid2 + vf_gidx(J, xr, yr, z0 + 8 * q)) =
-            make_uint4(r32[0], r32[1], r32[2], r32[3]);
-      }
-    }
+    rows_out(J, J.grid2, x0, y0, z0, vrows);
   }
 }
 

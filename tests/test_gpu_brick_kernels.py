@@ -36,3 +36,31 @@ def test_nearest_seed(vf, ctx, shape, nseeds, spread, dfunc):
     g = _grid(vf, ctx, occ)
     vf.NaiveFracturer().build(g, seeds, vf.Params.default(distance=dfunc))
     assert np.array_equal(g.data(), O.naive(occ, seeds, dfunc))
+
+
+def _labels(shape, cell, marked, seed):
+    """Blocks of one label with empty voxels between; some voxels marked already."""
+    rng = np.random.default_rng(seed)
+    n = [(s + c - 1) // c for s, c in zip(shape, cell)]
+    lab = rng.integers(2, 6, n).astype(np.uint16)
+    for a in range(3):
+        lab = np.repeat(lab, cell[a], axis=a)
+    lab = np.ascontiguousarray(lab[: shape[0], : shape[1], : shape[2]])
+    lab[rng.random(shape) < 0.4] = 0
+    lab[rng.random(shape) < 0.05] = 1
+    lab[(rng.random(shape) < marked) & (lab > 1)] |= 0x8000
+    return lab
+
+
+SHAPES = [((2, 2, 2), (1, 1, 1)), ((16, 16, 32), (16, 16, 32)), ((33, 17, 65), (16, 16, 32)),
+          ((40, 50, 70), (17, 15, 34)), ((35, 36, 100), (19, 19, 31)), ((50, 50, 37), (50, 50, 37))]
+
+
+@pytest.mark.parametrize("bs", [0, 1, 2, 3])
+@pytest.mark.parametrize("marked", [0.0, 0.01])
+@pytest.mark.parametrize("shape,cell", SHAPES)
+def test_boundaries(vf, ctx, shape, cell, marked, bs):
+    lab = _labels(shape, cell, marked, 3)
+    g = _grid(vf, ctx, lab)
+    g.detectBoundaries(bs)
+    assert np.array_equal(g.data(), O.detect_boundaries(lab, bs))

@@ -64,3 +64,20 @@ def test_boundaries(vf, ctx, shape, cell, marked, bs):
     g = _grid(vf, ctx, lab)
     g.detectBoundaries(bs)
     assert np.array_equal(g.data(), O.detect_boundaries(lab, bs))
+
+
+@pytest.mark.parametrize("etype,size,iters", [(0, 1, 1), (0, 3, 2), (1, 5, 1), (2, 7, 1), (0, 7, 2), (1, 3, 1)])
+@pytest.mark.parametrize("shape,cell", SHAPES)
+def test_erosion(vf, ctx, shape, cell, etype, size, iters):
+    lab = _labels(shape, cell, 0.0, 5)
+    g = _grid(vf, ctx, lab)
+    g.erode(etype, size, iters, 0.7, 0.5, 11)
+    assert np.array_equal(g.data(), O.erode(lab, etype, size, iters, 0.7, 0.5, 11))
+
+
+@pytest.mark.parametrize("shape,cell", SHAPES)
+def test_isolated(vf, ctx, shape, cell):
+    lab = _labels(shape, cell, 0.02, 7)
+    g = _grid(vf, ctx, lab)
+    g.removeIsolatedRegions()
+    assert np.array_equal(g.data(), O.remove_isolated(lab))

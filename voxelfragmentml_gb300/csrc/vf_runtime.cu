@@ -155,7 +155,7 @@ void Batch::release() {
   for (DevBuf* b : {&grid0, &grid1, &keys, &par, &tets, &range, &ys, &seeds, &counts, &lat,
                     &verts, &faces, &emask, &etab, &tables, &state, &brick_job, &live, &list, &lcount,
                     &scal, &uf, &wst, &win, &wzero, &wsched, &front[0], &front[1], &pcnt, &pbase,
-                    &psums, &srec, &stage_out, &rle_cnt, &rle_base, &rle_sums, &rle_tot, &rle_starts,
+                    &psums, &stage_out, &rle_cnt, &rle_base, &rle_sums, &rle_tot, &rle_starts,
                     &rle_rec})
     ctx->free_buf(*b);
   if (h_tables) cudaFreeHost(h_tables);
@@ -472,7 +472,6 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
   ALLOC(pcnt, nf * 4);
   ALLOC(pbase, nf * 8);
   ALLOC(psums, ((nf + 1023) / 1024 + 1) * 8);
-  ALLOC(srec, nf * 96);
   if (sz.out) ALLOC(stage_out, sz.out * 2);
 #undef ALLOC
     return VF_OK;
@@ -723,7 +722,6 @@ static void voxelize_stages(Batch& B, const std::function<void(int)>& mark) {
   fsc.pbase = static_cast<unsigned long long*>(B.pbase.p);
   fsc.psums = static_cast<unsigned long long*>(B.psums.p);
   fsc.ptotal = static_cast<unsigned long long*>(B.scal.p) + 256;  // bytes 2048..2055
-  fsc.srec = static_cast<float4*>(B.srec.p);
   vfk::centroid_and_slices(st, tv, ds, n);
   vfk::tetra_prep(st, tv, ds, n, B.sz.faces_total, fsc);
   mark(2);

@@ -67,7 +67,7 @@ struct Batch {
   DevBuf tables, state, brick_job, live, list, lcount, scal, front[2];
   DevBuf uf;         // union-find over the seed slots of jobs with sub-seed prefixes
   DevBuf wst, win, wzero, wsched;  // flood: row states; what reaches their ends; candidates + barriers; wave jobs + gangs
-  DevBuf pcnt, pbase, psums, srec;  // flattened per-face work lists, shell setup
+  DevBuf pcnt, pbase, psums;  // flattened per-face work lists
   DevBuf stage_out;  // packed labels of the DMA download
   // the plain path floods on u32 keys, the batched one on row states
   bool plain = false;

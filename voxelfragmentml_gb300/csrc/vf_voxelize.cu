@@ -17,9 +17,10 @@
 //                         used an odd number of times, then a prefix XOR
 //                         along x turns the per-row crossing markers into the
 //                         parity plane
-//   shell_sat           : per-face work items (columns of the triangle's
-//                         footprint) flattened by a prefix sum; warps test
-//                         runs of items with the exact SAT
+//   shell_sat           : columns of each triangle's footprint in even units
+//                         (prefix sum over groups of 32 faces); interval forms
+//                         with margins decide nearly all cells, the exact SAT
+//                         the rest
 //   combine             : one CTA per brick; bit planes -> uint16 0/1 rows,
 //                         brick liveness
 // All float arithmetic uses the _rn intrinsics (and the file is compiled
@@ -463,23 +464,8 @@ __device__ __forceinline__ void mm3(float a, float b, float c, float& mn, float&
   if (c < mn) mn = c;
   if (c > mx) mx = c;
 }
-// The SAT as a conjunction of tests, each evaluated exactly as
-// Intersections3D.h:204-258 does; MASK selects which run (a separating axis
-// makes the result false whatever the order).  Bits 0-8: the edge-cross-axis
-// tests (edge e0: x01 y02 z12; e1: x01 y02 z0; e2: x2 y1 z12), bits 9-11: the
-// box axes x, y, z, bit 12: the plane-box test.
-constexpr uint32_t SAT_ALL = 0x1FFFu;
-// tests that use only the two axes other than C: the same for every cell of
-// a column along C (the x-axis family uses y, z; the box axes other than C)
-__host__ __device__ constexpr uint32_t sat_column_mask(int C) {
-  return C == 0 ? ((1u << 0) | (1u << 3) | (1u << 6) | (1u << 10) | (1u << 11))
-       : C == 1 ? ((1u << 1) | (1u << 4) | (1u << 7) | (1u << 9) | (1u << 11))
-                : ((1u << 2) | (1u << 5) | (1u << 8) | (1u << 9) | (1u << 10));
-}
-
-template <uint32_t MASK>
-__device__ __forceinline__ bool tri_box_sel(const tv& p0, const tv& p1, const tv& p2, const tv& c,
-                                            const tv& r) {
+// The SAT, every test evaluated as Intersections3D.h:204-258 does.
+__device__ __forceinline__ bool tri_box(const tv& p0, const tv& p1, const tv& p2, const tv& c, const tv& r) {
   satd d;
   d.r = r;
   d.v0 = {SUB(p0.x, c.x), SUB(p0.y, c.y), SUB(p0.z, c.z)};
@@ -489,31 +475,24 @@ __device__ __forceinline__ bool tri_box_sel(const tv& p0, const tv& p1, const tv
   tv e1 = {SUB(d.v2.x, d.v1.x), SUB(d.v2.y, d.v1.y), SUB(d.v2.z, d.v1.z)};
   tv e2 = {SUB(d.v0.x, d.v2.x), SUB(d.v0.y, d.v2.y), SUB(d.v0.z, d.v2.z)};
   float fx = fabsf(e0.x), fy = fabsf(e0.y), fz = fabsf(e0.z);
-  if ((MASK & (1u << 0)) && !x01(d, e0.z, e0.y, fz, fy)) return false;
-  if ((MASK & (1u << 1)) && !y02(d, e0.z, e0.x, fz, fx)) return false;
-  if ((MASK & (1u << 2)) && !z12(d, e0.y, e0.x, fy, fx)) return false;
+  if (!x01(d, e0.z, e0.y, fz, fy)) return false;
+  if (!y02(d, e0.z, e0.x, fz, fx)) return false;
+  if (!z12(d, e0.y, e0.x, fy, fx)) return false;
   fx = fabsf(e1.x); fy = fabsf(e1.y); fz = fabsf(e1.z);
-  if ((MASK & (1u << 3)) && !x01(d, e1.z, e1.y, fz, fy)) return false;
-  if ((MASK & (1u << 4)) && !y02(d, e1.z, e1.x, fz, fx)) return false;
-  if ((MASK & (1u << 5)) && !z0(d, e1.y, e1.x, fy, fx)) return false;
+  if (!x01(d, e1.z, e1.y, fz, fy)) return false;
+  if (!y02(d, e1.z, e1.x, fz, fx)) return false;
+  if (!z0(d, e1.y, e1.x, fy, fx)) return false;
   fx = fabsf(e2.x); fy = fabsf(e2.y); fz = fabsf(e2.z);
-  if ((MASK & (1u << 6)) && !x2(d, e2.z, e2.y, fz, fy)) return false;
-  if ((MASK & (1u << 7)) && !y1(d, e2.z, e2.x, fz, fx)) return false;
-  if ((MASK & (1u << 8)) && !z12(d, e2.y, e2.x, fy, fx)) return false;
+  if (!x2(d, e2.z, e2.y, fz, fy)) return false;
+  if (!y1(d, e2.z, e2.x, fz, fx)) return false;
+  if (!z12(d, e2.y, e2.x, fy, fx)) return false;
   float mn, mx;
-  if (MASK & (1u << 9)) {
-    mm3(d.v0.x, d.v1.x, d.v2.x, mn, mx);
-    if (mn > d.r.x || mx < -d.r.x) return false;
-  }
-  if (MASK & (1u << 10)) {
-    mm3(d.v0.y, d.v1.y, d.v2.y, mn, mx);
-    if (mn > d.r.y || mx < -d.r.y) return false;
-  }
-  if (MASK & (1u << 11)) {
-    mm3(d.v0.z, d.v1.z, d.v2.z, mn, mx);
-    if (mn > d.r.z || mx < -d.r.z) return false;
-  }
-  if (!(MASK & (1u << 12))) return true;
+  mm3(d.v0.x, d.v1.x, d.v2.x, mn, mx);
+  if (mn > d.r.x || mx < -d.r.x) return false;
+  mm3(d.v0.y, d.v1.y, d.v2.y, mn, mx);
+  if (mn > d.r.y || mx < -d.r.y) return false;
+  mm3(d.v0.z, d.v1.z, d.v2.z, mn, mx);
+  if (mn > d.r.z || mx < -d.r.z) return false;
   tv n = {SUB(MUL(e0.y, e1.z), MUL(e1.y, e0.z)), SUB(MUL(e0.z, e1.x), MUL(e1.z, e0.x)),
           SUB(MUL(e0.x, e1.y), MUL(e1.x, e0.y))};
   // planeBoxOverlap
@@ -546,64 +525,53 @@ __device__ __forceinline__ int float_cell(float f, int n) {
   return vf_clampi((int)floorf(f), -2, n + 1);
 }
 
-// the exact test of one voxel (reference operation order) and the mark.
-// column_done: the column tests of axis c already passed for this cell's
-// column, so only the rest of the SAT runs; c < 0: the whole SAT
-__device__ __forceinline__ void test_cell(const JobDesc& J, const float* cs, const tv& p0,
-                                          const tv& p1, const tv& p2, int i, int jj, int k, int c) {
-  tv ce, r;
-  cell_box(J, cs, i, jj, k, ce, r);
-  bool hit;
-  if (c == 0) hit = tri_box_sel<SAT_ALL ^ sat_column_mask(0)>(p0, p1, p2, ce, r);
-  else if (c == 1) hit = tri_box_sel<SAT_ALL ^ sat_column_mask(1)>(p0, p1, p2, ce, r);
-  else if (c == 2) hit = tri_box_sel<SAT_ALL ^ sat_column_mask(2)>(p0, p1, p2, ce, r);
-  else hit = tri_box_sel<SAT_ALL>(p0, p1, p2, ce, r);
-  if (hit) atomicOr(J.shell + ((size_t)i * J.Y + jj) * J.Zw + (k >> 5), 1u << (k & 31));
-}
-
-// Per-face setup of the shell test.  Candidates: the cells touching the
-// triangle's bounding box (widened by 0.01 cell + 256 ulp of the largest
-// coordinate: any cell further out fails the exact box-axis tests), as
-// columns along the dominant normal axis c.  Per
-// column, (1) the SAT tests that do not involve axis c (the c-family edge
-// axes and the two other box axes) run exactly, once: they are the same for
-// every cell of the column, and a column they reject holds no hit; (2) the
-// plane slab along c bounds the cells, with a margin (2% of a cell + 64 ulp
-// of the largest coordinate) far beyond the rounding of the float SAT, so no
-// cell the exact test accepts is dropped.  Each remaining cell then runs the
-// rest of the SAT.  The marked set equals testing the full bbox.
-// Work items: columns (a, b) when pruning, else every bbox cell (whole SAT).
-struct ShellSetup {
-  float cs[3];                 // cell size (x, y, z)
-  tv p0, p1, p2;               // the triangle
-  // pruning, in the axes (a, b, c) = (c+1, c+2, c) mod 3; without pruning
-  // (a, b, c) = (x, y, z) and every bbox cell is an item
-  float amin_a, amin_b, amin_c, cs_a, cs_b, q0_a, q0_b, q0_c, nr_a, nr_b;
-  float Pa1, Pb1, Pa2, Pb2;    // projected triangle relative to p0 (ccw)
-  float ha, hb, w, inr, ics;
-  int lo_a, lo_b, lo_c, n_b, n_c, hi_c;
-  int c;
-  bool prune;
+// The shell marks every cell whose box the float SAT above accepts.  The SAT
+// itself runs for few cells: with the face's column axis c (the axis of its
+// largest normal component) and a column of cells (a, b), each of its 13 tests
+// is, in exact arithmetic, either the same for the whole column or an interval
+// of positions along c.  Per face the tests are written as linear forms in cell
+// units relative to the face's first vertex; per column their intervals are
+// intersected twice, once widened and once narrowed by a margin m above the
+// rounding of the float SAT and of the forms:
+//   outside the wide one    no float test can accept: no hit
+//   inside the narrow one   no float test can reject: a hit, marked at once
+//   in between              the SAT decides
+// With M the largest coordinate in play and eps = 2^-24 M, the SAT's box centres,
+// half sizes and vertex offsets carry at most 10 eps, its edges 6 eps, so a test
+// on an edge (e, f) with offsets up to D carries at most
+// (24 (|e| + |f|) + 12 D + 6 cells) eps, and its form here (13 (|e| + |f|) + 6 D)
+// eps; the margin is 48 (|e| + |f| + D) eps, and likewise for the plane.
+// Coordinates far from the origin only widen it: then the SAT decides more cells.
+// Work items are columns; faces whose normal has no clear axis (slivers) leave
+// every cell of their box, in columns along z, to the SAT.
+struct ShellBox {
+  int lo[3], n[3];  // cells touching the triangle's box along x, y, z
+  float M;          // largest coordinate in play
+  int c;            // column axis
+  bool prune;       // by columns
   uint32_t items;
 };
 
-__device__ bool shell_setup(const JobDesc& J, uint32_t f, ShellSetup& S) {
-  const uint32_t dims[3] = {J.X, J.Y, J.Z};
-  for (int a = 0; a < 3; ++a) S.cs[a] = J.cs[a];
+template <class T>
+__device__ __forceinline__ T sel3(const T* v, int i) {  // a register select
+  return i == 0 ? v[0] : (i == 1 ? v[1] : v[2]);
+}
+
+__device__ bool shell_box(const JobDesc& J, uint32_t f, float q0[3], float q1[3], float q2[3], ShellBox& S) {
+  const int dims[3] = {(int)J.X, (int)J.Y, (int)J.Z};
   const uint32_t* fi = J.faces + 3 * (size_t)f;
-  if (fi[0] >= J.nverts || fi[1] >= J.nverts || fi[2] >= J.nverts) return false;
-  const float* q0 = J.verts + 3 * (size_t)fi[0];
-  const float* q1 = J.verts + 3 * (size_t)fi[1];
-  const float* q2 = J.verts + 3 * (size_t)fi[2];
-  // The largest coordinate in play sets the rounding scale of the float SAT
-  // (box bounds, centres, vertex offsets): its errors are a few ulp of M.
-  float M = 0.0f;
+  const uint32_t i0 = fi[0], i1 = fi[1], i2 = fi[2];
+  if (i0 >= J.nverts || i1 >= J.nverts || i2 >= J.nverts) return false;
+  S.M = 0.0f;
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
-    M = fmaxf(M, fmaxf(fabsf(J.amin[a]), fabsf(J.amax[a])));
-    M = fmaxf(M, fmaxf(fabsf(q0[a]), fmaxf(fabsf(q1[a]), fabsf(q2[a]))));
+    q0[a] = J.verts[3 * (size_t)i0 + a];
+    q1[a] = J.verts[3 * (size_t)i1 + a];
+    q2[a] = J.verts[3 * (size_t)i2 + a];
+    S.M = fmaxf(S.M, fmaxf(fabsf(J.amin[a]), fabsf(J.amax[a])));
+    S.M = fmaxf(S.M, fmaxf(fabsf(q0[a]), fmaxf(fabsf(q1[a]), fabsf(q2[a]))));
   }
-  const float ulp64 = M * 7.62939453125e-6f;  // 64 * 2^-23 * M
-  int lo[3], n[3];
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
     float mn, mx;
     mm3(q0[a], q1[a], q2[a], mn, mx);
@@ -611,242 +579,340 @@ __device__ bool shell_setup(const JobDesc& J, uint32_t f, ShellSetup& S) {
     // 256 ulp of M: a cell further out fails the exact SAT's box-axis test,
     // whose roundings are a few ulp of M; the 0.01 cell covers the rounding
     // of these index computations (below 2^-11 cell for 4096 cells).
-    const float mc = 0.01f + 4.0f * ulp64 * J.ics[a];
-    lo[a] = vf_clampi(float_cell(SUB(mn, J.amin[a]) * J.ics[a] - mc, dims[a]), 0, dims[a] - 1);
+    const float mc = 0.01f + 4.0f * (S.M * 7.62939453125e-6f) * J.ics[a];
+    S.lo[a] = vf_clampi(float_cell(SUB(mn, J.amin[a]) * J.ics[a] - mc, dims[a]), 0, dims[a] - 1);
     const int hi = vf_clampi(float_cell(SUB(mx, J.amin[a]) * J.ics[a] + mc, dims[a]), 0, dims[a] - 1);
-    n[a] = hi - lo[a] + 1;
+    S.n[a] = hi - S.lo[a] + 1;
   }
-  S.p0 = {q0[0], q0[1], q0[2]};
-  S.p1 = {q1[0], q1[1], q1[2]};
-  S.p2 = {q2[0], q2[1], q2[2]};
   const float e1[3] = {q1[0] - q0[0], q1[1] - q0[1], q1[2] - q0[2]};
   const float e2[3] = {q2[0] - q0[0], q2[1] - q0[1], q2[2] - q0[2]};
-  const float nr[3] = {e1[1] * e2[2] - e1[2] * e2[1], e1[2] * e2[0] - e1[0] * e2[2],
-                       e1[0] * e2[1] - e1[1] * e2[0]};
-  int c = fabsf(nr[1]) > fabsf(nr[0]) ? 1 : 0;
-  if (fabsf(nr[2]) > fabsf(c ? nr[1] : nr[0])) c = 2;
+  const float nr[3] = {fabsf(e1[1] * e2[2] - e1[2] * e2[1]), fabsf(e1[2] * e2[0] - e1[0] * e2[2]),
+                       fabsf(e1[0] * e2[1] - e1[1] * e2[0])};
+  int c = nr[1] > nr[0] ? 1 : 0;
+  if (nr[2] > (c ? nr[1] : nr[0])) c = 2;
   const float e1n = fabsf(e1[0]) + fabsf(e1[1]) + fabsf(e1[2]);
   const float e2n = fabsf(e2[0]) + fabsf(e2[1]) + fabsf(e2[2]);
-  const float nrc_abs = fabsf(c == 0 ? nr[0] : (c == 1 ? nr[1] : nr[2]));
-  S.prune = nrc_abs > 1e-3f * e1n * e2n && nrc_abs > 0.0f;
-  if (!S.prune) {
-    S.c = 2;
-    S.lo_a = lo[0]; S.lo_b = lo[1]; S.lo_c = lo[2];
-    S.n_b = n[1]; S.n_c = n[2]; S.hi_c = lo[2] + n[2] - 1;
-    S.nr_a = S.nr_b = S.inr = S.Pa1 = S.Pb1 = S.Pa2 = S.Pb2 = S.ha = S.hb = S.w = 0.0f;
-    S.items = (uint32_t)(n[0] * n[1] * n[2]);
-    return true;
-  }
-  const int ax = (c + 1) % 3, bx = (c + 2) % 3;
-  // register selects instead of dynamic indexing (keeps the arrays out of
-  // local memory)
-#define SEL(v, i) ((i) == 0 ? (v)[0] : ((i) == 1 ? (v)[1] : (v)[2]))
-  S.c = c;
-  S.lo_a = SEL(lo, ax); S.lo_b = SEL(lo, bx); S.lo_c = SEL(lo, c);
-  const int n_a = SEL(n, ax);
-  S.n_b = SEL(n, bx); S.n_c = SEL(n, c); S.hi_c = S.lo_c + S.n_c - 1;
-  S.amin_a = SEL(J.amin, ax); S.amin_b = SEL(J.amin, bx); S.amin_c = SEL(J.amin, c);
-  S.cs_a = SEL(S.cs, ax); S.cs_b = SEL(S.cs, bx);
-  const float cs_c = SEL(S.cs, c);
-  S.q0_a = SEL(q0, ax); S.q0_b = SEL(q0, bx); S.q0_c = SEL(q0, c);
-  S.nr_a = SEL(nr, ax); S.nr_b = SEL(nr, bx);
-  const float nr_c = SEL(nr, c);
-  float P1a = SEL(e1, ax), P1b = SEL(e1, bx), P2a = SEL(e2, ax), P2b = SEL(e2, bx);
-#define SEL2(v, i) ((i) == 0 ? (v)[0] : ((i) == 1 ? (v)[1] : (v)[2]))
-#undef SEL
-  if (nr_c < 0.0f) { float t = P1a; P1a = P2a; P2a = t; t = P1b; P1b = P2b; P2b = t; }
-  S.Pa1 = P1a; S.Pb1 = P1b; S.Pa2 = P2a; S.Pb2 = P2b;
-  // half cell + margin.  The margin (2% of a cell + 64 ulp of the largest
-  // coordinate in play) is far above the rounding of the exact float SAT and
-  // of these bounds, so no cell the exact test accepts is dropped.
-  S.ha = 0.52f * S.cs_a + ulp64;
-  S.hb = 0.52f * S.cs_b + ulp64;
-  const float hc = 0.52f * cs_c + ulp64;
-  S.inr = __frcp_rn(nr_c);
-  S.w = hc + (fabsf(S.nr_a) * S.ha + fabsf(S.nr_b) * S.hb) * fabsf(S.inr);
-  S.ics = SEL2(J.ics, c);
-#undef SEL2
-  S.items = (uint32_t)(n_a * S.n_b);
+  const float nrc = sel3(nr, c);
+  S.prune = nrc > 1e-3f * e1n * e2n && nrc > 0.0f;
+  S.c = S.prune ? c : 2;
+  const int ax = c == 2 ? 0 : c + 1, bx = c == 0 ? 2 : c - 1;
+  S.items = S.prune ? (uint32_t)(sel3(S.n, ax) * sel3(S.n, bx)) : (uint32_t)(S.n[0] * S.n[1]);
   return true;
 }
 
-// the candidate cells of work item q: column (ia, ib) along c, cells
-// klo .. klo + n - 1 (n = 0: the column is pruned).  Items of a face without
-// pruning are single cells (ia, ib, klo) = (i, j, k) with c = z.
-__device__ __forceinline__ void shell_column(const ShellSetup& S, uint32_t q, int& ia, int& ib,
-                                             int& klo, int& n) {
-  n = 0;
-  if (!S.prune) {
-    klo = S.lo_c + (int)(q % S.n_c);
-    ib = S.lo_b + (int)((q / S.n_c) % S.n_b);
-    ia = S.lo_a + (int)(q / (S.n_c * S.n_b));
-    n = 1;
-    return;
-  }
-  ia = S.lo_a + (int)(q / S.n_b);
-  ib = S.lo_b + (int)(q % S.n_b);
-  // the SAT tests that do not involve axis c, exactly, once per column: the
-  // box of every cell of the column has the same extent along a and b
-  {
-    const float bmin_a = ADD(S.amin_a, MUL(S.cs_a, (float)ia)), bmax_a = ADD(bmin_a, S.cs_a);
-    const float bmin_b = ADD(S.amin_b, MUL(S.cs_b, (float)ib)), bmax_b = ADD(bmin_b, S.cs_b);
-    const float ce_a = MUL(ADD(bmax_a, bmin_a), 0.5f), ce_b = MUL(ADD(bmax_b, bmin_b), 0.5f);
-    const float r_a = SUB(bmax_a, ce_a), r_b = SUB(bmax_b, ce_b);
-    bool keep;
-    if (S.c == 0) keep = tri_box_sel<sat_column_mask(0)>(S.p0, S.p1, S.p2, tv{0.0f, ce_a, ce_b}, tv{0.0f, r_a, r_b});
-    else if (S.c == 1) keep = tri_box_sel<sat_column_mask(1)>(S.p0, S.p1, S.p2, tv{ce_b, 0.0f, ce_a}, tv{r_b, 0.0f, r_a});
-    else keep = tri_box_sel<sat_column_mask(2)>(S.p0, S.p1, S.p2, tv{ce_a, ce_b, 0.0f}, tv{r_a, r_b, 0.0f});
-    if (!keep) return;
-  }
-  const float ca = (S.amin_a + S.cs_a * ((float)ia + 0.5f)) - S.q0_a;
-  const float cb = (S.amin_b + S.cs_b * ((float)ib + 0.5f)) - S.q0_b;
-  // slab bounds (conservative: the margin is far above these roundings)
-  const float tc = S.q0_c - (S.nr_a * ca + S.nr_b * cb) * S.inr;
-  // cells whose centre is within w of the plane along c
-  klo = max(S.lo_c, (int)ceilf((tc - S.w - S.amin_c) * S.ics - 0.5f));
-  const int khi = min(S.hi_c, (int)floorf((tc + S.w - S.amin_c) * S.ics - 0.5f));
-  n = max(khi - klo + 1, 0);
+// The faces are taken in groups of 32, a lane each; a group's items in even units
+// of at most `run`.  A unit builds the forms of its faces again, so units are
+// long, but no longer than what gives every warp of the GPU a few.
+__host__ __device__ inline uint32_t shell_run(uint32_t groups) {
+  const uint32_t r = groups / 32 & ~31u;
+  return r < 64 ? 64 : (r > 1024 ? 1024 : r);
 }
-
-// Per-face setup packed into 6 float4 (computed once per face here, then
-// read by every lane that takes an item of the face):
-//   (p0.xyz, p1.x) (p1.yz, p2.xy) (p2.z, nr_a, nr_b, 1/nr_c) (Pa1, Pb1, Pa2, Pb2)
-//   (ha, hb, w, job) (c | prune << 2, lo_a | lo_b << 16, lo_c | hi_c << 16, n_b | n_c << 16)
-__global__ void k_shell_count(const JobDesc* jobs, int njobs, uint32_t total, uint32_t* scnt,
-                              float4* srec) {
-  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-    const int j = job_of_face(jobs, njobs, g);
-    const JobDesc& J = jobs[j];
-    ShellSetup S;
-    if (!shell_setup(J, g - J.face_base, S)) {
-      scnt[g] = 0u;
-      continue;
-    }
-    scnt[g] = S.items;
-    float4* r = srec + 6 * (size_t)g;
-    r[0] = make_float4(S.p0.x, S.p0.y, S.p0.z, S.p1.x);
-    r[1] = make_float4(S.p1.y, S.p1.z, S.p2.x, S.p2.y);
-    r[2] = make_float4(S.p2.z, S.nr_a, S.nr_b, S.inr);
-    r[3] = make_float4(S.Pa1, S.Pb1, S.Pa2, S.Pb2);
-    r[4] = make_float4(S.ha, S.hb, S.w, __int_as_float(j));
-    r[5] = make_float4(__int_as_float(S.c | (S.prune ? 4 : 0)), __int_as_float(S.lo_a | (S.lo_b << 16)),
-                       __int_as_float(S.lo_c | (S.hi_c << 16)), __int_as_float(S.n_b | (S.n_c << 16)));
-  }
-}
-
-__device__ __forceinline__ int shell_unpack(const JobDesc* jobs, const float4* rec, ShellSetup& S) {
-  const float4 r0 = rec[0], r1 = rec[1], r2 = rec[2], r3 = rec[3], r4 = rec[4], r5 = rec[5];
-  S.p0 = {r0.x, r0.y, r0.z};
-  S.p1 = {r0.w, r1.x, r1.y};
-  S.p2 = {r1.z, r1.w, r2.x};
-  S.nr_a = r2.y; S.nr_b = r2.z; S.inr = r2.w;
-  S.Pa1 = r3.x; S.Pb1 = r3.y; S.Pa2 = r3.z; S.Pb2 = r3.w;
-  S.ha = r4.x; S.hb = r4.y; S.w = r4.z;
-  const int j = __float_as_int(r4.w);
-  const int cp = __float_as_int(r5.x), lab = __float_as_int(r5.y), lch = __float_as_int(r5.z),
-            nbc = __float_as_int(r5.w);
-  S.c = cp & 3;
-  S.prune = (cp & 4) != 0;
-  S.lo_a = lab & 0xFFFF; S.lo_b = lab >> 16;
-  S.lo_c = lch & 0xFFFF; S.hi_c = lch >> 16;
-  S.n_b = nbc & 0xFFFF; S.n_c = nbc >> 16;
-  const JobDesc& J = jobs[j];
-  const int c = S.c, ax = c == 2 ? 0 : c + 1, bx = c == 0 ? 2 : (c == 1 ? 0 : 1);
-#define SEL(v, i) ((i) == 0 ? (v)[0] : ((i) == 1 ? (v)[1] : (v)[2]))
-  const float p0[3] = {S.p0.x, S.p0.y, S.p0.z};
-  S.cs[0] = J.cs[0]; S.cs[1] = J.cs[1]; S.cs[2] = J.cs[2];
-  S.amin_a = SEL(J.amin, ax); S.amin_b = SEL(J.amin, bx); S.amin_c = SEL(J.amin, c);
-  S.cs_a = SEL(J.cs, ax); S.cs_b = SEL(J.cs, bx);
-  S.ics = SEL(J.ics, c);
-  S.q0_a = SEL(p0, ax); S.q0_b = SEL(p0, bx); S.q0_c = SEL(p0, c);
-#undef SEL
+__device__ __forceinline__ int group_job(const JobDesc* jobs, int njobs, uint32_t g0, uint32_t g) {
+  int j = job_of_face(jobs, njobs, g0);
+  while (j + 1 < njobs && jobs[j + 1].face_base <= g) ++j;
   return j;
 }
+__global__ void __launch_bounds__(256) k_shell_count(const JobDesc* jobs, int njobs, uint32_t total, uint32_t* units) {
+  const uint32_t groups = (total + 31) / 32, run = shell_run(groups), lane = threadIdx.x & 31;
+  for (uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < groups; p += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t g = 32 * p + lane;
+    unsigned long long items = 0;
+    if (g < total) {
+      const JobDesc& J = jobs[group_job(jobs, njobs, 32 * p, g)];
+      ShellBox S;
+      float q0[3], q1[3], q2[3];
+      if (shell_box(J, g - J.face_base, q0, q1, q2, S)) items = S.items;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) items += __shfl_xor_sync(0xFFFFFFFFu, items, o);
+    if (lane == 0) units[p] = (uint32_t)((items + run - 1) / run);
+  }
+}
 
-// Warp-interleaved runs over the (face, column) items.  Each lane prunes its
-// column to a range of candidate cells; the cells of all 32 columns are then
-// dealt out to the lanes, one exact SAT per lane per round, so lanes with
-// pruned or short columns do not idle while others test.
-__global__ void __launch_bounds__(256, 3) k_shell_flat(const JobDesc* jobs, const uint32_t* scnt,
-                                                       const unsigned long long* sbase,
-                                                       const unsigned long long* stotal,
-                                                       uint32_t total_faces, const float4* srec) {
-  const unsigned long long total = *stotal;
+// A face's forms in shared memory, 13 uint4 (an odd number: 8 faces' loads of
+// one uint4 fall on distinct bank groups):
+//   0 first item of the face in the unit, 2^32 / n_b, n_b | n_c << 16, job
+//   1 lo_a | lo_b << 16, lo_c | c << 16, sure cells a, b (lo | end << 16)
+//   2 centre of cell (lo_a, lo_b, lo_c) fa fb fc, sure cells c
+//   3-5 column tests: |x a + y b - z| <= 1, sure below w
+//   6-11 tests along c: centre x v + y, half widths z (wide), w (narrow), v = b
+//        (6-8) or a (9-11)
+//   12 plane: centre x a + y b, half widths z, w
+constexpr int SHELL_REC = 13;
+__device__ __forceinline__ void shell_forms(const JobDesc& J, const ShellBox& S, const float q0[3], const float q1[3],
+                                            const float q2[3], uint32_t first, uint32_t job, uint4* rec) {
+  const int c = S.c, ax = c == 2 ? 0 : c + 1, bx = c == 0 ? 2 : c - 1;
+  const int lo_a = sel3(S.lo, ax), lo_b = sel3(S.lo, bx), lo_c = sel3(S.lo, c);
+  const int n_a = sel3(S.n, ax), n_b = sel3(S.n, bx), n_c = sel3(S.n, c);
+  rec[0] = make_uint4(first, 0xFFFFFFFFu / (uint32_t)n_b, (uint32_t)(n_b | n_c << 16), job);
+  const uint32_t w10 = (uint32_t)(lo_a | lo_b << 16), w11 = (uint32_t)(lo_c | c << 16);
+  rec[1] = make_uint4(w10, w11, 0u, 0u);
+  // cell units: vertices relative to the first
+  float V1[3], V2[3], F[3], mn[3], mx[3], ext = 0.0f, mics = 0.0f;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    V1[a] = (q1[a] - q0[a]) * J.ics[a];
+    V2[a] = (q2[a] - q0[a]) * J.ics[a];
+    F[a] = ((J.amin[a] - q0[a]) + J.cs[a] * ((float)S.lo[a] + 0.5f)) * J.ics[a];
+    mn[a] = fminf(0.0f, fminf(V1[a], V2[a]));
+    mx[a] = fmaxf(0.0f, fmaxf(V1[a], V2[a]));
+    ext = fmaxf(ext, mx[a] - mn[a]);
+    mics = fmaxf(mics, J.ics[a]);
+  }
+  const float V1a = sel3(V1, ax), V1b = sel3(V1, bx), V1c = sel3(V1, c);
+  const float V2a = sel3(V2, ax), V2b = sel3(V2, bx), V2c = sel3(V2, c);
+  const float fa = sel3(F, ax), fb = sel3(F, bx), fc = sel3(F, c);
+  const float u = S.M * mics * 2.86102294921875e-6f;  // 48 * 2^-24
+  const float D = ext + 0.6f + 12.0f * u;             // largest offset of a vertex from a cell of the box
+  const float Na = V1b * V2c - V1c * V2b, Nb = V1c * V2a - V1a * V2c, Nc = V1a * V2b - V1b * V2a;
+  float4* const r4 = reinterpret_cast<float4*>(rec);
+  if (!S.prune || !(u < 1.0f) || !(fabsf(Nc) > 1e-20f)) {
+    // no clear axis, or a margin above a cell: every cell of the box through the SAT
+    r4[2] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int i = 3; i < 6; ++i) r4[i] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+    for (int i = 6; i < 13; ++i) r4[i] = make_float4(0.0f, 0.0f, 1e30f, -1.0f);
+    return;
+  }
+  // sure cells of the box axes, relative to lo: lo | end << 16
+  auto sure = [&](float lo, float hi, float f, int n) {
+    const float m = 0.001f + u;
+    const int k0 = max(0, min(n, __float2int_ru(lo - 0.5f - f + m)));
+    const int k1 = max(k0, min(n - 1, __float2int_rd(hi + 0.5f - f - m)) + 1);
+    return (uint32_t)(k0 | k1 << 16);
+  };
+  rec[1] = make_uint4(w10, w11, sure(sel3(mn, ax), sel3(mx, ax), fa, n_a), sure(sel3(mn, bx), sel3(mx, bx), fb, n_b));
+  rec[2] = make_uint4(__float_as_uint(fa), __float_as_uint(fb), __float_as_uint(fc),
+                      sure(sel3(mn, c), sel3(mx, c), fc, n_c));
+  // edges 0 (V0 -> V1), 1 (V1 -> V2), 2 (V2 -> V0); (on) a vertex of the edge, (off) the third
+  const float Ea[3] = {V1a, V2a - V1a, -V2a}, Eb[3] = {V1b, V2b - V1b, -V2b}, Ec[3] = {V1c, V2c - V1c, -V2c};
+  const float on_a[3] = {0.0f, V2a, 0.0f}, on_b[3] = {0.0f, V2b, 0.0f}, on_c[3] = {0.0f, V2c, 0.0f};
+  const float off_a[3] = {V2a, 0.0f, V1a}, off_b[3] = {V2b, 0.0f, V1b}, off_c[3] = {V2c, 0.0f, V1c};
+#pragma unroll
+  for (int e = 0; e < 3; ++e) {
+    {  // axis e x c: e_a x_b - e_b x_a, the same along the column
+      const float s0 = Ea[e] * on_b[e] - Eb[e] * on_a[e], s1 = Ea[e] * off_b[e] - Eb[e] * off_a[e];
+      const float E = fabsf(Ea[e]) + fabsf(Eb[e]), half = 0.5f * (fabsf(s1 - s0) + E), m = u * (E + D);
+      const float r = __fdividef(1.0f, half + m);
+      r4[3 + e] = make_float4(-Eb[e] * r, Ea[e] * r, 0.5f * (s0 + s1) * r, (half - m) * r);
+    }
+    {  // axis e x a: e_c x_b - e_b x_c; a slope divisor below u is taken as u (the second D covers it)
+      const float s0 = Ec[e] * on_b[e] - Eb[e] * on_c[e], s1 = Ec[e] * off_b[e] - Eb[e] * off_c[e];
+      const float E = fabsf(Ec[e]) + fabsf(Eb[e]), half = 0.5f * (fabsf(s1 - s0) + E), m = u * (E + 2.0f * D);
+      const float ir = __fdividef(1.0f, fmaxf(fabsf(Eb[e]), u)), r = copysignf(ir, Eb[e]);
+      r4[6 + e] = make_float4(Ec[e] * r, -0.5f * (s0 + s1) * r, (half + m) * ir, (half - m) * ir);
+    }
+    {  // axis e x b: e_c x_a - e_a x_c
+      const float s0 = Ec[e] * on_a[e] - Ea[e] * on_c[e], s1 = Ec[e] * off_a[e] - Ea[e] * off_c[e];
+      const float E = fabsf(Ec[e]) + fabsf(Ea[e]), half = 0.5f * (fabsf(s1 - s0) + E), m = u * (E + 2.0f * D);
+      const float ir = __fdividef(1.0f, fmaxf(fabsf(Ea[e]), u)), r = copysignf(ir, Ea[e]);
+      r4[9 + e] = make_float4(Ec[e] * r, -0.5f * (s0 + s1) * r, (half + m) * ir, (half - m) * ir);
+    }
+  }
+  const float En = fabsf(V1a) + fabsf(V1b) + fabsf(V1c) + fabsf(V2a) + fabsf(V2b) + fabsf(V2c);
+  const float Nn = fabsf(Na) + fabsf(Nb) + fabsf(Nc), in = 1.0f / Nc;
+  const float m = u * (2.0f * En * D + Nn);
+  r4[12] = make_float4(-Na * in, -Nb * in, (0.5f * Nn + m) * fabsf(in), (0.5f * Nn - m) * fabsf(in));
+}
+
+__device__ __forceinline__ void red_or(uint32_t* p, uint32_t v) {
+  asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// the SAT of one queued cell (face, job, x | y << 16, z) and the mark
+__device__ __forceinline__ void shell_cell(const JobDesc* jobs, const uint4& e) {
+  const JobDesc& J = jobs[e.y];
+  const uint32_t* fi = J.faces + 3 * (size_t)(e.x - J.face_base);
+  const float* p0 = J.verts + 3 * (size_t)fi[0];
+  const float* p1 = J.verts + 3 * (size_t)fi[1];
+  const float* p2 = J.verts + 3 * (size_t)fi[2];
+  const int x = e.z & 0xFFFF, y = e.z >> 16, z = e.w;
+  tv ce, r;
+  cell_box(J, J.cs, x, y, z, ce, r);
+  if (tri_box({p0[0], p0[1], p0[2]}, {p1[0], p1[1], p1[2]}, {p2[0], p2[1], p2[2]}, ce, r))
+    red_or(J.shell + ((size_t)x * J.Y + y) * J.Zw + (z >> 5), 1u << (z & 31));
+}
+
+// A warp per unit: a lane builds a face's forms in shared memory, then the lanes
+// take the columns of the unit's faces.  Cells the forms leave open go to the
+// warp's queue, and through the SAT 32 at a time.
+// Bound by instruction issue (69% of cycles; 0.5 cells a face go to the SAT): 128
+// meshes, 6.4 M faces of 8 to 19 columns, 1575 us, and 48 of them 494 us, against
+// 3396 and 1104 us with the SAT's column tests and then the SAT for every cell.
+constexpr int SHELL_WARPS = 8;
+struct ShellWarp {
+  uint4 rec[32 * SHELL_REC];
+  uint4 queue[64];     // cells for the SAT
+  uint32_t cols[64];   // columns kept: face of the group | da << 5 | db << 18 | sure << 31
+  uint32_t start[36];  // first item of each face in the unit, and the end
+};
+__global__ void __launch_bounds__(SHELL_WARPS * 32, 3)
+    k_shell_flat(const JobDesc* jobs, int njobs, const unsigned long long* ubase, const unsigned long long* utotal,
+                 uint32_t total_faces) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ShellWarp& W = reinterpret_cast<ShellWarp*>(smem_raw)[threadIdx.x >> 5];
+  const unsigned long long total = *utotal;
   const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-  const uint32_t run = warp_run(total, nwarps);
-  const unsigned long long nwruns = (total + run - 1) / run;
-  for (unsigned long long wr = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
-       wr < nwruns; wr += nwarps) {
-    const unsigned long long base = wr * run;
-    const unsigned long long end = min(base + run, total);
-    uint32_t g = 0;
-    if (lane == 0) g = face_of_item(sbase, total_faces, base);
-    g = __shfl_sync(0xFFFFFFFFu, g, 0);
-    uint32_t cached = 0xFFFFFFFFu;
-    ShellSetup S;
-    S.c = 2;
-    S.p0 = S.p1 = S.p2 = {0.0f, 0.0f, 0.0f};
-    S.cs[0] = S.cs[1] = S.cs[2] = 0.0f;
-    int jidx = 0;
-    unsigned long long fb = 0;
-    for (unsigned long long p0 = base; p0 < end; p0 += 32) {
-      const unsigned long long p = p0 + lane;
-      int ia = 0, ib = 0, klo = 0, n = 0;
-      if (p < end) {
-        while (p >= sbase[g] + scnt[g]) ++g;
-        if (g != cached) {
-          cached = g;
-          jidx = shell_unpack(jobs, srec + 6 * (size_t)g, S);
-          fb = sbase[g];
-        }
-        shell_column(S, (uint32_t)(p - fb), ia, ib, klo, n);
-      }
-      // exclusive scan of the lanes' cell counts
-      int incl = n;
+  const uint32_t groups = (total_faces + 31) / 32, run = shell_run(groups);
+  uint32_t queued = 0;  // the same in all lanes, below 32 between rounds
+  for (unsigned long long unit = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5; unit < total;
+       unit += nwarps) {
+    uint32_t p = 0;
+    if (lane == 0) p = face_of_item(ubase, groups, unit);
+    p = __shfl_sync(0xFFFFFFFFu, p, 0);
+    const unsigned long long ub = ubase[p], units = (p + 1 < groups ? ubase[p + 1] : total) - ub;
+    const uint32_t g0 = 32 * p, g = g0 + lane;
+    {
+      const int j = g < total_faces ? group_job(jobs, njobs, g0, g) : 0;
+      ShellBox S;
+      float q0[3], q1[3], q2[3];
+      const bool ok = g < total_faces && shell_box(jobs[j], g - jobs[j].face_base, q0, q1, q2, S);
+      const unsigned long long items = ok ? S.items : 0u;
+      unsigned long long upto = items;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += t;
+        const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, upto, o);
+        if (lane >= o) upto += t;
       }
-      const int ncells = __shfl_sync(0xFFFFFFFFu, incl, 31);
-      const int excl = incl - n;
-      for (int t0 = 0; t0 < ncells; t0 += 32) {
-        const int t = t0 + lane;
-        // owner: the last lane whose first cell is <= t
-        int src = 0;
+      const unsigned long long first = upto - items;
+      // the unit's share of the group's items
+      const unsigned long long all = __shfl_sync(0xFFFFFFFFu, upto, 31);
+      const uint32_t share = units == 1 ? run : (uint32_t)((all + units - 1) / units);
+      const unsigned long long from = (unit - ub) * share;
+      auto clip = [&](unsigned long long i) { return (uint32_t)min((unsigned long long)share, i > from ? i - from : 0ull); };
+      const uint32_t s0 = clip(first), s1 = clip(upto);
+      __syncwarp();  // the previous unit's forms are read
+      W.start[lane] = s0;
+      if (lane == 31) W.start[32] = s1;
+      if (s0 < s1) shell_forms(jobs[j], S, q0, q1, q2, (uint32_t)(first - from), (uint32_t)j, W.rec + lane * SHELL_REC);
+      __syncwarp();
+    }
+    // Columns (slot, da, db) the tests across the face keep are collected, then
+    // taken 32 at a time.
+    const uint32_t stop = W.start[32];
+    uint32_t slot = 0, ncols = 0;
+    for (uint32_t i0 = 0; i0 < stop || ncols; i0 += 32) {
+      const uint32_t i = i0 + lane;
+      bool keep = false;
+      uint32_t col = 0;
+      if (i < stop) {
+        while (i >= W.start[slot + 1]) ++slot;
+        const uint4* rec = W.rec + slot * SHELL_REC;
+        const float4* r4 = reinterpret_cast<const float4*>(rec);
+        const uint4 h0 = rec[0], h1 = rec[1];
+        const uint32_t q = i - h0.x, n_b = h0.z & 0xFFFFu;
+        uint32_t da = __umulhi(q, h0.y), db = q - da * n_b;
+        if (db >= n_b) { ++da; db -= n_b; }  // the rounded-down reciprocal is at most 1 short
+        const float4 h2 = r4[2];
+        const float xa = (float)da + h2.x, xb = (float)db + h2.y;
+        uint32_t sure = da >= (h1.z & 0xFFFFu) && da < (h1.z >> 16) && db >= (h1.w & 0xFFFFu) && db < (h1.w >> 16);
+        keep = true;
 #pragma unroll
-        for (int step = 16; step >= 1; step >>= 1) {
-          const int e = __shfl_sync(0xFFFFFFFFu, excl, src + step);
-          if (e <= t) src += step;
+        for (int e = 0; e < 3; ++e) {
+          const float4 t = r4[3 + e];
+          const float d = fabsf(fmaf(t.x, xa, fmaf(t.y, xb, -t.z)));
+          keep &= !(d > 1.0f);
+          sure &= d < t.w;
         }
-        const tv q0 = {__shfl_sync(0xFFFFFFFFu, S.p0.x, src), __shfl_sync(0xFFFFFFFFu, S.p0.y, src),
-                       __shfl_sync(0xFFFFFFFFu, S.p0.z, src)};
-        const tv q1 = {__shfl_sync(0xFFFFFFFFu, S.p1.x, src), __shfl_sync(0xFFFFFFFFu, S.p1.y, src),
-                       __shfl_sync(0xFFFFFFFFu, S.p1.z, src)};
-        const tv q2 = {__shfl_sync(0xFFFFFFFFu, S.p2.x, src), __shfl_sync(0xFFFFFFFFu, S.p2.y, src),
-                       __shfl_sync(0xFFFFFFFFu, S.p2.z, src)};
-        const float cs[3] = {__shfl_sync(0xFFFFFFFFu, S.cs[0], src),
-                             __shfl_sync(0xFFFFFFFFu, S.cs[1], src),
-                             __shfl_sync(0xFFFFFFFFu, S.cs[2], src)};
-        const int sj = __shfl_sync(0xFFFFFFFFu, jidx, src);
-        // test mode: the face's axis c (column tests already passed) or -1
-        // (faces without pruning: every item is one cell, whole SAT)
-        const int mode = __shfl_sync(0xFFFFFFFFu, S.prune ? S.c : -1, src);
-        const int sc = mode < 0 ? 2 : mode;
-        const int sa = __shfl_sync(0xFFFFFFFFu, ia, src);
-        const int sb = __shfl_sync(0xFFFFFFFFu, ib, src);
-        const int sk = __shfl_sync(0xFFFFFFFFu, klo, src) + t - __shfl_sync(0xFFFFFFFFu, excl, src);
-        if (t < ncells) {
-          // (a, b, c) -> (x, y, z): c = 0: (k, a, b); c = 1: (b, k, a); c = 2: (a, b, k)
-          const int x = sc == 0 ? sk : (sc == 1 ? sb : sa);
-          const int y = sc == 0 ? sa : (sc == 1 ? sk : sb);
-          const int z = sc == 0 ? sb : (sc == 1 ? sa : sk);
-          test_cell(jobs[sj], cs, q0, q1, q2, x, y, z, mode);
+        col = slot | da << 5 | db << 18 | sure << 31;
+      }
+      const unsigned mk = __ballot_sync(0xFFFFFFFFu, keep);
+      if (keep) W.cols[ncols + __popc(mk & lt)] = col;
+      ncols += __popc(mk);
+      if (ncols < 32 && i0 + 32 < stop) continue;
+      __syncwarp();
+      uint32_t face = 0, job = 0;
+      int c = 2, ia = 0, ib = 0;  // the column, and cells open to the SAT:
+      int k0 = 0, n0 = 0, k1 = 0, n1 = 0;
+      if (lane < (int)ncols) {
+        const uint32_t e = W.cols[lane], da = (e >> 5) & 0x1FFFu, db = (e >> 18) & 0x1FFFu;
+        const uint4* rec = W.rec + (e & 31u) * SHELL_REC;
+        const float4* r4 = reinterpret_cast<const float4*>(rec);
+        const uint4 h0 = rec[0], h1 = rec[1];
+        const float4 h2 = r4[2];
+        face = g0 + (e & 31u);
+        job = h0.w;
+        const int lo_c = h1.y & 0xFFFF, n_c = (int)(h0.z >> 16);
+        c = (h1.y >> 16) & 3;
+        ia = (int)((h1.x & 0xFFFFu) + da);
+        ib = (int)((h1.x >> 16) + db);
+        const float xa = (float)da + h2.x, xb = (float)db + h2.y;
+        float wlo = -1e30f, whi = 1e30f, nlo = -1e30f, nhi = 1e30f;
+        auto along = [&](float at, float w, float n) {
+          wlo = fmaxf(wlo, at - w); whi = fminf(whi, at + w);
+          nlo = fmaxf(nlo, at - n); nhi = fminf(nhi, at + n);
+        };
+#pragma unroll
+        for (int t3 = 0; t3 < 3; ++t3) {
+          const float4 t = r4[6 + t3];
+          along(fmaf(t.x, xb, t.y), t.z, t.w);
+        }
+#pragma unroll
+        for (int t3 = 0; t3 < 3; ++t3) {
+          const float4 t = r4[9 + t3];
+          along(fmaf(t.x, xa, t.y), t.z, t.w);
+        }
+        const float4 t = r4[12];
+        along(fmaf(t.x, xa, t.y * xb), t.z, t.w);
+        // cells relative to lo_c; 0.001 covers the rounding of these sums
+        const uint32_t kc = __float_as_uint(h2.w);
+        const int a0 = max(0, __float2int_ru(wlo - h2.z - 0.001f));
+        const int a1 = min(n_c - 1, __float2int_rd(whi - h2.z + 0.001f)) + 1;
+        int b0 = max(max((int)(kc & 0xFFFFu), a0), __float2int_ru(nlo - h2.z + 0.001f));
+        int b1 = min(min((int)(kc >> 16), a1) - 1, __float2int_rd(nhi - h2.z - 0.001f)) + 1;
+        if (!(e >> 31) || b1 <= b0) b0 = b1 = max(a0, a1);
+        // [a0, b0) open, [b0, b1) hits, [b1, a1) open
+        k0 = lo_c + a0; n0 = max(b0 - a0, 0);
+        k1 = lo_c + b1; n1 = max(a1 - b1, 0);
+        if (b1 > b0) {
+          const JobDesc& J = jobs[job];
+          int k = lo_c + b0;
+          const int ke = lo_c + b1;
+          if (c == 2) {
+            uint32_t* row = J.shell + ((size_t)ia * J.Y + ib) * J.Zw;
+            while (k < ke) {
+              const int w = k >> 5, stop_k = min(ke, (w + 1) << 5);
+              red_or(row + w, (0xFFFFFFFFu << (k & 31)) & (0xFFFFFFFFu >> (31 - ((stop_k - 1) & 31))));
+              k = stop_k;
+            }
+          } else {
+            // c = 0: (x, y, z) = (k, a, b); c = 1: (b, k, a)
+            const int z = c == 0 ? ib : ia;
+            const size_t row = c == 0 ? (size_t)k * J.Y + ia : (size_t)ib * J.Y + k;
+            const size_t step = c == 0 ? (size_t)J.Y * J.Zw : J.Zw;
+            uint32_t* w = J.shell + row * J.Zw + (z >> 5);
+            for (; k < ke; ++k, w += step) red_or(w, 1u << (z & 31));
+          }
+        }
+      }
+      const uint32_t done = min(ncols, 32u);
+      ncols -= done;
+      const uint32_t left = W.cols[32 + lane];
+      __syncwarp();
+      if (lane < (int)ncols) W.cols[lane] = left;
+      for (unsigned m; (m = __ballot_sync(0xFFFFFFFFu, n0 + n1 > 0)) != 0;) {
+        if (n0 + n1 > 0) {
+          const int k = n0 > 0 ? k0 : k1;
+          if (n0 > 0) { ++k0; --n0; } else { ++k1; --n1; }
+          const int x = c == 0 ? k : (c == 1 ? ib : ia), y = c == 0 ? ia : (c == 1 ? k : ib),
+                    z = c == 0 ? ib : (c == 1 ? ia : k);
+          W.queue[queued + __popc(m & lt)] = make_uint4(face, job, (uint32_t)(x | y << 16), (uint32_t)z);
+        }
+        queued += __popc(m);
+        if (queued >= 32) {
+          __syncwarp();
+          shell_cell(jobs, W.queue[lane]);
+          queued -= 32;
+          const uint4 rest = W.queue[32 + lane];
+          __syncwarp();
+          if (lane < (int)queued) W.queue[lane] = rest;
         }
       }
     }
   }
+  __syncwarp();
+  if (lane < (int)queued) shell_cell(jobs, W.queue[lane]);
 }
 #undef MUL
 #undef ADD
@@ -1013,13 +1079,16 @@ void exclusive_scan(cudaStream_t st, const uint32_t* in, unsigned long long* out
 void shell_sat(cudaStream_t st, const JobDesc* dj, int njobs, uint32_t total_faces,
                const FaceScratch& fs, int num_sms, int grid_mult) {
   if (!total_faces) return;
-  const uint32_t nb = (total_faces + 1023) / 1024;
-  k_shell_count<<<grid_for(total_faces, 256, 65535), 256, 0, st>>>(dj, njobs, total_faces, fs.pcnt,
-                                                                   fs.srec);
-  k_scan_local<<<nb, 1024, 0, st>>>(fs.pcnt, fs.pbase, fs.psums, total_faces);
-  k_scan_sums<<<1, 1024, 0, st>>>(fs.psums, nb, fs.ptotal);
-  k_scan_add<<<(total_faces + 255) / 256, 256, 0, st>>>(fs.pbase, fs.psums, total_faces);
-  k_shell_flat<<<num_sms * grid_mult, 256, 0, st>>>(dj, fs.pcnt, fs.pbase, fs.ptotal, total_faces, fs.srec);
+  k_shell_count<<<grid_for(total_faces, 256, 65535), 256, 0, st>>>(dj, njobs, total_faces, fs.pcnt);
+  exclusive_scan(st, fs.pcnt, fs.pbase, fs.psums, (total_faces + 31) / 32, fs.ptotal);
+  constexpr int bytes = SHELL_WARPS * sizeof(ShellWarp);
+  static bool attr[64] = {};  // per device
+  const int dv = cur_dev();
+  if (!attr[dv]) {
+    cudaFuncSetAttribute(k_shell_flat, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    attr[dv] = true;
+  }
+  k_shell_flat<<<num_sms * grid_mult, SHELL_WARPS * 32, bytes, st>>>(dj, njobs, fs.pbase, fs.ptotal, total_faces);
 }
 void combine(cudaStream_t st, const JobDesc* dj, const uint32_t* brick_job,
              uint32_t total_bricks, uint8_t* live, int dual) {

@@ -902,27 +902,40 @@ static vfk::ImpactGrid impact_grid(const vf_grid* g) {
 vf_status vf_ray_entry_voxels(vf_grid* g, const float* rays, uint32_t n, uint32_t* out) {
   if (!g || (n && (!rays || !out))) return fail(VF_ERR_INVALID, "NULL argument");
   if (!n) return VF_OK;
-  for (uint32_t r = 0; r < n; ++r)
-    if (rays[6 * r + 3] == 0.0f && rays[6 * r + 4] == 0.0f && rays[6 * r + 5] == 0.0f)
-      return fail(VF_ERR_INVALID, "ray " + std::to_string(r) + " has a zero direction");
+  // batches of rays walk a packed occupancy bitmap (built once per call), and
+  // the kernel looks for zero directions (a host loop over 2^20 rays takes 0.8 ms);
+  // a few rays read the labels directly
+  const bool many = n >= 4096 && n <= 1u << 31;
+  auto zero_direction = [](uint32_t r) {
+    return fail(VF_ERR_INVALID, "ray " + std::to_string(r) + " has a zero direction");
+  };
+  for (uint32_t r = 0; r < n && !many; ++r)
+    if (rays[6 * r + 3] == 0.0f && rays[6 * r + 4] == 0.0f && rays[6 * r + 5] == 0.0f) return zero_direction(r);
   cudaSetDevice(g->ctx->c.device);
   vfr::Ctx& c = g->ctx->c;
   ImpactState& I = g->impact;
   vf_status s;
   if ((s = c.alloc(I.rays, (size_t)n * 24)) || (s = c.alloc(I.hits, (size_t)n * 12))) return s;
-  // batches of rays walk a packed occupancy bitmap (built once per call);
-  // a few rays read the labels directly
   const vfr::JobPlan& p = g->b.plans[0];
-  const size_t bitbytes = (size_t)p.X * p.Y * ((p.Z + 31) / 32) * 4;
+  const vfk::RayCells cells = vfk::ray_cells(p.X, p.Y, p.Z);
+  const size_t bitwords = (size_t)p.X * p.Y * ((p.Z + 31) / 32);
   uint32_t* bits = nullptr;
-  if (n >= 4096) {
-    if ((s = c.alloc(I.bits, bitbytes))) return s;
+  uint32_t* state = nullptr;
+  if (many) {
+    if ((s = c.alloc(I.bits, (bitwords + cells.words + 2) * 4))) return s;
     bits = static_cast<uint32_t*>(I.bits.p);
+    state = bits + bitwords + cells.words;
   }
   cudaStream_t st = g->b.stream;
   VF_CK(cudaMemcpyAsync(I.rays.p, rays, (size_t)n * 24, cudaMemcpyHostToDevice, st));
-  vfk::ray_entry(st, impact_grid(g), static_cast<const float*>(I.rays.p), n,
-                 static_cast<uint32_t*>(I.hits.p), bits, c.num_sms);
+  VF_CK(vfk::ray_entry(st, impact_grid(g), static_cast<const float*>(I.rays.p), n,
+                       static_cast<uint32_t*>(I.hits.p), bits, cells, state, c.num_sms));
+  if (many) {  // refused before the caller's array is written
+    uint32_t r = 0xFFFFFFFFu;
+    VF_CK(cudaMemcpyAsync(&r, state + 1, 4, cudaMemcpyDeviceToHost, st));
+    VF_CK(cudaStreamSynchronize(st));
+    if (r != 0xFFFFFFFFu) return zero_direction(r);
+  }
   VF_CK(cudaMemcpyAsync(out, I.hits.p, (size_t)n * 12, cudaMemcpyDeviceToHost, st));
   VF_CK(cudaStreamSynchronize(st));
   VF_CK(cudaGetLastError());

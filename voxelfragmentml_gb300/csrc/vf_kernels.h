@@ -115,12 +115,18 @@ struct ImpactGrid {
   uint32_t X, Y, Z, Zp;
   float amin[3], amax[3], cell[3];  // the grid's box and (amax - amin) / dims
 };
-// per ray (origin xyz, direction xyz): the 1-based index of the first
-// occupied voxel, 0xFFFFFFFF x3 when none; zero directions are rejected by
-// the caller.  bits (X * Y * ceil(Z / 32) words, or NULL): scratch for the
-// packed occupancy the walks read instead of the labels
-void ray_entry(cudaStream_t st, const ImpactGrid& G, const float* rays, uint32_t n, uint32_t* out,
-               uint32_t* bits, int num_sms);
+// cells of 2^shift voxels a side with an occupied voxel, one bit each
+struct RayCells {
+  uint32_t shift, ny, nz, words;
+};
+RayCells ray_cells(uint32_t X, uint32_t Y, uint32_t Z);
+// per ray (origin xyz, direction xyz): the 1-based index of the first occupied
+// voxel, 0xFFFFFFFF x3 when none.  bits (X * Y * ceil(Z / 32) + cells.words words,
+// or NULL): scratch for the packed occupancy the walks read instead of the labels;
+// state (with bits; 2 words): scratch, and the lowest ray without a direction or
+// 0xFFFFFFFF (without bits the caller looks for them)
+cudaError_t ray_entry(cudaStream_t st, const ImpactGrid& G, const float* rays, uint32_t n, uint32_t* out,
+                      uint32_t* bits, const RayCells& cells, uint32_t* state, int num_sms);
 // Seeder::nearSeeds: the new seeds (4 uint32 each, labels label0 + 1, ...)
 // in (x, y, z) order into out; status[0] = count, status[1] = 0 or
 // VF_ERR_SEED_SEARCH.  Needs nfrags >= 1, num_seeds <= 4095 and

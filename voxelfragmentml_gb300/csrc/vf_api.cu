@@ -545,9 +545,7 @@ vf_status vf_grid_triangulate(vf_grid* g, const vf_mc_params* mp, uint32_t* nmes
   auto rbase = static_cast<unsigned long long*>(M.rbase.p);
   auto tbase = static_cast<unsigned long long*>(M.tbase.p);
   auto err = static_cast<uint32_t*>(M.err.p);
-  // counts: vertices (exposed faces of fragment voxels) and triangles; the
-  // mask kernel stores non-zero masks only
-  VF_CK(cudaMemsetAsync(mask, 0, npad, st));
+  // counts: vertices (exposed faces of fragment voxels) and triangles
   vfk::mc_vertex_count(st, G, mask, static_cast<uint32_t*>(M.rcnt.p),
                        static_cast<uint8_t*>(M.present.p), nsm);
   vfk::exclusive_scan(st, static_cast<uint32_t*>(M.rcnt.p), rbase, sums, (uint32_t)rows, tot);

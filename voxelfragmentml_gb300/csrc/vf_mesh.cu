@@ -87,18 +87,12 @@ __device__ __forceinline__ uint4 load8w(const uint16_t* row, uint32_t z0, uint32
   return q;
 }
 
-// label e (0..7, a compile-time index after unrolling) of a packed load
-__device__ __forceinline__ uint32_t lab_of(const uint4& q, int e) {
-  const uint32_t wd = e < 2 ? q.x : (e < 4 ? q.y : (e < 6 ? q.z : q.w));
-  return (e & 1) ? (wd >> 16) : (wd & 0xFFFFu);
-}
-
-// every label of the packed load equals l0 (bit 15 ignored)
-__device__ __forceinline__ bool all_equal(const uint4& q, uint32_t l0) {
-  const uint32_t L = l0 | (l0 << 16);
-  return ((q.x & 0x7FFF7FFFu) == L) & ((q.y & 0x7FFF7FFFu) == L) & ((q.z & 0x7FFF7FFFu) == L) &
-         ((q.w & 0x7FFF7FFFu) == L);
-}
+// Pairs of labels (bit 15 cleared) compared in one word: bit 15 of a half is set
+// where the labels differ (sums of two 15-bit values do not carry over).
+constexpr uint32_t LAB2 = 0x7FFF7FFFu;
+__device__ __forceinline__ uint32_t ne2(uint32_t a, uint32_t b) { return ((a ^ b) + LAB2) & 0x80008000u; }
+// the pair one label before / after: (last of p, first of c) / (last of c, first of n)
+__device__ __forceinline__ uint32_t pair_of(uint32_t p, uint32_t c) { return __byte_perm(p, c, 0x5432); }
 
 __device__ __forceinline__ const uint16_t* row_ptr(const vfk::MeshGrid& G, int64_t x, int64_t y) {
   return (x >= 0 && y >= 0 && x < (int64_t)G.X && y < (int64_t)G.Y)
@@ -121,8 +115,11 @@ __device__ __forceinline__ uint32_t byte_of(uint2 m, int e) {
 
 // warp per grid row, 16 voxels per lane: face masks (bit d: the neighbour in
 // direction -x,+x,-y,+y,-z,+z carries another label), stored at the grid's
-// pitch into a zeroed buffer (all-FREE lanes store nothing); vertices per
-// row; present[value] for every fragment value
+// pitch; vertices per row; present[value] for every fragment value.  Labels are
+// compared two to a word.  Bound by the latency of a row's loads, few rows in
+// flight: 476 x 476 x 512 voxels, 64 fragments, 245 us, and k_mc_tcount 275 and
+// k_mc_temit 534 us, which find their cells alike (405, 448 and 712 us a label at a
+// time).
 __global__ void __launch_bounds__(256) k_mc_vcount(vfk::MeshGrid G, uint8_t* mask, uint32_t* rcnt,
                                                    uint8_t* present) {
   const int lane = threadIdx.x & 31;
@@ -140,50 +137,47 @@ __global__ void __launch_bounds__(256) k_mc_vcount(vfk::MeshGrid G, uint8_t* mas
       const uint32_t last = qb.w >> 16;
       const uint32_t before = __shfl_up_sync(FULL, last, 1);
       uint32_t after = __shfl_down_sync(FULL, qa.x & 0xFFFFu, 1);
-      const uint32_t zm1 = (lane == 0 ? carry : before) & 0x7FFFu;
+      const uint32_t zm1 = lane == 0 ? carry : before;
       if (lane == 31) after = (z0 + 512 < G.Z) ? (uint32_t)__ldg(rc + z0 + 512) : FREE;
-      after &= 0x7FFFu;
       carry = __shfl_sync(FULL, last, 31);
-      uint32_t cnt = 0;
+      uint32_t M[4] = {0u, 0u, 0u, 0u};  // masks, 4 voxels to a word
       // a label >= 2 somewhere in the lane's 16 voxels (bits 1..14 of a half)
       if (((qa.x | qa.y | qa.z | qa.w | qb.x | qb.y | qb.z | qb.w) & 0x7FFE7FFEu) != 0u) {
-        uint32_t c[16], mk[16];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          c[e] = lab_of(qa, e) & 0x7FFFu;
-          c[8 + e] = lab_of(qb, e) & 0x7FFFu;
-        }
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          const uint32_t zl = e ? c[e - 1] : zm1, zh = e < 15 ? c[e + 1] : after;
-          mk[e] = c[e] > FREE ? (((uint32_t)(zl != c[e]) << 4) | ((uint32_t)(zh != c[e]) << 5)) : 0u;
-        }
+        const uint32_t c[10] = {(zm1 << 16) & LAB2, qa.x & LAB2, qa.y & LAB2, qa.z & LAB2, qa.w & LAB2,
+                                qb.x & LAB2,        qb.y & LAB2, qb.z & LAB2, qb.w & LAB2, after & LAB2};
+        // flags of direction d end at bit 10 + d of each half
+        uint32_t f[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint4 oa = load8w(nb[k], zb, G.Z, G.Zp), ob = load8w(nb[k], zb + 8, G.Z, G.Zp);
+          const uint32_t o[8] = {oa.x, oa.y, oa.z, oa.w, ob.x, ob.y, ob.z, ob.w};
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const uint32_t o = lab_of(e < 8 ? oa : ob, e & 7) & 0x7FFFu;
-            if (c[e] > FREE) mk[e] |= (uint32_t)(o != c[e]) << k;
+          for (int i = 0; i < 8; ++i) f[i] = (f[i] >> 1) | ne2(o[i] & LAB2, c[i + 1]);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          f[i] = (f[i] >> 1) | ne2(pair_of(c[i], c[i + 1]), c[i + 1]);
+          f[i] = (f[i] >> 1) | ne2(pair_of(c[i + 1], c[i + 2]), c[i + 1]);
+          // fragment voxels only (labels >= 2)
+          const uint32_t own = ((c[i + 1] + 0x7FFE7FFEu) & 0x80008000u) >> 15;
+          f[i] = (f[i] >> 10) & (own * 0x3Fu);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) M[i] = __byte_perm(f[2 * i], f[2 * i + 1], 0x6420);
+        // every fragment has a voxel exposed towards -x (its lowest-x voxel); of
+        // a run of one label, the first
+        if ((M[0] | M[1] | M[2] | M[3]) & 0x01010101u) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            if ((f[i] & 1u) && (i == 0 || (f[i] & 0x10u))) present[c[i + 1] & 0xFFFFu] = 1;
+            if ((f[i] & 0x10000u) && (f[i] & 0x100000u)) present[c[i + 1] >> 16] = 1;
           }
         }
-#pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          cnt += (uint32_t)__popc(mk[e]);
-          // every fragment has a voxel exposed towards -x (its lowest-x voxel)
-          if ((mk[e] & 1u) && (e == 0 || c[e - 1] != c[e])) present[c[e]] = 1;
-        }
-        uint8_t* dst = mask + r * G.Zp + zb;
-        if (zb < G.Zp)
-          *reinterpret_cast<uint2*>(dst) =
-              make_uint2(mk[0] | (mk[1] << 8) | (mk[2] << 16) | (mk[3] << 24),
-                         mk[4] | (mk[5] << 8) | (mk[6] << 16) | (mk[7] << 24));
-        if (zb + 8 < G.Zp)
-          *reinterpret_cast<uint2*>(dst + 8) =
-              make_uint2(mk[8] | (mk[9] << 8) | (mk[10] << 16) | (mk[11] << 24),
-                         mk[12] | (mk[13] << 8) | (mk[14] << 16) | (mk[15] << 24));
       }
-      n += __reduce_add_sync(FULL, cnt);
+      uint8_t* dst = mask + r * G.Zp + zb;
+      if (zb < G.Zp) *reinterpret_cast<uint2*>(dst) = make_uint2(M[0], M[1]);
+      if (zb + 8 < G.Zp) *reinterpret_cast<uint2*>(dst + 8) = make_uint2(M[2], M[3]);
+      n += __reduce_add_sync(FULL, (uint32_t)(__popc(M[0]) + __popc(M[1]) + __popc(M[2]) + __popc(M[3])));
     }
     if (lane == 0) rcnt[r] = n;
   }
@@ -279,17 +273,6 @@ __device__ __forceinline__ void cell_rows_init(const vfk::MeshGrid& G, int64_t a
   for (int k = 0; k < 4; ++k) R.carry[k] = FREE;
 }
 
-__device__ __forceinline__ void cell_rows_load(const vfk::MeshGrid& G, CellRows& R, uint32_t c0,
-                                               int lane, uint32_t cur[4][8], uint32_t prv0[4]) {
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    load8(R.r[k], c0 + 8 * lane, G.Z, G.Zp, cur[k]);
-    prv0[k] = __shfl_up_sync(FULL, cur[k][7], 1);
-    if (lane == 0) prv0[k] = R.carry[k];
-    R.carry[k] = __shfl_sync(FULL, cur[k][7], 31);
-  }
-}
-
 // corner labels (bit 15 cleared) in VF_MC_CORNER order from the previous (z =
 // c-1) and current (z = c) label of each row
 __device__ __forceinline__ void corners(const uint32_t prv[4], const uint32_t cur[4], uint32_t v[8]) {
@@ -334,14 +317,15 @@ __device__ __forceinline__ uint32_t cell_triangles(const McShared& S, const uint
   return k;
 }
 
-// per warp: the step's four rows (index 7: z = c0 - 1, 8 + j: z = c0 + j),
-// the queue of its cells whose corners are not all one label, and per queued
-// cell its triangle count, then its first triangle
+// per warp: the step's four rows (index 7: z = c0 - 1, 8 + j: z = c0 + j; a step
+// that ends with the row takes the row's last cell too, 257 in all), the queue of
+// its cells whose corners are not all one label, and per queued cell its triangle
+// count, then its first triangle
 struct CellShared {
   McShared T;
-  uint16_t rows[8][4][264];
-  uint16_t qcell[8][256];
-  uint32_t qtri[8][256];
+  uint16_t rows[8][4][272];
+  uint16_t qcell[8][264];
+  uint32_t qtri[8][288];
 };
 
 // Stage one step (256 cells) of cell row (a, b) in shared memory and queue
@@ -361,30 +345,39 @@ __device__ __forceinline__ uint32_t stage_cells(const vfk::MeshGrid& G, CellRows
     prv0[k] = lane == 0 ? old[k] : p;
     R.carry[k] = __shfl_sync(FULL, last, 31);
   }
-  // one label on all 36 lattice points of the lane's 8 cells: nothing mixed
-  const uint32_t l0 = prv0[0] & 0x7FFFu;
-  bool same = true;
+  // cell e is mixed when the rows differ at e - 1 or e, or row 0 between them;
+  // labels two to a word, flags in bit 15 of each half
+  uint32_t mixed = 0;
+  {
+    const uint32_t c0w[4] = {q[0].x & LAB2, q[0].y & LAB2, q[0].z & LAB2, q[0].w & LAB2};
+    const uint32_t p0 = prv0[0] << 16;
+    uint32_t before = (((((prv0[1] << 16) ^ p0) | ((prv0[2] << 16) ^ p0) | ((prv0[3] << 16) ^ p0)) & LAB2) + LAB2) &
+                      0x80008000u,
+             last = p0 & LAB2;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) same &= all_equal(q[k], l0) & ((prv0[k] & 0x7FFFu) == l0);
-  if (__all_sync(FULL, same)) return 0;
+    for (int i = 0; i < 4; ++i) {
+      auto word = [&](const uint4& a) { return i == 0 ? a.x : (i == 1 ? a.y : (i == 2 ? a.z : a.w)); };
+      const uint32_t w0 = word(q[0]);
+      const uint32_t rows =
+          ((((word(q[1]) ^ w0) | (word(q[2]) ^ w0) | (word(q[3]) ^ w0)) & LAB2) + LAB2) & 0x80008000u;
+      const uint32_t m = rows | pair_of(before, rows) | ne2(pair_of(last, c0w[i]), c0w[i]);
+      mixed |= ((m >> 15 | m >> 30) & 3u) << (2 * i);
+      before = rows;
+      last = c0w[i];
+    }
+    const uint32_t z = c0 + 8 * lane;  // cells up to Z
+    mixed &= z > G.Z ? 0u : (G.Z - z >= 7u ? 0xFFu : (2u << (G.Z - z)) - 1u);
+    // the row's last cell, past a step that ends with the row: FREE above
+    if (z + 8 == G.Z && lane == 31) mixed |= (uint32_t)((before >> 31) | ((last >> 16) != FREE)) << 8;
+  }
+  if (!__any_sync(FULL, mixed)) return 0;
   if (lane == 0)
 #pragma unroll
     for (int k = 0; k < 4; ++k) S.rows[w][k][7] = (uint16_t)old[k];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(&S.rows[w][k][8 + 8 * lane]) = q[k];
-  uint32_t mixed = 0;
-  if (!same) {
-#pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      uint32_t pr[4], cu[4], v[8];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        pr[k] = e ? lab_of(q[k], e - 1) : prv0[k];
-        cu[k] = lab_of(q[k], e);
-      }
-      corners(pr, cu, v);
-      if (!uniform8(v) && c0 + 8 * lane + e <= G.Z) mixed |= 1u << e;
-    }
+  for (int k = 0; k < 4; ++k) {
+    *reinterpret_cast<uint4*>(&S.rows[w][k][8 + 8 * lane]) = q[k];
+    if (lane == 31) S.rows[w][k][264] = FREE;
   }
   const uint32_t na = (uint32_t)__popc(mixed);
   const uint32_t incl = warp_incl_scan(na, lane);
@@ -423,7 +416,7 @@ __global__ void __launch_bounds__(256) k_mc_tcount(vfk::MeshGrid G, const unsign
     CellRows R;
     cell_rows_init(G, a, b, R);
     uint32_t n = 0;
-    for (uint32_t c0 = 0; c0 <= G.Z; c0 += 256) {
+    for (uint32_t c0 = 0; c0 < G.Z; c0 += 256) {
       const uint32_t nq = stage_cells(G, R, S, w, lane, c0);
       uint32_t k = 0;
       for (uint32_t i = lane; i < nq; i += 32) {
@@ -460,20 +453,20 @@ __global__ void __launch_bounds__(256, 2) k_mc_temit(vfk::MeshGrid G, const unsi
     CellRows R;
     cell_rows_init(G, a, b, R);
     uint64_t base = rbase[r];
-    for (uint32_t c0 = 0; c0 <= G.Z; c0 += 256) {
+    for (uint32_t c0 = 0; c0 < G.Z; c0 += 256) {
       const uint32_t nq = stage_cells(G, R, S, w, lane, c0);
       if (!nq) continue;
-      // triangles per queued cell, then their exclusive prefix (8 entries per lane)
+      // triangles per queued cell, then their exclusive prefix (9 entries per lane)
       for (uint32_t i = lane; i < nq; i += 32) {
         uint32_t v[8], raw0;
         staged_corners(S, w, S.qcell[w][i], v, raw0);
         S.qtri[w][i] = cell_triangles(S.T, v);
       }
       __syncwarp();
-      uint32_t part[8], sum = 0;
+      uint32_t part[9], sum = 0;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const uint32_t i = 8 * lane + e;
+      for (int e = 0; e < 9; ++e) {
+        const uint32_t i = 9 * lane + e;
         part[e] = i < nq ? S.qtri[w][i] : 0u;
         sum += part[e];
       }
@@ -481,8 +474,8 @@ __global__ void __launch_bounds__(256, 2) k_mc_temit(vfk::MeshGrid G, const unsi
       uint32_t run = incl - sum;
       __syncwarp();
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const uint32_t i = 8 * lane + e;
+      for (int e = 0; e < 9; ++e) {
+        const uint32_t i = 9 * lane + e;
         if (i < nq) S.qtri[w][i] = run;
         run += part[e];
       }

@@ -1,5 +1,7 @@
-"""Fragment meshes at the sizes where the packed row kernels (csrc/vf_mesh.cu)
-change: rows around 8, 16, 256 and 512 voxels.  Bit for bit against the oracle."""
+"""Fragment meshes at the sizes where the packed row kernels and the smoothing
+lists (csrc/vf_mesh.cu) change: rows around 8, 16, 256 and 512 voxels, 255 to 257
+fragments, vertices with many faces, chunks of 256 vertices.  Bit for bit against
+the oracle."""
 import numpy as np
 import pytest
 
@@ -39,3 +41,23 @@ def test_rows(vf, ctx, Z, empty, marked):
     lab[-1, -1, -1] = 5
     lab |= (rng.random(lab.shape) < marked).astype(np.uint16) << 15
     _check(vf, ctx, lab, vf.MCParams(2, 0.7, 3, 0.3))
+
+
+@pytest.mark.parametrize("values", [1, 254, 255, 256, 257])
+def test_fragments(vf, ctx, values):
+    rng = np.random.default_rng(values)
+    lab = rng.integers(2, 2 + values, (12, 13, 14)).astype(np.uint16)
+    lab.ravel()[:values] = np.arange(2, 2 + values)
+    _check(vf, ctx, lab, vf.MCParams(1, 0.9, 1, 0.2))
+
+
+@pytest.mark.parametrize("marked", [0.0, 1.0, 0.01])
+def test_passes(vf, ctx, marked):
+    # blocks of two fragments: every vertex in one pass, in the other, in both
+    rng = np.random.default_rng(3)
+    lab = np.ones((30, 41, 50), np.uint16)
+    lab[3:28, 4:39, 5:30] = 2
+    lab[3:28, 4:39, 30:47] = 3
+    lab |= (rng.random(lab.shape) < marked).astype(np.uint16) << 15
+    V, T, nb, inc, ent, bent = _check(vf, ctx, lab, vf.MCParams(4, 0.9, 4, 0.2))
+    assert (nb == 0) == (marked == 0.0) and nb <= V and bent <= ent <= 2 * inc

@@ -60,7 +60,7 @@ struct vf_ctx {
 struct MeshState {
   vfr::DevBuf mask, vbase, rcnt, rbase, trcnt, tbase, sums, tot, present, dense, table, vkey, vown,
       vflag, vperm, tmp, vinv, tkey, tv, tperm, hist, hbase, vert, gface, face, voff, foff, acc, err,
-      deg, start, ustart, ent, nbr, meta;
+      deg, start, ent, nbr, item, meta;
   std::vector<uint16_t> values;
   uint64_t V = 0, T = 0;
   bool ready = false;
@@ -81,7 +81,7 @@ struct MeshState {
     for (vfr::DevBuf* b : {&mask, &vbase, &rcnt, &rbase, &trcnt, &tbase, &sums, &tot, &present,
                            &dense, &table, &vkey, &vown, &vflag, &vperm, &tmp, &vinv, &tkey, &tv,
                            &tperm, &hist, &hbase, &vert, &gface, &face, &voff, &foff, &acc, &err,
-                           &deg, &start, &ustart, &ent, &nbr, &meta})
+                           &deg, &start, &ent, &nbr, &item, &meta})
       c.free_buf(*b);
     ready = false;
   }
@@ -583,8 +583,8 @@ vf_status vf_grid_triangulate(vf_grid* g, const vf_mc_params* mp, uint32_t* nmes
       (s = c.alloc(M.face, T1 * 16)) || (s = c.alloc(M.voff, (F + 1) * 8)) ||
       (s = c.alloc(M.foff, (F + 1) * 8)) || (s = c.alloc(M.acc, V1 * 16)) ||
       (s = c.alloc(M.deg, V1 * 4)) || (s = c.alloc(M.start, (V1 + 1) * 8)) ||
-      (s = c.alloc(M.ent, T1 * 3 * 8)) || (s = c.alloc(M.ustart, (V1 + 1) * 8)) ||
-      (s = c.alloc(M.nbr, T1 * 3 * 4)) || (s = c.alloc(M.meta, V1 * 8)) ||
+      (s = c.alloc(M.ent, T1 * 3 * 8)) || (s = c.alloc(M.item, V1 * 4)) ||
+      (s = c.alloc(M.nbr, vfk::inc_entries(V1, T1) * 4)) || (s = c.alloc(M.meta, V1 * 8)) ||
       (s = scan_scratch(std::max<uint64_t>(V1, hw))))
     return s;
   sums = static_cast<unsigned long long*>(M.sums.p);
@@ -608,8 +608,8 @@ vf_status vf_grid_triangulate(vf_grid* g, const vf_mc_params* mp, uint32_t* nmes
   auto tmp = static_cast<uint32_t*>(M.tmp.p);
   auto hist = static_cast<uint32_t*>(M.hist.p);
   auto hbase = static_cast<unsigned long long*>(M.hbase.p);
-  vfk::stable_split16(st, vkey, V, F, tmp, vperm, hist, hbase, sums, tot + 2);
-  vfk::stable_split16(st, tkey, T, F, tmp, tperm, hist, hbase, sums, tot + 3);
+  vfk::stable_split16(st, vkey, V, F, tmp, vperm, hist, hbase, sums, tot + 2, voff);
+  vfk::stable_split16(st, tkey, T, F, tmp, tperm, hist, hbase, sums, tot + 3, foff);
   // the grid's affine map (RegularGrid.cpp:478-480): s = size / dims, min - s
   float sc[3], c0[3];
   for (int a = 0; a < 3; ++a) {
@@ -617,22 +617,22 @@ vf_status vf_grid_triangulate(vf_grid* g, const vf_mc_params* mp, uint32_t* nmes
     sc[a] = size / (float)d[a];
     c0[a] = g->job.aabb_min[a] - sc[a];
   }
-  vfk::mc_outputs(st, G, vperm, vown, vflag, V, sc, c0, vinv, vert, tperm, tv, T, gface, nsm);
-  vfk::mc_offsets(st, vkey, vperm, V, F, voff);
-  vfk::mc_offsets(st, tkey, tperm, T, F, foff);
-  VF_CK(cudaEventRecord(M.ev[3], st));
-  auto ustart = static_cast<unsigned long long*>(M.ustart.p);
-  auto start = static_cast<unsigned long long*>(M.start.p);
+  // the split's scratch is free again: boundary vertices per chunk of 2048
   const bool smooth = (mp->nonboundary_iterations || mp->boundary_iterations) && V && T;
+  if (smooth) VF_CK(cudaMemsetAsync(hist, 0, ((V + 2047) / 2048) * 4, st));
+  vfk::mc_outputs(st, G, vperm, vown, vflag, V, sc, c0, vinv, vert, tperm, tv, T, gface, smooth ? hist : nullptr, nsm);
+  VF_CK(cudaEventRecord(M.ev[3], st));
+  auto item = static_cast<uint32_t*>(M.item.p);
+  auto start = static_cast<unsigned long long*>(M.start.p);
   if (smooth)
-    VF_CK(vfk::mc_smooth_lists(st, gface, T, vert, V, static_cast<uint32_t*>(M.deg.p), start, ustart,
-                               sums, static_cast<uint2*>(M.ent.p), static_cast<uint32_t*>(M.nbr.p),
+    VF_CK(vfk::mc_smooth_lists(st, gface, T, vert, V, hist, hbase, static_cast<uint32_t*>(M.deg.p), start, sums,
+                               static_cast<uint2*>(M.ent.p), static_cast<uint32_t*>(M.nbr.p), item,
                                static_cast<uint2*>(M.meta.p), err, tot + 4, nsm));
   VF_CK(cudaEventRecord(M.ev[4], st));
   if (smooth)
-    VF_CK(vfk::mc_smooth_iterate(st, vert, static_cast<float4*>(M.acc.p), V,
+    VF_CK(vfk::mc_smooth_iterate(st, vert, static_cast<float4*>(M.acc.p), V, item,
                                  static_cast<const uint2*>(M.meta.p),
-                                 static_cast<const uint32_t*>(M.nbr.p), mp->nonboundary_iterations,
+                                 static_cast<const uint32_t*>(M.nbr.p), tot + 4, mp->nonboundary_iterations,
                                  mp->nonboundary_weight, mp->boundary_iterations,
                                  mp->boundary_weight, nsm));
   VF_CK(cudaEventRecord(M.ev[5], st));
@@ -643,7 +643,7 @@ vf_status vf_grid_triangulate(vf_grid* g, const vf_mc_params* mp, uint32_t* nmes
   VF_CK(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
   if (smooth) {
     VF_CK(cudaMemcpyAsync(smc + 0, start + V, 8, cudaMemcpyDeviceToHost, st));
-    VF_CK(cudaMemcpyAsync(smc + 1, ustart + V, 8, cudaMemcpyDeviceToHost, st));
+    VF_CK(cudaMemcpyAsync(smc + 1, tot + 6, 8, cudaMemcpyDeviceToHost, st));
     VF_CK(cudaMemcpyAsync(smc + 2, tot + 4, 16, cudaMemcpyDeviceToHost, st));
   }
   VF_CK(cudaStreamSynchronize(st));

@@ -78,34 +78,35 @@ void mc_tri_emit(cudaStream_t st, const MeshGrid& G, const unsigned long long* t
                  uint32_t* vflag, uint32_t* err, int num_sms);
 // stable order of items 0..n-1 by key[item] (< nkeys <= 65536) into out;
 // tmp: n words (two passes), hist: split_hist_words(n) words, hbase the
-// same count of u64, sums/tot: exclusive_scan scratch for that many words
+// same count of u64, sums/tot: exclusive_scan scratch for that many words;
+// off[f] = first sorted position with key >= f, f = 0..nkeys
 size_t split_hist_words(uint64_t n);
 void stable_split16(cudaStream_t st, const uint16_t* key, uint64_t n, uint32_t nkeys, uint32_t* tmp,
                     uint32_t* out, uint32_t* hist, unsigned long long* hbase,
-                    unsigned long long* sums, unsigned long long* tot);
+                    unsigned long long* sums, unsigned long long* tot, unsigned long long* off);
+// bnd (or NULL): zeroed counts of the boundary vertices of each 2048 vertices
 void mc_outputs(cudaStream_t st, const MeshGrid& G, const uint32_t* vperm,
                 const unsigned long long* vown, const uint32_t* vflag, uint64_t V, const float s[3],
                 const float c[3], uint32_t* vinv, float4* vert, const uint32_t* tperm,
-                const uint4* tv, uint64_t T, uint4* gface, int num_sms);
-// off[f] = first sorted position with key >= f, f = 0..F
-void mc_offsets(cudaStream_t st, const uint16_t* key, const uint32_t* perm, uint64_t n, uint32_t F,
-                unsigned long long* off);
+                const uint4* tv, uint64_t T, uint4* gface, uint32_t* bnd, int num_sms);
 // smoothSurface (MarchingCubes.cpp:489-510), in two steps.  mc_smooth_lists:
 // per vertex, the distinct neighbours (with multiplicity) of the faces its
-// pass sums, and meta; scratch deg V u32, start / ustart V + 1 u64, sums
-// exclusive_scan scratch for V, ent / nbr one uint2 / u32 per counted face
-// incidence (at most 3 T), meta V uint2, stats 2 u64 (boundary vertices,
-// their neighbour entries); err bit 2 if a vertex has more incidences than
-// its meta holds; needs V < 2^28.  mc_smooth_iterate: nb_iters over the
+// pass sums; scratch deg V u32, start V + 1 u64, sums exclusive_scan scratch for
+// V, ent one uint2 per counted face incidence (at most 3 T), nbr
+// inc_entries(V, T) u32, item /
+// meta V u32 / uint2, bnd / bbase mc_outputs' counts and as many u64, stats 4 u64
+// (boundary vertices, their neighbour entries, all entries, scratch); err bit 2 if a vertex has more incidences
+// than its meta holds; needs V < 2^28.  mc_smooth_iterate: nb_iters over the
 // non-boundary vertices, then b_iters over the boundary ones (tmp: V float4).
+uint64_t inc_entries(uint64_t V, uint64_t T);
 cudaError_t mc_smooth_lists(cudaStream_t st, const uint4* gface, uint64_t T, const float4* vert,
-                            uint64_t V, uint32_t* deg, unsigned long long* start,
-                            unsigned long long* ustart, unsigned long long* sums, uint2* ent,
-                            uint32_t* nbr, uint2* meta, uint32_t* err, unsigned long long* stats,
-                            int num_sms);
+                            uint64_t V, const uint32_t* bnd, unsigned long long* bbase, uint32_t* deg,
+                            unsigned long long* start, unsigned long long* sums, uint2* ent, uint32_t* nbr,
+                            uint32_t* item, uint2* meta, uint32_t* err, unsigned long long* stats, int num_sms);
 cudaError_t mc_smooth_iterate(cudaStream_t st, float4* vert, float4* tmp, uint64_t V,
-                              const uint2* meta, const uint32_t* nbr, uint32_t nb_iters,
-                              float nb_weight, uint32_t b_iters, float b_weight, int num_sms);
+                              const uint32_t* item, const uint2* meta, const uint32_t* nbr,
+                              const unsigned long long* stats, uint32_t nb_iters, float nb_weight,
+                              uint32_t b_iters, float b_weight, int num_sms);
 void mc_local_faces(cudaStream_t st, const uint4* gface, const uint32_t* tperm, const uint16_t* tkey,
                     const unsigned long long* voff, uint64_t T, uint4* out, int num_sms);
 

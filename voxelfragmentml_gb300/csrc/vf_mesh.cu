@@ -30,9 +30,9 @@
 //                 fragment (LSD, 8-bit digits, one or two passes)
 //   k_mc_vout     vertex positions through the grid's affine map
 //   k_mc_fout     faces in sorted vertex ids, face flag = OR of vertex flags
-//   k_inc_count / k_inc_fill / k_inc_unique / k_inc_compact  per vertex, the
-//                 distinct neighbours (with multiplicity) of the faces its
-//                 smoothing pass sums
+//   k_inc_count / k_inc_fill / k_inc_lists  per vertex, the distinct
+//                 neighbours (with multiplicity) of the faces its smoothing
+//                 pass sums; the vertices of each pass
 //   k_lap_gather  one Laplacian iteration per launch (laplacianSmoothing +
 //                 finishLaplacianSmoothing-comp.glsl) as a per-vertex gather
 //                 of the same int32 fixed-point sums
@@ -612,16 +612,25 @@ __global__ void __launch_bounds__(256) k_ms_scatter(const uint16_t* key, const u
     if (dig[k] < 256u) out[cnt[w][dig[k]] + rank[k]] = item[k];
 }
 
+// a chunk of vertices of the neighbour lists: the CTA of k_inc_lists; bnd counts
+// the boundary vertices of each
+constexpr uint32_t INC_CHUNK = 2048;
+
 // ---- outputs ---------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_mc_vout(vfk::MeshGrid G, const uint32_t* vperm,
                                                  const unsigned long long* vown,
                                                  const uint32_t* vflag, uint64_t V, float sx,
                                                  float sy, float sz, float cx, float cy, float cz,
-                                                 uint32_t* vinv, float4* out) {
+                                                 uint32_t* vinv, float4* out, uint32_t* bnd) {
   const uint64_t YZ = (uint64_t)G.Y * G.Zp;
-  for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < V;
+  const uint64_t n = (V + 31) & ~31ull;  // whole warps, for the ballot
+  for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n;
        s += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t gv = vperm[s];
+    const uint32_t gv = s < V ? vperm[s] : 0u;
+    const uint32_t flag = s < V ? (vflag[gv >> 5] >> (gv & 31u)) & 1u : 0u;
+    const unsigned m = __ballot_sync(FULL, flag);
+    if (bnd && m && (threadIdx.x & 31) == 0) atomicAdd(bnd + s / INC_CHUNK, (uint32_t)__popc(m));
+    if (s >= V) continue;
     vinv[gv] = (uint32_t)s;
     const unsigned long long own = vown[gv];
     const uint64_t lin = own >> 3;
@@ -632,7 +641,7 @@ __global__ void __launch_bounds__(256) k_mc_vout(vfk::MeshGrid G, const uint32_t
     o.x = __fadd_rn(__fmul_rn(sx, p[0]), cx);
     o.y = __fadd_rn(__fmul_rn(sy, p[1]), cy);
     o.z = __fadd_rn(__fmul_rn(sz, p[2]), cz);
-    o.w = (float)((vflag[gv >> 5] >> (gv & 31u)) & 1u);
+    o.w = (float)flag;
     out[s] = o;
   }
 }
@@ -649,10 +658,15 @@ __global__ void __launch_bounds__(256) k_mc_fout(const uint32_t* tperm, const ui
   }
 }
 
-// first sorted position of every key 0..F (F: one past the last mesh)
+// first sorted position of every key 0..F (F: one past the last mesh); after a
+// one-pass split, where its first chunk of the key starts
 __global__ void k_mc_offsets(const uint16_t* key, const uint32_t* perm, uint64_t n, uint32_t F,
-                             unsigned long long* off) {
+                             const unsigned long long* hbase, uint32_t nchunks, unsigned long long* off) {
   for (uint32_t f = blockIdx.x * blockDim.x + threadIdx.x; f <= F; f += gridDim.x * blockDim.x) {
+    if (hbase) {
+      off[f] = f < F ? hbase[(uint64_t)f * nchunks] : n;
+      continue;
+    }
     uint64_t lo = 0, hi = n;
     while (lo < hi) {
       const uint64_t mid = lo + (hi - lo) / 2;
@@ -697,62 +711,142 @@ __global__ void __launch_bounds__(256) k_inc_fill(const uint4* gface, const floa
   }
 }
 
-// the incidence pairs of vertex u folded in place into distinct neighbours,
-// each entry (neighbour << 4 | multiplicity): on a closed surface every edge
-// lies in two faces, so this halves the entries and the gathers
-__global__ void __launch_bounds__(256) k_inc_unique(const unsigned long long* start, uint2* ent,
-                                                    uint64_t V, uint32_t* ucnt, uint32_t* err) {
-  for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < V;
-       u += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t* w = reinterpret_cast<uint32_t*>(ent + start[u]);
-    const uint32_t n2 = (uint32_t)(2 * (start[u + 1] - start[u]));
-    uint32_t out = 0;
-    for (uint32_t i = 0; i < n2; ++i) {
-      const uint32_t n = w[i];  // every slot below i was read already
-      uint32_t j = 0;
-      while (j < out && (w[j] >> 4) != n) ++j;
-      if (j < out) {
-        if ((w[j] & 15u) == 15u) atomicOr(err, 2u); else ++w[j];
-      } else {
-        w[out++] = (n << 4) | 1u;
+// Neighbour lists.  The incidence pairs of a vertex are folded into distinct
+// neighbours, each entry (neighbour << 4 | multiplicity): on a closed surface
+// every edge lies in two faces, so this halves the entries and the gathers.
+// item lists the vertices of one smoothing pass from its front (non-boundary) and
+// those of the other from its back, each with meta: x = first entry, y = count of
+// summed positions (2 per face incidence, 16 bits) | entries << 16 (15 bits).
+// Items keep the vertices' order (bbase: boundary vertices before each chunk), so
+// the passes find neighbours near each other; entries are reserved per warp, in
+// whole 128-byte lines (any place will do).  Up to INC_FAST incidences fold in registers, more in place.
+// stats: [0] boundary vertices, [1] neighbour entries of boundary vertices,
+// [2] entries, [3] entries reserved.
+// 2.3 M vertices
+// 165 us, and 320 us in separate passes that fold in memory, scan and copy.
+constexpr uint32_t INC_FAST = 8;
+__global__ void __launch_bounds__(256) k_inc_lists(const unsigned long long* start, uint2* ent,
+                                                   const float4* vert, uint64_t V, const unsigned long long* bbase, uint32_t* nbr,
+                                                   uint32_t* item, uint2* meta, uint32_t* err,
+                                                   unsigned long long* stats) {
+  __shared__ uint32_t stage[8][32 * 2 * INC_FAST];
+  __shared__ uint32_t wb[8], s_ents[2];
+  const float* vw = reinterpret_cast<const float*>(vert) + 3;
+  const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const uint64_t from = (uint64_t)blockIdx.x * INC_CHUNK, to = min(from + INC_CHUNK, V);
+  if (t < 2) s_ents[t] = 0;
+  const uint32_t bnds = (uint32_t)bbase[blockIdx.x];
+  uint32_t next0 = (uint32_t)from - bnds, next1 = (uint32_t)(V - stats[0]) + bnds, bent = 0, ents = 0;
+  for (uint64_t u0 = from; u0 < to; u0 += 256) {
+    const uint64_t u = u0 + t;
+    const bool ok = u < to;
+    const bool bnd = ok && vw[4 * u] == 1.0f;
+    // the vertex's place among the items of its pass
+    const unsigned mb = __ballot_sync(FULL, bnd), mo = __ballot_sync(FULL, ok);
+    __syncthreads();  // wb is read
+    if (lane == 0) wb[warp] = (uint32_t)__popc(mb) | (uint32_t)__popc(mo & ~mb) << 16;
+    __syncthreads();
+    uint32_t before = 0, all = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < 8; ++w) {
+      before += w < warp ? wb[w] : 0u;
+      all += wb[w];
+    }
+    const uint32_t place = bnd ? next1 + (before & 0xFFFFu) + (uint32_t)__popc(mb & lt)
+                               : next0 + (before >> 16) + (uint32_t)__popc(mo & ~mb & lt);
+    next1 += all & 0xFFFFu;
+    next0 += all >> 16;
+    const unsigned long long a = ok ? start[u] : 0ull;
+    const uint64_t faces = ok ? start[u + 1] - a : 0ull;
+    const bool fast = faces <= INC_FAST;
+    uint32_t e[2 * INC_FAST], keep = 0, len = 0;
+    uint32_t* const w32 = reinterpret_cast<uint32_t*>(ent + a);
+    if (fast) {
+#pragma unroll
+      for (uint32_t k = 0; k < INC_FAST; ++k) {
+        const uint2 p = k < faces ? ent[a + k] : make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);
+        e[2 * k] = p.x;
+        e[2 * k + 1] = p.y;
+      }
+      uint32_t n[2 * INC_FAST];
+#pragma unroll
+      for (uint32_t i = 0; i < 2 * INC_FAST; ++i) n[i] = 1;
+#pragma unroll
+      for (uint32_t i = 0; i < 2 * INC_FAST; ++i) {
+        bool first = i < 2 * faces;
+#pragma unroll
+        for (uint32_t j = 0; j < i; ++j) {
+          const bool same = e[j] == e[i];
+          first &= !same;
+          n[j] += same;
+        }
+        keep |= (uint32_t)first << i;
+      }
+      uint32_t most = 0;
+#pragma unroll
+      for (uint32_t i = 0; i < 2 * INC_FAST; ++i) {
+        if ((keep >> i) & 1u) most = max(most, n[i]);
+        e[i] = (e[i] << 4) | (n[i] & 15u);
+      }
+      if (most > 15u) atomicOr(err, 2u);
+      len = (uint32_t)__popc(keep);
+    } else {
+      const uint64_t n2 = 2 * faces;
+      for (uint64_t i = 0; i < n2; ++i) {
+        const uint32_t v = w32[i];  // every slot below i was read already
+        uint32_t j = 0;
+        while (j < len && (w32[j] >> 4) != v) ++j;
+        if (j < len) {
+          if ((w32[j] & 15u) == 15u) atomicOr(err, 2u); else ++w32[j];
+        } else {
+          w32[len++] = (v << 4) | 1u;
+        }
       }
     }
-    ucnt[u] = out;
-  }
-}
-
-// dense neighbour lists and per-vertex meta: x = first entry, y = count of
-// summed positions (2 per face incidence, 16 bits) | entries << 16 (15 bits)
-// | boundary type << 31
-// stats: [0] boundary vertices, [1] neighbour entries of boundary vertices
-__global__ void __launch_bounds__(256) k_inc_compact(const unsigned long long* start,
-                                                     const uint2* ent,
-                                                     const unsigned long long* ustart,
-                                                     const float4* vert, uint64_t V,
-                                                     uint32_t* nbr, uint2* meta, uint32_t* err,
-                                                     unsigned long long* stats) {
-  const float* vw = reinterpret_cast<const float*>(vert) + 3;
-  const uint64_t n = (V + 31) & ~31ull;  // whole warps, for the reductions
-  for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n;
-       u += (uint64_t)gridDim.x * blockDim.x) {
-    uint32_t type = 0, len = 0;
-    if (u < V) {
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(ent + start[u]);
-      const uint64_t b = ustart[u];
-      len = (uint32_t)(ustart[u + 1] - b);
-      const uint64_t cnt = 2 * (start[u + 1] - start[u]);
-      if (cnt > 0xFFFFu || len > 0x7FFFu) atomicOr(err, 2u);
-      for (uint32_t k = 0; k < len; ++k) nbr[b + k] = w[k];
-      type = vw[4 * u] == 1.0f ? 1u : 0u;
-      meta[u] = make_uint2((uint32_t)b,
-                           (uint32_t)(cnt & 0xFFFFu) | ((len & 0x7FFFu) << 16) | (type << 31));
+    if (2 * faces > 0xFFFFu || len > 0x7FFFu) atomicOr(err, 2u);
+    uint32_t upto = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t v = __shfl_up_sync(FULL, upto, o);
+      if (lane >= (uint32_t)o) upto += v;
     }
-    const uint32_t nb = __reduce_add_sync(FULL, type), ne = __reduce_add_sync(FULL, type ? len : 0u);
-    if ((threadIdx.x & 31) == 0 && nb) {
-      atomicAdd(stats + 0, (unsigned long long)nb);
-      atomicAdd(stats + 1, (unsigned long long)ne);
+    const uint32_t total = __shfl_sync(FULL, upto, 31);
+    unsigned long long base = 0;
+    if (lane == 0 && total) base = atomicAdd(stats + 3, (unsigned long long)((total + 31u) & ~31u));
+    base = __shfl_sync(FULL, base, 0);
+    const uint32_t at = upto - len;
+    if (__all_sync(FULL, fast)) {
+      uint32_t o = at;
+#pragma unroll
+      for (uint32_t i = 0; i < 2 * INC_FAST; ++i)
+        if ((keep >> i) & 1u) stage[warp][o++] = e[i];
+      __syncwarp();
+      for (uint32_t k = lane; k < total; k += 32) nbr[base + k] = stage[warp][k];
+      __syncwarp();
+    } else if (fast) {
+      uint64_t o = base + at;
+#pragma unroll
+      for (uint32_t i = 0; i < 2 * INC_FAST; ++i)
+        if ((keep >> i) & 1u) nbr[o++] = e[i];
+    } else {
+      for (uint32_t k = 0; k < len; ++k) nbr[base + at + k] = w32[k];
     }
+    if (ok) {
+      item[place] = (uint32_t)u;
+      meta[place] = make_uint2((uint32_t)(base + at), (uint32_t)(2 * faces & 0xFFFFu) | ((len & 0x7FFFu) << 16));
+    }
+    bent += bnd ? len : 0u;
+    ents += len;
   }
+  bent = __reduce_add_sync(FULL, bent);
+  ents = __reduce_add_sync(FULL, ents);
+  if (lane == 0 && ents) {
+    atomicAdd(&s_ents[0], bent);
+    atomicAdd(&s_ents[1], ents);
+  }
+  __syncthreads();
+  if (t < 2 && s_ents[t]) atomicAdd(stats + 1 + t, (unsigned long long)s_ents[t]);
 }
 
 __device__ __forceinline__ uint32_t to_fixed(float p) {
@@ -760,29 +854,34 @@ __device__ __forceinline__ uint32_t to_fixed(float p) {
 }
 
 // one Jacobi iteration (laplacianSmoothing + finishLaplacianSmoothing) for the
-// vertices of type `target`; other vertices are read from src, never written
-// (both buffers hold them)
-__global__ void __launch_bounds__(256) k_lap_gather(const float4* src, float4* dst, const uint2* meta,
-                                                    const uint32_t* nbr, uint64_t V, uint32_t target,
-                                                    float omw, float weight) {
-  for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < V;
-       u += (uint64_t)gridDim.x * blockDim.x) {
-    const uint2 m = meta[u];
-    if ((m.y >> 31) != target) continue;
+// vertices of one pass: the first V - stats[0] of item, or (back) the others; other
+// vertices are read from src, never written (both buffers hold them).  Bound by
+// the latency of the gathers: 1.75 M and 0.55 M vertices 31 and 18 us, where a scan
+// of all vertices took 31 and 26; consecutive items per CTA took 40 and 20.
+constexpr uint32_t LAP_FLIGHT = 8;
+__global__ void __launch_bounds__(256) k_lap_gather(const float4* src, float4* dst, const uint32_t* item,
+                                                    const uint2* meta, const uint32_t* nbr, uint64_t V,
+                                                    const unsigned long long* stats, int back, float omw,
+                                                    float weight) {
+  const uint64_t nb = V - stats[0], to = back ? V : nb;
+  for (uint64_t i = (back ? nb : 0) + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < to;
+       i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint2 m = meta[i];
+    const uint32_t u = item[i];
     float4 p = src[u];
     const uint32_t cnt = m.y & 0xFFFFu, len = (m.y >> 16) & 0x7FFFu;
     if (cnt) {
       uint32_t sx = 0, sy = 0, sz = 0;
-      // four entries, then their four positions, in flight at a time
-      for (uint32_t k = 0; k < len; k += 4) {
-        uint32_t e[4];
+      // LAP_FLIGHT entries, then their positions, at a time (most have 6)
+      for (uint32_t k = 0; k < len; k += LAP_FLIGHT) {
+        uint32_t e[LAP_FLIGHT];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) e[j] = k + j < len ? __ldg(nbr + m.x + k + j) : 0u;
-        float4 a[4];
+        for (uint32_t j = 0; j < LAP_FLIGHT; ++j) e[j] = k + j < len ? __ldg(nbr + m.x + k + j) : 0u;
+        float4 a[LAP_FLIGHT];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) a[j] = e[j] ? src[e[j] >> 4] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (uint32_t j = 0; j < LAP_FLIGHT; ++j) a[j] = e[j] ? src[e[j] >> 4] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (uint32_t j = 0; j < LAP_FLIGHT; ++j) {
           const uint32_t mult = e[j] & 15u;  // 0 for the padding slots
           sx += mult * to_fixed(a[j].x);
           sy += mult * to_fixed(a[j].y);
@@ -881,8 +980,12 @@ size_t split_hist_words(uint64_t n) { return 256 * std::max<uint64_t>(1, (n + MS
 
 void stable_split16(cudaStream_t st, const uint16_t* key, uint64_t n, uint32_t nkeys, uint32_t* tmp,
                     uint32_t* out, uint32_t* hist, unsigned long long* hbase,
-                    unsigned long long* sums, unsigned long long* tot) {
-  if (!n) return;
+                    unsigned long long* sums, unsigned long long* tot, unsigned long long* off) {
+  const int ob = (int)(nkeys + 256) / 256;
+  if (!n) {
+    k_mc_offsets<<<ob, 256, 0, st>>>(key, out, n, nkeys, nullptr, 0, off);
+    return;
+  }
   const uint32_t nchunks = (uint32_t)((n + MS_CHUNK - 1) / MS_CHUNK);
   const int passes = nkeys > 256 ? 2 : 1;
   const uint32_t* in = nullptr;
@@ -893,46 +996,45 @@ void stable_split16(cudaStream_t st, const uint16_t* key, uint64_t n, uint32_t n
     k_ms_scatter<<<nchunks, 256, 0, st>>>(key, in, n, 8 * p, nchunks, hbase, dst);
     in = dst;
   }
+  k_mc_offsets<<<ob, 256, 0, st>>>(key, out, n, nkeys, passes == 1 ? hbase : nullptr, nchunks, off);
 }
 
 void mc_outputs(cudaStream_t st, const MeshGrid& G, const uint32_t* vperm,
                 const unsigned long long* vown, const uint32_t* vflag, uint64_t V, const float s[3],
                 const float c[3], uint32_t* vinv, float4* vert, const uint32_t* tperm,
-                const uint4* tv, uint64_t T, uint4* gface, int num_sms) {
+                const uint4* tv, uint64_t T, uint4* gface, uint32_t* bnd, int num_sms) {
   if (V)
     k_mc_vout<<<grid_for(V, num_sms), 256, 0, st>>>(G, vperm, vown, vflag, V, s[0], s[1], s[2], c[0],
-                                                    c[1], c[2], vinv, vert);
+                                                    c[1], c[2], vinv, vert, bnd);
   if (T) k_mc_fout<<<grid_for(T, num_sms), 256, 0, st>>>(tperm, tv, vinv, vflag, T, gface);
 }
 
-void mc_offsets(cudaStream_t st, const uint16_t* key, const uint32_t* perm, uint64_t n, uint32_t F,
-                unsigned long long* off) {
-  k_mc_offsets<<<(F + 256) / 256, 256, 0, st>>>(key, perm, n, F, off);
-}
+// entries of all vertices, and each warp's up to its 128-byte line
+uint64_t inc_entries(uint64_t V, uint64_t T) { return 3 * T + V + 31; }
 
 cudaError_t mc_smooth_lists(cudaStream_t st, const uint4* gface, uint64_t T, const float4* vert,
-                            uint64_t V, uint32_t* deg, unsigned long long* start,
-                            unsigned long long* ustart, unsigned long long* sums, uint2* ent,
-                            uint32_t* nbr, uint2* meta, uint32_t* err, unsigned long long* stats,
-                            int num_sms) {
+                            uint64_t V, const uint32_t* bnd, unsigned long long* bbase, uint32_t* deg,
+                            unsigned long long* start, unsigned long long* sums, uint2* ent, uint32_t* nbr,
+                            uint32_t* item, uint2* meta, uint32_t* err, unsigned long long* stats, int num_sms) {
   if (!V || !T) return cudaSuccess;
   cudaError_t e;
-  const int gv = grid_for(V, num_sms), gt = grid_for(T, num_sms);
+  const int gt = grid_for(T, num_sms);
   if ((e = cudaMemsetAsync(deg, 0, V * 4, st))) return e;
-  if ((e = cudaMemsetAsync(stats, 0, 16, st))) return e;
+  if ((e = cudaMemsetAsync(stats, 0, 32, st))) return e;
   k_inc_count<<<gt, 256, 0, st>>>(gface, vert, T, deg);
   exclusive_scan(st, deg, start, sums, (uint32_t)V, start + V);
   if ((e = cudaMemsetAsync(deg, 0, V * 4, st))) return e;
   k_inc_fill<<<gt, 256, 0, st>>>(gface, vert, T, start, deg, ent);
-  k_inc_unique<<<gv, 256, 0, st>>>(start, ent, V, deg, err);
-  exclusive_scan(st, deg, ustart, sums, (uint32_t)V, ustart + V);
-  k_inc_compact<<<gv, 256, 0, st>>>(start, ent, ustart, vert, V, nbr, meta, err, stats);
+  const uint32_t chunks = (uint32_t)((V + INC_CHUNK - 1) / INC_CHUNK);
+  exclusive_scan(st, bnd, bbase, sums, chunks, stats);
+  k_inc_lists<<<chunks, 256, 0, st>>>(start, ent, vert, V, bbase, nbr, item, meta, err, stats);
   return cudaGetLastError();
 }
 
 cudaError_t mc_smooth_iterate(cudaStream_t st, float4* vert, float4* tmp, uint64_t V,
-                              const uint2* meta, const uint32_t* nbr, uint32_t nb_iters,
-                              float nb_weight, uint32_t b_iters, float b_weight, int num_sms) {
+                              const uint32_t* item, const uint2* meta, const uint32_t* nbr,
+                              const unsigned long long* stats, uint32_t nb_iters, float nb_weight,
+                              uint32_t b_iters, float b_weight, int num_sms) {
   if (!V || (!nb_iters && !b_iters)) return cudaSuccess;
   cudaError_t e;
   const int gv = grid_for(V, num_sms);
@@ -946,7 +1048,7 @@ cudaError_t mc_smooth_iterate(cudaStream_t st, float4* vert, float4* tmp, uint64
     const float weight = pass ? b_weight : nb_weight;
     const float omw = 1.0f - weight;
     for (uint32_t it = 0; it < iters; ++it) {
-      k_lap_gather<<<gv, 256, 0, st>>>(cur, nxt, meta, nbr, V, pass, omw, weight);
+      k_lap_gather<<<gv, 256, 0, st>>>(cur, nxt, item, meta, nbr, V, stats, (int)pass, omw, weight);
       std::swap(cur, nxt);
     }
     // the finished type must match in both buffers before the other pass

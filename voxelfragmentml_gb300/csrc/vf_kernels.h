@@ -270,7 +270,8 @@ uint32_t flood_schedule(const WaveGang* gangs, uint32_t n, const WaveShape& shap
 void flood_seed_bricks(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs, uint8_t* live,
                        uint32_t* list, uint32_t* count);
 // row states from the labels
-void flood_init(cudaStream_t st, const JobDesc* dj, const FloodScratch& fs, const uint8_t* live);
+// planes: the labels are the voxelizer's occupancy, still in its bit planes
+void flood_init(cudaStream_t st, const JobDesc* dj, const FloodScratch& fs, const uint8_t* live, bool planes);
 cudaError_t flood_seed(cudaStream_t st, const JobDesc* dj, const JobState* ds, const FloodScratch& fs);
 cudaError_t flood_waves(cudaStream_t st, JobState* ds, const FloodScratch& fs);
 void flood_labels(cudaStream_t st, const JobDesc* dj, const JobState* ds, const uint32_t* list,

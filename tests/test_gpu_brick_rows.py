@@ -43,3 +43,29 @@ def test_job(vf, ctx, dims, dfunc):
     want = O.run_job(v, f, dims, mn, mx, q, ncounts=256)
     assert r.status == 0
     assert np.array_equal(spec.labels, want[0]) and np.array_equal(spec.counts, want[1][:256])
+
+
+def _labels(shape, seed):
+    rng = np.random.default_rng(seed)
+    lab = rng.integers(0, 5, [(s + 6) // 7 for s in shape]).astype(np.uint16)
+    for a in range(3):
+        lab = np.repeat(lab, 7, axis=a)
+    lab = np.ascontiguousarray(lab[: shape[0], : shape[1], : shape[2]])
+    lab[rng.random(shape) < 0.02] = 0
+    return lab
+
+
+@pytest.mark.parametrize("shape", [(2, 3, 2), (16, 16, 32), (33, 35, 66), (9, 40, 130)])
+@pytest.mark.parametrize("labels", [3, 255, 256, 300])
+def test_counts(vf, ctx, shape, labels):
+    rng = np.random.default_rng(labels)
+    lab = _labels(shape, 1)
+    noisy = rng.random(shape) < 0.3
+    lab[noisy] = rng.integers(0, labels + 1, int(noisy.sum()))
+    lab |= (rng.random(shape) < 0.3).astype(np.uint16) << 15
+    g = vf.RegularGrid(shape, None, None, ctx)
+    g.upload(lab)
+    want = np.bincount((lab & 0x7FFF)[(lab > 1)].ravel(), minlength=512)[:512]
+    counts, occupied = g.countValues(512)
+    assert np.array_equal(counts[2:], want[2:]) and occupied == (lab > 1).sum()
+    g.close()

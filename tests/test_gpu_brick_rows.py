@@ -69,3 +69,15 @@ def test_counts(vf, ctx, shape, labels):
     counts, occupied = g.countValues(512)
     assert np.array_equal(counts[2:], want[2:]) and occupied == (lab > 1).sum()
     g.close()
+
+
+@pytest.mark.parametrize("period", [1, 3, 5, 6, 7, 15, 16, 17, 40, 1000])
+@pytest.mark.parametrize("shape", [(2, 3, 2), (33, 35, 66), (16, 16, 32), (40, 17, 100)])
+def test_perturb(vf, ctx, shape, period):
+    lab = _labels(shape, period)
+    for amp in (0.7, 5.0, 64.0):
+        g = vf.RegularGrid(shape, None, None, ctx)
+        g.upload(lab)
+        g.perturb(amp, period, 9)
+        assert np.array_equal(g.data(), O.perturb(lab, amp, period, 9))
+        g.close()

@@ -120,6 +120,7 @@ struct JobState {
   unsigned long long occupied;
   uint32_t passes;
   uint32_t nranks;
+  uint32_t odd_edges;       // mesh edges used an odd number of times
 };
 
 // ---------------------------------------------------------------------------

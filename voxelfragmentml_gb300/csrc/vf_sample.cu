@@ -4,14 +4,14 @@
 // once.
 //
 //   k_pc_area     one thread per face: area |cross(v2-v1, v3-v1)| / 2
-//   k_pc_chunks   one thread per 1024-face chunk of a mesh: double sum and max
+//   k_pc_chunks   one warp per 1024-face chunk of a mesh: double sum and max
 //   k_pc_mesh     one thread per mesh: sumArea (chunk sums in order, rounded to
 //                 float), maxArea, the noise length NB
 //   k_pc_select   one CTA per mesh with S <= T: S distinct faces, the first ones
 //                 of the draw sequence; 256 draws per round tested in parallel
-//                 (already chosen, or drawn earlier in the round), then ranked
-//                 in draw order, so the set equals the sequential rejection
-//                 sampler's
+//                 (already chosen, or drawn earlier in the round: a hash table
+//                 of the round's faces), then ranked in draw order, so the set
+//                 equals the sequential rejection sampler's
 //   k_pc_count    samples per face: max(ceil(a / sumArea * S), 1) when S > T,
 //                 else 1 for a chosen face; an exclusive scan places them
 //   k_pc_points   one thread per face: its samples (noise pair, fold, v1 + u r.x
@@ -22,8 +22,6 @@
 #include "vf_kernels.h"
 
 namespace {
-
-constexpr uint32_t CHUNK = 1024;
 
 __device__ __forceinline__ int ceil_count(float x) {
   const float c = ceilf(x);
@@ -73,19 +71,60 @@ __global__ void __launch_bounds__(256) k_pc_area(const float4* V, const uint4* F
   }
 }
 
-// chunk c covers faces [cstart[c], min(cstart[c] + CHUNK, end of its mesh))
+// Chunk c covers faces [cstart[c], cend[c]), at most 1024; its areas are added in
+// order in double.  Where every partial sum is exact the order does not matter: the
+// areas are whole multiples of one power of two (2^-149 of the smallest exponent),
+// and their sum is below 2^53 of it.  Then the lanes add them as integers; a chunk
+// with a wider range (or an area that is not finite) is added face by face, a
+// dependent double add each: 138 k faces 5 us (122 us face by face, a thread a chunk).
 __global__ void __launch_bounds__(256) k_pc_chunks(const float* area, const unsigned long long* cstart,
                                                    const unsigned long long* cend, uint32_t nchunks,
                                                    double* csum, float* cmax) {
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < nchunks; c += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    float mx = 0.0f;
-    for (uint64_t t = cstart[c]; t < cend[c]; ++t) {
-      s = __dadd_rn(s, (double)area[t]);
-      mx = fmaxf(mx, area[t]);
+  constexpr uint32_t FULL = 0xFFFFFFFFu;
+  const uint32_t lane = threadIdx.x & 31;
+  for (uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nchunks; c += (gridDim.x * blockDim.x) >> 5) {
+    const uint64_t from = cstart[c], to = cend[c];
+    uint32_t bits[32], lo = 255u, hi = 0u, top = 0u;  // exponent fields (a subnormal's is 1), largest area
+#pragma unroll
+    for (uint32_t k = 0; k < 32; ++k) {
+      const uint64_t t = from + 32 * k + lane;
+      bits[k] = t < to ? __float_as_uint(area[t]) : 0u;  // areas are roots: never negative
+      const uint32_t e = bits[k] ? max(bits[k] >> 23, 1u) : 0u;
+      hi = max(hi, e);
+      lo = e ? min(lo, e) : lo;
+      top = max(top, bits[k]);
     }
-    csum[c] = s;
-    cmax[c] = mx;
+    lo = __reduce_min_sync(FULL, lo);
+    hi = __reduce_max_sync(FULL, hi);
+    top = __reduce_max_sync(FULL, top);
+    bool exact = to - from <= 1024 && hi < 255u && hi <= lo + 29u;
+    unsigned long long sum = 0;  // in units of 2^(lo - 150); below 1024 * 2^53
+    if (exact) {
+#pragma unroll
+      for (uint32_t k = 0; k < 32; ++k) {
+        const uint32_t e = bits[k] >> 23, m = (bits[k] & 0x7FFFFFu) | (e ? 0x800000u : 0u);
+        sum += bits[k] ? (unsigned long long)m << (max(e, 1u) - lo) : 0ull;
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(FULL, sum, o);
+      exact = sum < 1ull << 53;
+    }
+    if (lane == 0) {
+      if (exact) {
+        const double unit = __longlong_as_double((long long)((uint64_t)(lo - 150u + 1023u) << 52));
+        csum[c] = hi ? __dmul_rn((double)sum, unit) : 0.0;
+        cmax[c] = __uint_as_float(top);
+      } else {
+        double s = 0.0;
+        float mx = 0.0f;
+        for (uint64_t t = from; t < to; ++t) {
+          s = __dadd_rn(s, (double)area[t]);
+          mx = fmaxf(mx, area[t]);
+        }
+        csum[c] = s;
+        cmax[c] = mx;
+      }
+    }
   }
 }
 
@@ -110,7 +149,8 @@ __global__ void k_pc_mesh(const double* csum, const float* cmax, const unsigned 
 __global__ void __launch_bounds__(256) k_pc_select(const uint32_t* sel, const unsigned long long* face_off,
                                                    const uint32_t* keys, uint32_t S, uint64_t seed,
                                                    uint32_t* chosen, uint32_t* err) {
-  __shared__ uint32_t face[256];
+  constexpr uint32_t SLOTS = 1024, NONE = 0xFFFFFFFFu;
+  __shared__ uint32_t face[SLOTS], first[SLOTS];  // a face of the round, its first draw
   __shared__ uint32_t s_got;
   __shared__ uint32_t wsum[8];
   const uint32_t m = sel[blockIdx.x];
@@ -126,11 +166,21 @@ __global__ void __launch_bounds__(256) k_pc_select(const uint32_t* sel, const un
     const float uf = vf_u01(vf_hash(seed, VF_STREAM_SAMPLE_FACE, ((uint64_t)key << 40) + j));
     uint32_t f = (uint32_t)__fmul_rn(uf, (float)T);
     if (f > T - 1) f = T - 1;
-    face[t] = f;
+    for (uint32_t k = t; k < SLOTS; k += 256) {
+      face[k] = NONE;
+      first[k] = NONE;
+    }
     __syncthreads();
     const uint64_t g = base + f;
-    bool fresh = j < limit && !((chosen[g >> 5] >> (g & 31)) & 1u);
-    for (uint32_t k = 0; k < t && fresh; ++k) fresh = face[k] != f;  // drawn earlier this round
+    const bool open = j < limit && !((chosen[g >> 5] >> (g & 31)) & 1u);
+    uint32_t h = (f * 2654435761u) >> 22;  // of 1024 slots; 256 faces at most are in
+    for (;; h = (h + 1) & (SLOTS - 1)) {
+      const uint32_t old = atomicCAS(&face[h], NONE, f);
+      if (old == NONE || old == f) break;
+    }
+    atomicMin(&first[h], t);
+    __syncthreads();
+    const bool fresh = open && first[h] == t;
     // rank of the fresh draws in draw order
     const unsigned b = __ballot_sync(0xFFFFFFFFu, fresh);
     if (lane == 0) wsum[w] = (uint32_t)__popc(b);
@@ -228,7 +278,7 @@ void pc_areas(cudaStream_t st, const SampleMeshes& M, float* area, const unsigne
   if (M.nfaces) {
     k_pc_area<<<blocks_for(M.nfaces, num_sms), 256, 0, st>>>(M.verts, M.faces, M.vert_off, M.face_off, M.F,
                                                              M.nfaces, area);
-    k_pc_chunks<<<blocks_for(nchunks, num_sms), 256, 0, st>>>(area, cstart, cend, nchunks, csum, cmax);
+    k_pc_chunks<<<blocks_for((uint64_t)nchunks * 32, num_sms), 256, 0, st>>>(area, cstart, cend, nchunks, csum, cmax);
   }
   k_pc_mesh<<<(M.F + 255) / 256, 256, 0, st>>>(csum, cmax, mchunk, M.F, S, msum, nb);
 }

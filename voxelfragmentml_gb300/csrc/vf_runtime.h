@@ -86,6 +86,7 @@ struct Batch {
   size_t h_tables_cap = 0;
   JobState* h_state = nullptr;  // pinned
   size_t h_state_cap = 0;
+  uint32_t* h_counts = nullptr; // behind h_state: the counts of all jobs
   uint32_t* h_scal = nullptr;   // pinned: [0..3] flood stats, [4] err, [8] fcount
   cudaEvent_t ev_flood0 = nullptr, ev_flood1 = nullptr, ev_done = nullptr;
   // stage boundaries: 0 start, 1 inputs uploaded, 2 tetrahedra built,
@@ -106,6 +107,7 @@ struct Batch {
   // per-launch bookkeeping
   uint64_t launches = 0;
   bool flood_timed = false;
+  bool counts_copied = false;  // the counts are on their way to h_counts
 
   vf_status init(Ctx* c, bool own);
   void release();
@@ -120,6 +122,7 @@ struct Batch {
   void drop_graphs();
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};  // [download]
   uint64_t glaunches[2] = {0, 0};
+  bool gcounts[2] = {false, false};
   bool graphs_ok = true;
   bool last_run_graph = false;
   bool capturing = false;

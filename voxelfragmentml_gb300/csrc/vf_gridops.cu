@@ -1159,15 +1159,16 @@ __global__ void __launch_bounds__(256) k_pack16(const JobDesc* jobs, int njobs) 
 // per row (rows are 64..384 labels: 8..48 16-byte units), so a warp has four
 // rows' loads in flight.  A warp's rows only increase, so its job is found by
 // walking forward from the previous one.
-__global__ void __launch_bounds__(256) k_pack(const JobDesc* jobs, int njobs,
+__global__ void __launch_bounds__(256) k_pack(const JobDesc* jobs, int njobs, unsigned long long row0,
                                               unsigned long long total_rows) {
   const int lane = threadIdx.x & 31, sub = lane & 7;
   const unsigned long long nw = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   int j = 0;
   for (unsigned long long r0 = (((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4;
        r0 < total_rows; r0 += nw * 4) {
-    const unsigned long long r = r0 + (lane >> 3);
+    unsigned long long r = r0 + (lane >> 3);
     if (r >= total_rows) continue;
+    r += row0;
     while (j + 1 < njobs && jobs[j + 1].row_base <= r) ++j;
     const JobDesc& J = jobs[j];
     if (!J.out) continue;
@@ -1286,11 +1287,12 @@ void count_values(cudaStream_t st, const JobDesc* dj, JobState* ds, const uint32
   if (max_count) k_counts<<<brick_grid(max_count), 256, 0, st>>>(dj, ds, list, count, brick_job);
 }
 
-void pack_labels(cudaStream_t st, const JobDesc* dj, int njobs, uint64_t total_rows, int num_sms) {
-  if (njobs <= 0 || !total_rows) return;
-  const int per_job = std::max(1, num_sms * 8 / njobs);
+void pack_labels(cudaStream_t st, const JobDesc* dj, int njobs, uint64_t row0, uint64_t rows, int num_sms,
+                 int ctas_per_sm) {
+  if (njobs <= 0 || !rows) return;
+  const int per_job = std::max(1, num_sms * ctas_per_sm / njobs);
   k_pack16<<<dim3(per_job, std::min(njobs, 65535)), 256, 0, st>>>(dj, njobs);
-  k_pack<<<num_sms * 8, 256, 0, st>>>(dj, njobs, (unsigned long long)total_rows);
+  k_pack<<<num_sms * ctas_per_sm, 256, 0, st>>>(dj, njobs, row0, (unsigned long long)rows);
 }
 
 }  // namespace vfk

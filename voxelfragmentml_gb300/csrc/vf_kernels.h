@@ -33,12 +33,14 @@ void combine(cudaStream_t st, const JobDesc* dj, const uint32_t* brick_job,
              uint32_t total_bricks, uint8_t* live, int dual);
 void mark_live(cudaStream_t st, const JobDesc* dj, const uint32_t* brick_job,
                uint32_t total_bricks, uint8_t* live);
-void compact_live(cudaStream_t st, const uint8_t* live, uint32_t total_bricks,
+void compact_live(cudaStream_t st, const uint8_t* live, uint32_t first, uint32_t total_bricks,
                   uint32_t* list, uint32_t* count);
 
 // labels of every job with a device-accessible `out` (T_CNT table: the
 // final buffer) into `out`, rows of Z without the z padding
-void pack_labels(cudaStream_t st, const JobDesc* dj, int njobs, uint64_t total_rows, int num_sms);
+// rows [row0, row0 + rows) of the batch are those of the njobs jobs at dj
+void pack_labels(cudaStream_t st, const JobDesc* dj, int njobs, uint64_t row0, uint64_t rows, int num_sms,
+                 int ctas_per_sm);
 
 // exclusive prefix sum of n u32 into u64 (sums: ceil(n / 1024) + 1 scratch
 // words); *total = the sum

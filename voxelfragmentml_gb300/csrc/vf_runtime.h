@@ -92,7 +92,8 @@ struct Batch {
   // stage boundaries: 0 start, 1 inputs uploaded, 2 tetrahedra built,
   // 3 parity rasterised, 4 shell tested, 5 voxelized (combine + live list),
   // 6 seeded, 7 fractured, 8 perturbed, 9 eroded/boundaries, 10 counted,
-  // 11 downloaded
+  // 11 downloaded; with groups, 8 is the end of all groups' last stages and 9 and
+  // 10 follow at once
   static constexpr int NSTAGE_EV = 12;
   cudaEvent_t ev_stage[NSTAGE_EV] = {};
   bool stage_rec[NSTAGE_EV] = {};
@@ -115,6 +116,12 @@ struct Batch {
   vf_status enqueue_batched(bool upload_inputs = true, bool download = true);
   cudaError_t waves_serialized(cudaStream_t st, JobState* ds, const vfk::FloodScratch& fs);
   vf_status wave_tables(vfk::FloodScratch& fs);
+  // the download beside the last stages: the end of each group of jobs, the
+  // stream that writes their labels, after (and the join)
+  std::vector<uint32_t> groups;
+  cudaStream_t side = nullptr;
+  cudaEvent_t ev_group = nullptr;
+  vf_status plan_groups();
   // the resident stage chain (no uploads) as a CUDA graph: captured on the
   // first execute after plan(), replayed afterwards; falls back to direct
   // launches when the chain has sub-seed prefixes or cannot be captured

@@ -1070,18 +1070,19 @@ __global__ void __launch_bounds__(256) k_mark_live(const JobDesc* jobs, const ui
   }
 }
 
-__global__ void k_compact(const uint8_t* live, uint32_t total, uint32_t* list, uint32_t* count) {
+// the live ones of bricks [first, first + total)
+__global__ void k_compact(const uint8_t* live, uint32_t first, uint32_t total, uint32_t* list, uint32_t* count) {
   const int lane = threadIdx.x & 31;
   // grid-stride over bricks, warp-aggregated append (ballot + popc)
   for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < total;
        i0 += gridDim.x * blockDim.x) {
     const uint32_t i = i0 + lane;
-    const bool keep = i < total && live[i];
+    const bool keep = i < total && live[first + i];
     const unsigned m = __ballot_sync(0xFFFFFFFFu, keep);
     uint32_t base = 0;
     if (lane == 0 && m) base = atomicAdd(count, __popc(m));
     base = __shfl_sync(0xFFFFFFFFu, base, 0);
-    if (keep) list[base + __popc(m & ((1u << lane) - 1u))] = i;
+    if (keep) list[base + __popc(m & ((1u << lane) - 1u))] = first + i;
   }
 }
 
@@ -1160,11 +1161,11 @@ void mark_live(cudaStream_t st, const JobDesc* dj, const uint32_t* brick_job,
   if (total_bricks)
     k_mark_live<<<grid_for(total_bricks, 1, 1 << 20), 256, 0, st>>>(dj, brick_job, total_bricks, live);
 }
-void compact_live(cudaStream_t st, const uint8_t* live, uint32_t total_bricks, uint32_t* list,
+void compact_live(cudaStream_t st, const uint8_t* live, uint32_t first, uint32_t total_bricks, uint32_t* list,
                   uint32_t* count) {
   cudaMemsetAsync(count, 0, sizeof(uint32_t), st);
   if (total_bricks)
-    k_compact<<<grid_for(total_bricks, 256, 4096), 256, 0, st>>>(live, total_bricks, list, count);
+    k_compact<<<grid_for(total_bricks, 256, 4096), 256, 0, st>>>(live, first, total_bricks, list, count);
 }
 
 }  // namespace vfk

@@ -1,4 +1,4 @@
-"""Ray batches (csrc/vf_impact.cu) where their path changes: 4096 rays, cells of
+"""Ray batches (csrc/vf_impact.cu) where their path changes: 32768 rays, cells of
 8 and of 16 voxels with ragged last ones, directions of zero.  Entry voxels must
 equal the oracle's."""
 import numpy as np
@@ -24,8 +24,8 @@ def _rays(dims, n, rng):
     return r
 
 
-@pytest.mark.parametrize("dims,n", [((9, 17, 33), 4095), ((9, 17, 33), 4096), ((2, 2, 2), 5000), ((70, 64, 95), 40001),
-                                    ((1000, 300, 520), 9000)])
+@pytest.mark.parametrize("dims,n", [((9, 17, 33), 4095), ((9, 17, 33), 32767), ((9, 17, 33), 32768), ((2, 2, 2), 33000),
+                                    ((70, 64, 95), 40001), ((12, 14, 600), 33000), ((1000, 300, 520), 33000)])
 def test_entry_voxels(vf, ctx, dims, n):
     rng = np.random.default_rng(n)
     lab = np.zeros(dims, np.uint16)
@@ -40,7 +40,7 @@ def test_entry_voxels(vf, ctx, dims, n):
     g.close()
 
 
-@pytest.mark.parametrize("n", [10, 5000])
+@pytest.mark.parametrize("n", [10, 5000, 40000])
 def test_zero_direction(vf, ctx, n):
     g = vf.RegularGrid((8, 8, 8), np.zeros(3, np.float32), np.full(3, 8, np.float32), ctx)
     rays = _rays(np.array((8, 8, 8)), n, np.random.default_rng(1))

@@ -339,13 +339,35 @@ __device__ unsigned long long block_excl_scan(unsigned long long v, unsigned lon
   return r;
 }
 __global__ void __launch_bounds__(1024) k_scan_local(const uint32_t* in, unsigned long long* out,
-                                                     unsigned long long* sums, uint32_t n) {
+                                                     unsigned long long* sums, uint32_t n,
+                                                     unsigned long long* grand) {
   const uint32_t i = blockIdx.x * 1024u + threadIdx.x;
   const unsigned long long v = i < n ? in[i] : 0ull;
   __shared__ unsigned long long tot;
   const unsigned long long r = block_excl_scan(v, &tot);
   if (i < n) out[i] = r;
-  if (threadIdx.x == 0) sums[blockIdx.x] = tot;
+  if (threadIdx.x == 0) {
+    sums[blockIdx.x] = tot;
+    if (gridDim.x == 1) *grand = tot;  // nothing to add
+  }
+}
+// up to 1024 blocks: each adds up the sums before it, and adds them to its own
+// values; the last one knows the total
+__global__ void __launch_bounds__(1024) k_scan_base(unsigned long long* out, const unsigned long long* sums, uint32_t n,
+                                                    unsigned long long* grand) {
+  const uint32_t b = blockIdx.x, t = threadIdx.x;
+  __shared__ unsigned long long ws[32];
+  unsigned long long v = t < b ? sums[t] : 0ull;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+  if ((t & 31) == 0) ws[t >> 5] = v;
+  __syncthreads();
+  v = ws[t & 31];
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+  const uint32_t i = b * 1024u + t;
+  if (i < n) out[i] += v;
+  if (b == gridDim.x - 1 && t == 0) *grand = v + sums[b];
 }
 __global__ void __launch_bounds__(1024) k_scan_sums(unsigned long long* sums, uint32_t nb,
                                                     unsigned long long* grand) {
@@ -1115,10 +1137,7 @@ void tetra_prep(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs,
 void parity_raster(cudaStream_t st, const JobDesc* dj, const JobState* ds, int njobs,
                    uint32_t total_faces, const FaceScratch& fs, int num_sms, int grid_mult) {
   if (!total_faces) return;
-  const uint32_t nb = (total_faces + 1023) / 1024;
-  k_scan_local<<<nb, 1024, 0, st>>>(fs.pcnt, fs.pbase, fs.psums, total_faces);
-  k_scan_sums<<<1, 1024, 0, st>>>(fs.psums, nb, fs.ptotal);
-  k_scan_add<<<(total_faces + 255) / 256, 256, 0, st>>>(fs.pbase, fs.psums, total_faces);
+  exclusive_scan(st, fs.pcnt, fs.pbase, fs.psums, total_faces, fs.ptotal);
   k_parity_flat<<<num_sms * grid_mult, 256, 0, st>>>(dj, njobs, fs.pcnt, fs.pbase, fs.ptotal, total_faces);
   const unsigned gy = (unsigned)(njobs < 65535 ? njobs : 65535);
   k_odd_edges<<<dim3(std::max(1, num_sms * 8 / njobs), gy), 256, 0, st>>>(dj, ds, njobs);
@@ -1132,7 +1151,12 @@ void exclusive_scan(cudaStream_t st, const uint32_t* in, unsigned long long* out
     return;
   }
   const uint32_t nb = (n + 1023) / 1024;
-  k_scan_local<<<nb, 1024, 0, st>>>(in, out, sums, n);
+  k_scan_local<<<nb, 1024, 0, st>>>(in, out, sums, n, total);
+  if (nb == 1) return;
+  if (nb <= 1024) {  // a launch less (3 us); the blocks read nb * nb / 2 sums in all
+    k_scan_base<<<nb, 1024, 0, st>>>(out, sums, n, total);
+    return;
+  }
   k_scan_sums<<<1, 1024, 0, st>>>(sums, nb, total);
   k_scan_add<<<(n + 255) / 256, 256, 0, st>>>(out, sums, n);
 }

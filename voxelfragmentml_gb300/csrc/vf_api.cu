@@ -617,9 +617,9 @@ vf_status vf_grid_triangulate(vf_grid* g, const vf_mc_params* mp, uint32_t* nmes
     sc[a] = size / (float)d[a];
     c0[a] = g->job.aabb_min[a] - sc[a];
   }
-  // the split's scratch is free again: boundary vertices per chunk of 2048
+  // the split's scratch is free again: boundary vertices per chunk
   const bool smooth = (mp->nonboundary_iterations || mp->boundary_iterations) && V && T;
-  if (smooth) VF_CK(cudaMemsetAsync(hist, 0, ((V + 2047) / 2048) * 4, st));
+  if (smooth) VF_CK(cudaMemsetAsync(hist, 0, (size_t)vfk::inc_chunks(V) * 4, st));
   vfk::mc_outputs(st, G, vperm, vown, vflag, V, sc, c0, vinv, vert, tperm, tv, T, gface, smooth ? hist : nullptr, nsm);
   VF_CK(cudaEventRecord(M.ev[3], st));
   auto item = static_cast<uint32_t*>(M.item.p);

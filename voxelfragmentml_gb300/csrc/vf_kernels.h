@@ -86,7 +86,10 @@ size_t split_hist_words(uint64_t n);
 void stable_split16(cudaStream_t st, const uint16_t* key, uint64_t n, uint32_t nkeys, uint32_t* tmp,
                     uint32_t* out, uint32_t* hist, unsigned long long* hbase,
                     unsigned long long* sums, unsigned long long* tot, unsigned long long* off);
-// bnd (or NULL): zeroed counts of the boundary vertices of each 2048 vertices
+// bnd (or NULL): inc_chunks(V) zeroed counts, of the boundary vertices of each
+// inc_chunk(V) vertices
+uint32_t inc_chunk(uint64_t V);
+uint32_t inc_chunks(uint64_t V);
 void mc_outputs(cudaStream_t st, const MeshGrid& G, const uint32_t* vperm,
                 const unsigned long long* vown, const uint32_t* vflag, uint64_t V, const float s[3],
                 const float c[3], uint32_t* vinv, float4* vert, const uint32_t* tperm,

@@ -612,16 +612,12 @@ __global__ void __launch_bounds__(256) k_ms_scatter(const uint16_t* key, const u
     if (dig[k] < 256u) out[cnt[w][dig[k]] + rank[k]] = item[k];
 }
 
-// a chunk of vertices of the neighbour lists: the CTA of k_inc_lists; bnd counts
-// the boundary vertices of each
-constexpr uint32_t INC_CHUNK = 2048;
-
 // ---- outputs ---------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_mc_vout(vfk::MeshGrid G, const uint32_t* vperm,
                                                  const unsigned long long* vown,
                                                  const uint32_t* vflag, uint64_t V, float sx,
                                                  float sy, float sz, float cx, float cy, float cz,
-                                                 uint32_t* vinv, float4* out, uint32_t* bnd) {
+                                                 uint32_t* vinv, float4* out, uint32_t chunk, uint32_t* bnd) {
   const uint64_t YZ = (uint64_t)G.Y * G.Zp;
   const uint64_t n = (V + 31) & ~31ull;  // whole warps, for the ballot
   for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < n;
@@ -629,7 +625,7 @@ __global__ void __launch_bounds__(256) k_mc_vout(vfk::MeshGrid G, const uint32_t
     const uint32_t gv = s < V ? vperm[s] : 0u;
     const uint32_t flag = s < V ? (vflag[gv >> 5] >> (gv & 31u)) & 1u : 0u;
     const unsigned m = __ballot_sync(FULL, flag);
-    if (bnd && m && (threadIdx.x & 31) == 0) atomicAdd(bnd + s / INC_CHUNK, (uint32_t)__popc(m));
+    if (bnd && m && (threadIdx.x & 31) == 0) atomicAdd(bnd + (uint32_t)s / chunk, (uint32_t)__popc(m));
     if (s >= V) continue;
     vinv[gv] = (uint32_t)s;
     const unsigned long long own = vown[gv];
@@ -717,7 +713,8 @@ __global__ void __launch_bounds__(256) k_inc_fill(const uint4* gface, const floa
 // item lists the vertices of one smoothing pass from its front (non-boundary) and
 // those of the other from its back, each with meta: x = first entry, y = count of
 // summed positions (2 per face incidence, 16 bits) | entries << 16 (15 bits).
-// Items keep the vertices' order (bbase: boundary vertices before each chunk), so
+// Items keep the vertices' order (bbase: boundary vertices before each chunk of
+// vertices, a CTA's), so
 // the passes find neighbours near each other; entries are reserved per warp, in
 // whole 128-byte lines (any place will do).  Up to INC_FAST incidences fold in registers, more in place.
 // stats: [0] boundary vertices, [1] neighbour entries of boundary vertices,
@@ -726,7 +723,8 @@ __global__ void __launch_bounds__(256) k_inc_fill(const uint4* gface, const floa
 // 165 us, and 320 us in separate passes that fold in memory, scan and copy.
 constexpr uint32_t INC_FAST = 8;
 __global__ void __launch_bounds__(256) k_inc_lists(const unsigned long long* start, uint2* ent,
-                                                   const float4* vert, uint64_t V, const unsigned long long* bbase, uint32_t* nbr,
+                                                   const float4* vert, uint64_t V, uint32_t chunk,
+                                                   const unsigned long long* bbase, uint32_t* nbr,
                                                    uint32_t* item, uint2* meta, uint32_t* err,
                                                    unsigned long long* stats) {
   __shared__ uint32_t stage[8][32 * 2 * INC_FAST];
@@ -734,7 +732,7 @@ __global__ void __launch_bounds__(256) k_inc_lists(const unsigned long long* sta
   const float* vw = reinterpret_cast<const float*>(vert) + 3;
   const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const unsigned lt = (1u << lane) - 1u;
-  const uint64_t from = (uint64_t)blockIdx.x * INC_CHUNK, to = min(from + INC_CHUNK, V);
+  const uint64_t from = (uint64_t)blockIdx.x * chunk, to = min(from + chunk, V);
   if (t < 2) s_ents[t] = 0;
   const uint32_t bnds = (uint32_t)bbase[blockIdx.x];
   uint32_t next0 = (uint32_t)from - bnds, next1 = (uint32_t)(V - stats[0]) + bnds, bent = 0, ents = 0;
@@ -863,11 +861,13 @@ __global__ void __launch_bounds__(256) k_lap_gather(const float4* src, float4* d
                                                     const uint2* meta, const uint32_t* nbr, uint64_t V,
                                                     const unsigned long long* stats, int back, float omw,
                                                     float weight) {
-  const uint64_t nb = V - stats[0], to = back ? V : nb;
-  for (uint64_t i = (back ? nb : 0) + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < to;
-       i += (uint64_t)gridDim.x * blockDim.x) {
+  // the other pass from the back, so that no load waits for the count
+  const uint64_t nb = V - stats[0];
+  for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < V; k += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t i = back ? V - 1 - k : k;
     const uint2 m = meta[i];
     const uint32_t u = item[i];
+    if (back ? i < nb : i >= nb) break;
     float4 p = src[u];
     const uint32_t cnt = m.y & 0xFFFFu, len = (m.y >> 16) & 0x7FFFu;
     if (cnt) {
@@ -999,13 +999,20 @@ void stable_split16(cudaStream_t st, const uint16_t* key, uint64_t n, uint32_t n
   k_mc_offsets<<<ob, 256, 0, st>>>(key, out, n, nkeys, passes == 1 ? hbase : nullptr, nchunks, off);
 }
 
+// vertices of a CTA of k_inc_lists: 256 at a time, 2048 at most; small meshes are
+// spread over up to 1024 CTAs (100 k vertices: lists 53 us, 113 in chunks of 2048)
+uint32_t inc_chunk(uint64_t V) {
+  return 256u * (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(8, (V + 256 * 1024 - 1) / (256 * 1024)));
+}
+uint32_t inc_chunks(uint64_t V) { return (uint32_t)((V + inc_chunk(V) - 1) / inc_chunk(V)); }
+
 void mc_outputs(cudaStream_t st, const MeshGrid& G, const uint32_t* vperm,
                 const unsigned long long* vown, const uint32_t* vflag, uint64_t V, const float s[3],
                 const float c[3], uint32_t* vinv, float4* vert, const uint32_t* tperm,
                 const uint4* tv, uint64_t T, uint4* gface, uint32_t* bnd, int num_sms) {
   if (V)
     k_mc_vout<<<grid_for(V, num_sms), 256, 0, st>>>(G, vperm, vown, vflag, V, s[0], s[1], s[2], c[0],
-                                                    c[1], c[2], vinv, vert, bnd);
+                                                    c[1], c[2], vinv, vert, inc_chunk(V), bnd);
   if (T) k_mc_fout<<<grid_for(T, num_sms), 256, 0, st>>>(tperm, tv, vinv, vflag, T, gface);
 }
 
@@ -1025,9 +1032,9 @@ cudaError_t mc_smooth_lists(cudaStream_t st, const uint4* gface, uint64_t T, con
   exclusive_scan(st, deg, start, sums, (uint32_t)V, start + V);
   if ((e = cudaMemsetAsync(deg, 0, V * 4, st))) return e;
   k_inc_fill<<<gt, 256, 0, st>>>(gface, vert, T, start, deg, ent);
-  const uint32_t chunks = (uint32_t)((V + INC_CHUNK - 1) / INC_CHUNK);
+  const uint32_t chunk = inc_chunk(V), chunks = inc_chunks(V);
   exclusive_scan(st, bnd, bbase, sums, chunks, stats);
-  k_inc_lists<<<chunks, 256, 0, st>>>(start, ent, vert, V, bbase, nbr, item, meta, err, stats);
+  k_inc_lists<<<chunks, 256, 0, st>>>(start, ent, vert, V, chunk, bbase, nbr, item, meta, err, stats);
   return cudaGetLastError();
 }
 

@@ -19,7 +19,7 @@ Printed JSON line (rank 0):
   plain     the reference-shaped per-job path (vf_plain_run) on a subset;
   serving   Poisson arrivals through vf_server (continuous batching):
             p50/p99 latency submit -> labels on host, sustained voxels/s;
-  roofline  the flood relaxation kernel against the measured HBM peak;
+  roofline  the flood kernel against the measured HBM peak;
   cpu_baseline the CPU oracle on a bounded sample of the same workload.
 
 `--impl reference` times the reference algorithm's CPU restatement (the

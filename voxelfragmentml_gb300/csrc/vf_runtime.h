@@ -165,7 +165,7 @@ struct Ctx {
   bool dry = false;
   size_t dry_need = 0, dry_freed = 0;
   cudaEvent_t ev[16] = {};
-  // the last flood relaxation issued on any of the context's streams: the
+  // the last flood issued on any of the context's streams: the
   // next one waits for it, so two cooperative (grid-barrier) launches of
   // batches in flight never share the GPU
   cudaEvent_t ev_relax = nullptr;

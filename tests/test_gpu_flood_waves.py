@@ -101,3 +101,21 @@ def test_flood_prefixes_in_a_batch(vf, ctx):
         wants.append(O.run_job(v, f, specs[-1].dims, mn, mx, q, ncounts=256)[:2])
     for r, s, (lab, cnt) in zip(vf.batch_run(specs, ctx), specs, wants):
         assert r.status == 0 and np.array_equal(s.labels, lab) and np.array_equal(s.counts, cnt)
+
+
+def test_labels_dealt_to_resident_blocks(vf, ctx):
+    # more live bricks than resident blocks, jobs changing under a block,
+    # slot planes in one load and past it, bricks that reach past their grid
+    specs, wants = [], []
+    for i in range(48):
+        v, f = Vs.vessel_mesh(20 + i % 5, 15, i)
+        mn, mx = Vs.mesh_aabb(v)
+        p = vf.Params.default(distance=i % 3, num_seeds=(3, 64, 65, 200)[i % 4], seed=i + 1, seed_location=vf.BOTH,
+                              num_extra_seeds=400 if i % 3 == 2 and i % 4 else 0)
+        specs.append(vf.JobSpec(v, f, p, dims=(113 + i % 4, 97 + i % 9, 96 + i), aabb=(mn, mx), ncounts=256))
+        q = O.Params()
+        for name, _ in O.Params._fields_:
+            setattr(q, name, getattr(p, name))
+        wants.append(O.run_job(v, f, specs[-1].dims, mn, mx, q, ncounts=256)[:2])
+    for r, s, (lab, cnt) in zip(vf.batch_run(specs, ctx), specs, wants):
+        assert r.status == 0 and np.array_equal(s.labels, lab) and np.array_equal(s.counts, cnt)

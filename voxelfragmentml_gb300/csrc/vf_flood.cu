@@ -878,81 +878,99 @@ __global__ void __launch_bounds__(256) k_flat_labels(WaveArrays arr, WaveJob W, 
   }
 }
 
-// 8 bits -> 8 bytes of 0 / 1 (low four in .x)
-__device__ __forceinline__ uint2 spread8(uint32_t b) {
-  return make_uint2(((b & 15u) * 0x00204081u) & 0x01010101u, ((b >> 4) * 0x00204081u) & 0x01010101u);
-}
-
 // row states -> labels (undoMask fused: & 0xFF).
-// Live bricks, one per CTA; four lanes per row, each 8 voxels (16 bytes of
-// labels).  EMPTY 0, unclaimed FREE, claimed: the slot's label.
-__global__ void __launch_bounds__(256) k_wave_labels(const JobDesc* jobs, const JobState* st,
-                                                     const uint32_t* list, const uint32_t* count,
-                                                     const uint32_t* brick_job) {
+// Live bricks, dealt to resident CTAs; four lanes per row, each 8 voxels (16 bytes
+// of labels).  EMPTY 0, unclaimed FREE, claimed: the slot's label.  Bound by the
+// chain brick -> job -> rows -> labels, so a CTA keeps its job's label table from
+// brick to brick and reads the next brick's number beside this one's rows (a CTA per
+// brick, each with its own table: 42 us in a 476x476x512 job, 535 us in 128 mixed
+// ones; four CTAs per SM: 30 and 420).  A lane takes the slots of its voxels one
+// after another (most have one, at a border two): a slot's voxels are an and of the
+// planes.
+__global__ void __launch_bounds__(256, 4) k_wave_labels(const JobDesc* jobs, const JobState* st,
+                                                        const uint32_t* list, const uint32_t* count,
+                                                        const uint32_t* brick_job) {
   // fragment of each slot for the job of the current brick (reloaded when the
   // job changes): the seed's, or after a second flood the rank's
   __shared__ uint16_t lab[4096];
-  __shared__ int cached;
-  if (threadIdx.x == 0) cached = -1;
-  __syncthreads();
-  const uint32_t n = *count;
-  for (uint32_t it = blockIdx.x; it < n; it += gridDim.x) {
-    const uint32_t b = list[it];
-    const uint32_t j = brick_job[b];
+  int cached = -1;
+  const uint32_t n = *count, part = threadIdx.x & 3u, sh = 8 * part, row = threadIdx.x >> 2;
+  uint32_t b = blockIdx.x < n ? list[blockIdx.x] : 0u;
+  uint32_t j = blockIdx.x < n ? brick_job[b] : 0u;
+  for (uint32_t it = blockIdx.x; it < n;) {
     const JobDesc& J = jobs[j];
-    if (!J.active) continue;  // uniform across the CTA
     const JobState& s = st[j];
-    if ((int)j != cached) {  // uniform: cached changes only between barriers
+    const bool active = J.active != 0;  // uniform across the CTA
+    const uint32_t lb = b - J.brick_base;
+    const uint32_t bz = lb % J.nbz, by = (lb / J.nbz) % J.nby, bx = lb / (J.nbz * J.nby);
+    const uint32_t x = bx * VF_BX + row / VF_BY, y = by * VF_BY + row % VF_BY, z = bz * VF_BZ + sh;
+    const uint32_t nq = J.wsw / 4;
+    static_assert(64 % VF_BY == 0, "a pass is whole columns of rows");
+    constexpr uint32_t DX = 64 / VF_BY;  // rows of a pass: DX columns
+    const uint4* src = reinterpret_cast<const uint4*>(J.wstate + (size_t)(J.wrow0 + x * J.wsx + bz * J.wsy + y) * J.wsw);
+    const size_t step = (size_t)DX * J.wsx * nq;  // from pass to pass
+    const bool in = active && y < J.Y && z < J.Zp;
+    const uint32_t X = J.X;
+    uint16_t* const grid = J.grid + vf_gidx(J, x, y, z);
+    const size_t gstep = (size_t)DX * J.Y * J.Zp;
+    if (active && (int)j != cached) {  // uniform
       __syncthreads();
       const bool second = s.has_prefix && s.disjoint;
       const uint32_t nl = second ? 256u : min(s.nseeds, 4096u);
       for (uint32_t k = threadIdx.x; k < nl; k += blockDim.x)
         lab[k] = (uint16_t)((second ? s.rank_value[k] : J.seeds[4 * k + 3]) & 0xFFu);
-      if (threadIdx.x == 0) cached = (int)j;
+      cached = (int)j;
       __syncthreads();
     }
-    const uint32_t lb = b - J.brick_base;
-    const uint32_t bz = lb % J.nbz, by = (lb / J.nbz) % J.nby, bx = lb / (J.nbz * J.nby);
-    const uint32_t part = threadIdx.x & 3u, z = bz * VF_BZ + 8 * part;
-    if (z >= J.Zp) continue;
-    const uint32_t nq = J.wsw / 4;
+    it += gridDim.x;
+    if (it < n) {  // the next brick, on its way beside this one's rows
+      b = list[it];
+      j = brick_job[b];
+    }
 #pragma unroll
-    for (int pass = 0; pass < 4; ++pass) {
-      const uint32_t row = (threadIdx.x >> 2) + 64u * pass;
-      const uint32_t x = bx * VF_BX + row / VF_BY, y = by * VF_BY + row % VF_BY;
-      if (x >= J.X || y >= J.Y) continue;
-      const uint4* src = reinterpret_cast<const uint4*>(J.wstate + (size_t)(J.wrow0 + x * J.wsx + bz * J.wsy + y) * J.wsw);
-      const uint4 a = __ldcs(src);
-      const uint32_t sh = 8 * part;
-      const uint32_t v = (a.x >> sh) & 0xFFu, u = ((a.y & ~a.x) >> sh) & 0xFFu;
-      uint4 out = make_uint4(0, 0, 0, 0);
-      if (v | u) {
-        const uint2 us = spread8(u);
-        const uint2 l0 = spread8((a.z >> sh) & 0xFFu), l1 = spread8((a.w >> sh) & 0xFFu);
-        uint2 lo = make_uint2(l0.x | (l1.x << 1), l0.y | (l1.y << 1)), hi = make_uint2(0, 0);  // slot bits 0-7, 8-
-        for (uint32_t k = 1; k < nq; ++k) {
-          const uint4 c = src[k];
-          const uint32_t p[4] = {c.x, c.y, c.z, c.w};
+    for (int pass = 0; pass < 4; pass += 2) {
+      uint4 a[2], c[2];  // planes A, B and slot bits 0 .. 5
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint32_t bit = 4 * k - 2 + i;  // slot bit of plane word 4 k + i
-            const uint2 sp = spread8((p[i] >> sh) & 0xFFu);
-            if (bit < 8) { lo.x |= sp.x << bit; lo.y |= sp.y << bit; }
-            else { hi.x |= sp.x << (bit - 8); hi.y |= sp.y << (bit - 8); }
-          }
+      for (int h = 0; h < 2; ++h) {
+        a[h] = c[h] = make_uint4(0, 0, 0, 0);
+        if (in && x + (pass + h) * DX < X) {
+          a[h] = __ldcs(src + (pass + h) * step);
+          c[h] = __ldcs(src + (pass + h) * step + 1);
         }
-        uint32_t l[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const uint32_t by8 = 8 * (i & 3);
-          const uint32_t slot = (((i < 4 ? lo.x : lo.y) >> by8) & 0xFFu) |
-                                ((((i < 4 ? hi.x : hi.y) >> by8) & 0xFu) << 8);
-          const uint32_t fr = ((i < 4 ? us.x : us.y) >> by8) & 1u;
-          l[i] = (v >> i) & 1u ? (uint32_t)lab[slot] : fr;
-        }
-        out = make_uint4(l[0] | (l[1] << 16), l[2] | (l[3] << 16), l[4] | (l[5] << 16), l[6] | (l[7] << 16));
       }
-      *reinterpret_cast<uint4*>(J.grid + vf_gidx(J, x, y, z)) = out;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (!in || x + (pass + h) * DX >= X) continue;
+        const uint32_t v = (a[h].x >> sh) & 0xFFu, u = ((a[h].y & ~a[h].x) >> sh) & 0xFFu;
+        auto pair = [](uint32_t m) { return ((m & 3u) * 0x8001u) & 0x00010001u; };
+        uint4 out = make_uint4(pair(u), pair(u >> 2), pair(u >> 4), pair(u >> 6));
+        const uint32_t p[6] = {a[h].z >> sh, a[h].w >> sh, c[h].x >> sh, c[h].y >> sh, c[h].z >> sh, c[h].w >> sh};
+        for (uint32_t rem = v; rem;) {
+          const uint32_t k = (uint32_t)__ffs(rem) - 1;
+          uint32_t slot = 0, m = rem;  // the first voxel's slot, and its voxels
+          auto plane = [&](uint32_t w, uint32_t bit) {
+            const uint32_t one = (w >> k) & 1u;
+            slot |= one << bit;
+            m &= w ^ (one - 1u);
+          };
+#pragma unroll
+          for (uint32_t bit = 0; bit < 6; ++bit) plane(p[bit], bit);
+          for (uint32_t q = 2; q < nq; ++q) {  // more than 64 seeds
+            const uint4 e = src[(pass + h) * step + q];
+            plane(e.x >> sh, 4 * q - 2);
+            plane(e.y >> sh, 4 * q - 1);
+            plane(e.z >> sh, 4 * q);
+            plane(e.w >> sh, 4 * q + 1);
+          }
+          const uint32_t L = lab[slot & 4095u];
+          out.x += pair(m) * L;
+          out.y += pair(m >> 2) * L;
+          out.z += pair(m >> 4) * L;
+          out.w += pair(m >> 6) * L;
+          rem &= ~m;
+        }
+        *reinterpret_cast<uint4*>(grid + (pass + h) * gstep) = out;
+      }
     }
   }
 }
@@ -1390,7 +1408,8 @@ void flat_labels(cudaStream_t st, const WaveArrays& arr, const WaveJob& W, const
 
 void flood_labels(cudaStream_t st, const JobDesc* dj, const JobState* ds, const uint32_t* list,
                   const uint32_t* count, uint32_t max_count, const uint32_t* brick_job) {
-  if (max_count) k_wave_labels<<<brick_grid(max_count), 256, 0, st>>>(dj, ds, list, count, brick_job);
+  // resident CTAs: four of 256 threads fit an SM beside their 64 registers
+  if (max_count) k_wave_labels<<<std::min(brick_grid(max_count), 152 * 4), 256, 0, st>>>(dj, ds, list, count, brick_job);
 }
 
 cudaError_t flood_prefixes(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs, const FloodScratch& fs) {

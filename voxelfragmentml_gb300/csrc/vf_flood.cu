@@ -11,8 +11,8 @@
 // The GPU runs those waves bit-parallel.  32 voxels along z are one word of
 // bit planes:
 //
-//   A, B         00 EMPTY, 01 occupied and not claimed yet (U), 10 / 11 claimed
-//                in a wave of even / odd parity (E0, E1)
+//   A, B         EMPTY, occupied and not claimed yet (U), or claimed in a wave of
+//                either parity (E0, E1): vf_wave_state.h
 //   L0 .. L(n-1) the claiming seed's slot, bit by bit
 //
 // and, apart from them, the smallest slot that reaches the word's two end
@@ -23,9 +23,10 @@
 // claims the unclaimed occupied bits it reaches into E((t + 1) & 1).  Every
 // voxel is claimed once.  E(t & 1) also holds the bits of waves t-2, t-4,
 // ..., but no unclaimed voxel is next to one of those (it would have been
-// claimed by the following wave), so they change nothing; and a word's
-// owner changes only bits that the same wave's readers mask out.  So there
-// is no frontier to clear and no race between the words of a wave.
+// claimed by the following wave), so they change nothing; and a row's owner
+// claims with one bit of one plane, which the same wave's readers mask out
+// whether they see it or not, and its slot with it.  So there is no frontier to
+// clear, and no order is needed between the rows' loads and stores of a wave.
 //
 // A lane takes one row (x, y, word) of 32 voxels with its 8 neighbour rows.
 // Rows are numbered linearly with rows of zeros around each axis (WaveJob), so
@@ -74,6 +75,7 @@
 #include <vector>
 
 #include "vf_kernels.h"
+#include "vf_wave_state.h"
 
 namespace {
 
@@ -220,10 +222,8 @@ __device__ __forceinline__ uint32_t visit_row(const WaveArrays& arr, const JobRo
   // a claim at a word end names rows beyond it unseen: the ones in the zeros
   // around the grid whose own neighbours would lie outside the job
   if (i < J.lo || i >= J.hi) return 0;
-  const bool par = t & 1u;
   uint32_t* const p0 = arr.state + (size_t)i * SW;
   const size_t xs = (size_t)sx * SW;
-  const uint32_t pm = par ? 0u : FULL;  // A & (B ^ pm): claimed with this wave's parity
   uint32_t A4, B4, O[NB], U[9], F[9], P[9][NB];
   // the 3 x 3 rows around the row (6: the cross)
 #pragma unroll
@@ -235,8 +235,8 @@ __device__ __forceinline__ uint32_t visit_row(const WaveArrays& arr, const JobRo
     }
     uint32_t w[SW];
     load_row<NB>((dx < 0 ? p0 - xs : (dx > 0 ? p0 + xs : p0)) + dy * SW, w);
-    U[r] = w[1] & ~w[0];
-    F[r] = w[0] & (w[1] ^ pm);
+    U[r] = wave_unclaimed(w[0], w[1]);
+    F[r] = wave_front(w[0], w[1], t);
 #pragma unroll
     for (int b = 0; b < NB; ++b) P[r][b] = w[2 + b];
     if (r == 4) {
@@ -286,8 +286,9 @@ __device__ __forceinline__ uint32_t visit_row(const WaveArrays& arr, const JobRo
   U[4] &= ~N;
   {
     uint32_t w[SW];
-    w[0] = A4 | N;
-    w[1] = par ? B4 & ~N : B4;  // B is set for U: claims of odd waves + 1 clear it
+    w[0] = A4;
+    w[1] = B4;
+    wave_claim(w[0], w[1], N, t);
 #pragma unroll
     for (int b = 0; b < SW - 2; ++b) w[2 + b] = b < NB ? (O[b < NB ? b : 0] & ~N) | (L[b < NB ? b : 0] & N) : 0u;
 #pragma unroll
@@ -616,7 +617,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_wave(WaveAr
 }
 
 // ---------------------------------------------------------------------------
-// Row states from the label grid: occupied voxels unclaimed, all else zero,
+// Row states from the label grid: occupied voxels unclaimed, all else EMPTY,
 // the rows around the grid included (bricks without occupied voxels are not
 // read).  A CTA takes 256 consecutive rows of one job, eight lanes per row, 4
 // voxels per lane (a warp instruction reads 4 whole 64-byte rows); the lanes
@@ -655,7 +656,7 @@ __global__ void __launch_bounds__(256) k_wave_init(const JobDesc* jobs, WaveArra
     for (int o = 1; o < 8; o <<= 1) w |= __shfl_xor_sync(FULL, w, o);
     uint32_t* d = arr.state + (size_t)row * J.wsw;  // up to the next job's base
 
-    for (uint32_t k = q; k < J.wsw; k += 8) d[k] = k == 1 ? w : 0u;
+    for (uint32_t k = q; k < J.wsw; k += 8) d[k] = k == 0 ? wave_empty_a(w) : (k == 1 ? wave_empty_b(w) : 0u);
     if (q < 4) reinterpret_cast<uint32_t*>(arr.in + 2 * (size_t)row)[q] = 0xFFFFFFFFu;
   }
 }
@@ -683,7 +684,7 @@ __global__ void __launch_bounds__(256) k_wave_planes(const JobDesc* jobs, WaveAr
       }
     }
     uint4* const d = reinterpret_cast<uint4*>(arr.state + (size_t)row * J.wsw);  // up to the next job's base
-    d[0] = make_uint4(0u, w, 0u, 0u);
+    d[0] = make_uint4(wave_empty_a(w), wave_empty_b(w), 0u, 0u);
     for (uint32_t k = 1; k < J.wsw / 4; ++k) d[k] = make_uint4(0u, 0u, 0u, 0u);
     reinterpret_cast<uint4*>(arr.in)[row] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
   }
@@ -754,7 +755,7 @@ __device__ void seed_waves(const WaveArrays& arr, const WaveJob& W, uint32_t* uf
     const uint32_t zw = z >> 5, bit = 1u << (z & 31u);
     const uint32_t row = W.row0 + x * W.sx + zw * W.sy + y;
     uint32_t* d = arr.state + (size_t)row * sw;
-    atomicOr(d, bit);  // E0
+    atomicAnd(d, ~bit);  // E0
     atomicAnd(d + 1, ~bit);
     for (int b = 0; b < nb; ++b)
       if ((i >> b) & 1u) atomicOr(d + 2 + b, bit);
@@ -808,7 +809,8 @@ __global__ void __launch_bounds__(256) k_flat_init(const uint16_t* grid, WaveArr
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t box = (A.nx + 2) * W.sx, nwarps = (gridDim.x * blockDim.x) >> 5;
   auto put = [&](uint32_t row, uint32_t m) {
-    if (lane < sw) arr.state[(size_t)row * sw + lane] = lane == 1 ? m : 0u;
+    if (lane < sw)
+      arr.state[(size_t)row * sw + lane] = lane == 0 ? wave_empty_a(m) : (lane == 1 ? wave_empty_b(m) : 0u);
     if (lane < 4) reinterpret_cast<uint32_t*>(arr.in + 2 * (size_t)row)[lane] = 0xFFFFFFFFu;
   };
   for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < box; k += nwarps) {
@@ -866,12 +868,12 @@ __global__ void __launch_bounds__(256) k_flat_labels(WaveArrays arr, WaveJob W, 
     const bool in = flat_row(W, A, k, lane, row, at);
     if (!__any_sync(FULL, in)) continue;
     const uint32_t word = lane < sw ? arr.state[(size_t)row * sw + lane] : 0u;
-    const uint32_t v = __shfl_sync(FULL, word, 0);
-    const uint32_t u = __shfl_sync(FULL, word, 1) & ~v;
+    const uint32_t a = __shfl_sync(FULL, word, 0), b = __shfl_sync(FULL, word, 1);
+    const uint32_t v = wave_claimed(a, b), u = wave_unclaimed(a, b);
     uint32_t l = (u >> lane) & 1u;
     if (v) {  // uniform
       uint32_t slot = 0;
-      for (uint32_t b = 0; b + 2 < sw; ++b) slot |= ((__shfl_sync(FULL, word, 2 + b) >> lane) & 1u) << b;
+      for (uint32_t k = 0; k + 2 < sw; ++k) slot |= ((__shfl_sync(FULL, word, 2 + k) >> lane) & 1u) << k;
       if ((v >> lane) & 1u) l = seeds[4 * slot + 3] & 0xFFu;
     }
     if (in) labels[at] = (uint16_t)l;
@@ -941,7 +943,8 @@ __global__ void __launch_bounds__(256, 4) k_wave_labels(const JobDesc* jobs, con
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         if (!in || x + (pass + h) * DX >= X) continue;
-        const uint32_t v = (a[h].x >> sh) & 0xFFu, u = ((a[h].y & ~a[h].x) >> sh) & 0xFFu;
+        const uint32_t v = (wave_claimed(a[h].x, a[h].y) >> sh) & 0xFFu,
+                       u = (wave_unclaimed(a[h].x, a[h].y) >> sh) & 0xFFu;
         auto pair = [](uint32_t m) { return ((m & 3u) * 0x8001u) & 0x00010001u; };
         uint4 out = make_uint4(pair(u), pair(u >> 2), pair(u >> 4), pair(u >> 6));
         const uint32_t p[6] = {a[h].z >> sh, a[h].w >> sh, c[h].x >> sh, c[h].y >> sh, c[h].z >> sh, c[h].w >> sh};
@@ -1023,7 +1026,7 @@ __global__ void __launch_bounds__(256) k_slot_unions(const JobDesc* jobs, const 
   const uint32_t i = blockIdx.x * 256u + threadIdx.x, sw = J.wsw, nb = sw - 2;
   if (i < W.row0 || i + W.sx + W.sy + 1 >= W.base + W.nrows) return;
   const uint32_t* p = arr.state + (size_t)i * sw;
-  const uint32_t V = p[0];
+  const uint32_t V = wave_claimed(p[0], p[1]);
   if (!V) return;
   uint32_t L[14];
 #pragma unroll
@@ -1032,7 +1035,7 @@ __global__ void __launch_bounds__(256) k_slot_unions(const JobDesc* jobs, const 
   auto join = [&](uint32_t r, int s) {
     const uint32_t* q = arr.state + (size_t)r * sw;
     auto shift = [s](uint32_t v) { return s == 0 ? v : (s == 1 ? v >> 1 : (s == -1 ? v << 1 : v << 31)); };
-    const uint32_t both = V & shift(q[0]);
+    const uint32_t both = V & shift(wave_claimed(q[0], q[1]));
     if (!both) return;
     uint32_t d = 0;
 #pragma unroll
@@ -1159,7 +1162,7 @@ __global__ void __launch_bounds__(256) k_slot_reset(const JobDesc* jobs, const J
   const uint32_t i = blockIdx.x * 256u + threadIdx.x, sw = J.wsw;
   if (i < W.row0 || i + W.sx + W.sy + 1 >= W.base + W.nrows) return;
   uint32_t* p = arr.state + (size_t)i * sw;
-  uint32_t v = p[0], u = p[1] & ~v;
+  uint32_t v = wave_claimed(p[0], p[1]), u = wave_unclaimed(p[0], p[1]);
   if (!(u | v)) return;
   uint32_t L[14], w[14];
 #pragma unroll
@@ -1191,8 +1194,8 @@ __global__ void __launch_bounds__(256) k_slot_reset(const JobDesc* jobs, const J
     }
   }
   u |= v & ~keep;
-  p[0] = keep;
-  p[1] = u;
+  p[0] = wave_empty_a(u | keep);  // the survivors as E0
+  p[1] = wave_empty_b(u);
 #pragma unroll
   for (uint32_t b = 0; b < 14; ++b)
     if (b < sw - 2) p[2 + b] = w[b];

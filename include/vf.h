@@ -354,7 +354,9 @@ vf_status vf_batch_execute(vf_ctx* ctx, int download, vf_job_result* results);
  * host read per BFS wave (the reference's execution shape). */
 vf_status vf_plain_run(vf_ctx* ctx, const vf_job* jobs, uint32_t njobs,
                        vf_job_result* results);
-/* device bytes vf_batch_run needs for these jobs (admission control) */
+/* device bytes vf_batch_run needs for this job alone (admission control).  Jobs of one
+ * batch can need more together: their floods share the widest job's state width,
+ * which the server counts when it packs a micro-batch. */
 size_t vf_job_footprint(const vf_job* job);
 
 /* ---- serving: continuous batching ---------------------------------------

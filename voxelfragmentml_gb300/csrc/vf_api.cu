@@ -1438,7 +1438,6 @@ struct vf_server {
     vf_job job;
     uint64_t ticket;
     double submit_ms;
-    size_t footprint;
   };
   struct Slot {
     vfr::Batch b;
@@ -1492,11 +1491,15 @@ void vf_server::loop() {
     for (Slot& s : slots) {
       if (s.busy || pending.empty()) continue;
       std::vector<Pending> take;
+      vfr::Footprint need;  // of `take` as one batch
       size_t fp = 0;
-      while (!pending.empty() && take.size() < max_batch &&
-             (take.empty() ? in_flight_bytes + pending.front().footprint <= budget || in_flight_bytes == 0
-                           : in_flight_bytes + fp + pending.front().footprint <= budget)) {
-        fp += pending.front().footprint;
+      while (!pending.empty() && take.size() < max_batch) {
+        vfr::Footprint with = need;
+        with.add(pending.front().job);
+        // a job alone is taken when nothing else is in flight, whatever it needs
+        if (in_flight_bytes + with.bytes() > budget && !(take.empty() && in_flight_bytes == 0)) break;
+        need = with;
+        fp = need.bytes();
         take.push_back(pending.front());
         pending.pop_front();
       }
@@ -1578,7 +1581,6 @@ vf_status vf_server_submit(vf_server* s, const vf_job* job, uint64_t* ticket) {
   p.job = *job;
   p.ticket = s->next_ticket++;
   p.submit_ms = s->now_ms();
-  p.footprint = vfr::job_footprint(*job);
   s->pending.push_back(p);
   if (ticket) *ticket = p.ticket;
   s->cv.notify_all();

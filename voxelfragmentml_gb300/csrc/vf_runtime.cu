@@ -286,24 +286,36 @@ static uint32_t edge_slots(uint32_t nfaces) {
   return (uint32_t)std::min<uint64_t>(c, 1ull << 31);
 }
 
-// most seeds a flood of these parameters can have (Batch::plan's given seeds aside)
+// most seeds a flood of these parameters can have (Batch::plan's given seeds aside);
+// the parameters may not have been checked yet
 static uint32_t wave_seeds(const vf_params& q) {
-  const int32_t n = q.num_seeds + (q.num_impacts > 0 ? q.bias_seeds : 0);
-  return (uint32_t)std::max(q.num_extra_seeds > 0 ? 2 * n + q.num_extra_seeds : n, 1);
+  const int64_t n = (int64_t)q.num_seeds + (q.num_impacts > 0 ? q.bias_seeds : 0);
+  const int64_t all = q.num_extra_seeds > 0 ? 2 * n + q.num_extra_seeds : n;
+  return (uint32_t)std::min<int64_t>(std::max<int64_t>(all, 1), VF_MAX_SEEDS);
 }
 
-size_t job_footprint(const vf_job& j) {
+void Footprint::add(const vf_job& j) {
   uint32_t d[3] = {j.dims[0], j.dims[1], j.dims[2]};
   if (!d[0] && !d[1] && !d[2]) d[0] = d[1] = d[2] = j.max_dim;
   const size_t X = d[0], Y = d[1], Z = d[2];
   const size_t Zp = vf_roundup((uint32_t)Z, 8), Zw = (Z + 31) / 32;
-  size_t b = X * Y * Zp * 2 * 2 + X * Y * Zw * 4 * 2 + (size_t)j.nfaces * (48 + 4 + 12) +
-             (size_t)edge_slots(j.nfaces) * 8 + (size_t)j.nverts * 12 + 65536;
-  if (j.params.algorithm == VF_FLOOD)  // row states, what reaches their ends, two sets of candidate words
-    b += vfk::wave_rows((uint32_t)X, (uint32_t)Y, (uint32_t)Zw) * (4 * vfk::wave_state_words(wave_seeds(j.params)) + 17);
+  // labels twice, bit planes; per face: tetrahedron, range, indices, work list
+  fixed += X * Y * Zp * 2 * 2 + X * Y * Zw * 4 * 2 + (size_t)j.nfaces * (48 + 4 + 12 + 12) +
+           (size_t)edge_slots(j.nfaces) * 8 + (size_t)j.nverts * 12 + 65536;
+  if (j.params.algorithm == VF_FLOOD) {
+    rows += (vfk::wave_rows((uint32_t)X, (uint32_t)Y, (uint32_t)Zw) + 255) / 256 * 256;
+    words = std::max(words, vfk::wave_state_words(wave_seeds(j.params)));
+  }
   // per brick: owner, live flag, list
-  b += ((X + VF_BX - 1) / VF_BX) * ((Y + VF_BY - 1) / VF_BY) * ((Z + VF_BZ - 1) / VF_BZ) * (4 + 1 + 4);
-  return b;
+  fixed += ((X + VF_BX - 1) / VF_BX) * ((Y + VF_BY - 1) / VF_BY) * ((Z + VF_BZ - 1) / VF_BZ) * (4 + 1 + 4);
+}
+size_t Footprint::bytes() const {  // row states, what reaches their ends, two sets of candidate words
+  return fixed + (size_t)rows * (4 * words + 17);
+}
+size_t job_footprint(const vf_job& j) {
+  Footprint f;
+  f.add(j);
+  return f.bytes();
 }
 
 vf_status Batch::plan(const vf_job* const* js, uint32_t n) {

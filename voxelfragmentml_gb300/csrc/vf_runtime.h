@@ -193,6 +193,15 @@ struct Ctx {
   void free_buf(DevBuf& b);
 };
 
+// Device memory of a batch of jobs.  The floods of a batch share one state width, the
+// widest of its jobs (Batch::plan), so a batch can need more than its jobs one by one.
+struct Footprint {
+  size_t fixed = 0;
+  uint64_t rows = 0;   // of the floods' states
+  uint32_t words = 8;  // of a row, at least 8
+  void add(const vf_job& j);
+  size_t bytes() const;
+};
 size_t job_footprint(const vf_job& j);
 
 }  // namespace vfr

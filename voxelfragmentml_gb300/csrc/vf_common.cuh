@@ -121,6 +121,7 @@ struct JobState {
   uint32_t passes;
   uint32_t nranks;
   uint32_t odd_edges;       // mesh edges used an odd number of times
+  uint32_t wave_voxels;     // occupied voxels of a small flood
 };
 
 // ---------------------------------------------------------------------------

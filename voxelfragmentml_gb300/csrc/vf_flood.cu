@@ -42,10 +42,11 @@
 // CTAs that flood a set of jobs in step (vfk::WaveGang): wave t of all of them,
 // then the gang's barrier.  A batch has two gangs of one CTA per SM, so that
 // one gang's scan and barrier run under the other's visits; jobs of a batch of
-// small ones, and a small job alone, have a CTA each, which synchronises with
-// __syncthreads and keeps the candidate words in shared memory.  The barrier
-// of a larger gang is a counter in global memory whose spin is bounded (it
-// sets an error word and the kernel returns instead of hanging).
+// small ones, and a small job alone, have a gang each, of one CTA where they hold
+// few voxels, which synchronises with __syncthreads and keeps the candidate words
+// in shared memory.  The barrier of a larger gang is a counter in global memory
+// whose spin is bounded (it sets an error word and the kernel returns instead of
+// hanging).
 //
 // What bounds it: the latency of a wave's four steps (scan, row list, visits,
 // barrier), each 1300 to 4000 cycles, while the front is small, and the L1's
@@ -92,10 +93,16 @@ constexpr int SCAN = 4;                   // times 32 candidate words a warp rea
 constexpr uint32_t WORDS = 1024;          // words with candidates listed per round
 constexpr uint32_t LIST = 2048;           // rows of each kind listed per round
 constexpr uint32_t UNITS = 2048;          // units of 256 rows a CTA keeps a list of
-// floods of at most this many rows get a CTA of their own: a wave of theirs is one
-// or two passes of 512 threads, and without a global barrier 60 x 57 x 64 voxels
-// (10.8 k rows) take 0.29 ms against 0.31 on three CTAs and 0.33 on six
+// Floods of at most SMALL_ROWS rows (64^3 voxels: 12.9 k) have a gang each in a batch,
+// and the candidate words of one CTA hold them.  One with at most LONE_VOXELS occupied
+// voxels, counted with its row states, runs on the first CTA of its gang alone,
+// without a global barrier: its waves are a pass or two of one CTA.  Flood of 64 x 64
+// x 64 voxels, Manhattan, on one CTA and on 13: a wall of 40 k voxels 287 and 293 us,
+// a vessel of 38 k in 60 x 57 x 64 268 and 291; a ball of 58 k in 48^3 225 and 184, of
+// 137 k 410 and 229, a full cube 918 and 334 (328 us by relaxing bricks; the rows
+// alone do not tell these apart).
 constexpr uint32_t SMALL_ROWS = 16384;
+constexpr uint32_t LONE_VOXELS = 48 << 10;
 constexpr uint32_t PRUNE = 16;            // waves between dropping the finished jobs' units
 
 struct WaveArgs {
@@ -112,6 +119,7 @@ struct WaveArgs {
   uint32_t* wave_sizes;      // rows visited in each of the first 256 waves (or null)
   uint32_t wait_spins;       // polls of a gang barrier before it gives up
   uint32_t smem_words;       // candidate words that fit the shared memory of a one-CTA gang
+  uint32_t lone_voxels;      // small floods of at most so many voxels run on one CTA
 };
 
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
@@ -372,9 +380,13 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_wave(WaveAr
       G = a.gangs[en.gang];
       s_rank = en.rank;
       s_size = en.size;
+      if (en.size > 1 && G.count == 1 && G.units * 256 <= SMALL_ROWS &&
+          a.st[a.jobs[G.first].job].wave_voxels <= a.lone_voxels)
+        s_size = 1;  // the first CTA's alone
       s_n[0][0] = s_n[0][1] = s_n[1][0] = s_n[1][1] = s_w[0] = s_w[1] = s_any[0] = s_any[1] = s_again[0] = s_again[1] = 0;
     }
     __syncthreads();
+    if (s_rank >= s_size) continue;
     const uint32_t rank = s_rank, size = s_size, first = G.first, njobs = G.count;
     const uint32_t word_lo = G.unit_lo * 8, words = G.units * 8;
     for (uint32_t j = tid; j < njobs; j += THREADS) {
@@ -617,12 +629,19 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1) k_wave(WaveAr
 }
 
 // ---------------------------------------------------------------------------
+__device__ __forceinline__ void add_voxels(uint32_t* to, uint32_t n) {
+  n = __reduce_add_sync(FULL, n);
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(to, n);
+}
+
 // Row states from the label grid: occupied voxels unclaimed, all else EMPTY,
 // the rows around the grid included (bricks without occupied voxels are not
 // read).  A CTA takes 256 consecutive rows of one job, eight lanes per row, 4
 // voxels per lane (a warp instruction reads 4 whole 64-byte rows); the lanes
 // then write the row's state together.
-__global__ void __launch_bounds__(256) k_wave_init(const JobDesc* jobs, WaveArrays arr, const WaveJob* wj,
+//
+// Small floods have their occupied voxels counted (LONE_VOXELS).
+__global__ void __launch_bounds__(256) k_wave_init(const JobDesc* jobs, JobState* st, WaveArrays arr, const WaveJob* wj,
                                                    uint32_t njobs, const uint8_t* live) {
   uint32_t lo = 0, hi = njobs - 1;  // the job of these rows: the last that starts at or before them
   while (lo < hi) {
@@ -646,6 +665,7 @@ __global__ void __launch_bounds__(256) k_wave_init(const JobDesc* jobs, WaveArra
     if (z < J.Zk && live[J.brick_base + ((x / VF_BX) * J.nby + y / VF_BY) * J.nbz + zw])
       a[i] = *reinterpret_cast<const uint2*>(J.grid + vf_gidx(J, x, y, z));
   }
+  uint32_t voxels = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const uint32_t row = first + r0 + 32u * i;
@@ -654,17 +674,19 @@ __global__ void __launch_bounds__(256) k_wave_init(const JobDesc* jobs, WaveArra
     w <<= 4 * q;
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) w |= __shfl_xor_sync(FULL, w, o);
+    if (q == 0) voxels += (uint32_t)__popc(w);
     uint32_t* d = arr.state + (size_t)row * J.wsw;  // up to the next job's base
 
     for (uint32_t k = q; k < J.wsw; k += 8) d[k] = k == 0 ? wave_empty_a(w) : (k == 1 ? wave_empty_b(w) : 0u);
     if (q < 4) reinterpret_cast<uint32_t*>(arr.in + 2 * (size_t)row)[q] = 0xFFFFFFFFu;
   }
+  if (W.nrows <= SMALL_ROWS) add_voxels(&st[W.job].wave_voxels, voxels);
 }
 
 // The same from the voxelizer's bit planes, which hold the rows' words already: a
 // thread per row writes its state.  Bound by the stores: 128 mixed jobs 377 us, from
 // the labels 1018 us.
-__global__ void __launch_bounds__(256) k_wave_planes(const JobDesc* jobs, WaveArrays arr, const WaveJob* wj,
+__global__ void __launch_bounds__(256) k_wave_planes(const JobDesc* jobs, JobState* st, WaveArrays arr, const WaveJob* wj,
                                                      uint32_t njobs, uint32_t units) {
   for (uint32_t unit = blockIdx.x; unit < units; unit += gridDim.x) {
     uint32_t lo = 0, hi = njobs - 1;  // the job of these rows: the last that starts at or before them
@@ -683,6 +705,7 @@ __global__ void __launch_bounds__(256) k_wave_planes(const JobDesc* jobs, WaveAr
         w = J.par[at] | J.shell[at];
       }
     }
+    if (W.nrows <= SMALL_ROWS) add_voxels(&st[W.job].wave_voxels, (uint32_t)__popc(w));
     uint4* const d = reinterpret_cast<uint4*>(arr.state + (size_t)row * J.wsw);  // up to the next job's base
     d[0] = make_uint4(wave_empty_a(w), wave_empty_b(w), 0u, 0u);
     for (uint32_t k = 1; k < J.wsw / 4; ++k) d[k] = make_uint4(0u, 0u, 0u, 0u);
@@ -805,7 +828,7 @@ __device__ __forceinline__ bool flat_row(const WaveJob& W, const vfk::FlatAxes& 
 }
 
 __global__ void __launch_bounds__(256) k_flat_init(const uint16_t* grid, WaveArrays arr, WaveJob W,
-                                                   vfk::FlatAxes A, uint32_t sw) {
+                                                   vfk::FlatAxes A, uint32_t sw, JobState* st) {
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t box = (A.nx + 2) * W.sx, nwarps = (gridDim.x * blockDim.x) >> 5;
   auto put = [&](uint32_t row, uint32_t m) {
@@ -817,7 +840,9 @@ __global__ void __launch_bounds__(256) k_flat_init(const uint16_t* grid, WaveArr
     uint32_t row;
     size_t at;
     const bool in = flat_row(W, A, k, lane, row, at);
-    put(row, __ballot_sync(FULL, in && grid[at] != VOXEL_EMPTY));
+    const uint32_t m = __ballot_sync(FULL, in && grid[at] != VOXEL_EMPTY);
+    put(row, m);
+    if (W.nrows <= SMALL_ROWS && lane == 0 && m) atomicAdd(&st->wave_voxels, (uint32_t)__popc(m));
   }
   // the rows before and after the box
   const uint32_t before = W.row0 - W.sx, after = W.nrows - before - box;
@@ -1233,13 +1258,13 @@ void flood_seed_bricks(cudaStream_t st, const JobDesc* dj, JobState* ds, int njo
   if (njobs > 0) k_seed_bricks<<<njobs, 128, 0, st>>>(dj, ds, live, list, count);
 }
 
-void flood_init(cudaStream_t st, const JobDesc* dj, const FloodScratch& fs, const uint8_t* live, bool planes) {
+void flood_init(cudaStream_t st, const JobDesc* dj, JobState* ds, const FloodScratch& fs, const uint8_t* live, bool planes) {
   if (!fs.units) return;
   if (planes)
-    k_wave_planes<<<std::min<uint32_t>(fs.units, (uint32_t)fs.shape.sms * 32), 256, 0, st>>>(dj, fs.arr, fs.jobs, fs.njobs,
-                                                                                           fs.units);
+    k_wave_planes<<<std::min<uint32_t>(fs.units, (uint32_t)fs.shape.sms * 32), 256, 0, st>>>(dj, ds, fs.arr, fs.jobs,
+                                                                                           fs.njobs, fs.units);
   else
-    k_wave_init<<<fs.units, 256, 0, st>>>(dj, fs.arr, fs.jobs, fs.njobs, live);
+    k_wave_init<<<fs.units, 256, 0, st>>>(dj, ds, fs.arr, fs.jobs, fs.njobs, live);
 }
 
 // launch shape of k_wave: threads per CTA and dynamic shared memory
@@ -1283,11 +1308,11 @@ WaveShape flood_shape(uint32_t sw, uint32_t njobs, int num_sms, int ctas_per_sm)
 }
 
 uint32_t flood_gang(uint64_t rows, uint32_t blocks, uint32_t min_size) {
-  // rows per CTA: 525 k rows (240 x 240 x 256) take 0.56 ms with 4096, 0.59
-  // with 2048 and 0.62 with 8192
-  constexpr uint64_t GANG_ROWS = 4096;
-  if (rows <= SMALL_ROWS) return std::min(min_size, blocks);
-  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>((rows + GANG_ROWS - 1) / GANG_ROWS, 2), blocks);
+  // A CTA per 1024 rows up to 128 of them, then per 4096.  Full cubes, Manhattan, with
+  // 4096 and 1024 rows a CTA throughout: 128^3 965 and 760 us, 160^3 1200 and 987, 200^3
+  // 1405 and 1306; a vessel of 240 x 240 x 256 (525 k rows) 510 on 129 CTAs, 520 on 152.
+  const uint64_t size = std::max<uint64_t>(std::min<uint64_t>((rows + 1023) / 1024, 128), (rows + 4095) / 4096);
+  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>(size, min_size), blocks);
 }
 
 uint32_t flood_gangs(const uint64_t* rows, uint32_t n, uint32_t* gang_of) {
@@ -1322,21 +1347,29 @@ uint32_t flood_gangs(const uint64_t* rows, uint32_t n, uint32_t* gang_of) {
 }
 
 // One-CTA gangs are dealt to all CTAs, the largest first, each to the least
-// loaded one; larger gangs alternate between as many sets of CTAs as fit an SM.
+// loaded one.  Larger gangs of small floods lie side by side, as wide as all of them
+// fit; those of large floods alternate between as many sets of CTAs as fit an SM.
+// Every CTA runs its gangs of several CTAs in their order, so that none waits for one
+// that waits for it.
 uint32_t flood_schedule(const WaveGang* gangs, uint32_t n, const WaveShape& shape, uint32_t min_size, WaveCta* cta,
                         WaveEntry* entries) {
-  const uint32_t C = (uint32_t)shape.blocks;
+  const uint32_t C = (uint32_t)shape.blocks, sms = (uint32_t)std::max(shape.sms, 1);
   std::vector<std::vector<WaveEntry>> lists(C);
-  const uint32_t sets = n > 1 ? std::max(1u, std::min(n, C / (uint32_t)std::max(shape.sms, 1))) : 1u;
-  const uint32_t width = std::max(1u, std::min(C / sets, (uint32_t)std::max(shape.sms, 1)));
+  bool small_floods = true;
+  for (uint32_t g = 0; g < n; ++g) small_floods &= gangs[g].units * 256 <= SMALL_ROWS;
+  const uint32_t sets = n > 1 ? std::max(1u, std::min(n, C / sms)) : 1u;
+  const uint32_t width = std::max(1u, std::min(small_floods && n ? std::max(C / n, min_size) : C / sets, sms));
   std::vector<uint32_t> small;
+  uint32_t next = 0;  // of small floods: the first CTA past the last gang's
   for (uint32_t g = 0; g < n; ++g) {
-    const uint32_t size = flood_gang((uint64_t)gangs[g].units * 256, width, min_size);
+    const uint32_t size = flood_gang((uint64_t)gangs[g].units * 256, std::min(width, C), min_size);
     if (size < 2) {
       small.push_back(g);
       continue;
     }
-    const uint32_t at = (g % sets) * width;
+    if (next + size > C) next = 0;
+    const uint32_t at = small_floods ? next : (g % sets) * width;
+    next += size;
     for (uint32_t r = 0; r < size; ++r) lists[at + r].push_back({g, r, size, 0});
   }
   std::sort(small.begin(), small.end(), [&](uint32_t a, uint32_t b) {
@@ -1385,6 +1418,7 @@ cudaError_t flood_waves(cudaStream_t st, JobState* ds, const FloodScratch& fs) {
   a.wave_sizes = fs.wave_sizes;
   a.wait_spins = fs.wait_spins ? fs.wait_spins : (1u << 23);
   a.smem_words = (uint32_t)((WAVE_SMEM - sizeof(WaveShared)) / 4);
+  a.lone_voxels = fs.wait_spins ? 0u : LONE_VOXELS;  // a wait limit is for gangs that wait
   void* args[] = {&a};
   return cudaLaunchCooperativeKernel(fs.shape.threads == 512 ? wave_kernel<512>(fs.sw) : wave_kernel<256>(fs.sw),
                                      dim3(fs.shape.blocks), dim3(fs.shape.threads), args, WAVE_SMEM, st);
@@ -1394,8 +1428,8 @@ static int flat_grid(const WaveJob& W) {
   return (int)std::max<uint32_t>(1, std::min<uint32_t>((W.nrows + 7) / 8, 2432));
 }
 void flat_init(cudaStream_t st, const uint16_t* grid, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A,
-               uint32_t sw) {
-  k_flat_init<<<flat_grid(W), 256, 0, st>>>(grid, arr, W, A, sw);
+               uint32_t sw, JobState* ds) {
+  k_flat_init<<<flat_grid(W), 256, 0, st>>>(grid, arr, W, A, sw, ds);
 }
 void flat_seed(cudaStream_t st, const WaveJob& W, const FlatAxes& A, const FloodScratch& fs, const uint32_t* seeds,
                uint32_t ns, JobState* ds) {

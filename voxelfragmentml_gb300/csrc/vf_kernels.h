@@ -266,7 +266,7 @@ struct FloodScratch {
 WaveShape flood_shape(uint32_t sw, uint32_t njobs, int num_sms, int ctas_per_sm);
 // the gangs of n floods of rows[i] rows: their number, the gang of each
 uint32_t flood_gangs(const uint64_t* rows, uint32_t n, uint32_t* gang_of);
-// CTAs of a gang
+// CTAs of a gang, min_size to blocks
 uint32_t flood_gang(uint64_t rows, uint32_t blocks, uint32_t min_size);
 // the CTAs of n gangs: cta[shape.blocks], entries (at most n * shape.sms + n);
 // returns the entries
@@ -276,7 +276,8 @@ void flood_seed_bricks(cudaStream_t st, const JobDesc* dj, JobState* ds, int njo
                        uint32_t* list, uint32_t* count);
 // row states from the labels
 // planes: the labels are the voxelizer's occupancy, still in its bit planes
-void flood_init(cudaStream_t st, const JobDesc* dj, const FloodScratch& fs, const uint8_t* live, bool planes);
+void flood_init(cudaStream_t st, const JobDesc* dj, JobState* ds, const FloodScratch& fs, const uint8_t* live,
+                bool planes);
 cudaError_t flood_seed(cudaStream_t st, const JobDesc* dj, const JobState* ds, const FloodScratch& fs);
 cudaError_t flood_waves(cudaStream_t st, JobState* ds, const FloodScratch& fs);
 void flood_labels(cudaStream_t st, const JobDesc* dj, const JobState* ds, const uint32_t* list,
@@ -293,7 +294,7 @@ struct FlatAxes {
   uint32_t order;    // nibble a: the grid axis of state axis a
 };
 void flat_init(cudaStream_t st, const uint16_t* grid, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A,
-               uint32_t sw);
+               uint32_t sw, JobState* ds);
 // checks and places the seeds; writes the wave job and its gang's tables
 void flat_seed(cudaStream_t st, const WaveJob& W, const FlatAxes& A, const FloodScratch& fs, const uint32_t* seeds,
                uint32_t ns, JobState* ds);

@@ -160,7 +160,7 @@ extern "C" vf_status vf_flood_noalloc(const uint16_t* d_grid, uint16_t* d_labels
       return fail(VF_ERR_CUDA, std::string("vf_flood_noalloc: ") + cudaGetErrorString(e_)); \
   } while (0)
   NA_CK(cudaMemsetAsync(S, 0, cleared, st));
-  vfk::flat_init(st, d_grid, fs.arr, W, A, sw);
+  vfk::flat_init(st, d_grid, fs.arr, W, A, sw, dstate);
   // Without seeds nothing is claimed: occupied voxels come out FREE (1), as
   // FloodFracturer::build leaves them after homogenize.
   if (nseeds) {

@@ -916,7 +916,7 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
     const JobDesc* tf = dtable(T_FLOOD);
     if ((s = wave_tables(fs))) return s;
     vfk::flood_seed_bricks(st, tf, ds, n, lv, lst, lc);
-    vfk::flood_init(st, tf, fs, lv, (stages & ST_VOX) != 0);
+    vfk::flood_init(st, tf, ds, fs, lv, (stages & ST_VOX) != 0);
     VF_CK(vfk::flood_seed(st, tf, ds, fs));
     VF_CK(record_event(ev_flood0, st));
     cudaError_t e = waves_serialized(st, ds, fs);

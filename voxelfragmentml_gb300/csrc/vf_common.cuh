@@ -60,6 +60,7 @@ struct JobDesc {
   uint2* win;
   uint32_t* wcand;
   uint32_t wsw, wrow0, wsx, wsy;
+  uint32_t wflat;   // its words do not lie along z
   uint32_t* uf;     // [seeds_cap] union-find over the slots (null: no sub-seed prefixes)
   uint32_t* par;
   uint32_t* shell;

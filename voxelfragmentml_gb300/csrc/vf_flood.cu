@@ -8,8 +8,8 @@
 // (6-neighbourhood for Manhattan, 26 for Euclidean and Chebyshev), ties to
 // the lowest seed index.
 //
-// The GPU runs those waves bit-parallel.  32 voxels along z are one word of
-// bit planes:
+// The GPU runs those waves bit-parallel.  32 voxels along z (in a large flat
+// grid along its longest axis: wave_order) are one word of bit planes:
 //
 //   A, B         EMPTY, occupied and not claimed yet (U), or claimed in a wave of
 //                either parity (E0, E1): vf_wave_state.h
@@ -649,6 +649,7 @@ __global__ void __launch_bounds__(256) k_wave_init(const JobDesc* jobs, JobState
     if (wj[mid].base <= blockIdx.x * 256u) lo = mid; else hi = mid - 1;
   }
   const WaveJob& W = wj[lo];
+  if (W.order != vfk::WAVE_XYZ) return;  // k_flat_init's
   const JobDesc& J = jobs[W.job];
   const uint32_t q = threadIdx.x & 7, r0 = threadIdx.x >> 3;
   const uint32_t first = blockIdx.x * 256u;
@@ -695,6 +696,7 @@ __global__ void __launch_bounds__(256) k_wave_planes(const JobDesc* jobs, JobSta
       if (wj[mid].base <= unit * 256u) lo = mid; else hi = mid - 1;
     }
     const WaveJob& W = wj[lo];
+    if (W.order != vfk::WAVE_XYZ) continue;  // k_flat_init's
     const JobDesc& J = jobs[W.job];
     const uint32_t row = unit * 256u + threadIdx.x;
     uint32_t w = 0;
@@ -809,19 +811,20 @@ __global__ void __launch_bounds__(256) k_wave_seed(const JobDesc* jobs, const Jo
     __syncthreads();
   }
   if (s.err) return;
-  seed_waves(arr, W, J.uf, J.seeds, min(s.nseeds, 4096u), J.wsw, (int)J.wsw - 2, 0x210u, pos);
+  seed_waves(arr, W, J.uf, J.seeds, min(s.nseeds, 4096u), J.wsw, (int)J.wsw - 2, W.order, pos);
 }
 
-// ---- a flood on a caller's unpadded device grid, any axis order -----------
-// (vf_flood_noalloc).  Voxel (a, b, c) of the state, c along the words, is the
-// caller's element a * sa + b * sb + c * sc.
+// ---- a flood on a grid of any strides, any axis order ----------------------
+// (vf_flood_noalloc on a caller's device grid; flat grids of the batched path).
+// Voxel (a, b, c) of the state, c along the words, is the grid's element
+// a * s[0] + b * s[1] + c * s[2].
 // One warp per row, a lane per voxel; consecutive warps take consecutive words
 // of a grid row, whose voxels are contiguous.
 __device__ __forceinline__ bool flat_row(const WaveJob& W, const vfk::FlatAxes& A, uint32_t k, uint32_t lane,
                                          uint32_t& row, size_t& at) {
   // k numbers the rows of the padded box [nx + 2][ny + 1][nw + 1], words fastest
   const uint32_t nw1 = W.sx / W.sy, zw = k % nw1, y = (k / nw1) % W.sy, x = k / W.sx;
-  row = W.row0 - W.sx + x * W.sx + zw * W.sy + y;  // base 0
+  row = W.row0 - W.sx + x * W.sx + zw * W.sy + y;
   const uint32_t z = 32 * zw + lane;
   at = (x - 1) * A.s[0] + y * A.s[1] + z * A.s[2];
   return x >= 1 && x <= A.nx && y < A.ny && z < A.nz;
@@ -845,9 +848,9 @@ __global__ void __launch_bounds__(256) k_flat_init(const uint16_t* grid, WaveArr
     if (W.nrows <= SMALL_ROWS && lane == 0 && m) atomicAdd(&st->wave_voxels, (uint32_t)__popc(m));
   }
   // the rows before and after the box
-  const uint32_t before = W.row0 - W.sx, after = W.nrows - before - box;
+  const uint32_t before = W.row0 - W.sx - W.base, after = W.nrows - before - box;
   for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < before + after; k += nwarps)
-    put(k < before ? k : box + k, 0u);
+    put(W.base + (k < before ? k : box + k), 0u);
 }
 
 // wave job and gang table, then the seeds (labels 2..255 without prefix)
@@ -883,9 +886,11 @@ __global__ void __launch_bounds__(256) k_flat_seed(WaveArrays arr, WaveJob W, vf
   if (!bad && !prefix) seed_waves(arr, W, nullptr, seeds, ns, sw, (int)sw - 2, A.order, pos);
 }
 
+// st: the job of a batch (null: no sub-seed prefixes)
 __global__ void __launch_bounds__(256) k_flat_labels(WaveArrays arr, WaveJob W, vfk::FlatAxes A, uint32_t sw,
-                                                     const uint32_t* seeds, uint16_t* labels) {
+                                                     const uint32_t* seeds, const JobState* st, uint16_t* labels) {
   const uint32_t lane = threadIdx.x & 31;
+  const bool second = st && st->has_prefix && st->disjoint;  // slots are ranks
   const uint32_t box = (A.nx + 2) * W.sx, nwarps = (gridDim.x * blockDim.x) >> 5;
   for (uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; k < box; k += nwarps) {
     uint32_t row;
@@ -899,7 +904,7 @@ __global__ void __launch_bounds__(256) k_flat_labels(WaveArrays arr, WaveJob W, 
     if (v) {  // uniform
       uint32_t slot = 0;
       for (uint32_t k = 0; k + 2 < sw; ++k) slot |= ((__shfl_sync(FULL, word, 2 + k) >> lane) & 1u) << k;
-      if ((v >> lane) & 1u) l = seeds[4 * slot + 3] & 0xFFu;
+      if ((v >> lane) & 1u) l = (second ? st->rank_value[slot] : seeds[4 * slot + 3]) & 0xFFu;
     }
     if (in) labels[at] = (uint16_t)l;
   }
@@ -927,7 +932,7 @@ __global__ void __launch_bounds__(256, 4) k_wave_labels(const JobDesc* jobs, con
   for (uint32_t it = blockIdx.x; it < n;) {
     const JobDesc& J = jobs[j];
     const JobState& s = st[j];
-    const bool active = J.active != 0;  // uniform across the CTA
+    const bool active = J.active != 0 && !J.wflat;  // uniform across the CTA
     const uint32_t lb = b - J.brick_base;
     const uint32_t bz = lb % J.nbz, by = (lb / J.nbz) % J.nby, bx = lb / (J.nbz * J.nby);
     const uint32_t x = bx * VF_BX + row / VF_BY, y = by * VF_BY + row % VF_BY, z = bz * VF_BZ + sh;
@@ -1252,6 +1257,29 @@ void wave_layout(WaveJob& W, uint32_t base, uint32_t nx, uint32_t ny, uint32_t n
   W.row0 = base + W.sx + W.sy + 1;
   W.nrows = (uint32_t)wave_rows(nx, ny, nw);
 }
+uint32_t wave_order(uint32_t X, uint32_t Y, uint32_t Z) {
+  // Words along z, also in a flat grid, whose words are mostly empty bits: a front
+  // that runs along the plane claims such a row in one wave (1024 x 1024 x 8 voxels,
+  // full, Manhattan: 2.29 ms, 2.55 with words along x).  Where a large grid has at
+  // least 8 times fewer rows with words along its longest axis (z up to 5 voxels), the
+  // scans and the memory of the others count: 4096 x 4096 x 2 8.4 against 13.3 ms and
+  // 0.1 against 1.6 GB, 2048 x 2048 x 4 4.9 against 5.0 ms.
+  constexpr uint64_t FLAT_ROWS = 4 << 20, FLAT_GAIN = 8;
+  const uint32_t D[3] = {X, Y, Z}, w = X > Y ? 0u : 1u, l = 1u - w;
+  const uint64_t rows = wave_rows(X, Y, (Z + 31) / 32);
+  if (rows < FLAT_ROWS || wave_rows(Z, D[l], (D[w] + 31) / 32) * FLAT_GAIN > rows) return WAVE_XYZ;
+  return 2u | l << 4 | w << 8;
+}
+uint64_t wave_job_rows(uint32_t X, uint32_t Y, uint32_t Z) {
+  const FlatAxes A = wave_axes(X, Y, Z, Z);
+  return wave_rows(A.nx, A.ny, (A.nz + 31) / 32);
+}
+FlatAxes wave_axes(uint32_t X, uint32_t Y, uint32_t Z, uint32_t pitch) {
+  const uint32_t D[3] = {X, Y, Z}, order = wave_order(X, Y, Z);
+  const size_t stride[3] = {(size_t)Y * pitch, pitch, 1};
+  const uint32_t a = order & 15u, b = (order >> 4) & 15u, c = order >> 8;
+  return {{stride[a], stride[b], stride[c]}, D[a], D[b], D[c], {X, Y, Z}, order};
+}
 
 void flood_seed_bricks(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs, uint8_t* live,
                        uint32_t* list, uint32_t* count) {
@@ -1439,8 +1467,8 @@ void flat_seed(cudaStream_t st, const WaveJob& W, const FlatAxes& A, const Flood
                                  const_cast<WaveCta*>(fs.cta), const_cast<WaveEntry*>(fs.entries));
 }
 void flat_labels(cudaStream_t st, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A, uint32_t sw,
-                 const uint32_t* seeds, uint16_t* labels) {
-  k_flat_labels<<<flat_grid(W), 256, 0, st>>>(arr, W, A, sw, seeds, labels);
+                 const uint32_t* seeds, const JobState* ds, uint16_t* labels) {
+  k_flat_labels<<<flat_grid(W), 256, 0, st>>>(arr, W, A, sw, seeds, ds, labels);
 }
 
 void flood_labels(cudaStream_t st, const JobDesc* dj, const JobState* ds, const uint32_t* list,

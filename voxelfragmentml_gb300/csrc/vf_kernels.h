@@ -219,8 +219,20 @@ struct WaveJob {
   uint32_t base, nrows, row0, sx, sy;
   uint32_t conn6;  // 6-neighbourhood (Manhattan), else 26
   uint32_t job;    // its JobState
+  uint32_t order;  // nibble a: the grid axis of state axis a (outer, rows, words)
+};
+constexpr uint32_t WAVE_XYZ = 0x210u;  // words along z
+struct FlatAxes {
+  size_t s[3];       // element strides of the state's axes (outer, rows, words)
+  uint32_t nx, ny, nz;  // voxels along them
+  uint32_t dims[3];  // X, Y, Z
+  uint32_t order;    // nibble a: the grid axis of state axis a
 };
 uint64_t wave_rows(uint32_t nx, uint32_t ny, uint32_t nw);
+// the axes of a job's state, the rows it needs with them; pitch: elements of a z row
+uint32_t wave_order(uint32_t X, uint32_t Y, uint32_t Z);
+FlatAxes wave_axes(uint32_t X, uint32_t Y, uint32_t Z, uint32_t pitch);
+uint64_t wave_job_rows(uint32_t X, uint32_t Y, uint32_t Z);
 void wave_layout(WaveJob& W, uint32_t base, uint32_t nx, uint32_t ny, uint32_t nw);
 // Jobs flooded in step: wave jobs first .. first + count, whose rows are units
 // unit_lo .. unit_lo + units of 256 rows
@@ -287,19 +299,13 @@ void flood_labels(cudaStream_t st, const JobDesc* dj, const JobState* ds, const 
 cudaError_t flood_prefixes(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs, const FloodScratch& fs);
 
 // ---- a flood on an unpadded device grid (vf_flood_noalloc) ----
-struct FlatAxes {
-  size_t s[3];       // element strides of the state's axes (outer, rows, words)
-  uint32_t nx, ny, nz;  // voxels along them
-  uint32_t dims[3];  // X, Y, Z
-  uint32_t order;    // nibble a: the grid axis of state axis a
-};
 void flat_init(cudaStream_t st, const uint16_t* grid, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A,
                uint32_t sw, JobState* ds);
 // checks and places the seeds; writes the wave job and its gang's tables
 void flat_seed(cudaStream_t st, const WaveJob& W, const FlatAxes& A, const FloodScratch& fs, const uint32_t* seeds,
                uint32_t ns, JobState* ds);
 void flat_labels(cudaStream_t st, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A, uint32_t sw,
-                 const uint32_t* seeds, uint16_t* labels);
+                 const uint32_t* seeds, const JobState* ds, uint16_t* labels);
 
 // ---- plain (reference-shaped) per-voxel kernels for one job ----
 void plain_init_keys(cudaStream_t st, const JobDesc* dj, const JobDesc& hj);

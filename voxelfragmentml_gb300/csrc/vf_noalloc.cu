@@ -117,6 +117,7 @@ extern "C" vf_status vf_flood_noalloc(const uint16_t* d_grid, uint16_t* d_labels
   vfk::WaveJob W = {};
   vfk::wave_layout(W, 0, D[o], D[l], (D[w] + 31) / 32);
   W.conn6 = distance == VF_MANHATTAN ? 1u : 0u;
+  W.order = A.order;
   const vfk::WaveShape shape = vfk::flood_shape(sw, 1, num_sms, 0);
   const size_t blocks = (size_t)shape.blocks, rows = ((size_t)W.nrows + 255) / 256 * 256;
   // layout of the scratch array: job state, flood words, barrier and masks
@@ -167,7 +168,7 @@ extern "C" vf_status vf_flood_noalloc(const uint16_t* d_grid, uint16_t* d_labels
     vfk::flat_seed(st, W, A, fs, d_seeds_xyzw, nseeds, dstate);
     NA_CK(vfk::flood_waves(st, dstate, fs));
   }
-  vfk::flat_labels(st, fs.arr, W, A, sw, d_seeds_xyzw, d_labels);
+  vfk::flat_labels(st, fs.arr, W, A, sw, d_seeds_xyzw, nullptr, d_labels);
   NA_CK(cudaGetLastError());
   static_assert(offsetof(JobState, disjoint) == offsetof(JobState, err) + 8, "err, has_prefix, disjoint in a row");
   uint32_t status[3] = {0, 0, 0};

@@ -182,6 +182,9 @@ void Batch::release() {
 }
 
 size_t Batch::table_off(uint32_t t) const { return (size_t)t * jobs.size(); }
+const JobDesc* Batch::htable(uint32_t t) const {
+  return reinterpret_cast<const JobDesc*>(h_tables) + table_off(t);
+}
 const JobDesc* Batch::dtable(uint32_t t) const {
   return reinterpret_cast<const JobDesc*>(tables.p) + table_off(t);
 }
@@ -303,7 +306,7 @@ void Footprint::add(const vf_job& j) {
   fixed += X * Y * Zp * 2 * 2 + X * Y * Zw * 4 * 2 + (size_t)j.nfaces * (48 + 4 + 12 + 12) +
            (size_t)edge_slots(j.nfaces) * 8 + (size_t)j.nverts * 12 + 65536;
   if (j.params.algorithm == VF_FLOOD) {
-    rows += (vfk::wave_rows((uint32_t)X, (uint32_t)Y, (uint32_t)Zw) + 255) / 256 * 256;
+    rows += (vfk::wave_job_rows((uint32_t)X, (uint32_t)Y, (uint32_t)Z) + 255) / 256 * 256;
     words = std::max(words, vfk::wave_state_words(wave_seeds(j.params)));
   }
   // per brick: owner, live flag, list
@@ -414,7 +417,7 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
     for (uint32_t i = 0; i < n; ++i)
       if (js[i]->params.algorithm == VF_FLOOD) {
         fl.push_back(i);
-        rows.push_back(vfk::wave_rows(plans[i].X, plans[i].Y, plans[i].nbz));
+        rows.push_back(vfk::wave_job_rows(plans[i].X, plans[i].Y, plans[i].Z));
       }
     gang.resize(fl.size());
     const uint32_t ng = fl.empty() ? 0u : vfk::flood_gangs(rows.data(), (uint32_t)fl.size(), gang.data());
@@ -426,9 +429,13 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
     for (uint32_t k : order) {
       const uint32_t i = fl[k];
       const uint64_t u = (rows[k] + 255) / 256;
-      if ((units + u) * 256 > 1ull << 31) return fail(VF_ERR_RANGE, "the batch's floods have 2^31 rows or more");
+      // rows are numbered in 32 bits, the last number stands for none (their states
+      // alone take 196 GiB there)
+      if ((units + u) * 256 >= 1ull << 32) return fail(VF_ERR_RANGE, "the batch's floods have 2^32 rows or more");
       vfk::WaveJob w = {};
-      vfk::wave_layout(w, (uint32_t)(units * 256), plans[i].X, plans[i].Y, plans[i].nbz);
+      const vfk::FlatAxes A = vfk::wave_axes(plans[i].X, plans[i].Y, plans[i].Z, plans[i].Zp);
+      vfk::wave_layout(w, (uint32_t)(units * 256), A.nx, A.ny, (A.nz + 31) / 32);
+      w.order = A.order;
       w.conn6 = js[i]->params.distance == VF_MANHATTAN ? 1u : 0u;
       w.job = i;
       vfk::WaveGang& g = wave_gangs[gang[k]];
@@ -654,6 +661,7 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
       d.wrow0 = w.row0;
       d.wsx = w.sx;
       d.wsy = w.sy;
+      d.wflat = w.order != vfk::WAVE_XYZ ? 1u : 0u;
     }
   return plan_groups();
 }
@@ -917,6 +925,12 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
     if ((s = wave_tables(fs))) return s;
     vfk::flood_seed_bricks(st, tf, ds, n, lv, lst, lc);
     vfk::flood_init(st, tf, ds, fs, lv, (stages & ST_VOX) != 0);
+    for (const vfk::WaveJob& w : wave_jobs)
+      if (w.order != vfk::WAVE_XYZ) {
+        const JobDesc& d = htable(T_FLOOD)[w.job];
+        vfk::flat_init(st, d.grid, fs.arr, w, vfk::wave_axes(d.X, d.Y, d.Z, d.Zp), wsw, ds + w.job);
+        launches += 1;
+      }
     VF_CK(vfk::flood_seed(st, tf, ds, fs));
     VF_CK(record_event(ev_flood0, st));
     cudaError_t e = waves_serialized(st, ds, fs);
@@ -932,9 +946,19 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
       launches += 5;
     }
   }
-  // the stages from the labels on, for the live bricks of a list
-  auto finish_bricks = [&](uint32_t* bl, uint32_t* bc, uint32_t most, const std::function<void(int)>& mk) {
-    if (any_flood) { vfk::flood_labels(st, dtable(T_FLOOD), ds, bl, bc, most, bj); launches += 1; }
+  // the stages from the labels on, for the live bricks of a list, of jobs [j0, j1)
+  auto finish_bricks = [&](uint32_t j0, uint32_t j1, uint32_t* bl, uint32_t* bc, uint32_t most,
+                           const std::function<void(int)>& mk) {
+    if (any_flood) {
+      vfk::flood_labels(st, dtable(T_FLOOD), ds, bl, bc, most, bj);
+      launches += 1;
+      for (const vfk::WaveJob& w : wave_jobs)
+        if (w.order != vfk::WAVE_XYZ && w.job >= j0 && w.job < j1) {
+          const JobDesc& d = htable(T_FLOOD)[w.job];
+          vfk::flat_labels(st, fs.arr, w, vfk::wave_axes(d.X, d.Y, d.Z, d.Zp), wsw, d.seeds, ds + w.job, d.grid);
+          launches += 1;
+        }
+    }
     if (any_naive) { vfk::naive(st, dtable(T_NAIVE), ds, bl, bc, most, bj); launches += 1; }
     mk(7);
     if (any_pert) { vfk::perturb(st, dtable(T_PERT), bl, bc, most, bj); launches += 1; }
@@ -968,7 +992,7 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
       }
       // the whole batch's list is not needed any more; its part of the group is
       vfk::compact_live(st, lv, b0, nb, lst + b0, lc + 16 + g);
-      finish_bricks(lst + b0, lc + 16 + g, nb, [](int) {});
+      finish_bricks(j0, groups[g], lst + b0, lc + 16 + g, nb, [](int) {});
       VF_CK(cudaEventRecord(ev_group, st));
       VF_CK(cudaStreamWaitEvent(side, ev_group, 0));
       vfk::pack_labels(side, dtable(T_CNT) + j0, (int)(groups[g] - j0), r0, nr, ctx->num_sms, GROUP_PACK_CTAS);
@@ -981,7 +1005,7 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
     mark(9);
     mark(10);
   } else {
-    finish_bricks(lst, lc, maxc, mark);
+    finish_bricks(0, n, lst, lc, maxc, mark);
   }
   if (chain) {
     std::lock_guard<std::mutex> lk(ctx->relax_mu);

@@ -139,6 +139,7 @@ struct Batch {
   vf_status finish(vf_job_result* res);
   size_t table_off(uint32_t t) const;
   const JobDesc* dtable(uint32_t t) const;
+  const JobDesc* htable(uint32_t t) const;  // its host copy
 };
 
 // launch settings chosen by vf_autotune (results never depend on them)

@@ -1315,15 +1315,25 @@ vf_status vf_autotune(vf_ctx* ctx, const vf_job* jobs, uint32_t njobs, int32_t* 
   };
   float warm = 0.f;
   if ((s = run(0, &warm))) return s;
+  // flood CTAs/SM (0: as many as fit), one candidate of those that are the same launch
+  std::vector<int32_t> flood_ctas;
+  for (int32_t v : {0, 3, 2}) {
+    auto blocks = [&](int32_t ctas) {
+      return vfk::flood_shape(B.wsw, (uint32_t)B.wave_jobs.size(), c.num_sms, ctas).blocks;
+    };
+    bool same = false;
+    for (int32_t o : flood_ctas) same |= blocks(o) == blocks(v);
+    if (!same) flood_ctas.push_back(v);
+  }
   struct Knob { int index, stage; std::vector<int32_t> cand; };
   const Knob knobs[] = {{0, 2, {4, 8, 16, 32}},      // parity grid   (stage: parity)
                         {1, 3, {6, 12, 24}},         // shell grid    (stage: shell)
-                        {2, 6, {8, 16, 32, 96}},     // sweeps/visit  (stage: fracture)
-                        {3, 6, {2, 3, 0}}};          // flood CTAs/SM (stage: fracture)
+                        {3, 6, flood_ctas}};         // flood CTAs/SM (stage: fracture)
   for (const Knob& k : knobs) {
-    int32_t best_v = 0;
+    int32_t best_v = k.cand[0];
     float best = 3.0e38f;
     for (int32_t v : k.cand) {
+      if (k.cand.size() == 1) break;  // nothing to decide
       int32_t cur[4];
       vf_ctx_get_tuning(ctx, cur, 4);
       cur[k.index] = v;

@@ -29,6 +29,7 @@
 #include <cuda_pipeline_primitives.h>
 
 #include "vf_kernels.h"
+#include "vf_slices.h"
 
 namespace {
 
@@ -131,15 +132,6 @@ __device__ __forceinline__ tv to_ndc(const float* v, const float* ctr, const flo
   return r;
 }
 
-// first slice plane above v, or n.  The planes are -1, -1 + 2 / n, ... added up, so
-// one is near (v + 1) n / 2 and its neighbours are looked at from there.
-__device__ __forceinline__ uint32_t upper_bound_f(const float* a, uint32_t n, float v) {
-  uint32_t i = (uint32_t)min((int)n, max(0, __float2int_rd((v + 1.0f) * (0.5f * (float)n)) + 1));
-  while (i > 0 && a[i - 1] > v) --i;
-  while (i < n && !(a[i] > v)) ++i;
-  return i;
-}
-
 // ---- parity by edge crossings ---------------------------------------------
 // The reference rasterises, for every slice plane, the cross-section of every
 // tetrahedron (face + centroid) with XOR at pixel centres (GL rules: 8
@@ -220,8 +212,8 @@ __device__ __forceinline__ int tetra_face(const JobDesc& J, JobState& st, uint32
   o[0] = make_float4(v[0].x, v[0].y, v[0].z, v[1].x);
   o[1] = make_float4(v[1].y, v[1].z, v[2].x, v[2].y);
   o[2] = make_float4(v[2].z, 0.0f, 0.0f, 0.0f);
-  const uint32_t s0 = upper_bound_f(J.ys, J.Y, v[0].y);
-  const uint32_t s1e = upper_bound_f(J.ys, J.Y, v[2].y);
+  const uint32_t s0 = slice_above(J.ys, J.Y, v[0].y);
+  const uint32_t s1e = slice_above(J.ys, J.Y, v[2].y);
   J.tet_range[f] = (s1e > s0) ? (s0 | ((s1e - 1) << 16)) : 0xFFFFu;
   *pcnt = s1e > s0 ? s1e - s0 : 0u;  // (face, slice) items
   return edge_use(J, i0, i1) + edge_use(J, i1, i2) + edge_use(J, i2, i0);
@@ -481,8 +473,8 @@ __global__ void __launch_bounds__(256) k_odd_edges(const JobDesc* jobs, const Jo
         p[1] = to_ndc(J.verts + 3 * (size_t)(uint32_t)key, ctr, dim);
         p[2] = to_ndc(st[j].centroid, ctr, dim);
         sort3_y(p);
-        const uint32_t s0 = upper_bound_f(J.ys, J.Y, p[0].y);
-        const uint32_t s1e = upper_bound_f(J.ys, J.Y, p[2].y);
+        const uint32_t s0 = slice_above(J.ys, J.Y, p[0].y);
+        const uint32_t s1e = slice_above(J.ys, J.Y, p[2].y);
         for (uint32_t s = s0 + lane; s < s1e; s += 32) face_segment(J, p[0], p[1], p[2], s);
       }
     }

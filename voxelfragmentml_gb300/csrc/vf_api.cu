@@ -1357,8 +1357,8 @@ vf_status vf_autotune(vf_ctx* ctx, const vf_job* jobs, uint32_t njobs, int32_t* 
 vf_status vf_ctx_flood_stats(vf_ctx* ctx, uint64_t* passes, uint64_t* sweeps, uint64_t* maxit_hits) {
   if (!ctx) return fail(VF_ERR_INVALID, "ctx is NULL");
   if (passes) *passes = ctx->c.last_flood_passes;
-  if (sweeps) *sweeps = ctx->c.last_flood_sweeps;
-  if (maxit_hits) *maxit_hits = ctx->c.last_flood_maxit;
+  if (sweeps) *sweeps = 0;
+  if (maxit_hits) *maxit_hits = 0;
   return VF_OK;
 }
 

@@ -54,11 +54,9 @@ struct JobDesc {
   uint16_t* grid;   // stage source (and in-place target)
   uint16_t* grid2;  // stage destination for double-buffered stages
   uint32_t* keys;   // plain path only
-  // flood: row states of wsw words, what reaches their ends, candidate bits; row
-  // (x, z word, y) is wrow0 + x * wsx + word * wsy + y (vfk::WaveJob)
+  // flood: row states of wsw words; row (x, z word, y) is wrow0 + x * wsx + word * wsy
+  // + y (vfk::WaveJob)
   uint32_t* wstate;
-  uint2* win;
-  uint32_t* wcand;
   uint32_t wsw, wrow0, wsx, wsy;
   uint32_t wflat;   // its words do not lie along z
   uint32_t* uf;     // [seeds_cap] union-find over the slots (null: no sub-seed prefixes)

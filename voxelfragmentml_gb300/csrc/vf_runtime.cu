@@ -559,8 +559,6 @@ vf_status Batch::plan(const vf_job* const* js, uint32_t n) {
     uint16_t* g1 = static_cast<uint16_t*>(grid1.p) + p.o_grid;
     d.keys = static_cast<uint32_t*>(keys.p) + p.o_keys;
     d.wstate = static_cast<uint32_t*>(wst.p);
-    d.win = static_cast<uint2*>(win.p);
-    d.wcand = static_cast<uint32_t*>(wzero.p);
     d.wsw = wsw;
     d.wrow0 = d.wsx = d.wsy = 0;  // from its wave job, below
     d.uf = p.prefix_possible && !plain ? static_cast<uint32_t*>(uf.p) + p.o_uf : nullptr;
@@ -1070,8 +1068,7 @@ vf_status Batch::finish(vf_job_result* res) {
       first = st;
       set_error("job " + std::to_string(i) + ": " +
                 (st == VF_ERR_SEED_SEARCH ? "seed search exceeded 1e6 tries"
-                 : st == VF_ERR_TIMEOUT   ? ((ferr & 8u) ? "flood skipped an out-of-range access"
-                                                        : "flood did not converge (bounded wait expired)")
+                 : st == VF_ERR_TIMEOUT   ? "flood did not converge (bounded wait expired)"
                  : st == VF_ERR_RANGE     ? "value out of range (prefix, distance or count)"
                                           : "invalid seeds or parameters"));
     }
@@ -1094,8 +1091,6 @@ vf_status Batch::finish(vf_job_result* res) {
     if (cudaEventElapsedTime(&ms, ev_flood0, ev_flood1) == cudaSuccess) ctx->last_flood_ms = ms;
     ctx->last_flood_visits = h_scal[16];
     ctx->last_flood_passes = h_scal[17];
-    ctx->last_flood_sweeps = h_scal[20];
-    ctx->last_flood_maxit = h_scal[21];
     for (int i = 0; i < VF_FLOOD_NCOUNTERS; ++i) ctx->last_flood_counters[i] = h_scal[16 + i];
     for (int i = 0; i < 256; ++i) ctx->last_pass_sizes[i] = h_scal[128 + i];
   } else {

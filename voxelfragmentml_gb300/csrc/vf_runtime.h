@@ -186,10 +186,8 @@ struct Ctx {
   bool resident = false;  // batch inputs uploaded by vf_batch_prepare
   uint64_t last_flood_visits = 0;
   uint64_t last_flood_passes = 0;
-  uint64_t last_flood_sweeps = 0;
   uint64_t last_flood_counters[VF_FLOOD_NCOUNTERS] = {};  // raw flood counters of the last batched run
-  uint32_t last_pass_sizes[256] = {};    // bricks queued per flood pass (first 256)
-  uint64_t last_flood_maxit = 0;
+  uint32_t last_pass_sizes[256] = {};    // rows visited per flood wave (first 256)
   vf_status alloc(DevBuf& b, size_t bytes);
   void free_buf(DevBuf& b);
 };

@@ -1452,12 +1452,12 @@ cudaError_t flood_waves(cudaStream_t st, JobState* ds, const FloodScratch& fs) {
                                      dim3(fs.shape.blocks), dim3(fs.shape.threads), args, WAVE_SMEM, st);
 }
 
-static int flat_grid(const WaveJob& W) {
-  return (int)std::max<uint32_t>(1, std::min<uint32_t>((W.nrows + 7) / 8, 2432));
+static int flat_grid(const WaveJob& W, int num_sms) {  // a warp per row, 16 CTAs per SM at most
+  return (int)std::max<uint32_t>(1, std::min<uint32_t>((W.nrows + 7) / 8, 16u * (uint32_t)num_sms));
 }
 void flat_init(cudaStream_t st, const uint16_t* grid, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A,
-               uint32_t sw, JobState* ds) {
-  k_flat_init<<<flat_grid(W), 256, 0, st>>>(grid, arr, W, A, sw, ds);
+               uint32_t sw, JobState* ds, int num_sms) {
+  k_flat_init<<<flat_grid(W, num_sms), 256, 0, st>>>(grid, arr, W, A, sw, ds);
 }
 void flat_seed(cudaStream_t st, const WaveJob& W, const FlatAxes& A, const FloodScratch& fs, const uint32_t* seeds,
                uint32_t ns, JobState* ds) {
@@ -1467,14 +1467,15 @@ void flat_seed(cudaStream_t st, const WaveJob& W, const FlatAxes& A, const Flood
                                  const_cast<WaveCta*>(fs.cta), const_cast<WaveEntry*>(fs.entries));
 }
 void flat_labels(cudaStream_t st, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A, uint32_t sw,
-                 const uint32_t* seeds, const JobState* ds, uint16_t* labels) {
-  k_flat_labels<<<flat_grid(W), 256, 0, st>>>(arr, W, A, sw, seeds, ds, labels);
+                 const uint32_t* seeds, const JobState* ds, uint16_t* labels, int num_sms) {
+  k_flat_labels<<<flat_grid(W, num_sms), 256, 0, st>>>(arr, W, A, sw, seeds, ds, labels);
 }
 
 void flood_labels(cudaStream_t st, const JobDesc* dj, const JobState* ds, const uint32_t* list,
-                  const uint32_t* count, uint32_t max_count, const uint32_t* brick_job) {
+                  const uint32_t* count, uint32_t max_count, const uint32_t* brick_job, int num_sms) {
   // resident CTAs: four of 256 threads fit an SM beside their 64 registers
-  if (max_count) k_wave_labels<<<std::min(brick_grid(max_count), 152 * 4), 256, 0, st>>>(dj, ds, list, count, brick_job);
+  if (max_count)
+    k_wave_labels<<<std::min(brick_grid(max_count), std::max(num_sms, 1) * 4), 256, 0, st>>>(dj, ds, list, count, brick_job);
 }
 
 cudaError_t flood_prefixes(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs, const FloodScratch& fs) {

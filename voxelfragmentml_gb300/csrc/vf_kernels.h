@@ -293,19 +293,19 @@ void flood_init(cudaStream_t st, const JobDesc* dj, JobState* ds, const FloodScr
 cudaError_t flood_seed(cudaStream_t st, const JobDesc* dj, const JobState* ds, const FloodScratch& fs);
 cudaError_t flood_waves(cudaStream_t st, JobState* ds, const FloodScratch& fs);
 void flood_labels(cudaStream_t st, const JobDesc* dj, const JobState* ds, const uint32_t* list,
-                  const uint32_t* count, uint32_t max_count, const uint32_t* brick_job);
+                  const uint32_t* count, uint32_t max_count, const uint32_t* brick_job, int num_sms);
 // sub-seed prefix competition and the disjoint cleanup after a flood: the jobs
 // whose voxels were reset are ready for the second flood
 cudaError_t flood_prefixes(cudaStream_t st, const JobDesc* dj, JobState* ds, int njobs, const FloodScratch& fs);
 
 // ---- a flood on an unpadded device grid (vf_flood_noalloc) ----
 void flat_init(cudaStream_t st, const uint16_t* grid, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A,
-               uint32_t sw, JobState* ds);
+               uint32_t sw, JobState* ds, int num_sms);
 // checks and places the seeds; writes the wave job and its gang's tables
 void flat_seed(cudaStream_t st, const WaveJob& W, const FlatAxes& A, const FloodScratch& fs, const uint32_t* seeds,
                uint32_t ns, JobState* ds);
 void flat_labels(cudaStream_t st, const WaveArrays& arr, const WaveJob& W, const FlatAxes& A, uint32_t sw,
-                 const uint32_t* seeds, const JobState* ds, uint16_t* labels);
+                 const uint32_t* seeds, const JobState* ds, uint16_t* labels, int num_sms);
 
 // ---- plain (reference-shaped) per-voxel kernels for one job ----
 void plain_init_keys(cudaStream_t st, const JobDesc* dj, const JobDesc& hj);

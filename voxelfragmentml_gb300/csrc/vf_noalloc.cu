@@ -161,14 +161,14 @@ extern "C" vf_status vf_flood_noalloc(const uint16_t* d_grid, uint16_t* d_labels
       return fail(VF_ERR_CUDA, std::string("vf_flood_noalloc: ") + cudaGetErrorString(e_)); \
   } while (0)
   NA_CK(cudaMemsetAsync(S, 0, cleared, st));
-  vfk::flat_init(st, d_grid, fs.arr, W, A, sw, dstate);
+  vfk::flat_init(st, d_grid, fs.arr, W, A, sw, dstate, num_sms);
   // Without seeds nothing is claimed: occupied voxels come out FREE (1), as
   // FloodFracturer::build leaves them after homogenize.
   if (nseeds) {
     vfk::flat_seed(st, W, A, fs, d_seeds_xyzw, nseeds, dstate);
     NA_CK(vfk::flood_waves(st, dstate, fs));
   }
-  vfk::flat_labels(st, fs.arr, W, A, sw, d_seeds_xyzw, nullptr, d_labels);
+  vfk::flat_labels(st, fs.arr, W, A, sw, d_seeds_xyzw, nullptr, d_labels, num_sms);
   NA_CK(cudaGetLastError());
   static_assert(offsetof(JobState, disjoint) == offsetof(JobState, err) + 8, "err, has_prefix, disjoint in a row");
   uint32_t status[3] = {0, 0, 0};

@@ -926,7 +926,7 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
     for (const vfk::WaveJob& w : wave_jobs)
       if (w.order != vfk::WAVE_XYZ) {
         const JobDesc& d = htable(T_FLOOD)[w.job];
-        vfk::flat_init(st, d.grid, fs.arr, w, vfk::wave_axes(d.X, d.Y, d.Z, d.Zp), wsw, ds + w.job);
+        vfk::flat_init(st, d.grid, fs.arr, w, vfk::wave_axes(d.X, d.Y, d.Z, d.Zp), wsw, ds + w.job, ctx->num_sms);
         launches += 1;
       }
     VF_CK(vfk::flood_seed(st, tf, ds, fs));
@@ -948,12 +948,13 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
   auto finish_bricks = [&](uint32_t j0, uint32_t j1, uint32_t* bl, uint32_t* bc, uint32_t most,
                            const std::function<void(int)>& mk) {
     if (any_flood) {
-      vfk::flood_labels(st, dtable(T_FLOOD), ds, bl, bc, most, bj);
+      vfk::flood_labels(st, dtable(T_FLOOD), ds, bl, bc, most, bj, ctx->num_sms);
       launches += 1;
       for (const vfk::WaveJob& w : wave_jobs)
         if (w.order != vfk::WAVE_XYZ && w.job >= j0 && w.job < j1) {
           const JobDesc& d = htable(T_FLOOD)[w.job];
-          vfk::flat_labels(st, fs.arr, w, vfk::wave_axes(d.X, d.Y, d.Z, d.Zp), wsw, d.seeds, ds + w.job, d.grid);
+          vfk::flat_labels(st, fs.arr, w, vfk::wave_axes(d.X, d.Y, d.Z, d.Zp), wsw, d.seeds, ds + w.job, d.grid,
+                           ctx->num_sms);
           launches += 1;
         }
     }

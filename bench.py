@@ -197,6 +197,15 @@ def reference_arm(args):
     return 0
 
 
+# The flood is bound by the latency of its waves, not by memory: the roofline's bytes are
+# what it has to move once, however often a row is visited.
+FLOOD_BYTES_RULE = "one occupancy bit per voxel in, one u16 label per claimed voxel out"
+
+
+def flood_once_bytes(voxels, claimed):
+    return voxels / 8.0 + 2.0 * claimed
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -274,14 +283,13 @@ def main():
     R.barrier()
     ctx.synchronize()
     L.vf_ctx_event_record(ctx.h, 0)
-    launches, flood_ms, flood_bytes, visits, passes, key_changes = 0, 0.0, 0, 0, 0, 0
+    launches, flood_ms, visits, passes, key_changes = 0, 0.0, 0, 0, 0
     stage_tot = {}
     for _ in range(args.steps):
         rb.execute(download=False)
         st = ctx.last_stats()
         launches += st["launches"]
         flood_ms += st["flood_ms"]
-        flood_bytes += st["flood_bytes"]
         visits += st["flood_visits"]
         passes += st["flood_passes"]
         key_changes += st["flood_key_changes"]
@@ -415,13 +423,13 @@ def main():
 
     peak, peak_kind = _peaks()
     flood_launch_ms = flood_ms / args.steps
-    flood_launch_bytes = flood_bytes / args.steps
+    flood_launch_bytes = flood_once_bytes(voxels, key_changes / args.steps)
     achieved = (flood_launch_bytes / 1e9) / (flood_launch_ms / 1000.0) if flood_launch_ms else 0.0
     roof = {"kernel": "k_wave (bit-parallel flood waves, one cooperative launch per step)",
-            "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "bound": "latency", "achieved": achieved, "peak": peak, "unit": "GB/s",
             "frac": achieved / peak, "peak_kind": f"{peak_kind} copy bandwidth",
             "algorithmic_bytes_per_launch": flood_launch_bytes,
-            "bytes_rule": "4 B (u16 label read + write) per voxel of every row visit (32 voxels)",
+            "bytes_rule": FLOOD_BYTES_RULE,
             "row_visits_per_launch": visits / args.steps,
             "waves_per_launch": passes / args.steps,
             "claims_per_visit": key_changes / max(visits, 1),
@@ -589,7 +597,7 @@ def single_configs(args):
         t = time.perf_counter()
         lab, cnt, _ = O.run_job(v, f, spec.dims, spec.aabb[0], spec.aabb[1], q)
         cpu_ms = 1000.0 * (time.perf_counter() - t)
-        flood_bytes = st["flood_bytes"]
+        flood_bytes = flood_once_bytes(vox, st["flood_key_changes"])
         print(json.dumps({
             "config": name, "dims": list(spec.dims), "voxels": vox, "triangles": int(spec.faces.shape[0]),
             "batched_device_ms": dev_ms, "batched_voxels_per_s": vox / (dev_ms / 1e3),

@@ -431,8 +431,9 @@ vf_status vf_ctx_last_stats(vf_ctx* ctx, uint64_t* kernel_launches,
  * [1] tetrahedra, [2] parity raster, [3] shell SAT, [4] combine + live
  * bricks, [5] seeds, [6] fracture, [7] perturb, [8] erode/boundaries,
  * [9] counts, [10] download (n <= 11 entries written).  Where the labels go
- * to the host group by group, [7] is all stages from the labels to the counts
- * and [8], [9] are about 0 */
+ * to the host group by group beside the last stages, [6] to [9] are added up over
+ * the groups and [10] is what is left of the download after them; in a replayed
+ * graph [7] is all stages from the labels to the counts and [8], [9] are about 0 */
 vf_status vf_ctx_stage_ms(vf_ctx* ctx, float* ms, uint32_t n);
 /* flood of the last batched run: passes = waves; sweeps and maxit_hits are 0
  * (counts of an earlier flood that relaxed bricks) */

@@ -146,6 +146,7 @@ vf_status Batch::execute_resident(bool download) {
   }
   launches = glaunches[gi];
   counts_copied = gcounts[gi];
+  parts = 0;
   VF_CK(cudaGraphLaunch(gexec[gi], stream));
   last_run_graph = true;
   return VF_OK;
@@ -176,6 +177,11 @@ void Batch::release() {
   if (ev_group) cudaEventDestroy(ev_group);
   side = nullptr;
   ev_group = nullptr;
+  for (auto& part : ev_part)
+    for (cudaEvent_t& e : part) {
+      if (e) cudaEventDestroy(e);
+      e = nullptr;
+    }
   if (own_stream && stream) cudaStreamDestroy(stream);
   stream = nullptr;
   ctx = nullptr;
@@ -830,7 +836,6 @@ cudaError_t Batch::waves_serialized(cudaStream_t st, JobState* ds, const vfk::Fl
 // time), all of them written by the pack kernel.  Empty: one group.  128 mixed jobs
 // with labels: 18.9 -> 17.6 ms, 48 jobs 7.1 -> 6.7 ms with 8 groups and 2 pack CTAs per
 // SM (4 groups 17.9 and 6.8; 4 CTAs 17.6 and 6.9; 1 CTA 19.3 and 7.1).
-constexpr uint32_t MAX_GROUPS = 8;
 constexpr uint64_t GROUP_BYTES = 16ull << 20;  // labels of a group, at least
 constexpr int GROUP_PACK_CTAS = 2;             // pack CTAs per SM beside the next group's stages
 vf_status Batch::plan_groups() {
@@ -855,6 +860,8 @@ vf_status Batch::plan_groups() {
     VF_CK(cudaDeviceGetStreamPriorityRange(&lo, &hi));
     VF_CK(cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, hi));
     VF_CK(cudaEventCreateWithFlags(&ev_group, cudaEventDisableTiming));
+    for (auto& part : ev_part)
+      for (cudaEvent_t& e : part) VF_CK(cudaEventCreate(&e));
   }
   return VF_OK;
 }
@@ -865,6 +872,7 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
   launches = 0;
   flood_timed = false;
   counts_copied = false;
+  parts = 0;
   for (int i = 0; i < NSTAGE_EV; ++i) stage_rec[i] = false;
   std::function<void(int)> mark = [&](int i) {
     if (record_event(ev_stage[i], st) == cudaSuccess) stage_rec[i] = true;
@@ -978,10 +986,13 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
   const bool grouped = !groups.empty() && (stages & ST_DOWNLOAD) && do_download;
   if (grouped) {
     // Group by group, each one's labels on their way to the host while the next
-    // group's stages run (stage times: all of it counts as the perturbation).
+    // group's stages run.
     uint32_t j0 = 0, b0 = 0;
     uint64_t r0 = 0;
-    mark(7);
+    // a stage's time is added up over the groups; in a graph, where a record between two
+    // kernels costs 6 us (128 jobs: 17.6 -> 17.8 ms), all of it counts as the perturbation
+    if (capturing) mark(7);
+    else parts = (uint32_t)groups.size();
     for (size_t g = 0; g < groups.size(); ++g) {
       uint32_t nb = 0;
       uint64_t nr = 0;
@@ -991,7 +1002,9 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
       }
       // the whole batch's list is not needed any more; its part of the group is
       vfk::compact_live(st, lv, b0, nb, lst + b0, lc + 16 + g);
-      finish_bricks(j0, groups[g], lst + b0, lc + 16 + g, nb, [](int) {});
+      finish_bricks(j0, groups[g], lst + b0, lc + 16 + g, nb, [&](int i) {
+        if (parts && record_event(ev_part[g][i - 7], st) != cudaSuccess) parts = 0;
+      });
       VF_CK(cudaEventRecord(ev_group, st));
       VF_CK(cudaStreamWaitEvent(side, ev_group, 0));
       vfk::pack_labels(side, dtable(T_CNT) + j0, (int)(groups[g] - j0), r0, nr, ctx->num_sms, GROUP_PACK_CTAS);
@@ -1000,9 +1013,7 @@ vf_status Batch::enqueue_batched(bool do_upload, bool do_download) {
       b0 += nb;
       r0 += nr;
     }
-    mark(8);
-    mark(9);
-    mark(10);
+    for (int i = 8; capturing && i <= 10; ++i) mark(i);
   } else {
     finish_bricks(0, n, lst, lc, maxc, mark);
   }
@@ -1109,6 +1120,17 @@ vf_status Batch::finish(vf_job_result* res) {
     else
       ctx->last_stage_ms[i] = 0.f;
   }
+  if (parts) {  // stages 6 to 9 added up over the groups, the download after the last
+    auto between = [](cudaEvent_t a, cudaEvent_t b) {
+      float ms = 0.f;
+      return cudaEventElapsedTime(&ms, a, b) == cudaSuccess ? ms : 0.f;
+    };
+    for (uint32_t g = 0; g < parts; ++g)
+      for (int k = 0; k < 4; ++k)
+        ctx->last_stage_ms[6 + k] +=
+            between(k ? ev_part[g][k - 1] : (g ? ev_part[g - 1][3] : ev_stage[6]), ev_part[g][k]);
+    ctx->last_stage_ms[10] = between(ev_part[parts - 1][3], ev_stage[11]);
+  }
   return first;
 }
 
@@ -1118,6 +1140,7 @@ vf_status Batch::enqueue_plain_and_wait(vf_job_result* res, bool skip_vox) {
   cudaStream_t st = stream;
   launches = 0;
   counts_copied = false;
+  parts = 0;
   flood_timed = false;
   for (int i = 0; i < NSTAGE_EV; ++i) stage_rec[i] = false;
   const vf_job& j = *jobs[0];

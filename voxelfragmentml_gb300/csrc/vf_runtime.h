@@ -92,8 +92,8 @@ struct Batch {
   // stage boundaries: 0 start, 1 inputs uploaded, 2 tetrahedra built,
   // 3 parity rasterised, 4 shell tested, 5 voxelized (combine + live list),
   // 6 seeded, 7 fractured, 8 perturbed, 9 eroded/boundaries, 10 counted,
-  // 11 downloaded; with groups, 8 is the end of all groups' last stages and 9 and
-  // 10 follow at once
+  // 11 downloaded; with groups, 7 to 10 are recorded once per group (ev_part), and in a
+  // graph 8 is the end of all groups' last stages and 9 and 10 follow at once
   static constexpr int NSTAGE_EV = 12;
   cudaEvent_t ev_stage[NSTAGE_EV] = {};
   bool stage_rec[NSTAGE_EV] = {};
@@ -119,8 +119,11 @@ struct Batch {
   // the download beside the last stages: the end of each group of jobs, the
   // stream that writes their labels, after (and the join)
   std::vector<uint32_t> groups;
+  static constexpr uint32_t MAX_GROUPS = 8;
   cudaStream_t side = nullptr;
   cudaEvent_t ev_group = nullptr;
+  cudaEvent_t ev_part[MAX_GROUPS][4] = {};  // stage boundaries 7 to 10 of each group
+  uint32_t parts = 0;                       // groups of the last run (0: not by groups)
   vf_status plan_groups();
   // the resident stage chain (no uploads) as a CUDA graph: captured on the
   // first execute after plan(), replayed afterwards; falls back to direct

@@ -1,13 +1,15 @@
 // vf_gridops.cu -- seeding, naive Voronoi, perturbation, boundary detection,
 // erosion, isolated-voxel removal and per-fragment counts on sm_103a.
 //
-// Brick kernels: one CTA (256 threads) per live brick, one thread per (x,y)
-// row of VF_BZ = 32 voxels.  The brick plus an xy halo of H voxels and a z
-// window [z0-8, z0+40) is staged in shared memory with 16-byte loads (rows
-// are 16-byte aligned because Zp % 8 == 0), results are written back as
-// 16-byte stores of whole rows (padding z >= Z written as 0).  Halo voxels
-// outside the grid read as EMPTY; voxels of bricks that are not live are
-// EMPTY in memory (both grid buffers start as the voxelizer output).
+// Brick kernels: one CTA (256 threads) per live brick of 16 x 16 rows of VF_BZ = 32
+// voxels.  A stencil stages the brick with an xy halo of H voxels and a z window
+// [z0-8, z0+40) in shared memory with 16-byte loads (rows are 16-byte aligned
+// because Zp % 8 == 0); boundaries of size 1 keep their units of 8 voxels in
+// registers, the others stage the rows alone.  The voxels that have work are dealt
+// to the threads from a queue (units of 8 for boundaries of size 1).  Results go
+// back as 16-byte stores of whole units (padding z >= Z written as 0).  Halo voxels
+// outside the grid read as EMPTY; voxels of bricks that are not live are EMPTY in
+// memory (both grid buffers start as the voxelizer output).
 //
 // The CTAs of a launch loop over the live-brick list (its length is read on
 // the device, so launches need no host synchronisation).
@@ -1102,14 +1104,12 @@ __global__ void __launch_bounds__(256) k_counts(const JobDesc* jobs, JobState* s
 
 
 // ---------------------------------------------------------------------------
-// label download, 16-byte path (Z % 4 == 0, destination 16-byte aligned):
-// the job's output is a flat array of X*Y*Z labels written in 16-byte units
-// (8 labels); each unit is two 8-byte halves, and a half never crosses a row
-// (Z % 4 == 0), so it is one 8-byte load from row (e / Z) at z = e % Z.  Units
-// go to consecutive lanes, so every warp store is 512 contiguous bytes.
-// Labels into a caller's buffer the GPU writes directly (mapped pinned host
-// memory): 16-byte units that may straddle rows (Z a multiple of 4), one
-// 32-bit division per unit.
+// Label download, 16-byte path: a caller's buffer the GPU writes directly (mapped
+// pinned host memory, 16-byte aligned), Z a multiple of 4.  The job's output is a
+// flat array of X*Y*Z labels written in 16-byte units (8 labels); each unit is two
+// 8-byte halves, and a half never crosses a row, so it is one 8-byte load from row
+// (e / Z) at z = e % Z.  Units go to consecutive lanes, so every warp store is 512
+// contiguous bytes.
 __global__ void __launch_bounds__(256) k_pack16(const JobDesc* jobs, int njobs) {
   for (int j = blockIdx.y; j < njobs; j += gridDim.y) {
     const JobDesc& J = jobs[j];
@@ -1147,18 +1147,12 @@ __global__ void __launch_bounds__(256) k_pack16(const JobDesc* jobs, int njobs) 
   }
 }
 
-// label download: one warp per (x, y) row, the final grid (row pitch Zp) into
-// the caller's buffer (row pitch Z); 8-byte stores when Z % 4 == 0 and the
-// destination is 8-byte aligned
-// Labels without the z padding into J.out (a device staging buffer, or a
-// caller's buffer k_pack16 does not take): one warp per (x, y) row of any job (rows of all jobs are
-// numbered consecutively, row_base per job), copied with the widest access
-// the row's alignment allows.
-// Packs each row's labels (z padded to Zp) into the job's staging buffer
-// (J.out, Z per row).  A warp takes 4 consecutive rows of the batch, 8 lanes
-// per row (rows are 64..384 labels: 8..48 16-byte units), so a warp has four
-// rows' loads in flight.  A warp's rows only increase, so its job is found by
-// walking forward from the previous one.
+// Labels without the z padding into J.out (a device staging buffer, or a caller's
+// buffer k_pack16 does not take).  The rows of all jobs are numbered consecutively
+// (row_base per job); a warp takes 4 consecutive ones, 8 lanes per row (rows are
+// 64..384 labels: 8..48 16-byte units), so it has four rows' loads in flight, and
+// copies each with the widest access its alignment allows.  A warp's rows only
+// increase, so its job is found by walking forward from the previous one.
 __global__ void __launch_bounds__(256) k_pack(const JobDesc* jobs, int njobs, unsigned long long row0,
                                               unsigned long long total_rows) {
   const int lane = threadIdx.x & 31, sub = lane & 7;

@@ -51,6 +51,7 @@
 struct JobDesc {
   uint32_t X, Y, Z, Zp, Zk, Zw;
   uint32_t nbx, nby, nbz, brick_base, nbricks;
+  uint32_t wflat;   // the words of its flood's rows do not lie along z
   uint16_t* grid;   // stage source (and in-place target)
   uint16_t* grid2;  // stage destination for double-buffered stages
   uint32_t* keys;   // plain path only
@@ -58,7 +59,6 @@ struct JobDesc {
   // + y (vfk::WaveJob)
   uint32_t* wstate;
   uint32_t wsw, wrow0, wsx, wsy;
-  uint32_t wflat;   // its words do not lie along z
   uint32_t* uf;     // [seeds_cap] union-find over the slots (null: no sub-seed prefixes)
   uint32_t* par;
   uint32_t* shell;

@@ -29,7 +29,7 @@
 // clear, and no order is needed between the rows' loads and stores of a wave.
 //
 // A lane takes one row (x, y, word) of 32 voxels with its 8 neighbour rows.
-// Rows are numbered linearly with rows of zeros around each axis (WaveJob), so
+// Rows are numbered linearly with EMPTY rows around each axis (WaveJob), so
 // a neighbour is an index difference and no bounds are tested.  Which rows a
 // wave looks at is a candidate bit per row, set by the claims of the previous
 // wave: a row is a candidate when a claimed bit reaches one of its unclaimed
@@ -55,8 +55,10 @@
 // bricks of keys in shared memory to local convergence, a queue of bricks per
 // pass, took 10.56 ms (7 key updates per voxel claimed, bound by the chain
 // along each row); 48 jobs 1.64 against 4.01 ms; one job of 476 x 476 x 512
-// 0.87 against 2.15 ms, of 240 x 240 x 256 0.56 against 1.36 ms; of 60 x 57 x
-// 64 0.29 against 0.26 ms.  A gang per job in proportion to its size instead of
+// 0.79 against 2.15 ms, of 240 x 240 x 256 0.51 against 1.36 ms; of 60 x 57 x
+// 64 0.27 against 0.26 ms.  Solids by Manhattan, whose fronts cross a row's 32 voxels
+// in 32 waves, and large thin plates take longer than by bricks (full cubes of 128^3
+// 0.78 against 0.63 ms, of 400^3 4.1 against 2.6).  A gang per job in proportion to its size instead of
 // two gangs in step took 6.1 ms for the 128 jobs (the longest job's gang
 // finished last), a word of 30 neighbouring rows per warp 15.3 ms.
 //
@@ -227,8 +229,8 @@ __device__ __forceinline__ uint32_t visit_row(const WaveArrays& arr, const JobRo
                                               uint32_t* next, uint32_t* err, uint32_t& claims) {
   constexpr int SW = state_words(NB);
   const uint32_t sy = J.sy & 0x7FFFFFFFu, sx = J.sx;
-  // a claim at a word end names rows beyond it unseen: the ones in the zeros
-  // around the grid whose own neighbours would lie outside the job
+  // a claim at a word end names rows beyond it unseen: of the EMPTY ones around the
+  // grid, some have neighbours of their own that would lie outside the job
   if (i < J.lo || i >= J.hi) return 0;
   uint32_t* const p0 = arr.state + (size_t)i * SW;
   const size_t xs = (size_t)sx * SW;

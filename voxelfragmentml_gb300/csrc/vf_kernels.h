@@ -212,7 +212,7 @@ struct WaveArrays {
 };
 // One flood: rows base .. base + nrows of the arrays (base a multiple of 256, up
 // to the next job's base).  Row (outer x, word, y) is row0 + x * sx + word * sy
-// + y, with at least one row of zeros on each side of every axis, so the
+// + y, with at least one EMPTY row on each side of every axis, so the
 // neighbours of a row are rows +- sx, +- sy, +- 1.  A job's axes are (x, y, z) with
 // words along z, or any permutation.
 struct WaveJob {
